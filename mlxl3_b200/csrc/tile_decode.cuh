@@ -17,6 +17,19 @@ __device__ __forceinline__ constexpr uint32_t hash_mul() { return CB == 0 ? 8922
 template <int CB>
 __device__ __forceinline__ constexpr uint32_t hash_add() { return CB == 0 ? 64248484u : 0u; }
 
+// bits [O, O + 16) of v, O at most 16.  The left shift is spelled in PTX so that it stays one (folded with the right shift
+// it becomes a shift and a mask, both on the logic pipe).
+template <int O>
+__device__ __forceinline__ uint32_t window(uint32_t v) {
+    if constexpr (O == 0) return v & 0xffffu;
+    else if constexpr (O == 16) return v >> 16;
+    else {
+        uint32_t d;
+        asm("shl.b32 %0, %1, %2;" : "=r"(d) : "r"(v), "n"(16 - O));
+        return d >> 16;
+    }
+}
+
 // b[j] = state_j * M + C for the lane's states j = 0..7 (32-bit wrap-around).  (w0:w1:w2) are the
 // stream words that end at the word holding the lane's last bit; `slack` bits of w2 lie past it.
 template <int K, int CB>
@@ -48,20 +61,42 @@ __device__ __forceinline__ void lane_hashes(uint32_t w2, uint32_t w1, uint32_t w
             }
         }
     } else {
-        const uint32_t n2 = __funnelshift_r(w2, w1, slack);
-        const uint32_t n1 = __funnelshift_r(w1, w0, slack);
-        const uint32_t n0 = w0 >> slack;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int c = (7 - j) * K;
-            uint32_t v;
-            if (c + 16 <= 32) v = n2 >> c;
-            else if (c < 32) v = __funnelshift_r(n2, n1, c);
-            else if (c + 16 <= 64) v = n1 >> (c - 32);
-            else if (c < 64) v = __funnelshift_r(n1, n0, c - 32);
-            else v = n0 >> (c - 64);
-            b[j] = (v & 0xffffu) * M + C;
+        // The states are 16-bit windows at bit offsets 0, K, .., 7K from the lane's end.  A few registers are funnelled out
+        // of the stream words so that every window lies at an offset 0..16 of one of them; there it costs ONE logic-pipe
+        // instruction: nothing but a shift at offset 16, a mask at 0, and in between a left shift, which the integer
+        // multiply-add pipe takes, followed by the right shift that drops what lies below (shifting right and masking,
+        // two logic-pipe instructions per state, made the decode of a tile 53 cycles at K = 3; now 41, the multiply-add
+        // pipe being busy as long as the logic pipe).
+        uint32_t v[8];
+        const uint32_t n = __funnelshift_r(w2, w1, slack);                       // offsets 0..31
+        if constexpr (K <= 2) {
+            v[7] = window<0>(n); v[6] = window<K>(n); v[5] = window<2 * K>(n); v[4] = window<3 * K>(n);
+            v[3] = window<4 * K>(n); v[2] = window<5 * K>(n); v[1] = window<6 * K>(n); v[0] = window<7 * K>(n);
+        } else if constexpr (K == 3) {
+            const uint32_t m = __funnelshift_r(w2, w1, slack + 5);                  // offsets 5..36 (slack is at most 24)
+            v[7] = window<0>(n); v[6] = window<3>(n);
+            v[5] = window<1>(m); v[4] = window<4>(m); v[3] = window<7>(m); v[2] = window<10>(m); v[1] = window<13>(m); v[0] = window<16>(m);
+        } else {
+            const uint32_t n1 = __funnelshift_r(w1, w0, slack);                     // offsets 32..63
+            if constexpr (K == 5) {
+                const uint32_t m = __funnelshift_r(n, n1, 19);                      // offsets 19..50
+                v[7] = window<0>(n); v[6] = window<5>(n); v[5] = window<10>(n); v[4] = window<15>(n);
+                v[3] = window<1>(m); v[2] = window<6>(m); v[1] = window<11>(m); v[0] = window<16>(m);
+            } else if constexpr (K == 6) {
+                const uint32_t m = __funnelshift_r(n, n1, 14);                      // offsets 14..45
+                v[7] = window<0>(n); v[6] = window<6>(n); v[5] = window<12>(n);
+                v[4] = window<4>(m); v[3] = window<10>(m); v[2] = window<16>(m);
+                v[1] = window<4>(n1); v[0] = window<10>(n1);
+            } else {
+                const uint32_t m = __funnelshift_r(n, n1, 19);                      // offsets 19..50
+                const uint32_t l = __funnelshift_r(n1, w0 >> slack, 1);             // offsets 33..64
+                v[7] = window<0>(n); v[6] = window<7>(n); v[5] = window<14>(n);
+                v[4] = window<2>(m); v[3] = window<9>(m); v[2] = window<16>(m);
+                v[1] = window<9>(l); v[0] = window<16>(l);
+            }
         }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) b[j] = v[j] * M + C;
     }
 }
 
