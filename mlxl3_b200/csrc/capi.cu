@@ -174,7 +174,7 @@ int b200exl3_plan_query(const char* kind, int in, int out, int k, int64_t rows, 
         return 0;
     }
     if (!strcmp(kind, "qmm")) {
-        const QmmPlan p = plan_qmm(in, out, rows);
+        const QmmPlan p = plan_qmm(in, out, rows);   // rows of a pass in tiles of 512, each in halves of up to 256
         out_values[0] = p.splits; out_values[1] = p.token_tiles; out_values[2] = p.small ? 1 : 0; out_values[3] = in / 64;
         return 0;
     }
@@ -383,24 +383,28 @@ static size_t xhat_bytes(const LayerCore& c, int64_t rows) {
     return rows > kQmvFusedRows ? round256(static_cast<size_t>(c.groups) * rows * c.in * sizeof(__half)) : 0;
 }
 
-// From this many rows on, a plain layer's forward runs the tensor-core product (rotate all rows, tcgen05 product,
-// output rotation) instead of the fused kernel: its small shape (two CTAs per SM) takes 43 us for 9..64 rows of a
-// 4096 -> 14336 layer where the fused kernel's two-block form takes 61 us for 9..16 rows.
+// From this many rows on, a plain layer's forward runs the tensor-core product (rotate all rows, tcgen05 product with the
+// output rotation in its epilogue) instead of the fused kernel, whose two-block form takes twice its one-block form's time.
 constexpr int64_t kQmmMinRows = 9;
+
+// tensor-core path: [counters | rotated rows of a pass, once per member | pieces of shared items | fp32 sums of a row shard]
+struct QmmLayout { QmmPlan plan; size_t xhat, pieces, sums, total; };
+static QmmLayout qmm_layout(const LayerCore& c, int64_t rows, bool whole_items = false) {
+    QmmLayout l;
+    l.plan = plan_qmm(c.in, c.out, rows, whole_items);
+    l.xhat = kCounterBytes;
+    l.pieces = l.xhat + xhat_bytes(c, std::min(rows, l.plan.pass_rows));
+    l.sums = l.pieces + round256(l.plan.piece_bytes);
+    l.total = l.sums + (whole_items ? 0 : round256(static_cast<size_t>(std::min(rows, l.plan.pass_rows)) * c.out * sizeof(float)));
+    return l;
+}
 
 static int core_workspace_bytes(const LayerCore& c, int64_t rows, size_t* out_bytes) {
     if (!out_bytes) return fail("NULL argument");
     if (rows <= 0) return fail("EXL3 linear input cannot be empty");
     QmvPlan plan = plan_qmv(c.in, c.out, c.k, rows);
     size_t bytes = kCounterBytes + qmv_partial_bytes(plan, c.out, rows) + xhat_bytes(c, rows);
-    if (rows >= kQmmMinRows) {
-        // tensor-core path: one rotated copy of the rows at a time (per member of a group) and the member's partials
-        for (int g = 0; g < c.groups; ++g) {
-            const QmmPlan qp = plan_qmm(c.in, c.gout[g], rows);
-            bytes = std::max(bytes, kCounterBytes + round256(static_cast<size_t>(rows) * c.in * sizeof(__half)) +
-                                        qmm_partial_bytes(qp, c.gout[g], rows));
-        }
-    }
+    if (rows >= kQmmMinRows) bytes = std::max(bytes, qmm_layout(c, rows).total);
     *out_bytes = bytes;
     return 0;
 }
@@ -416,10 +420,11 @@ static TpPeers tp_peers(const b200exl3_tp* tp);
 
 static int forward_common(const LayerCore& c, const void* d_x, int x_dtype, const uint16_t* d_xhat, int64_t rows,
                           void* const* ys, float* d_yhat, void* ws, size_t ws_bytes, cudaStream_t stream,
-                          const b200exl3_tp* tp = nullptr, const b200exl3_prologue* pro = nullptr) {
+                          const b200exl3_tp* tp = nullptr, const b200exl3_prologue* pro = nullptr, bool whole_items = false) {
     if (rows <= 0) return fail("EXL3 linear input cannot be empty");
     size_t need = 0;
-    if (core_workspace_bytes(c, rows, &need)) return -1;
+    if (whole_items) need = qmm_layout(c, rows, true).total;
+    else if (core_workspace_bytes(c, rows, &need)) return -1;
     if (!ws || ws_bytes < need) return fail("workspace too small: %zu bytes given, %zu needed", ws_bytes, need);
     if (!aligned16(ws)) return fail("device pointers must be 16-byte aligned");
     char* base = static_cast<char*>(ws);
@@ -434,34 +439,34 @@ static int forward_common(const LayerCore& c, const void* d_x, int x_dtype, cons
         pro = nullptr;
     }
     if (rows >= kQmmMinRows && ys && !d_xhat && g_qmm_enabled) {
-        // many rows: input rotation -> tensor-core product (fp32 partials per input split) -> output rotation.
-        // A group runs member by member (each member has its own input scales, so its own rotated rows); a row shard
-        // of a tensor-parallel layer keeps one split, and the sum over ranks and the rotation follow as one kernel.
-        __half* buf = reinterpret_cast<__half*>(base + kCounterBytes);
-        float* partials = reinterpret_cast<float*>(base + kCounterBytes + round256(static_cast<size_t>(rows) * c.in * sizeof(__half)));
-        unsigned int* status = reinterpret_cast<unsigned int*>(base + kCounterBytes - sizeof(unsigned int));
-        for (int g = 0; g < c.groups; ++g) {
-            QmmPlan qp = plan_qmm(c.in, c.gout[g], rows);
-            const __half* svh = c.svh + c.gcol0[g];
-            const __half* bias = c.bias ? c.bias + c.gcol0[g] : nullptr;
-            const int ld = c.out / 16, col0 = c.gcol0[g] / 16;
-            B200_TRY(launch_prepare(d_x, x_dtype, c.suh + static_cast<size_t>(g) * c.in, 1, rows, c.in, buf, stream, glu_up), "prepare");
+        // many rows: input rotation (once per member of a group, each has its own input scales) -> tensor-core product
+        // over all members with the output rotation in its epilogue; of a row shard of a tensor-parallel layer the sums
+        // over the inputs are kept, and the sum over ranks and the rotation follow as one kernel
+        const QmmLayout l = qmm_layout(c, rows, whole_items);
+        for (int64_t r0 = 0; r0 < rows; r0 += l.plan.pass_rows) {
+            const int64_t n = std::min(l.plan.pass_rows, rows - r0);
+            __half* buf = reinterpret_cast<__half*>(base + l.xhat);
+            B200_TRY(launch_prepare(static_cast<const char*>(d_x) + static_cast<size_t>(r0) * c.in * x_size, x_dtype, c.suh, 1, n, c.in, buf, stream,
+                                    glu_up ? glu_up + r0 * c.in : nullptr, c.groups), "prepare");
+            QmmArgs a{};
+            a.wq = c.wq; a.svh = c.svh; a.bias = c.bias;
+            a.pieces = reinterpret_cast<float*>(base + l.pieces);
+            a.counters = reinterpret_cast<unsigned int*>(base);
+            a.error = reinterpret_cast<unsigned int*>(base + kCounterBytes - sizeof(unsigned int));
+            a.in = c.in; a.out = c.out; a.rows = static_cast<int>(n); a.y_dtype = x_dtype;
+            a.groups = c.groups;
+            for (int g = 0; g < c.groups; ++g) {
+                a.gcol0[g] = c.gcol0[g];
+                a.gout[g] = c.gout[g];
+                a.gy[g] = static_cast<char*>(ys[g]) + static_cast<size_t>(r0) * c.gout[g] * x_size;
+            }
+            if (tp) { a.yhat = reinterpret_cast<float*>(base + l.sums); a.yhat_ld = c.out; }
+            B200_TRY(launch_qmm(a, buf, c.k, c.cb, l.plan, stream), "tensor-core product kernel");
             if (tp) {
-                qp.splits = 1;
-                B200_TRY(launch_qmm(c.wq, c.in, c.gout[g], c.k, c.cb, buf, rows, qp, partials, status, nullptr, nullptr, nullptr, 0, stream, ld, col0),
-                         "tensor-core product kernel");
-                TpArgs a{};
-                a.yhat = partials; a.peers = tp_peers(tp); a.svh = svh; a.bias = bias; a.y = ys[g];
-                a.rows = static_cast<int>(rows); a.out = c.gout[g]; a.y_dtype = x_dtype;
-                B200_TRY(launch_tp_finish(a, stream), "tensor-parallel finish kernel");
-            } else if (qp.splits == 1) {
-                // one CTA holds the whole input range of its columns: the output rotation runs in its epilogue
-                B200_TRY(launch_qmm(c.wq, c.in, c.gout[g], c.k, c.cb, buf, rows, qp, partials, status, svh, bias, ys[g], x_dtype, stream, ld, col0),
-                         "tensor-core product kernel");
-            } else {
-                B200_TRY(launch_qmm(c.wq, c.in, c.gout[g], c.k, c.cb, buf, rows, qp, partials, status, nullptr, nullptr, nullptr, 0, stream, ld, col0),
-                         "tensor-core product kernel");
-                B200_TRY(launch_finish(partials, qp.splits, rows * c.gout[g], svh, 1, bias, rows, c.gout[g], x_dtype, ys[g], stream), "finish");
+                TpArgs t{};
+                t.yhat = a.yhat; t.peers = tp_peers(tp); t.svh = c.svh; t.bias = c.bias; t.y = a.gy[0];
+                t.rows = static_cast<int>(n); t.out = c.out; t.y_dtype = x_dtype;
+                B200_TRY(launch_tp_finish(t, stream), "tensor-parallel finish kernel");
             }
         }
         return 0;
@@ -470,9 +475,7 @@ static int forward_common(const LayerCore& c, const void* d_x, int x_dtype, cons
         // more than two rows: rotate all of them once per group, the product kernel reads the rotated rows
         const QmvPlan first = plan_qmv(c.in, c.out, c.k, rows);
         __half* buf = reinterpret_cast<__half*>(base + kCounterBytes + qmv_partial_bytes(first, c.out, rows));
-        for (int g = 0; g < c.groups; ++g)
-            B200_TRY(launch_prepare(d_x, x_dtype, c.suh + static_cast<size_t>(g) * c.in, 1, rows, c.in,
-                                    buf + static_cast<size_t>(g) * rows * c.in, stream, glu_up), "prepare");
+        B200_TRY(launch_prepare(d_x, x_dtype, c.suh, 1, rows, c.in, buf, stream, glu_up, c.groups), "prepare");
         xhat = buf;
     }
     for (int64_t r0 = 0; r0 < rows; r0 += kMaxBatchRows) {
@@ -655,6 +658,13 @@ int b200exl3_linear_forward_static(const b200exl3_linear* h, const void* d_x, in
     if (!d_x || !d_y) return fail("NULL buffer");
     size_t need = 0;
     if (core_workspace_bytes(h->c, rows, &need)) return -1;
+    bool whole_items = false;
+    if (need > kStaticScratchBytes && rows >= kQmmMinRows) {
+        // many rows: without parts of items shared by CTAs the call needs less (what counts against the array is the
+        // rotated rows and one fp32 copy of the result, as it always did)
+        const size_t smallest = qmm_layout(h->c, rows, true).total + static_cast<size_t>(rows) * h->c.out * sizeof(float);
+        if (smallest <= kStaticScratchBytes) { whole_items = true; need = smallest; }
+    }
     if (need > kStaticScratchBytes)
         return fail("this call needs %zu bytes of scratch but the allocation-free entry point owns %zu; "
                     "use b200exl3_linear_forward with a caller workspace", need, kStaticScratchBytes);
@@ -666,7 +676,7 @@ int b200exl3_linear_forward_static(const b200exl3_linear* h, const void* d_x, in
     // until that call clears it, as it does in a caller's workspace.
     B200_TRY(cudaMemsetAsync(scratch, 0, kCounterBytes - sizeof(unsigned int), as_stream(s)), "clear static scratch");
     void* ys[1] = {d_y};
-    return forward_common(h->c, d_x, x_dtype, nullptr, rows, ys, nullptr, scratch, kStaticScratchBytes, as_stream(s));
+    return forward_common(h->c, d_x, x_dtype, nullptr, rows, ys, nullptr, scratch, kStaticScratchBytes, as_stream(s), nullptr, nullptr, whole_items);
 }
 
 int b200exl3_static_status(int* out_status, int clear) {
@@ -962,17 +972,12 @@ static MoeLayout moe_layout(const b200exl3_moe* h, int64_t rows) {
     return l;
 }
 
-// Expert-sorted form, used from this many slots on: slots are grouped by expert into segments of kMoeSegRows rows,
+// Expert-sorted form, used from this many slots on: slots are grouped by expert into segments of kQmmSegRows rows,
 // so an expert's columns are decoded once per segment instead of once per slot.
 constexpr int64_t kMoeSortedMinSlots = 33;
 
-static int64_t moe_max_segments(const b200exl3_moe* h, int64_t slots, int seg_rows) {
-    return std::min<int64_t>(h->experts, slots) + slots / seg_rows;   // one partly filled segment per expert at most
-}
-// Segments of 8 rows run in the fused kernel; once most experts see many rows, segments of 64 rows run on the tensor cores.
-constexpr int64_t kMoeTensorSlotsPerExpert = 12;
-static int moe_seg_rows(const b200exl3_moe* h, int64_t rows) {
-    return g_qmm_enabled && rows * h->top_k >= kMoeTensorSlotsPerExpert * h->experts ? kQmmSegRows : kMoeSegRows;
+static int64_t moe_max_segments(const b200exl3_moe* h, int64_t slots) {
+    return std::min<int64_t>(h->experts, slots) + slots / kQmmSegRows;   // one partly filled segment per expert at most
 }
 // rows per pass (bounds the scratch); the passes of a call get equal shares
 constexpr int64_t kMoeSortedPassSlots = 16384;
@@ -983,44 +988,36 @@ static int64_t moe_sorted_chunk_rows(const b200exl3_moe* h, int64_t rows) {
 }
 
 struct MoeSortedLayout {
-    size_t counters, counter_bytes, seg_count, seg_expert, row_slot, slot_row, xgu, ygu, xdown, ydown, partials, total;
-    int max_segments, seg_rows;
-    QmvPlan gu_plan, down_plan;
+    size_t counters, counter_bytes, seg_count, seg_expert, seg_rows, slot_row, xgu, ygu, xdown, ydown, pieces, total;
+    int max_segments;
 };
 
 static MoeSortedLayout moe_sorted_layout(const b200exl3_moe* h, int64_t rows) {
     MoeSortedLayout l{};
     const int64_t slots = moe_sorted_chunk_rows(h, rows) * h->top_k;
-    const int seg_rows = moe_seg_rows(h, rows);
-    const int64_t segs = moe_max_segments(h, slots, seg_rows);
+    const size_t segs = static_cast<size_t>(moe_max_segments(h, slots)), padded = segs * kQmmSegRows;
     l.max_segments = static_cast<int>(segs);
-    l.seg_rows = seg_rows;
-    l.gu_plan = plan_qmv(h->in, static_cast<int>(segs * 2 * h->hidden), h->k, kMoeSegRows);
-    l.down_plan = plan_qmv(h->hidden, static_cast<int>(segs * h->in), h->k, kMoeSegRows);
     size_t at = kCounterBytes;
     // arrival counters of its own (one per virtual column block; the header's 16 KiB would cap a pass at 4093 blocks),
     // cleared at the start of every call
-    l.counter_bytes = round256((static_cast<size_t>(segs) * moe_blocks_per_slot(h->in, h->hidden) + 2) * sizeof(unsigned int));
+    l.counter_bytes = round256((segs * moe_blocks_per_slot(h->in, h->hidden) + 2) * sizeof(unsigned int));
     l.counters = at; at += l.counter_bytes;
     l.seg_count = at; at += 256;
-    l.seg_expert = at; at += round256(static_cast<size_t>(segs) * sizeof(uint32_t));
-    l.row_slot = at; at += round256(static_cast<size_t>(segs) * seg_rows * sizeof(uint32_t));
+    l.seg_expert = at; at += round256(segs * sizeof(uint32_t));
+    l.seg_rows = at; at += round256(segs * sizeof(int));
     l.slot_row = at; at += round256(static_cast<size_t>(slots) * sizeof(uint32_t));
-    l.xgu = at; at += round256(static_cast<size_t>(segs) * 2 * seg_rows * h->in * sizeof(__half));
-    l.ygu = at; at += round256(static_cast<size_t>(segs) * 2 * seg_rows * h->hidden * sizeof(float));
-    l.xdown = at; at += round256(static_cast<size_t>(segs) * seg_rows * h->hidden * sizeof(__half));
-    l.ydown = at; at += round256(static_cast<size_t>(segs) * seg_rows * h->in * sizeof(float));
-    l.partials = at;
-    if (seg_rows == kMoeSegRows)
-        at += std::max(qmv_partial_bytes(l.gu_plan, static_cast<int>(segs * 2 * h->hidden), kMoeSegRows),
-                       qmv_partial_bytes(l.down_plan, static_cast<int>(segs * h->in), kMoeSegRows));
+    l.xgu = at; at += round256(padded * 2 * h->in * sizeof(__half));
+    l.ygu = at; at += round256(padded * 2 * h->hidden * sizeof(float));
+    l.xdown = at; at += round256(padded * h->hidden * sizeof(__half));
+    l.ydown = at; at += round256(padded * h->in * sizeof(float));
+    l.pieces = at; at += round256(qmm_mapped_piece_bytes());
     l.total = at;
     return l;
 }
 
 static bool moe_sorted(const b200exl3_moe* h, int64_t rows) {
     // worth it once experts see several rows each: below two slots per expert one row per slot is faster
-    if (!g_moe_sorted || rows * h->top_k < std::max<int64_t>(kMoeSortedMinSlots, 2 * static_cast<int64_t>(h->experts))) return false;
+    if (!g_moe_sorted || !g_qmm_enabled || rows * h->top_k < std::max<int64_t>(kMoeSortedMinSlots, 2 * static_cast<int64_t>(h->experts))) return false;
     // the route plan keeps 2 * experts + 1 counters and one 16-bit expert id per slot of a pass in 48 KiB of shared
     // memory; shapes beyond that keep one row per slot
     const size_t plan_smem = (2 * static_cast<size_t>(h->experts) + 1) * sizeof(int) +
@@ -1114,59 +1111,42 @@ int b200exl3_moe_forward(const b200exl3_moe* h, const void* d_x, int x_dtype, in
         if (!ws || ws_bytes < l.total) return fail("workspace too small: %zu bytes given, %zu needed", ws_bytes, l.total);
         int* seg_count = reinterpret_cast<int*>(base + l.seg_count);
         uint32_t* seg_expert = reinterpret_cast<uint32_t*>(base + l.seg_expert);
-        uint32_t* row_slot = reinterpret_cast<uint32_t*>(base + l.row_slot);
+        int* seg_rows = reinterpret_cast<int*>(base + l.seg_rows);
         uint32_t* slot_row = reinterpret_cast<uint32_t*>(base + l.slot_row);
         __half* xgu = reinterpret_cast<__half*>(base + l.xgu);
         float* ygu = reinterpret_cast<float*>(base + l.ygu);
         __half* xdown = reinterpret_cast<__half*>(base + l.xdown);
         float* ydown = reinterpret_cast<float*>(base + l.ydown);
-        const int segs = l.max_segments, seg_rows = l.seg_rows;
+        const int segs = l.max_segments;
         const int64_t chunk = moe_sorted_chunk_rows(h, rows);
         B200_TRY(cudaMemsetAsync(base + l.counters, 0, l.counter_bytes, stream), "clear arrival counters");
         for (int64_t r0 = 0; r0 < rows; r0 += chunk) {
             const int64_t n = std::min(chunk, rows - r0), slots = n * h->top_k;
             const uint32_t* sel = d_selected + r0 * h->top_k;
-            // kMoeSegRows rows per segment against the columns of the segment's expert; segments past the count are skipped
-            auto mapped = [&](const uint32_t* wq, const __half* xhat, int in, int width, int proj, int stride_blocks, float* yhat,
-                              const QmvPlan& plan) {
-                const int out = segs * proj * width;
-                QmvArgs a{};
-                a.wq = wq; a.xhat = xhat; a.xhat_group_stride = static_cast<int64_t>(kMoeSegRows) * in;
+            // up to 64 rows per segment against the columns of the segment's expert; segments past the count do not exist
+            auto mapped = [&](const uint32_t* wq, const __half* xhat, int in, int width, int proj, int stride_blocks, float* yhat) {
+                QmmArgs a{};
+                a.wq = wq;
+                a.pieces = reinterpret_cast<float*>(base + l.pieces);
                 a.counters = reinterpret_cast<unsigned int*>(base + l.counters);
                 a.error = reinterpret_cast<unsigned int*>(base + kCounterBytes - sizeof(unsigned int));
-                a.partials = reinterpret_cast<float*>(base + l.partials);
-                a.yhat = yhat;
-                a.groups = 1; a.gcol0[0] = 0; a.gout[0] = out;
-                a.x_dtype = kF16; a.y_dtype = kF16;
-                a.in = in; a.out = out; a.rows = kMoeSegRows;
-                a.tiles_n = h->experts * proj * width / 16;
-                a.map_selected = seg_expert; a.map_count = seg_count;
+                a.yhat = yhat; a.yhat_ld = width;
+                a.in = in;
+                a.map_expert = seg_expert; a.map_rows = seg_rows; a.map_count = seg_count;
                 a.map_blocks = width / 128; a.map_proj = proj; a.map_stride_blocks = stride_blocks; a.map_experts = h->experts;
-                return launch_qmv(a, h->k, h->cb, exact, plan, stream);
+                return launch_qmm_mapped(a, xhat, segs, h->k, h->cb, stream);
             };
-            // the same on the tensor cores: 64 rows per segment, one CTA per (segment, projection, 128 columns)
-            auto mapped_tensor = [&](const uint32_t* wq, const __half* xhat, int in, int width, int proj, int stride_blocks, float* yhat) {
-                return launch_qmm_mapped(wq, in, width, h->experts * proj * width / 16, h->k, h->cb, xhat, segs, proj, stride_blocks,
-                                         h->experts, seg_expert, seg_count, yhat,
-                                         reinterpret_cast<unsigned int*>(base + kCounterBytes - sizeof(unsigned int)), stream);
-            };
-            const bool tensor = seg_rows == kQmmSegRows;
-            B200_TRY(launch_route_plan(sel, slots, h->experts, segs, seg_rows, seg_count, seg_expert, row_slot, slot_row, stream), "route plan");
-            B200_TRY(launch_routed_prepare_padded(static_cast<const char*>(d_x) + static_cast<size_t>(r0) * h->in * x_size, x_dtype,
-                                                  h->gu_suh, seg_expert, slot_row, slots, h->top_k, 2, segs, seg_rows, h->in, xgu,
-                                                  stream), "routed prepare");
-            B200_TRY(tensor ? mapped_tensor(h->gu_wq, xgu, h->in, h->hidden, 2, h->experts * (h->hidden / 128), ygu)
-                            : mapped(h->gu_wq, xgu, h->in, h->hidden, 2, h->experts * (h->hidden / 128), ygu, l.gu_plan),
-                     "expert gate/up kernel");
-            B200_TRY(launch_glu_down_input_padded(ygu, h->gu_svh, h->down_suh, seg_expert, row_slot, seg_count, h->experts, segs,
-                                                  seg_rows, h->hidden, h->hidden, xdown, stream), "SwiGLU glue");
-            B200_TRY(tensor ? mapped_tensor(h->down_wq, xdown, h->hidden, h->in, 1, 0, ydown)
-                            : mapped(h->down_wq, xdown, h->hidden, h->in, 1, 0, ydown, l.down_plan),
-                     "expert down kernel");
-            B200_TRY(launch_finish_and_reduce_padded(ydown, h->down_svh, sel, slot_row, h->experts,
-                                                     static_cast<const char*>(d_scores) + static_cast<size_t>(r0) * h->top_k * score_size,
-                                                     score_dtype, n, h->top_k, h->in, segs, seg_rows,
-                                                     static_cast<char*>(d_y) + static_cast<size_t>(r0) * h->in * score_size, stream),
+            B200_TRY(launch_route_plan(sel, slots, h->experts, segs, seg_count, seg_expert, seg_rows, slot_row, stream), "route plan");
+            B200_TRY(launch_routed_prepare(static_cast<const char*>(d_x) + static_cast<size_t>(r0) * h->in * x_size, x_dtype, h->gu_suh, sel,
+                                           slot_row, h->experts, slots, h->top_k, 2, segs, h->in, xgu, stream), "routed prepare");
+            B200_TRY(mapped(h->gu_wq, xgu, h->in, h->hidden, 2, h->experts * (h->hidden / 128), ygu), "expert gate/up kernel");
+            B200_TRY(launch_glu_down_input(ygu, h->gu_svh, h->down_suh, sel, h->experts, slots, h->hidden, h->hidden, xdown, stream, nullptr,
+                                           slot_row), "SwiGLU glue");
+            B200_TRY(mapped(h->down_wq, xdown, h->hidden, h->in, 1, 0, ydown), "expert down kernel");
+            B200_TRY(launch_finish_and_reduce(ydown, h->down_svh, sel, h->experts,
+                                              static_cast<const char*>(d_scores) + static_cast<size_t>(r0) * h->top_k * score_size,
+                                              score_dtype, n, h->top_k, h->in,
+                                              static_cast<char*>(d_y) + static_cast<size_t>(r0) * h->in * score_size, stream, slot_row),
                      "expert reduction");
         }
         return 0;

@@ -49,6 +49,54 @@ __device__ __forceinline__ void store_from_half(void* p, int dtype, int64_t i, _
     }
 }
 
+// four consecutive elements (i a multiple of 4) in one load
+__device__ __forceinline__ void load4_as_half(const void* p, int dtype, int64_t i, __half (&h)[4]) {
+    if (dtype == kF32) {
+        const float4 v = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p) + i);
+        h[0] = __float2half_rn(v.x); h[1] = __float2half_rn(v.y); h[2] = __float2half_rn(v.z); h[3] = __float2half_rn(v.w);
+    } else {
+        const uint2 v = *reinterpret_cast<const uint2*>(reinterpret_cast<const uint16_t*>(p) + i);
+        if (dtype == kF16) {
+            const __half* e = reinterpret_cast<const __half*>(&v);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) h[j] = e[j];
+        } else {
+            const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&v);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) h[j] = __float2half_rn(__bfloat162float(e[j]));
+        }
+    }
+}
+
+// store_from_half for four consecutive elements (i a multiple of 4) in one store; `bias` points at the first one's bias
+__device__ __forceinline__ void store4_from_half(void* p, int dtype, int64_t i, const __half (&v)[4], const __half* bias) {
+    __half b[4];
+    if (bias) {
+        const uint2 w = *reinterpret_cast<const uint2*>(bias);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) b[j] = reinterpret_cast<const __half*>(&w)[j];
+    }
+    if (dtype == kF16) {
+        __align__(8) __half o[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) o[j] = bias ? __hadd_rn(v[j], b[j]) : v[j];
+        *reinterpret_cast<uint2*>(reinterpret_cast<__half*>(p) + i) = *reinterpret_cast<const uint2*>(o);
+    } else if (dtype == kF32) {
+        float o[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) o[j] = bias ? __fadd_rn(__half2float(v[j]), __half2float(b[j])) : __half2float(v[j]);
+        *reinterpret_cast<float4*>(reinterpret_cast<float*>(p) + i) = make_float4(o[0], o[1], o[2], o[3]);
+    } else {
+        __align__(8) __nv_bfloat16 o[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            o[j] = __float2bfloat16_rn(__half2float(v[j]));
+            if (bias) o[j] = __float2bfloat16_rn(__fadd_rn(__bfloat162float(o[j]), __half2float(b[j])));
+        }
+        *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(p) + i) = *reinterpret_cast<const uint2*>(o);
+    }
+}
+
 __device__ __forceinline__ uint32_t lop3_and_xor(uint32_t a, uint32_t mask, uint32_t flip) {
     uint32_t d;
     asm("lop3.b32 %0, %1, %2, %3, 0x6a;" : "=r"(d) : "r"(a), "r"(mask), "r"(flip));  // (a & mask) ^ flip

@@ -42,9 +42,10 @@ cudaError_t launch_reconstruct(const uint16_t* trellis, int tiles_k, int tiles_n
                                cudaStream_t stream);
 
 // ---- rotations (kernels_rotate.cu) ----------------------------------------------------------------
-// xhat[r, :] = H128(half(half(x[r, :]) * suh[(r % scale_rows), :])); scale_rows is 1 or rows.
+// xhat[r, :] = H128(half(half(x[r, :]) * suh[(r % scale_rows), :])); scale_rows is 1 or rows.  With groups > 1 (scale_rows
+// 1) the rows are rotated once per member: suh [groups, in], xhat [groups, rows, in].
 cudaError_t launch_prepare(const void* x, int x_dtype, const __half* suh, int64_t scale_rows, int64_t rows, int in,
-                           __half* xhat, cudaStream_t stream, const __half* glu_up = nullptr);
+                           __half* xhat, cudaStream_t stream, const __half* glu_up = nullptr, int groups = 1);
 // y = half(H128(half(sum_s partials[s, r, :]))) * svh (+ bias), written in y_dtype.
 cudaError_t launch_finish(const float* partials, int splits, int64_t split_stride, const __half* svh,
                           int64_t scale_rows, const __half* bias, int64_t rows, int out, int y_dtype, void* y,
@@ -248,16 +249,17 @@ cudaError_t launch_stack(const StackArgs& args, int k, int cb, bool exact, const
 
 // ---- grouped experts (kernels_moe.cu) ------------------------------------------------------------------
 // SwiGLU glue between the expert projections (native/src/moe.rs:438-533, SiLU): raw gate/up sums
-// ygu[slot * 2 + {0,1}, :] -> rotated input of the down projection xhat[slot, :]
+// ygu[slot * 2 + {0,1}, :] -> rotated input of the down projection xhat[slot, :].  With slot_row (the expert-sorted form)
+// slot s is row r = slot_row[s] % 64 of segment g = slot_row[s] / 64: sums ygu[(g * 2 + {0,1}) * 64 + r, :], result xhat[g * 64 + r, :].
 // `count` (optional, device): only slots below *count are computed
 cudaError_t launch_glu_down_input(const float* ygu, const __half* gu_svh, const __half* down_suh, const uint32_t* selected,
                                   int experts, int64_t slots, int hidden, int logical_hidden, __half* xhat,
-                                  cudaStream_t stream, const int* count = nullptr);
+                                  cudaStream_t stream, const int* count = nullptr, const uint32_t* slot_row = nullptr);
 // y[row, :] = sum over the row's top_k slots of rotate(half(raw[slot, :])) * svh[selected[slot], :] * score
-// (native/src/moe.rs:586-609); scores and y are fp16 or fp32 (score_dtype)
+// (native/src/moe.rs:586-609); scores and y are fp16 or fp32 (score_dtype); with slot_row, slot s is row slot_row[s] of raw
 cudaError_t launch_finish_and_reduce(const float* raw, const __half* down_svh, const uint32_t* selected, int experts,
                                      const void* scores, int score_dtype, int64_t rows, int top_k, int out, void* y,
-                                     cudaStream_t stream);
+                                     cudaStream_t stream, const uint32_t* slot_row = nullptr);
 
 // ---- expert parallelism (kernels_ep.cu) -------------------------------------------------------------------------------
 struct EpPeers {
@@ -288,30 +290,17 @@ struct TpArgs {
 cudaError_t launch_tp_finish(const TpArgs& args, cudaStream_t stream);
 
 // Expert-sorted form for many slots (native/src/moe.rs:66-182 route_plan, 1001-1085): slots are grouped by expert
-// into segments of up to R rows (seg_rows), so that an expert's columns are decoded once per R rows that use them.
-// R = kMoeSegRows = 8 is one block of rows of the fused kernel, whose one-block form runs two CTAs per SM and decodes
-// almost twice as fast per tile as the two-block form that 16 rows would need; R = kQmmSegRows = 64 is the token tile
-// of the small tensor-core shape, for batches that give most experts many rows.
-//   seg_count[0]        number of segments
-//   seg_expert[s]       expert of segment s
-//   row_slot[R s + r]   slot in row r of segment s, or 0xffffffff for a padding row
-//   slot_row[slot]      padded row R s + r that holds the slot
-// max_segments bounds the arrays (min(experts, slots) + slots / R always suffices).
-constexpr int kMoeSegRows = 8;
-cudaError_t launch_route_plan(const uint32_t* selected, int64_t slots, int experts, int max_segments, int seg_rows, int* seg_count,
-                              uint32_t* seg_expert, uint32_t* row_slot, uint32_t* slot_row, cudaStream_t stream);
-// padded-row forms of the three glue kernels; activations and products are laid out per segment:
-// xhat[(s * proj + p) * R + r, :], products y[r, (s * proj + p) * width + col] with row stride max_segments * proj * width
-cudaError_t launch_routed_prepare_padded(const void* x, int x_dtype, const __half* suh, const uint32_t* seg_expert,
-                                         const uint32_t* slot_row, int64_t slots, int top_k, int proj, int max_segments,
-                                         int seg_rows, int in, __half* xhat, cudaStream_t stream);
-cudaError_t launch_glu_down_input_padded(const float* ygu, const __half* gu_svh, const __half* down_suh,
-                                         const uint32_t* seg_expert, const uint32_t* row_slot, const int* seg_count,
-                                         int experts, int max_segments, int seg_rows, int hidden, int logical_hidden, __half* xhat,
-                                         cudaStream_t stream);
-cudaError_t launch_finish_and_reduce_padded(const float* raw, const __half* down_svh, const uint32_t* selected,
-                                            const uint32_t* slot_row, int experts, const void* scores, int score_dtype,
-                                            int64_t rows, int top_k, int out, int max_segments, int seg_rows, void* y, cudaStream_t stream);
+// into segments of up to kQmmSegRows rows, so that an expert's columns are decoded once per 64 rows that use them.
+//   seg_count[0]     number of segments
+//   seg_expert[s]    expert of segment s
+//   seg_rows[s]      slots in segment s
+//   slot_row[slot]   padded row 64 * segment + r that holds the slot
+// max_segments bounds the arrays (min(experts, slots) + slots / 64 always suffices).
+cudaError_t launch_route_plan(const uint32_t* selected, int64_t slots, int experts, int max_segments, int* seg_count,
+                              uint32_t* seg_expert, int* seg_rows, uint32_t* slot_row, cudaStream_t stream);
+// every slot's token row rotated with its expert's input scales: xhat[(g * proj + p) * 64 + r, :]
+cudaError_t launch_routed_prepare(const void* x, int x_dtype, const __half* suh, const uint32_t* selected, const uint32_t* slot_row,
+                                  int experts, int64_t slots, int top_k, int proj, int max_segments, int in, __half* xhat, cudaStream_t stream);
 
 // ---- router (kernels_router.cu) --------------------------------------------------------------------------
 // stable top-k per row with index tie-break; values and scores fp16 or fp32; experts <= 1024.  With `softmax` the
@@ -344,26 +333,47 @@ cudaError_t launch_head_argmax(const __half* x, const __half* w, int64_t vocab, 
 
 // ---- tensor-core product for many rows (kernels_qmm.cu) ---------------------------------------------------
 struct QmmPlan {
-    int splits;        // CTAs that share one (128 columns x token tile) output tile along the input axis
-    int token_tiles;   // ceil(rows / 512), or ceil(rows / 64) for the small shape
-    bool small;        // up to 64 rows: 64 tokens per CTA, two CTAs per SM
+    int token_tiles;     // ceil(rows / 512) (taken in halves of up to 256), 1 for the small shape
+    bool small;          // up to 64 rows: the whole batch is one tile, no weight is decoded twice
+    bool fixed;          // every item goes to `splits` CTAs; otherwise one wave of CTAs gets equal runs of stages
+    int splits;
+    int tile_tokens;     // tokens of an item, a multiple of 16
+    int64_t pass_rows;   // rows of one launch (more rows go in passes)
+    size_t piece_bytes;  // scratch for the parts of items that CTAs share
 };
-QmmPlan plan_qmm(int in, int out, int64_t rows);
-size_t qmm_partial_bytes(const QmmPlan& plan, int out, int64_t rows);
-// partials[s, r, n] (fp32) = sum over the inputs of split s of xhat[r, :] (fp16, rotated) x W[:, n]; with one
-// split and y != nullptr the output rotation (half -> H128 -> * svh, + bias) is applied in the kernel's epilogue
-// and y[r, n] is stored in y_dtype instead.
-// A member of a group (projections concatenated on the output axis) is addressed by ld_tiles (tiles per row of the
-// whole weight array; 0 = out / 16) and col_tile0 (the member's first tile column, a multiple of 8).
-cudaError_t launch_qmm(const uint32_t* wq, int in, int out, int k, int cb, const __half* xhat, int64_t rows,
-                       const QmmPlan& plan, float* partials, unsigned int* error, const __half* svh, const __half* bias,
-                       void* y, int y_dtype, cudaStream_t stream, int ld_tiles = 0, int col_tile0 = 0);
-// Expert-mapped form of the small shape: segment s = 64 padded rows xhat[(s * proj + p) * 64 + r, :] that all use expert
-// seg_expert[s]; products[r, (s * proj + p) * width + col] (fp32, row stride max_segments * proj * width).
-constexpr int kQmmSegRows = 64;
-cudaError_t launch_qmm_mapped(const uint32_t* wq, int in, int width, int bank_tiles_n, int k, int cb, const __half* xhat,
-                              int max_segments, int proj, int stride_blocks, int experts, const uint32_t* seg_expert,
-                              const int* seg_count, float* products, unsigned int* error, cudaStream_t stream);
+// `out` counts all members of a group; `whole_items`: no item is shared, so no scratch for pieces
+QmmPlan plan_qmm(int in, int out, int64_t rows, bool whole_items = false);
+constexpr int kQmmSegRows = 64;      // rows of an expert segment
+struct QmmArgs {
+    const uint32_t* wq;        // quad layout
+    float* pieces;             // [parts, tile tokens, 128] fp32: the parts of items that CTAs share
+    unsigned int* counters;    // [items] arrival counters, zero on entry and on exit
+    unsigned int* error;
+    const __half* svh;         // [out] (output rotation; yhat == nullptr)
+    const __half* bias;        // [out] or nullptr
+    float* yhat;               // summed fp32 products (rows of yhat_ld floats) instead of rotated outputs, or nullptr
+    int64_t yhat_ld;
+    void* gy[kQmvMaxGroups];   // per member: [rows, gout[g]] output in y_dtype
+    int gcol0[kQmvMaxGroups];  // per member: first column in the concatenated output space
+    int gout[kQmvMaxGroups];
+    int groups;                // activation rows of member g start at row g * rows of xhat
+    int y_dtype;
+    int in, out, rows;
+    int tiles, tile_tokens, items, box_rows;     // filled by the launch
+    unsigned long long* trace; // optional [CTA, 8] nanosecond stamps of the phases
+    // Expert-mapped mode (map_expert != nullptr; yhat): an item is (segment, projection, 128 columns); segment s holds
+    // map_rows[s] of up to 64 rows that all use expert map_expert[s], whose columns start at column block
+    // projection * map_stride_blocks + expert * map_blocks of the bank.  Row r of (segment, projection) is row
+    // (s * map_proj + p) * 64 + r of both xhat and yhat.
+    const uint32_t* map_expert;
+    const int* map_rows;
+    const int* map_count;      // segments in use (device)
+    int map_blocks, map_proj, map_stride_blocks, map_experts;
+};
+// xhat [groups, rows, in] fp16 (rotated with each member's input scales) times the layer's columns; rows <= plan.pass_rows
+cudaError_t launch_qmm(QmmArgs args, const __half* xhat, int k, int cb, const QmmPlan& plan, cudaStream_t stream);
+size_t qmm_mapped_piece_bytes();
+cudaError_t launch_qmm_mapped(QmmArgs args, const __half* xhat, int max_segments, int k, int cb, cudaStream_t stream);
 void qmm_set_tuning(int splits);   // force the number of input splits (0 = automatic)
 
 // ---- weight layout (kernels_codec.cu) -----------------------------------------------------------------

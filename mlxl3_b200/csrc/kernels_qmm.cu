@@ -1,34 +1,36 @@
-// Tensor-core product for many activation rows (prefill, verify batches): decode trellis tiles into
-// shared memory and feed tcgen05.mma with the accumulator in tensor memory.
+// Tensor-core product for many activation rows (prefill, verify batches, grouped experts): trellis tiles are decoded into
+// tensor memory, where tcgen05.mma reads them as its A operand; the accumulator is in tensor memory too.
 //
 // Reference behaviour replaced: native/shaders/_qmm_tensor_shared_kernel.metal (decode a weight tile
 // once, share it across row groups, matrix-unit product with fp32 accumulation) driven by
-// native/src/linear.rs:1874-2081.  Output here: fp32 partial products partials[split, row, n], which
-// the output-rotation kernel sums and rotates (the reference stores the raw product and finishes it
-// in native/src/linear.rs:1940-1963).
+// native/src/linear.rs:1874-2081, with the output rotation of native/src/linear.rs:1940-1963.
 //
 // Mapping.  The product is computed transposed, D[out, token] = W^T[out, in] . Xhat^T[in, token]:
-//  * one CTA owns 128 output columns (the 128 lanes of tensor memory), up to 512 tokens (all 512 fp32
-//    columns of tensor memory, as two halves of 256) and a contiguous range of 64-input stages
-//    (split-K across CTAs), so a batch of up to 512 rows decodes every weight exactly once;
-//  * A operand = decoded weights, [128 out, 64 in] fp16, K-major with the 128-byte swizzle.  One thread streams the
-//    packed stages (4 tile rows x 8 tiles, contiguous in the quad layout) with bulk copies into a ring; eight
-//    decoder warps each own four tiles (one interleaved quad) of one 16-input tile row of the stage, decode them
-//    bit-exactly in registers (the lane's eight weights are two 4-byte pairs for rows g and g+8 of the A tile) and
-//    store them with the swizzle applied;
-//  * B operand = rotated activations, [256 token, 64 in] fp16 per half, K-major, loaded by one TMA
-//    tensor copy per half and stage with the 128-byte swizzle (rows past the batch are zero-filled);
-//    the B ring is decoupled from the A ring;
-//  * one thread issues four tcgen05.mma (M=128, N=256, K=16) per half and stage and one commit per stage, which
-//    frees the A stage and the B slots; in the large shape a watcher warp tests the barriers for it (one lane per
-//    barrier, one instruction) and publishes a count; after the last stage the decoder warps read the accumulator
-//    with tcgen05.ld and either store partial products or rotate and store the outputs.
-// Every wait on an mbarrier is bounded in time; a wait that gives up sets the status word and the
-// kernel still releases its tensor memory.
+//  * an item is 128 output columns (the 128 lanes of tensor memory) x one tile of up to NT tokens (the MMA's N); its
+//    inputs are walked in stages of 128.  The stages of all items, item after item, are dealt out to the CTAs of ONE wave
+//    in equal runs (one CTA per SM), so no SM idles whatever the shape; a CTA that holds a whole item rotates and stores
+//    it, CTAs that share one leave fp32 pieces and the last to arrive adds them in input order;
+//  * A operand: sixteen decoder warps in two groups that take alternate stages; a warp owns the 32 lanes of its quarter of
+//    tensor memory = two 16-column tiles, of four of the stage's eight tile rows.  A lane's eight weights of a tile are the
+//    fragment of the 16x128b store shape, so a decoded tile goes from registers to tensor memory in one instruction;
+//  * B operand: rotated activations, two TMA tensor copies of [tile tokens, 64 in] fp16 per stage, 128-byte swizzle;
+//  * packed words: one bulk copy per stage (8 tile rows x 8 tiles are contiguous in the quad layout);
+//  * one thread issues the stage's eight products and one commit, which frees the A stage and the activation slot.
+//
+// What bounds it: the decode (60 to 70 cycles per tile and scheduler with everything else running; 49 at 4 bits, 53 at 3
+// bits alone), at NT = 256 nearly the products as well (1024 cycles of a stage's 1400).  Stages of 128 inputs and a single
+// barrier per stage are there because the single-thread roles share the schedulers with decoders that keep the integer
+// pipes full: an instruction of theirs takes about eight cycles, a stage of any of them 400 to 600.  For the same reason
+// the issuing loop is unrolled over the ring and its thread picked by elect.sync, so that addresses and descriptors are
+// constants in uniform registers; the producers' loops stay rolled (all three unrolled: instruction fetch stalls, 714 ns
+// per 64 inputs against 523).  Measured: 64 rows 4096->14336, 4 bits, 42 -> 29.7 us with the input rotation; 16 rows
+// 5120->25600, 3 bits, 74 -> 48.2 us (A in shared memory, one CTA per item and 64-token tile before).
+// Every wait is bounded in time; a wait that gives up sets the status word and the kernel still releases its tensor memory.
 #include <cuda.h>
 
 #include <algorithm>
 #include <atomic>
+#include <type_traits>
 
 #include "kernels.h"
 #include "hadamard.cuh"
@@ -38,57 +40,31 @@ namespace b200exl3 {
 
 namespace {
 
-constexpr int kStages = 3;            // decoded A stages in flight
-// packed stages (4 tile rows x 8 tiles = 1024*K bytes) in flight: a 16 KiB ring, at most 8 slots
-constexpr int raw_depth(int k) { return 16 / k > 8 ? 8 : 16 / k; }
-constexpr int kRawDepthMax = 8;
-constexpr uint32_t kRawBytes = 16 * 1024;
-constexpr int kGroupWarps = 8;        // decoder warps of a group: (tile row of the stage, quad of the 8-tile row)
-// Warp roles.  The single-thread roles take the lowest warp numbers: the scheduler favours older warps, and a
-// producer starved by spinning decoder warps stalls the whole pipeline.
-constexpr int kMmaWarp = 0, kActWarp = 1, kWeightWarp = 2, kWatchWarp = 3, kFirstDecoder = 4;
-constexpr uint32_t kAStageBytes = 128 * 128;           // 128 rows x 64 fp16
+// The single-thread roles take the lowest warp numbers: the scheduler favours older warps.
+constexpr int kMmaWarp = 0, kWeightWarp = 1, kActWarp = 2, kFirstDecoder = 4;
+constexpr int kStageIn = 128;                          // inputs of a stage
+constexpr int kStageCols = 64;                         // tensor-memory columns of an A stage: two fp16 inputs each
+constexpr int kChunk = 16;                             // tokens four warps finish at a time
 
-// Two shapes of the same kernel.  Large (more than 64 rows): a CTA holds up to 512 tokens (two accumulator
-// halves of 256), sixteen decoder warps in two groups on alternate stages, one CTA per SM.  Small (up to 64
-// rows): 64 tokens per CTA, eight decoder warps, under half of the shared memory and registers, so two CTAs
-// share an SM and twice as many warps decode -- these batches are bound by the decode, not by the MMAs.
-template <bool SMALL>
+template <int NT>
 struct QmmShape {
-    static constexpr int kTokHalf = SMALL ? 64 : 256;          // tokens per accumulator half = MMA N
-    static constexpr int kMaxHalves = SMALL ? 1 : 2;
-    static constexpr int kTokTile = kTokHalf * kMaxHalves;     // tokens per CTA
-    static constexpr int kDecoderGroups = SMALL ? 1 : 2;       // groups of eight decoder warps that take alternate stages
-    static constexpr int kDecoders = kDecoderGroups * kGroupWarps;
+    static constexpr int kGroups = 2;                  // groups of eight decoder warps that take alternate stages
+    static constexpr int kDecoders = 8 * kGroups;
     static constexpr int kThreads = 32 * (kFirstDecoder + kDecoders);
-    static constexpr int kMinBlocks = SMALL ? 2 : 1;
-    static constexpr int kBSlots = SMALL ? 4 : 5;              // activation half-stages in flight
-    static constexpr uint32_t kBSlotBytes = kTokHalf * 128;    // kTokHalf rows x 64 fp16
-    static constexpr uint32_t kInstrDesc = (1u << 4)                      // D = fp32
-                                           | (0u << 7) | (0u << 10)       // A, B = fp16
-                                           | (0u << 15) | (0u << 16)      // both K-major
-                                           | ((kTokHalf >> 3) << 17)      // N
-                                           | ((128u >> 4) << 24);         // M
-    static constexpr size_t kSmemBytes = kStages * kAStageBytes + kBSlots * kBSlotBytes + kRawBytes + 1024;
+    static constexpr int kSlots = NT == 64 ? 6 : 4;    // A stages in tensor memory beside NT accumulator columns
+    static constexpr int kBSlots = NT == 64 ? 6 : 2;   // activation stages in shared memory; divides kSlots
+    static constexpr uint32_t kBHalfBytes = NT * 128;  // NT tokens x 64 fp16
+    static constexpr uint32_t kBSlotBytes = 2 * kBHalfBytes;
+    static constexpr uint32_t kEpilogueBytes = kDecoders / 4 * 2 * kChunk * 128 * sizeof(__half);
+    static_assert(NT + kSlots * kStageCols <= 512 && kSlots % kGroups == 0 && kSlots % kBSlots == 0, "tensor memory");
 };
-
-struct QmmArgs {
-    const uint32_t* wq;        // quad layout
-    float* partials;           // [splits, rows, out]
-    unsigned int* error;
-    int in, out, rows, tiles_n, splits, stages_total;   // stages_total = in / 64
-    unsigned long long* trace;   // optional [CTA, 8] nanosecond stamps of the phases
-    const __half* svh;           // fused output rotation (y != nullptr; one input split): [out]
-    const __half* bias;          // [out] or nullptr
-    void* y;                     // [rows, out] in y_dtype, or nullptr: store fp32 partial products
-    int y_dtype;
-    // Expert-mapped mode (map_expert != nullptr; small shape, one split, fp32 products): the `out` axis is virtual,
-    // [segments, map_proj, map_blocks * 128]; segment s holds 64 padded rows that all use expert map_expert[s], whose
-    // columns start at column block map_proj_index * map_stride_blocks + expert * map_blocks of the bank.
-    const uint32_t* map_expert;
-    const int* map_count;      // segments in use; the CTAs of later segments return at once
-    int map_blocks, map_proj, map_stride_blocks, map_experts;
-};
+// packed stages (2048 * K bytes) in flight: 32 to 48 KB
+template <int K, int NT>
+constexpr int raw_slots() { return NT == 64 ? (K <= 4 ? 6 : (K <= 6 ? 4 : 3)) : (K <= 4 ? 4 : 2); }
+template <int K, int NT>
+constexpr size_t qmm_smem_bytes() {
+    return 1024 + QmmShape<NT>::kBSlots * QmmShape<NT>::kBSlotBytes + static_cast<size_t>(raw_slots<K, NT>()) * 2048 * K + QmmShape<NT>::kEpilogueBytes;
+}
 
 __device__ __forceinline__ uint64_t umma_desc(uint32_t smem_byte_addr) {
     // K-major operand, 128-byte swizzle: 8-row groups 1024 bytes apart, descriptor version 1
@@ -108,10 +84,11 @@ __device__ __forceinline__ void tmem_alloc(uint32_t* smem_dst, uint32_t cols) {
 __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t cols) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
 }
-__device__ __forceinline__ void umma_f16(uint32_t taddr, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+// D[tmem] (+)= A[tmem] . B[smem]
+__device__ __forceinline__ void umma_f16_ts(uint32_t d, uint32_t a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
-        "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}"
-        ::"r"(taddr), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+        "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}"
+        ::"r"(d), "r"(a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
 // One lane of a converged warp, chosen so that the compiler knows the branch is warp-uniform: the descriptors then live
 // in uniform registers.  Under `if (lane == 0)` every product was wrapped in a loop that moves them there one lane at a
@@ -132,72 +109,87 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
         "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
         ::"r"(smem_addr(dst)), "l"(map), "r"(smem_addr(bar)), "r"(c0), "r"(c1) : "memory");
 }
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
     asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-          "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-          "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
         : "r"(taddr) : "memory");
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+// 16 lanes x 8 columns: the weights of one decoded tile, row g and g + 8, inputs 2q, 2q+1 and 2q+8, 2q+9 of the lane
+template <int OFFSET>
+__device__ __forceinline__ void tmem_st_tile(uint32_t taddr, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3) {
+    asm volatile("tcgen05.st.sync.aligned.16x128b.x2.b32 [%0+%5], {%1,%2,%3,%4};" ::"r"(taddr), "r"(a0), "r"(a1), "r"(a2), "r"(a3), "n"(OFFSET));
 }
 
 // Wait that gives up after about a quarter of a second, or at once when another role of the CTA has
 // already given up, so that a lost copy or a miscounted barrier ends the kernel instead of hanging it.
-__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n.reg .pred p;\nmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
-        : "=r"(ok) : "r"(smem_addr(bar)), "r"(parity) : "memory");
-    return ok != 0;
-}
-__device__ __forceinline__ bool qmm_wait(uint64_t* bar, uint32_t parity, volatile int* cta_failed) {
-    // non-blocking tests: a suspended try_wait was seen to resume long after the phase completed.
+__device__ __noinline__ bool qmm_wait_slow(uint64_t* bar, uint32_t parity, volatile int* cta_failed) {
     // Reading the global timer costs about 0.2 us, so the clock only starts after many plain polls.
     for (int i = 0; i < 4096; ++i)
-        if (mbar_test_wait(bar, parity)) return true;
+        if (mbar_try_wait(bar, parity)) return true;
     const unsigned long long t0 = global_ns();
     for (int i = 1;; ++i) {
-        if (mbar_test_wait(bar, parity)) return true;
+        if (mbar_try_wait(bar, parity)) return true;
         if ((i & 255) == 0 && (*cta_failed || global_ns() - t0 > 250000000ull)) { *cta_failed = 1; return false; }
     }
 }
-__device__ __forceinline__ uint32_t ld_acquire_shared(const uint32_t* ptr) {
-    uint32_t v;
-    asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(smem_addr(ptr)) : "memory");
-    return v;
+__device__ __forceinline__ bool qmm_wait(uint64_t* bar, uint32_t parity, volatile int* cta_failed) {
+    return mbar_try_wait(bar, parity) || qmm_wait_slow(bar, parity, cta_failed);
 }
-__device__ __forceinline__ void st_release_shared(uint32_t* ptr, uint32_t v) {
-    asm volatile("st.release.cta.shared::cta.u32 [%0], %1;" ::"r"(smem_addr(ptr)), "r"(v) : "memory");
-}
-// Bounded wait of one thread until the watcher's count has passed `it` (a shared-memory load answers in tens of
-// cycles, a barrier test in a few hundred).
-__device__ __forceinline__ bool qmm_wait_count(const uint32_t* count, int it, volatile int* cta_failed) {
-    for (int i = 0; i < 16384; ++i)
-        if (ld_acquire_shared(count) > static_cast<uint32_t>(it)) return true;
-    const unsigned long long t0 = global_ns();
-    for (int i = 1;; ++i) {
-        if (ld_acquire_shared(count) > static_cast<uint32_t>(it)) return true;
-        if ((i & 255) == 0 && (*cta_failed || global_ns() - t0 > 250000000ull)) { *cta_failed = 1; return false; }
+__device__ __forceinline__ void group_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+
+// What an item is: where its weights, its activation rows and its outputs are.
+struct QmmItem {
+    int wblock;      // column block of the weight array
+    int cblock;      // column block of the output space (dense) or of the projection's columns (experts)
+    int brow;        // first activation row
+    int n;           // tokens
+    int tok0;        // first token of the batch (dense) / first output row (experts)
+};
+template <int NT>
+__device__ __forceinline__ QmmItem qmm_item(const QmmArgs& p, uint32_t item) {
+    QmmItem it;
+    if (p.map_expert != nullptr) {
+        const int sp = static_cast<int>(item) / p.map_blocks, j = static_cast<int>(item) - sp * p.map_blocks;
+        const int seg = sp / p.map_proj, proj = sp - seg * p.map_proj;
+        const int expert = static_cast<int>(min(p.map_expert[seg], static_cast<uint32_t>(p.map_experts - 1)));
+        it.wblock = proj * p.map_stride_blocks + expert * p.map_blocks + j;
+        it.cblock = j;
+        it.brow = it.tok0 = sp * kQmmSegRows;
+        it.n = p.map_rows[seg];
+    } else {
+        const int cb = static_cast<int>(item) / p.tiles, t = static_cast<int>(item) - cb * p.tiles;
+        int grp = 0;
+        while (grp + 1 < p.groups && cb * 128 >= p.gcol0[grp + 1]) ++grp;
+        it.wblock = it.cblock = cb;
+        it.tok0 = t * p.tile_tokens;
+        it.brow = grp * p.rows + it.tok0;
+        it.n = min(p.rows - it.tok0, p.tile_tokens);
     }
-}
-// The same wait for a whole warp: one lane polls (32 lanes polling one barrier flood the shared-memory
-// pipe that the copies, the stores and the MMA issue also need), then every lane observes the completed
-// phase itself, which makes the data the barrier guards visible to it.
-__device__ __forceinline__ bool qmm_wait_warp(uint64_t* bar, uint32_t parity, volatile int* cta_failed, int lane) {
-    int ok = 1;
-    if (lane == 0) ok = qmm_wait(bar, parity, cta_failed);
-    ok = __shfl_sync(0xffffffffu, ok, 0);
-    if (!ok) return false;
-    return mbar_test_wait(bar, parity) || qmm_wait(bar, parity, cta_failed);
+    return it;
 }
 
-template <int K, int CB, bool SMALL>
-__global__ void __launch_bounds__(QmmShape<SMALL>::kThreads, QmmShape<SMALL>::kMinBlocks)
+// One finished row of 128 outputs (lane L: columns 4L..4L+3): fp32 sums as they are, or rounded, rotated, scaled and stored.
+__device__ __forceinline__ void qmm_store_row(const QmmArgs& p, const QmmItem& it, int t, const __half (&in)[4], int lane) {
+    const int col = it.cblock * 128 + lane * 4;
+    int grp = 0;
+    while (grp + 1 < p.groups && it.cblock * 128 >= p.gcol0[grp + 1]) ++grp;
+    const int gcol = col - p.gcol0[grp];
+    __half h[4] = {in[0], in[1], in[2], in[3]};
+    warp_hadamard128_f16(h, lane);
+    const uint2 svw = *reinterpret_cast<const uint2*>(p.svh + col);
+    const __half* sv = reinterpret_cast<const __half*>(&svw);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) h[e] = __hmul_rn(h[e], sv[e]);
+    store4_from_half(p.gy[grp], p.y_dtype, static_cast<int64_t>(it.tok0 + t) * p.gout[grp] + gcol, h, p.bias ? p.bias + col : nullptr);
+}
+
+template <int K, int CB, int NT>
+__global__ void __launch_bounds__(QmmShape<NT>::kThreads, 1)
 qmm_kernel(const __grid_constant__ CUtensorMap xmap, const QmmArgs p) {
-    using S = QmmShape<SMALL>;
+    using S = QmmShape<NT>;
     // Dependent launch: this kernel may be scheduled under the tail of the kernel before it (the input rotation, the
     // glue of the expert block).  The packed weights are nobody's output, so the barriers, the tensor memory and the
     // first weight copies do not wait; what that kernel wrote -- the rotated rows, the segment table -- is read only
@@ -207,304 +199,332 @@ qmm_kernel(const __grid_constant__ CUtensorMap xmap, const QmmArgs p) {
     pdl_launch_dependents();
     if (p.map_expert != nullptr) pdl_wait();
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    constexpr int kQuadWords = 32 * K;                       // four interleaved tiles
-    constexpr int kRawStageWords = 8 * kQuadWords;           // 4 tile rows x 2 quads
-    constexpr uint32_t kRawStageBytes = kRawStageWords * 4;
-    constexpr int kRawDepth = raw_depth(K);
-    __shared__ __align__(8) uint64_t full_a[kStages], done[kStages], full_b[S::kBSlots], accum_bar;
-    __shared__ __align__(8) uint64_t raw_full[kRawDepthMax], raw_empty[kRawDepthMax];
-    __shared__ uint32_t tmem_base_slot;
-    __shared__ uint32_t s_mma_ready;      // written by the watcher warp: product stages whose operands are in place
+    constexpr int kRawWords = 512 * K;                       // a packed stage: 8 tile rows x 2 quads x 32K words
+    constexpr uint32_t kRawBytes = kRawWords * 4;
+    constexpr int kRaw = raw_slots<K, NT>();
+    __shared__ __align__(8) uint64_t full[S::kSlots], done[S::kSlots], raw_full[kRaw], raw_empty[kRaw];
+    __shared__ __align__(8) uint64_t accum_full, accum_free;
+    __shared__ uint32_t tmem_base_slot, s_last;
     __shared__ volatile int s_failed;
 
-    const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;   // uniform
-    const int g = lane >> 2, q = lane & 3;
-    unsigned long long* tr = p.trace ? p.trace + (blockIdx.y * gridDim.x + blockIdx.x) * 8 : nullptr;
+    const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;   // warp: uniform
+    const uint32_t spi = static_cast<uint32_t>(p.in) / kStageIn;                       // stages of an item
+    const uint32_t items = p.map_expert != nullptr ? static_cast<uint32_t>(*p.map_count * p.map_proj * p.map_blocks) : static_cast<uint32_t>(p.items);
+    // one run per CTA, at least one stage each; the launch keeps total * CTAs below 2^32
+    const uint32_t total = items * spi, G = min(gridDim.x, total);
+    if (blockIdx.x >= G) return;
+    const uint32_t s0 = total * blockIdx.x / G, s1 = total * (blockIdx.x + 1) / G;
+    if (s0 == s1) return;                                                        // uniform for the CTA; nothing is allocated yet
+    const int count = static_cast<int>(s1 - s0);
+    unsigned long long* tr = p.trace ? p.trace + blockIdx.x * 8 : nullptr;
     if (tr && threadIdx.x == 0) tr[0] = global_ns();
-    const int col_blocks = p.out >> 7;
-    const int cblock = blockIdx.x % col_blocks;
-    const int split = blockIdx.x / col_blocks;
-    const int tok0 = blockIdx.y * S::kTokTile;
-    int wblock = cblock;            // column block of the weight array
-    int brow0 = tok0;               // first row of the activation tile
-    if (p.map_expert != nullptr) {
-        const int sp = cblock / p.map_blocks, j = cblock - sp * p.map_blocks;
-        const int seg = sp / p.map_proj, proj = sp - seg * p.map_proj;
-        if (seg >= *p.map_count) return;                          // uniform for the CTA; nothing is allocated yet
-        const int expert = static_cast<int>(min(p.map_expert[seg], static_cast<uint32_t>(p.map_experts - 1)));
-        wblock = proj * p.map_stride_blocks + expert * p.map_blocks + j;
-        brow0 = sp * S::kTokTile;
-    }
-    const int halves = (S::kMaxHalves == 2 && p.rows - tok0 > S::kTokHalf) ? 2 : 1;      // accumulator halves this CTA fills
-    const uint32_t tmem_cols = halves * S::kTokHalf;
-    const int st0 = static_cast<int>(static_cast<int64_t>(p.stages_total) * split / p.splits);
-    const int st1 = static_cast<int>(static_cast<int64_t>(p.stages_total) * (split + 1) / p.splits);
-    const int nst = st1 - st0;
 
-    // shared memory: A stages | B slots | raw rings; the swizzled operands need 1024-byte alignment
-    unsigned char* a_base = smem_raw + ((1024u - (smem_addr(smem_raw) & 1023u)) & 1023u);
-    unsigned char* b_base = a_base + kStages * kAStageBytes;
+    // shared memory: activation ring | packed ring | epilogue staging; the swizzled operand needs 1024-byte alignment
+    unsigned char* b_base = smem_raw + ((1024u - (smem_addr(smem_raw) & 1023u)) & 1023u);
     uint32_t* raw_base = reinterpret_cast<uint32_t*>(b_base + S::kBSlots * S::kBSlotBytes);
+    __half* stage_base = reinterpret_cast<__half*>(raw_base + kRaw * kRawWords);
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < kStages; ++s) { mbar_init(&full_a[s], kGroupWarps); mbar_init(&done[s], 1); }
-        for (int s = 0; s < S::kBSlots; ++s) mbar_init(&full_b[s], 1);
-        mbar_init(&accum_bar, 1);
-        for (int d = 0; d < kRawDepth; ++d) { mbar_init(&raw_full[d], 1); mbar_init(&raw_empty[d], kGroupWarps); }
+        // a stage is full when its eight decoder warps and its activation copies have arrived
+        for (int s = 0; s < S::kSlots; ++s) { mbar_init(&full[s], 9); mbar_init(&done[s], 1); }
+        for (int s = 0; s < kRaw; ++s) { mbar_init(&raw_full[s], 1); mbar_init(&raw_empty[s], 8); }
+        mbar_init(&accum_full, 1);
+        mbar_init(&accum_free, S::kDecoders);
         s_failed = 0;
-        s_mma_ready = 0;
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    if (warp == kMmaWarp) tmem_alloc(&tmem_base_slot, tmem_cols);
+    if (warp == kMmaWarp) tmem_alloc(&tmem_base_slot, 512);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_base_slot;
+    const uint32_t first_item = s0 / spi, k0 = s0 - first_item * spi;            // first item and its first stage here
     if (tr && threadIdx.x == 0) tr[1] = global_ns();
 
-    const int dec = warp - kFirstDecoder;                        // decoder index, negative for the other roles
-    if (dec >= 0) {
-        // ================= decoder warps: packed quad -> 16 inputs x 64 outputs of the A stage =================
-        // Two groups of eight warps take alternate stages, so that one group's barrier round trips and
-        // proxy fence overlap the other group's arithmetic.  Within a group: (tile row of the stage, quad).
-        const int group = dec >> 3, trow = dec & 3, quad = (dec >> 2) & 1;
+    if (warp >= kFirstDecoder) {
+        // ================= decoders: packed words -> A stages in tensor memory; then the epilogue of each item =================
+        const int dec = warp - kFirstDecoder, group = dec >> 3, rows4 = (dec >> 2) & 1, quarter = dec & 3;   // quarter == warp & 3: the lanes it may access
+        const int quad = dec >> 2;                               // four warps that hold all lanes
         const LaneGeom<K> geom(lane);
-        // this warp's quad of a packed stage: input tile 4*stage + trow, output tiles 8*cblock + 4*quad .. +3
-        const uint32_t* my_quad = raw_base + (trow * 2 + quad) * kQuadWords;
-        // A barrier test takes a few hundred cycles to answer, so the tests for the warp's next stage are
-        // issued before the current stage is decoded and their answer is only looked at afterwards.
-        // Large shape: lane 0 tests the packed words and lane 1 the A stage in ONE instruction, so the warp stalls
-        // once, not twice (the warp barrier below orders the other lanes' reads after the two observations).  With two
-        // small CTAs per SM that was measured slower than every lane testing both.
-        auto stage_ready = [&](int it) -> bool {
-            if constexpr (SMALL) {
-                return mbar_test_wait(&raw_full[it % kRawDepth], (it / kRawDepth) & 1u) &
-                       mbar_test_wait(&done[it % kStages], ((it / kStages) & 1u) ^ 1u);
-            } else {
-                uint64_t* bar = lane == 0 ? &raw_full[it % kRawDepth] : &done[it % kStages];
-                const uint32_t par = lane == 0 ? (it / kRawDepth) & 1u : ((it / kStages) & 1u) ^ 1u;
-                bool ok = true;
-                if (lane < 2) ok = mbar_test_wait(bar, par);
-                return ok;
-            }
+        // this warp's two tiles of each row: half of a quad of four interleaved tiles
+        const uint32_t* words = raw_base + rows4 * (256 * K) + (quarter >> 1) * (32 * K) + (quarter & 1) * 2;
+        const int j2 = geom.i2 * 4, j1 = geom.i1 * 4, j0 = geom.i0 * 4;
+        const uint32_t lanes = tmem + (static_cast<uint32_t>(quarter * 32) << 16);
+        int slot = group, rslot = group % kRaw;
+        uint32_t par = 0, rpar = (group / kRaw) & 1;
+        // A barrier test takes a few hundred cycles to answer beside busy decoders, so the tests for the warp's next stage
+        // are issued before the current stage is decoded: lane 0 tests the packed words and lane 1 the A stage in ONE
+        // instruction (the warp barrier orders the other lanes' reads after the two observations).
+        auto stage_ready = [&]() -> bool {
+            bool ok = true;
+            if (lane < 2) ok = mbar_test_wait(lane == 0 ? &raw_full[rslot] : &done[slot], lane == 0 ? rpar : par ^ 1u);
+            return ok;
         };
-        bool ready = group < nst && stage_ready(group);
-        for (int it = group; it < nst; it += S::kDecoderGroups) {
-            const int s = it % kStages, rslot = it % kRawDepth;
-            if (!__all_sync(0xffffffffu, ready)) {
-                // the packed stage has landed, and the MMAs that read this A stage last time are done
-                ready = qmm_wait(&raw_full[rslot], (it / kRawDepth) & 1u, &s_failed) &&
-                        qmm_wait(&done[s], ((it / kStages) & 1u) ^ 1u, &s_failed);
-                if (!__all_sync(0xffffffffu, ready)) break;
-            }
-            if constexpr (!SMALL) __syncwarp();
-            unsigned char* a_stage = a_base + s * kAStageBytes;
-            const uint4* qw = reinterpret_cast<const uint4*>(my_quad + rslot * kRawStageWords);
-            const uint4 W2 = qw[geom.i2];
-            const uint4 W1 = qw[geom.i1];
-            uint4 W0 = make_uint4(0, 0, 0, 0);
-            if constexpr (K >= 5) W0 = qw[geom.i0];
-            const uint32_t w2[4] = {W2.x, W2.y, W2.z, W2.w}, w1[4] = {W1.x, W1.y, W1.z, W1.w},
-                           w0[4] = {W0.x, W0.y, W0.z, W0.w};
-            ready = it + S::kDecoderGroups < nst && stage_ready(it + S::kDecoderGroups);
+        bool ready = group < count && stage_ready();
+        int it = group;
+        int seg_begin = 0, buf = 0;
+        uint32_t item = first_item, k_first = k0, seg = 0;
+        while (seg_begin < count) {
+            const int seg_end = min(count, seg_begin + static_cast<int>(spi - k_first));
+#pragma unroll 1
+            for (; it < seg_end; it += S::kGroups) {
+                if (!__all_sync(0xffffffffu, ready)) {
+                    // the packed stage has landed, and the MMAs that read this A stage last time are done
+                    ready = qmm_wait(&raw_full[rslot], rpar, &s_failed) && qmm_wait(&done[slot], par ^ 1u, &s_failed);
+                    if (!__all_sync(0xffffffffu, ready)) break;
+                }
+                __syncwarp();
+                const uint32_t* rw = words + rslot * kRawWords;
+                const uint32_t dst = lanes + NT + rows4 * 32 + slot * kStageCols;
+                uint64_t* stage_full = &full[slot];
+                uint64_t* empty = &raw_empty[rslot];
+                slot += S::kGroups;
+                if (slot >= S::kSlots) { slot -= S::kSlots; par ^= 1u; }
+                rslot += S::kGroups;
+                if (rslot >= kRaw) { rslot -= kRaw; rpar ^= 1u; }
+                ready = it + S::kGroups < count && stage_ready();
+                uint2 w2[4], w1[4], w0[4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                uint32_t a0, a1, a2, a3;
-                lane_weights_exact<K, CB>(w2[j], w1[j], w0[j], geom.slack, a0, a1, a2, a3);
-                // rows (= output columns) 16t+g and 16t+g+8 of the A tile; 16-byte chunks 2*trow and 2*trow+1 of
-                // the row, XORed with the row index modulo 8 (the 128-byte swizzle); 4q bytes into the chunk
-                const int t = quad * 4 + j;
-                unsigned char* r0 = a_stage + (16 * t + g) * 128 + 4 * q;
-                const int c0 = ((2 * trow) ^ g) << 4, c1 = ((2 * trow + 1) ^ g) << 4;
-                *reinterpret_cast<uint32_t*>(r0 + c0) = a0;
-                *reinterpret_cast<uint32_t*>(r0 + 8 * 128 + c0) = a1;
-                *reinterpret_cast<uint32_t*>(r0 + c1) = a2;
-                *reinterpret_cast<uint32_t*>(r0 + 8 * 128 + c1) = a3;
-            }
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic writes -> visible to the MMA unit
-            __syncwarp();
-            if (lane == 0) {
-                mbar_arrive(&raw_empty[rslot]);                         // the packed words were consumed: slot free for this warp
-                mbar_arrive(&full_a[s]);
-            }
-        }
-        if (tr && threadIdx.x == 32 * kFirstDecoder) tr[2] = global_ns();
-    } else if (warp == kActWarp) {
-        // ================= activation producer: one tensor copy per half and stage =================
-        if (lane < halves) {
-            // Lane h copies half h: the two halves' barrier tests (a few hundred cycles each) run side by side.
-            // A slot is free once the MMAs of the stage that used it last are done.
-            const int h = lane;
-            pdl_wait();
-            for (int it = 0; it < nst && !s_failed; ++it) {
-                const int u = it * halves + h, slot = u % S::kBSlots;
-                const int before = u - S::kBSlots;                       // the use of this slot one lap earlier
-                if (before >= 0) {
-                    const int st = before / halves;
-                    if (!qmm_wait(&done[st % kStages], (st / kStages) & 1u, &s_failed)) break;
+                for (int r = 0; r < 4; ++r) {
+                    const uint32_t* row = rw + r * (64 * K);
+                    w2[r] = *reinterpret_cast<const uint2*>(row + j2);
+                    w1[r] = *reinterpret_cast<const uint2*>(row + j1);
+                    w0[r] = make_uint2(0, 0);
+                    if constexpr (K >= 5) w0[r] = *reinterpret_cast<const uint2*>(row + j0);
                 }
-                mbar_expect_tx(&full_b[slot], S::kBSlotBytes);
-                tma_load_2d(b_base + slot * S::kBSlotBytes, &xmap, (st0 + it) * 64, brow0 + h * S::kTokHalf, &full_b[slot]);
-            }
-            if (tr && lane == 0) tr[7] = global_ns();
-        }
-    } else if (warp == kWeightWarp) {
-        // ================= weight producer: one bulk copy (4 tile rows x 8 tiles, contiguous) per stage =================
-        if (lane == 0) {
-            int slot = 0;
-            uint32_t par = 0;
-            for (int it = 0; it < nst && !s_failed; ++it) {
-                if (!qmm_wait(&raw_empty[slot], par ^ 1u, &s_failed)) break;
-                mbar_expect_tx(&raw_full[slot], kRawStageBytes);
-                bulk_copy_g2s(raw_base + slot * kRawStageWords, p.wq + quad_row_offset(4 * (st0 + it), wblock, p.in / 16, K), kRawStageBytes,
-                              &raw_full[slot]);
-                if (++slot == kRawDepth) { slot = 0; par ^= 1u; }
-            }
-        }
-    } else if (!SMALL && warp == kWatchWarp) {
-        // ================= watcher: all barriers of the next product stage in ONE test instruction =================
-        // A barrier test answers after a few hundred cycles and the thread that reads the answer stalls that long.
-        // Up to three tests in a row per stage (A stage, one or two activation slots) cost the issuing thread more
-        // time than issuing the stage's products: it, not the tensor pipe, set the pace.  Here lane 0 looks at the A
-        // stage and lanes 1, 2 at the activation slots, one instruction tests them all, and the count of stages whose
-        // operands are in place is published in shared memory, where the issuing thread reads it in tens of cycles.
-        // (Large shape only: with two small CTAs per SM the decoders set the pace and a second polling warp costs more
-        // than it saves -- measured.)
-        const uint32_t mask = halves == 2 ? 7u : 3u;
-        int idle = 0;
-        unsigned long long t0 = 0;
-        for (int it = 0; it < nst;) {
-            uint64_t* bar = nullptr;
-            uint32_t par = 0;
-            if (lane == 0) {
-                bar = &full_a[it % kStages]; par = (it / kStages) & 1u;
-            } else if (lane <= halves) {
-                const int u = it * halves + lane - 1;
-                bar = &full_b[u % S::kBSlots]; par = (u / S::kBSlots) & 1u;
-            }
-            bool ok = false;
-            if (bar != nullptr) ok = mbar_test_wait(bar, par);
-            if ((__ballot_sync(0xffffffffu, ok) & mask) == mask) {
-                ++it;
-                idle = 0;
-                if (lane == 0) st_release_shared(&s_mma_ready, static_cast<uint32_t>(it));
-                continue;
-            }
-            if ((++idle & 1023) == 0) {                                   // bounded like every other wait of the kernel
-                int give_up = 0;
+                auto tile_pair = [&](auto row) {
+                    constexpr int r = decltype(row)::value;
+                    uint32_t a0, a1, a2, a3;
+                    lane_weights_exact<K, CB>(w2[r].x, w1[r].x, w0[r].x, geom.slack, a0, a1, a2, a3);
+                    tmem_st_tile<r * 8>(dst, a0, a1, a2, a3);
+                    lane_weights_exact<K, CB>(w2[r].y, w1[r].y, w0[r].y, geom.slack, a0, a1, a2, a3);
+                    tmem_st_tile<r * 8 + (16 << 16)>(dst, a0, a1, a2, a3);
+                };
+                tile_pair(std::integral_constant<int, 0>{});
+                tile_pair(std::integral_constant<int, 1>{});
+                tile_pair(std::integral_constant<int, 2>{});
+                tile_pair(std::integral_constant<int, 3>{});
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 if (lane == 0) {
-                    if (idle == 1024) t0 = global_ns();
-                    give_up = s_failed || global_ns() - t0 > 250000000ull;
-                    if (give_up) s_failed = 1;
+                    mbar_arrive(stage_full);
+                    mbar_arrive(empty);                          // the packed words were consumed: slot free for this warp
                 }
-                if (__shfl_sync(0xffffffffu, give_up, 0)) break;
             }
+            // ---- epilogue of the item (or of this CTA's part of it) ----
+            if (seg == 0) {
+                pdl_wait();                                      // returns at once: the kernel before ended long ago
+                if (tr && dec == 0 && lane == 0) tr[2] = global_ns();
+            }
+            const QmmItem info = qmm_item<NT>(p, item);
+            qmm_wait(&accum_full, seg & 1u, &s_failed);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            __syncwarp();
+            const bool complete = seg_end - seg_begin == static_cast<int>(spi);
+            // parts of shared items in order of (CTA, item): CTA + item numbers them; with more items than CTAs, two per CTA
+            const size_t piece_floats = static_cast<size_t>(p.tile_tokens) * 128;
+            float* piece = p.pieces + (items < G ? blockIdx.x + item : 2 * blockIdx.x + (seg > 0 ? 1 : 0)) * piece_floats;
+            // chunks of 16 tokens: four warps hold 32 columns each of the same tokens
+            for (int c = quad * kChunk; c < info.n; c += S::kDecoders / 4 * kChunk) {
+                uint32_t r[16];
+                tmem_ld16(lanes + c, r);
+                if (!complete || p.yhat != nullptr) {
+                    float* dst = complete ? p.yhat + static_cast<int64_t>(info.tok0 + c) * p.yhat_ld + info.cblock * 128 + quarter * 32 + lane
+                                          : piece + c * 128 + quarter * 32 + lane;
+                    const int64_t ld = complete ? p.yhat_ld : 128;
+#pragma unroll
+                    for (int i = 0; i < kChunk; ++i)
+                        if (c + i < info.n) dst[i * ld] = __uint_as_float(r[i]);
+                } else {
+                    // the output rotation runs over the 128 columns of a token: transposed through shared memory, then
+                    // every warp rotates four tokens
+                    __half* stage = stage_base + (quad * 2 + buf) * (kChunk * 128);
+#pragma unroll
+                    for (int i = 0; i < kChunk; ++i) stage[i * 128 + quarter * 32 + lane] = __float2half_rn(__uint_as_float(r[i]));
+                    group_sync(1 + quad, 128);
+#pragma unroll 2
+                    for (int j = 0; j < 4; ++j) {
+                        const int t = quarter * 4 + j;
+                        if (c + t >= info.n) break;
+                        __align__(8) __half h[4];
+                        *reinterpret_cast<uint2*>(h) = *reinterpret_cast<const uint2*>(stage + t * 128 + lane * 4);
+                        qmm_store_row(p, info, c + t, h, lane);
+                    }
+                    buf ^= 1;
+                }
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&accum_free);             // the accumulator may be overwritten
+            if (!complete) {
+                // CTAs share the item: this one's part is a piece; the last to arrive adds the pieces in input order
+                const uint32_t x0 = item * spi;
+                const uint32_t c_first = ((x0 + 1) * G - 1) / total, c_last = ((x0 + spi) * G - 1) / total;
+                __threadfence();
+                group_sync(8, S::kDecoders * 32);
+                if (dec == 0 && lane == 0) {
+                    const unsigned int before = atomicAdd(p.counters + item, 1u);
+                    s_last = before == c_last - c_first;
+                    if (s_last) p.counters[item] = 0;            // leave the scratch ready for the next call
+                }
+                group_sync(8, S::kDecoders * 32);
+                if (s_last) {
+                    __threadfence();
+                    // the first CTA's part is its last one if it starts before the item, the others' their first
+                    const size_t stride = items < G ? piece_floats : 2 * piece_floats;
+                    const float* base = p.pieces + (items < G ? c_first + item : 2 * c_first) * piece_floats + lane * 4;
+                    const float* base0 = base + (items >= G && total * c_first / G < x0 ? piece_floats : 0);
+                    const int pieces = static_cast<int>(c_last - c_first) + 1;
+                    // a warp's rows two at a time, up to four parts of each in flight
+                    for (int t0 = dec; t0 < info.n; t0 += 2 * S::kDecoders) {
+                        const int t1 = t0 + S::kDecoders < info.n ? t0 + S::kDecoders : t0;
+                        float4 a[2] = {__ldcg(reinterpret_cast<const float4*>(base0 + t0 * 128)), __ldcg(reinterpret_cast<const float4*>(base0 + t1 * 128))};
+#pragma unroll 1
+                        for (int q0 = 1; q0 < pieces; q0 += 4) {
+                            float4 part[2][4];
+#pragma unroll
+                            for (int j = 0; j < 4; ++j)
+                                if (q0 + j < pieces) {
+                                    part[0][j] = __ldcg(reinterpret_cast<const float4*>(base + (q0 + j) * stride + t0 * 128));
+                                    part[1][j] = __ldcg(reinterpret_cast<const float4*>(base + (q0 + j) * stride + t1 * 128));
+                                }
+#pragma unroll
+                            for (int j = 0; j < 4; ++j)
+                                if (q0 + j < pieces)
+#pragma unroll
+                                    for (int i = 0; i < 2; ++i) {
+                                        a[i].x = __fadd_rn(a[i].x, part[i][j].x); a[i].y = __fadd_rn(a[i].y, part[i][j].y);
+                                        a[i].z = __fadd_rn(a[i].z, part[i][j].z); a[i].w = __fadd_rn(a[i].w, part[i][j].w);
+                                    }
+                        }
+#pragma unroll
+                        for (int i = 0; i < 2; ++i) {
+                            const int t = i == 0 ? t0 : t1;
+                            if (i == 1 && t1 == t0) break;
+                            if (p.yhat != nullptr) {
+                                *reinterpret_cast<float4*>(p.yhat + static_cast<int64_t>(info.tok0 + t) * p.yhat_ld + info.cblock * 128 + lane * 4) = a[i];
+                            } else {
+                                const __half h[4] = {__float2half_rn(a[i].x), __float2half_rn(a[i].y), __float2half_rn(a[i].z), __float2half_rn(a[i].w)};
+                                qmm_store_row(p, info, t, h, lane);
+                            }
+                        }
+                    }
+                }
+            }
+            seg_begin = seg_end;
+            k_first = 0;
+            ++item;
+            ++seg;
+        }
+        if (tr && dec == 0 && lane == 0) tr[5] = global_ns();
+    } else if (warp == kWeightWarp) {
+        // ================= weight producer: one bulk copy (8 tile rows x 8 tiles, contiguous) per stage =================
+        if (elect_one()) {
+            uint32_t item = first_item, par = 0;
+            int done_before = 0, rem = min(count, static_cast<int>(spi - k0)), run = rem;
+            const uint32_t* src = p.wq + quad_row_offset(8 * static_cast<int>(k0), qmm_item<NT>(p, item).wblock, p.in / 16, K);
+            bool running = true;
+            while (running) {
+#pragma unroll 1
+                for (int s = 0; s < kRaw; ++s) {
+                    if (!qmm_wait(&raw_empty[s], par ^ 1u, &s_failed)) { running = false; break; }
+                    mbar_expect_tx(&raw_full[s], kRawBytes);
+                    bulk_copy_g2s(raw_base + s * kRawWords, src, kRawBytes, &raw_full[s]);
+                    src += kRawWords;
+                    if (--rem == 0) {
+                        done_before += run;
+                        if (done_before == count) { running = false; break; }
+                        run = rem = min(count - done_before, static_cast<int>(spi));
+                        src = p.wq + quad_row_offset(0, qmm_item<NT>(p, ++item).wblock, p.in / 16, K);
+                    }
+                }
+                par ^= 1u;
+            }
+        }
+    } else if (warp == kActWarp) {
+        // ================= activation producer: tensor copies of [tokens, 64 inputs] =================
+        if (elect_one()) {
+            pdl_wait();
+            uint32_t item = first_item, par = 0;
+            int done_before = 0, rem = min(count, static_cast<int>(spi - k0)), x = static_cast<int>(k0) * kStageIn;
+            int run = rem;                                                       // stages of the current item here
+            QmmItem info = qmm_item<NT>(p, item);
+            int boxes = p.map_expert != nullptr ? (info.n + 15) >> 4 : 1;        // expert segments come in boxes of 16 rows
+            uint32_t box_bytes = static_cast<uint32_t>(boxes * p.box_rows) * 256u;
+            bool running = true;
+            while (running) {
+#pragma unroll 1
+                for (int s = 0; s < S::kSlots; ++s) {
+                    // the slot is free once the MMAs of the stage that used it last (kBSlots stages ago) are done
+                    constexpr int kB = S::kBSlots;
+                    const int before = (s + S::kSlots - kB) % S::kSlots;
+                    if (!qmm_wait(&done[before], s >= kB ? par : par ^ 1u, &s_failed)) { running = false; break; }
+                    unsigned char* dst = b_base + (s % kB) * S::kBSlotBytes;
+                    mbar_expect_tx(&full[s], box_bytes);
+                    tma_load_2d(dst, &xmap, x, info.brow, &full[s]);
+                    tma_load_2d(dst + S::kBHalfBytes, &xmap, x + 64, info.brow, &full[s]);
+                    for (int b = 1; b < boxes; ++b) {
+                        tma_load_2d(dst + b * 2048, &xmap, x, info.brow + b * 16, &full[s]);
+                        tma_load_2d(dst + S::kBHalfBytes + b * 2048, &xmap, x + 64, info.brow + b * 16, &full[s]);
+                    }
+                    x += kStageIn;
+                    if (--rem == 0) {
+                        done_before += run;
+                        if (done_before == count) { running = false; break; }
+                        run = rem = min(count - done_before, static_cast<int>(spi));
+                        x = 0;
+                        info = qmm_item<NT>(p, ++item);
+                        if (p.map_expert != nullptr) { boxes = (info.n + 15) >> 4; box_bytes = static_cast<uint32_t>(boxes) * 4096u; }
+                    }
+                }
+                par ^= 1u;
+            }
+            if (tr) tr[7] = global_ns();
         }
     } else if (warp == kMmaWarp) {
         // ================= MMA issuer =================
         if (elect_one()) {
-            // small shape: the thread tests the barriers itself, all tests of the next stage right after the commit
-            auto stage_ready = [&](int it) -> bool {
-                return mbar_test_wait(&full_a[it % kStages], (it / kStages) & 1u) &
-                       mbar_test_wait(&full_b[it % S::kBSlots], (it / S::kBSlots) & 1u);
+            uint32_t item = first_item, par = 0, seg = 0, accumulate = 0;
+            int left = count, rem = min(count, static_cast<int>(spi - k0));
+            auto instr_desc = [&](uint32_t i) -> uint32_t {
+                const int n16 = (qmm_item<NT>(p, i).n + 15) >> 4;
+                return (1u << 4) /* D = fp32; A, B = fp16, K-major */ | (static_cast<uint32_t>(n16 * 2) << 17) /* N */ | ((128u >> 4) << 24) /* M */;
             };
-            bool ready = SMALL && nst > 0 && stage_ready(0);
-            for (int it = 0; it < nst && !s_failed; ++it) {
-                const int s = it % kStages;
-                if constexpr (SMALL) {
-                    if (!ready && (!qmm_wait(&full_a[s], (it / kStages) & 1u, &s_failed) ||
-                                   !qmm_wait(&full_b[it % S::kBSlots], (it / S::kBSlots) & 1u, &s_failed)))
-                        break;
-                } else if (!qmm_wait_count(&s_mma_ready, it, &s_failed)) break;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t a_addr = smem_addr(a_base + s * kAStageBytes);
-                for (int h = 0; h < halves; ++h) {
-                    const uint32_t b_addr = smem_addr(b_base + ((it * halves + h) % S::kBSlots) * S::kBSlotBytes);
+            uint32_t idesc = instr_desc(item);
+            const uint64_t b_desc0 = umma_desc(smem_addr(b_base));
+            bool running = true;
+            while (running) {
 #pragma unroll
-                    for (int kk = 0; kk < 4; ++kk)                      // 4 x 16 inputs = one 64-input stage
-                        umma_f16(tmem + h * S::kTokHalf, umma_desc(a_addr + kk * 32), umma_desc(b_addr + kk * 32), S::kInstrDesc,
-                                 (it > 0 || kk > 0) ? 1u : 0u);
+                for (int s = 0; s < S::kSlots; ++s) {
+                    if (rem == 0) {
+                        umma_commit(&accum_full);                                // accumulator of this item complete
+                        if (left == 0) { running = false; break; }
+                        if (!qmm_wait(&accum_free, seg & 1u, &s_failed)) { running = false; break; }
+                        ++seg;
+                        idesc = instr_desc(++item);
+                        rem = min(left, static_cast<int>(spi));
+                        accumulate = 0;
+                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    }
+                    if (!qmm_wait(&full[s], par, &s_failed)) { running = false; break; }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint64_t bd = b_desc0 + (s % S::kBSlots) * (S::kBSlotBytes >> 4);
+#pragma unroll
+                    for (int kk = 0; kk < 8; ++kk)                               // 8 x 16 inputs: two halves of 64
+                        umma_f16_ts(tmem, tmem + NT + s * kStageCols + kk * 8, bd + (kk >> 2) * (S::kBHalfBytes >> 4) + (kk & 3) * 2, idesc,
+                                    kk > 0 ? 1u : accumulate);
+                    accumulate = 1;
+                    umma_commit(&done[s]);                                       // A stage and activation slot free once these MMAs have read them
+                    --rem;
+                    --left;
                 }
-                umma_commit(&done[s]);                                  // A stage and B slots free once these MMAs have read them
-                if constexpr (SMALL) ready = it + 1 < nst && stage_ready(it + 1);
+                par ^= 1u;
             }
-            umma_commit(&accum_bar);                                    // accumulator complete
+            if (s_failed) umma_commit(&accum_full);
             if (tr) tr[3] = global_ns();
         }
     }
-
-    // ================= epilogue: accumulator -> fp32 partial products =================
-    if (dec >= 0) {
-        pdl_wait();                                                     // returns at once: the kernel before ended long ago
-        if (nst > 0) {
-            qmm_wait_warp(&accum_bar, 0, &s_failed, lane);
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        }
-        if (tr && threadIdx.x == 32 * kFirstDecoder) tr[4] = global_ns();
-        // a warp may read the 32 lanes 32*(warp%4)..; the warps of a lane quarter share the token columns
-        const int lq = warp & 3, cpart = dec >> 2;
-        const int col = cblock * 128 + lq * 32 + lane;                  // this thread's output column = its TMEM lane
-        float* dst = p.partials + (static_cast<int64_t>(split) * p.rows) * p.out + col;
-        const int c_span = static_cast<int>(tmem_cols) / (S::kDecoders / 4);
-        const int c_begin = cpart * c_span, c_end = c_begin + c_span;
-        if (p.y == nullptr) {
-            for (int c = c_begin; c < c_end; c += 32) {
-                if (tok0 + c >= p.rows) break;
-                uint32_t r[32];
-                if (nst > 0) tmem_ld32(tmem + (static_cast<uint32_t>(lq * 32) << 16) + c, r);
-                else
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) r[i] = 0;
-#pragma unroll
-                for (int i = 0; i < 32; ++i) {
-                    const int tok = tok0 + c + i;
-                    if (tok < p.rows) dst[static_cast<int64_t>(tok) * p.out] = __uint_as_float(r[i]);
-                }
-            }
-        } else {
-            // Output rotation fused (one input split only): the four warps that share a range of token
-            // columns transpose 32 tokens x 128 outputs through shared memory (the operand rings are free
-            // once the accumulator is complete), then every warp rotates eight token rows:
-            // half(sum) -> H128 -> * svh (+ bias), stored in the caller's dtype.
-            __half* stage_base = reinterpret_cast<__half*>(b_base) + cpart * (2 * 32 * 128);
-            const __half* sv = p.svh + cblock * 128 + lane * 4;
-            const __half* bias = p.bias ? p.bias + cblock * 128 : nullptr;
-            int buf = 0;
-            for (int c = c_begin; c < c_end; c += 32) {
-                if (tok0 + c >= p.rows) break;
-                uint32_t r[32];
-                tmem_ld32(tmem + (static_cast<uint32_t>(lq * 32) << 16) + c, r);
-                __half* stage = stage_base + buf * (32 * 128);
-#pragma unroll
-                for (int i = 0; i < 32; ++i) stage[i * 128 + lq * 32 + lane] = __float2half_rn(__uint_as_float(r[i]));
-                asm volatile("bar.sync %0, %1;" ::"r"(1 + cpart), "r"(128) : "memory");
-#pragma unroll 2
-                for (int j = 0; j < 8; ++j) {                            // two rows' shuffle chains in flight
-                    const int t = lq * 8 + j, tok = tok0 + c + t;
-                    if (tok >= p.rows) break;
-                    __align__(8) __half h[4];
-                    *reinterpret_cast<uint2*>(h) = *reinterpret_cast<const uint2*>(stage + t * 128 + lane * 4);
-                    warp_hadamard128_f16(h, lane);
-                    if (p.y_dtype == kF16) {                            // one 8-byte store per lane
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            h[e] = __hmul_rn(h[e], sv[e]);
-                            if (bias) h[e] = __hadd_rn(h[e], bias[lane * 4 + e]);
-                        }
-                        *reinterpret_cast<uint2*>(reinterpret_cast<__half*>(p.y) + static_cast<int64_t>(tok) * p.out + cblock * 128 +
-                                                  lane * 4) = *reinterpret_cast<const uint2*>(h);
-                    } else {
-#pragma unroll
-                        for (int e = 0; e < 4; ++e)
-                            store_from_half(p.y, p.y_dtype, static_cast<int64_t>(tok) * p.out + cblock * 128 + lane * 4 + e,
-                                            __hmul_rn(h[e], sv[e]), bias, lane * 4 + e);
-                    }
-                }
-                buf ^= 1;
-            }
-        }
-    }
-    if (tr && threadIdx.x == 32 * kFirstDecoder) tr[5] = global_ns();
+    __syncwarp();
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (tr && threadIdx.x == 0) tr[6] = global_ns();
@@ -513,7 +533,7 @@ qmm_kernel(const __grid_constant__ CUtensorMap xmap, const QmmArgs p) {
         const unsigned long long t0 = global_ns();
         while (global_ns() - t0 < 2000000ull) __nanosleep(1000);
     }
-    if (warp == kMmaWarp) tmem_dealloc(tmem, tmem_cols);
+    if (warp == kMmaWarp) tmem_dealloc(tmem, 512);
     if (threadIdx.x == 0 && s_failed) {
         pdl_wait();
         atomicExch(p.error, 3u);
@@ -525,161 +545,127 @@ using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, voi
                               CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
 EncodeFn encode_fn() {
-    static EncodeFn fn = nullptr;
-    if (!fn) {
+    static EncodeFn fn = [] {
         void* ptr = nullptr;
         cudaDriverEntryPointQueryResult qres;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &qres) != cudaSuccess ||
-            qres != cudaDriverEntryPointSuccess)
-            return nullptr;
-        fn = reinterpret_cast<EncodeFn>(ptr);
-    }
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &qres) != cudaSuccess || qres != cudaDriverEntryPointSuccess)
+            return static_cast<EncodeFn>(nullptr);
+        return reinterpret_cast<EncodeFn>(ptr);
+    }();
     return fn;
 }
 
-template <int K, int CB, bool SMALL>
-cudaError_t qmm_launch_shape(const CUtensorMap& map, const QmmArgs& p, dim3 grid, cudaStream_t stream) {
-    using S = QmmShape<SMALL>;
-    constexpr size_t smem = S::kSmemBytes;
-    auto kernel = qmm_kernel<K, CB, SMALL>;
+// rotated activations [rows, in] fp16 as a 2-D tensor: boxes of 64 inputs x box_rows tokens, 128-byte swizzle
+bool encode_rows(CUtensorMap* map, const __half* xhat, int in, int64_t rows, int box_rows) {
+    EncodeFn encode = encode_fn();
+    const cuuint64_t dims[2] = {static_cast<cuuint64_t>(in), static_cast<cuuint64_t>(rows)};
+    const cuuint64_t strides[1] = {static_cast<cuuint64_t>(in) * sizeof(__half)};
+    const cuuint32_t box[2] = {64, static_cast<cuuint32_t>(box_rows)};
+    const cuuint32_t elem[2] = {1, 1};
+    return encode && encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<__half*>(xhat), dims, strides, box, elem,
+                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+template <int K, int CB, int NT>
+cudaError_t qmm_launch_shape(const CUtensorMap& map, const QmmArgs& p, int grid, cudaStream_t stream) {
+    constexpr size_t smem = qmm_smem_bytes<K, NT>();
+    auto kernel = qmm_kernel<K, CB, NT>;
     static PerDeviceOnce attribute;                         // once per kernel and device
     if (attribute.needed()) {
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
         if (e != cudaSuccess) return e;
         attribute.mark();
     }
-    return launch_dependent(kernel, grid, dim3(S::kThreads), smem, stream, map, p);
-}
-
-template <int K, int CB>
-cudaError_t qmm_launch_one(const CUtensorMap& map, const QmmArgs& p, dim3 grid, bool small, cudaStream_t stream) {
-    return small ? qmm_launch_shape<K, CB, true>(map, p, grid, stream) : qmm_launch_shape<K, CB, false>(map, p, grid, stream);
+    return launch_dependent(kernel, dim3(static_cast<unsigned>(grid)), dim3(QmmShape<NT>::kThreads), smem, stream, map, p);
 }
 
 template <int K>
-cudaError_t qmm_launch_k(int cb, const CUtensorMap& map, const QmmArgs& p, dim3 grid, bool small, cudaStream_t stream) {
-    if (cb == 0) return qmm_launch_one<K, 0>(map, p, grid, small, stream);
-    if (cb == 1) return qmm_launch_one<K, 1>(map, p, grid, small, stream);
-    return qmm_launch_one<K, 2>(map, p, grid, small, stream);
+cudaError_t qmm_launch_k(int cb, const CUtensorMap& map, const QmmArgs& p, int grid, bool small, cudaStream_t stream) {
+    if (cb == 0) return small ? qmm_launch_shape<K, 0, 64>(map, p, grid, stream) : qmm_launch_shape<K, 0, 256>(map, p, grid, stream);
+    if (cb == 1) return small ? qmm_launch_shape<K, 1, 64>(map, p, grid, stream) : qmm_launch_shape<K, 1, 256>(map, p, grid, stream);
+    return small ? qmm_launch_shape<K, 2, 64>(map, p, grid, stream) : qmm_launch_shape<K, 2, 256>(map, p, grid, stream);
+}
+
+cudaError_t qmm_dispatch(int k, int cb, const CUtensorMap& map, const QmmArgs& p, int grid, bool small, cudaStream_t stream) {
+    switch (k) {
+        case 1: return qmm_launch_k<1>(cb, map, p, grid, small, stream);
+        case 2: return qmm_launch_k<2>(cb, map, p, grid, small, stream);
+        case 3: return qmm_launch_k<3>(cb, map, p, grid, small, stream);
+        case 4: return qmm_launch_k<4>(cb, map, p, grid, small, stream);
+        case 5: return qmm_launch_k<5>(cb, map, p, grid, small, stream);
+        case 6: return qmm_launch_k<6>(cb, map, p, grid, small, stream);
+        case 7: return qmm_launch_k<7>(cb, map, p, grid, small, stream);
+        case 8: return qmm_launch_k<8>(cb, map, p, grid, small, stream);
+        default: return cudaErrorInvalidValue;
+    }
 }
 
 }  // namespace
 
 std::atomic<unsigned long long*> g_qmm_trace{nullptr};
-static std::atomic<int> g_qmm_splits{0};                              // 0 = chosen by the cost model below
+static std::atomic<int> g_qmm_splits{0};                              // 0 = one wave of CTAs with equal runs of stages
 void qmm_set_tuning(int splits) { g_qmm_splits = splits > 0 ? splits : 0; }
 
 constexpr int64_t kQmmSmallMaxRows = 64;     // one token tile: a second one would decode every weight twice
 
-QmmPlan plan_qmm(int in, int out, int64_t rows) {
+// CTAs of a launch over `items` items: one wave of equal runs, at least one stage each (below that a CTA would only add a
+// piece to be summed), or as many per item as asked for.
+static int64_t qmm_grid(const QmmPlan& plan, int64_t items, int64_t stages) {
+    return plan.fixed ? items * plan.splits : std::max<int64_t>(1, std::min<int64_t>(sm_count(), items * stages));
+}
+
+static size_t qmm_piece_count(int64_t items, int64_t grid) { return static_cast<size_t>(items < grid ? grid + items : 2 * grid); }
+
+QmmPlan plan_qmm(int in, int out, int64_t rows, bool whole_items) {
     QmmPlan plan{};
     plan.small = rows <= kQmmSmallMaxRows;
-    const int col_blocks = out / 128;
-    const int tile = plan.small ? QmmShape<true>::kTokTile : QmmShape<false>::kTokTile;
-    plan.token_tiles = static_cast<int>((rows + tile - 1) / tile);
-    const int stages_total = in / 64;
-    const int64_t base = static_cast<int64_t>(col_blocks) * plan.token_tiles;
-    const int max_splits = std::max(1, stages_total / 8);     // every split keeps at least 8 stages
-    if (const int forced = g_qmm_splits.load()) { plan.splits = std::min(forced, max_splits); return plan; }
-    // CTAs that run at once: one per SM for the large shape (the operand rings take most of the shared memory),
-    // two for the small one.  Estimated time of a choice: waves x (stages per CTA + fixed prologue/epilogue) + the
-    // fp32 partials that several splits write and the separate output rotation reads back.
-    const int64_t slots = static_cast<int64_t>(sm_count()) * (plan.small ? 2 : 1);
-    const double stage_us = plan.small ? 0.55 : (rows > 256 ? 0.6 : 0.35), fixed_us = 4.0;
-    const double partial_us = static_cast<double>(rows) * out * 8.0 / 8.0e6;
-    double best = 0;
-    for (int s = 1; s <= max_splits; ++s) {
-        const int64_t waves = (base * s + slots - 1) / slots;
-        // with one split the output rotation runs in the epilogue; more splits write fp32 partials and add a launch
-        const double t = waves * (((stages_total + s - 1) / s) * stage_us + fixed_us) + (s > 1 ? s * partial_us + 5.0 : 0.0);
-        if (s == 1 || t < best) { best = t; plan.splits = s; }
-    }
+    plan.token_tiles = static_cast<int>(plan.small ? 1 : (rows + 511) / 512);
+    const int nt = plan.small ? 64 : 256;
+    const int col_blocks = out / 128, stages = in / kStageIn;
+    // the items of one launch need an arrival counter each, and stages x CTAs must fit 32 bits: more rows go in passes
+    const int64_t max_items = std::min<int64_t>(4000, (int64_t{1} << 31) / (static_cast<int64_t>(stages) * 1024));
+    const int64_t max_tiles = std::max<int64_t>(1, max_items / col_blocks);
+    const int64_t tiles = (rows + nt - 1) / nt;
+    const int64_t passes = (tiles + max_tiles - 1) / max_tiles;
+    plan.pass_rows = passes == 1 ? rows : max_tiles * nt;
+    const int64_t pass_tiles = std::min(tiles, max_tiles);
+    // equal tiles of whole sixteens: N of the MMA is a multiple of 16
+    plan.tile_tokens = static_cast<int>(((std::min(rows, plan.pass_rows) + pass_tiles - 1) / pass_tiles + 15) / 16 * 16);
+    const int64_t items = pass_tiles * col_blocks;
+    const int forced = g_qmm_splits.load();
+    plan.fixed = whole_items || forced > 0;
+    plan.splits = whole_items || !forced ? 1 : std::max(1, std::min(forced, stages / 4));
+    plan.piece_bytes = plan.fixed && plan.splits == 1 ? 256 : qmm_piece_count(items, qmm_grid(plan, items, stages)) * plan.tile_tokens * 128 * sizeof(float);
     return plan;
 }
 
-size_t qmm_partial_bytes(const QmmPlan& plan, int out, int64_t rows) {
-    return (static_cast<size_t>(plan.splits) * rows * out * sizeof(float) + 255) / 256 * 256;
+cudaError_t launch_qmm(QmmArgs p, const __half* xhat, int k, int cb, const QmmPlan& plan, cudaStream_t stream) {
+    if (p.in % 128 || p.out % 128 || p.rows <= 0 || p.rows > plan.pass_rows || p.groups < 1) return cudaErrorInvalidValue;
+    CUtensorMap map;
+    if (!encode_rows(&map, xhat, p.in, static_cast<int64_t>(p.groups) * p.rows, plan.tile_tokens)) return cudaErrorInvalidValue;
+    p.tile_tokens = p.box_rows = plan.tile_tokens;
+    p.tiles = (p.rows + plan.tile_tokens - 1) / plan.tile_tokens;
+    p.items = p.tiles * (p.out / 128);
+    p.trace = g_qmm_trace.load();
+    const int64_t stages = p.in / kStageIn, grid = qmm_grid(plan, p.items, stages);
+    if (p.items * stages * grid >= (int64_t{1} << 32)) return cudaErrorInvalidValue;
+    return qmm_dispatch(k, cb, map, p, static_cast<int>(grid), plan.small, stream);
 }
 
-cudaError_t launch_qmm(const uint32_t* wq, int in, int out, int k, int cb, const __half* xhat, int64_t rows,
-                       const QmmPlan& plan, float* partials, unsigned int* error, const __half* svh, const __half* bias,
-                       void* y, int y_dtype, cudaStream_t stream, int ld_tiles, int col_tile0) {
-    if (in % 128 || out % 128 || rows <= 0 || col_tile0 % 8) return cudaErrorInvalidValue;
-    if (ld_tiles <= 0) ld_tiles = out / 16;
-    // a member of a group: its column blocks follow those of the members before it
-    (void)ld_tiles;
-    wq += quad_row_offset(0, col_tile0 / 8, in / 16, k);
-    if (y != nullptr && plan.splits != 1) return cudaErrorInvalidValue;     // the fused rotation needs the complete sum
-    EncodeFn encode = encode_fn();
-    if (!encode) return cudaErrorNotSupported;
-    // rotated activations [rows, in] fp16 as a 2-D tensor: boxes of 64 inputs x 256 tokens, 128-byte swizzle
-    CUtensorMap map;
-    const cuuint64_t dims[2] = {static_cast<cuuint64_t>(in), static_cast<cuuint64_t>(rows)};
-    const cuuint64_t strides[1] = {static_cast<cuuint64_t>(in) * sizeof(__half)};
-    const cuuint32_t box[2] = {64, static_cast<cuuint32_t>(plan.small ? QmmShape<true>::kTokHalf : QmmShape<false>::kTokHalf)};
-    const cuuint32_t elem[2] = {1, 1};
-    if (encode(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<__half*>(xhat), dims, strides, box, elem,
-               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-        return cudaErrorInvalidValue;
-    // packed weights: the four tile rows of a stage are contiguous in the quad layout, so the weight producer issues plain
-    // bulk copies and needs no tensor map
-    QmmArgs p{};
-    p.wq = wq; p.partials = partials; p.error = error;
-    p.svh = svh; p.bias = bias; p.y = y; p.y_dtype = y_dtype;
-    p.in = in; p.out = out; p.rows = static_cast<int>(rows); p.tiles_n = out / 16;
-    p.splits = plan.splits; p.stages_total = in / 64; p.trace = g_qmm_trace.load();
-    const dim3 grid(static_cast<unsigned>((out / 128) * plan.splits), static_cast<unsigned>(plan.token_tiles));
-    switch (k) {
-        case 1: return qmm_launch_k<1>(cb, map, p, grid, plan.small, stream);
-        case 2: return qmm_launch_k<2>(cb, map, p, grid, plan.small, stream);
-        case 3: return qmm_launch_k<3>(cb, map, p, grid, plan.small, stream);
-        case 4: return qmm_launch_k<4>(cb, map, p, grid, plan.small, stream);
-        case 5: return qmm_launch_k<5>(cb, map, p, grid, plan.small, stream);
-        case 6: return qmm_launch_k<6>(cb, map, p, grid, plan.small, stream);
-        case 7: return qmm_launch_k<7>(cb, map, p, grid, plan.small, stream);
-        case 8: return qmm_launch_k<8>(cb, map, p, grid, plan.small, stream);
-        default: return cudaErrorInvalidValue;
-    }
-}
+size_t qmm_mapped_piece_bytes() { return static_cast<size_t>(sm_count()) * 2 * kQmmSegRows * 128 * sizeof(float); }
 
-
-cudaError_t launch_qmm_mapped(const uint32_t* wq, int in, int width, int bank_tiles_n, int k, int cb, const __half* xhat,
-                              int max_segments, int proj, int stride_blocks, int experts, const uint32_t* seg_expert,
-                              const int* seg_count, float* products, unsigned int* error, cudaStream_t stream) {
-    using S = QmmShape<true>;
-    if (in % 128 || width % 128 || max_segments <= 0 || proj <= 0) return cudaErrorInvalidValue;
-    EncodeFn encode = encode_fn();
-    if (!encode) return cudaErrorNotSupported;
-    const int64_t rows = static_cast<int64_t>(max_segments) * proj * S::kTokTile;   // padded activation rows
-    const int out = max_segments * proj * width;                                   // virtual output width
+cudaError_t launch_qmm_mapped(QmmArgs p, const __half* xhat, int max_segments, int k, int cb, cudaStream_t stream) {
+    if (p.in % 128 || p.map_blocks <= 0 || max_segments <= 0 || p.map_proj <= 0 || p.yhat == nullptr) return cudaErrorInvalidValue;
+    const int64_t stages = static_cast<int64_t>(max_segments) * p.map_proj * p.map_blocks * (p.in / kStageIn);
+    if (stages * sm_count() >= (int64_t{1} << 32)) return cudaErrorInvalidValue;
     CUtensorMap map;
-    const cuuint32_t elem[2] = {1, 1};
-    const cuuint64_t dims[2] = {static_cast<cuuint64_t>(in), static_cast<cuuint64_t>(rows)};
-    const cuuint64_t strides[1] = {static_cast<cuuint64_t>(in) * sizeof(__half)};
-    const cuuint32_t box[2] = {64, static_cast<cuuint32_t>(S::kTokHalf)};
-    if (encode(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<__half*>(xhat), dims, strides, box, elem,
-               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-        return cudaErrorInvalidValue;
-    QmmArgs p{};
-    p.wq = wq; p.partials = products; p.error = error;
-    p.in = in; p.out = out; p.rows = S::kTokTile; p.tiles_n = bank_tiles_n;
-    p.splits = 1; p.stages_total = in / 64; p.trace = nullptr;
-    p.map_expert = seg_expert; p.map_count = seg_count;
-    p.map_blocks = width / 128; p.map_proj = proj; p.map_stride_blocks = stride_blocks; p.map_experts = experts;
-    const dim3 grid(static_cast<unsigned>(out / 128), 1);
-    switch (k) {
-        case 1: return qmm_launch_k<1>(cb, map, p, grid, true, stream);
-        case 2: return qmm_launch_k<2>(cb, map, p, grid, true, stream);
-        case 3: return qmm_launch_k<3>(cb, map, p, grid, true, stream);
-        case 4: return qmm_launch_k<4>(cb, map, p, grid, true, stream);
-        case 5: return qmm_launch_k<5>(cb, map, p, grid, true, stream);
-        case 6: return qmm_launch_k<6>(cb, map, p, grid, true, stream);
-        case 7: return qmm_launch_k<7>(cb, map, p, grid, true, stream);
-        case 8: return qmm_launch_k<8>(cb, map, p, grid, true, stream);
-        default: return cudaErrorInvalidValue;
-    }
+    constexpr int box = 16;                                   // segments are short: only the boxes that hold rows are fetched
+    if (!encode_rows(&map, xhat, p.in, static_cast<int64_t>(max_segments) * p.map_proj * kQmmSegRows, box)) return cudaErrorInvalidValue;
+    p.groups = 1; p.gcol0[0] = 0;
+    p.tile_tokens = kQmmSegRows; p.box_rows = box;
+    p.trace = nullptr;
+    return qmm_dispatch(k, cb, map, p, sm_count(), true, stream);
 }
 
 }  // namespace b200exl3

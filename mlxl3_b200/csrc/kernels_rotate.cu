@@ -8,7 +8,7 @@ namespace b200exl3 {
 
 __global__ void __launch_bounds__(256)
 prepare_kernel(const void* __restrict__ x, int x_dtype, const __half* __restrict__ suh, int64_t scale_rows,
-               int64_t rows, int in, __half* __restrict__ xhat, const __half* __restrict__ glu_up) {
+               int64_t rows, int in, __half* __restrict__ xhat, const __half* __restrict__ glu_up, int groups) {
     pdl_launch_dependents();                    // the kernel after this one may start; it waits for our memory itself
     pdl_wait();                                 // what the kernel before this one wrote is visible from here on
     const int lane = threadIdx.x & 31;
@@ -18,8 +18,7 @@ prepare_kernel(const void* __restrict__ x, int x_dtype, const __half* __restrict
          unit += static_cast<int64_t>(gridDim.x) * (blockDim.x >> 5)) {
         const int64_t row = unit / blocks_per_row;
         const int col = static_cast<int>(unit % blocks_per_row) * 128 + lane * 4;
-        const __half* s = suh + (scale_rows == 1 ? 0 : row * in) + col;
-        __align__(8) __half h[4];
+        __half v[4];
         if (glu_up != nullptr) {
             // SwiGLU of two fp16 row sets as the input (x = gate rows): half(gate * sigmoid(gate)) * up, each product
             // rounded to half, the arithmetic of the stand-alone SwiGLU kernel and of the small-batch prologue
@@ -31,16 +30,24 @@ prepare_kernel(const void* __restrict__ x, int x_dtype, const __half* __restrict
             for (int j = 0; j < 2; ++j) {
                 const float2 f = __half22float2(gh[j]);
                 const __half2 sg = __floats2half2_rn(1.0f / (1.0f + expf(-f.x)), 1.0f / (1.0f + expf(-f.y)));
-                const __half2 v = __hmul2_rn(__hmul2_rn(gh[j], sg), uh[j]);
-                h[2 * j] = __hmul_rn(__low2half(v), s[2 * j]);
-                h[2 * j + 1] = __hmul_rn(__high2half(v), s[2 * j + 1]);
+                const __half2 a = __hmul2_rn(__hmul2_rn(gh[j], sg), uh[j]);
+                v[2 * j] = __low2half(a);
+                v[2 * j + 1] = __high2half(a);
             }
         } else {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) h[j] = __hmul_rn(load_as_half(x, x_dtype, row * in + col + j), s[j]);
+            load4_as_half(x, x_dtype, row * in + col, v);
         }
-        warp_hadamard128_f16(h, lane);
-        *reinterpret_cast<uint2*>(xhat + row * in + col) = *reinterpret_cast<uint2*>(h);
+        // a group's members read the same row, each with its own input scales
+        const __half* s = suh + (scale_rows == 1 ? 0 : row * in) + col;
+        __half* dst = xhat + row * in + col;
+        for (int g = 0; g < groups; ++g, s += in, dst += rows * in) {
+            const uint2 sw = *reinterpret_cast<const uint2*>(s);
+            __align__(8) __half h[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) h[j] = __hmul_rn(v[j], reinterpret_cast<const __half*>(&sw)[j]);
+            warp_hadamard128_f16(h, lane);
+            *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<uint2*>(h);
+        }
     }
 }
 
@@ -73,9 +80,10 @@ finish_kernel(const float* __restrict__ partials, int splits, int64_t split_stri
         }
         __half h[4] = {__float2half_rn(acc.x), __float2half_rn(acc.y), __float2half_rn(acc.z), __float2half_rn(acc.w)};
         warp_hadamard128_f16(h, lane);
-        const __half* s = svh + (scale_rows == 1 ? 0 : row * out) + col;
+        const uint2 sw = *reinterpret_cast<const uint2*>(svh + (scale_rows == 1 ? 0 : row * out) + col);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) store_from_half(y, y_dtype, row * out + col + j, __hmul_rn(h[j], s[j]), bias, col + j);
+        for (int j = 0; j < 4; ++j) h[j] = __hmul_rn(h[j], reinterpret_cast<const __half*>(&sw)[j]);
+        store4_from_half(y, y_dtype, row * out + col, h, bias ? bias + col : nullptr);
     }
 }
 
@@ -86,11 +94,12 @@ static unsigned grid_for(int64_t units) {
 }
 
 cudaError_t launch_prepare(const void* x, int x_dtype, const __half* suh, int64_t scale_rows, int64_t rows, int in,
-                           __half* xhat, cudaStream_t stream, const __half* glu_up) {
+                           __half* xhat, cudaStream_t stream, const __half* glu_up, int groups) {
     if (rows == 0) return cudaSuccess;
+    if (groups > 1 && scale_rows != 1) return cudaErrorInvalidValue;
     if (glu_up != nullptr && x_dtype != kF16) return cudaErrorInvalidValue;
     return launch_dependent(prepare_kernel, dim3(grid_for(rows * (in / 128))), dim3(256), 0, stream, x, x_dtype, suh, scale_rows, rows, in, xhat,
-                            glu_up);
+                            glu_up, groups);
 }
 
 cudaError_t launch_finish(const float* partials, int splits, int64_t split_stride, const __half* svh,
