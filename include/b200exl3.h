@@ -87,6 +87,13 @@ int b200exl3_plan_query(const char* kind, int in, int out, int k, int64_t rows, 
  * native/ffi/mlx_bridge.cpp:337, 610, 233, 192).  Streams are created non-blocking. */
 int b200exl3_malloc(size_t bytes, void** out_device_ptr);
 int b200exl3_free(void* device_ptr);
+/* Device memory for calls that take host buffers: blocks are kept by the library, per device, up to 64 MiB, and what is
+ * released beyond that is freed (so is everything kept, when an allocation of b200exl3_malloc fails).  A block may be handed
+ * to any thread and stream as soon as it is released: release it only once the work that used it has completed.  Blocks of
+ * up to 1 MiB come with as much page-locked host memory (NULL otherwise), so that a copy through it needs no staging by the
+ * driver. */
+int b200exl3_scratch_acquire(size_t bytes, void** out_device_ptr, void** out_host_ptr);
+int b200exl3_scratch_release(void* device_ptr);
 int b200exl3_host_alloc(size_t bytes, void** out_pinned_ptr);
 int b200exl3_host_free(void* pinned_ptr);
 int b200exl3_memcpy_h2d(void* dst_device, const void* src_host, size_t bytes, b200exl3_stream stream);

@@ -28,6 +28,8 @@ SIGNATURES = {
     "b200exl3_plan_query": (c_int, [c_char_p, c_int, c_int, c_int, c_int64, POINTER(c_int64), c_int]),
     "b200exl3_malloc": (c_int, [c_size_t, POINTER(c_void_p)]),
     "b200exl3_free": (c_int, [c_void_p]),
+    "b200exl3_scratch_acquire": (c_int, [c_size_t, POINTER(c_void_p), POINTER(c_void_p)]),
+    "b200exl3_scratch_release": (c_int, [c_void_p]),
     "b200exl3_host_alloc": (c_int, [c_size_t, POINTER(c_void_p)]),
     "b200exl3_host_free": (c_int, [c_void_p]),
     "b200exl3_memcpy_h2d": (c_int, [c_void_p, c_void_p, c_size_t, c_void_p]),
@@ -143,5 +145,12 @@ def check(status: int) -> None:
         raise B200Exl3Error(load().b200exl3_last_error().decode("utf-8", "replace"))
 
 
+_bound: dict[str, object] = {}      # entry points that were called before
+
+
 def call(name: str, *args) -> None:
-    check(getattr(load(), name)(*args))
+    fn = _bound.get(name)
+    if fn is None:
+        fn = _bound[name] = getattr(load(), name)
+    if fn(*args) != 0:
+        check(-1)

@@ -64,6 +64,29 @@ std::atomic<bool> g_qmm_enabled{true};                   // "qmm" option: 0 send
 std::atomic<long long> g_tp_wait_ms{4000};
 std::atomic<long long> g_stack_wait_ms{2000};            // "stack_wait_ms" option: bound of a layer-boundary wait inside a step
 std::atomic<unsigned long long*> g_stack_trace{nullptr}; // "stack_trace_buffer" option               // "tp_wait_ms" option: how long a rank polls for its peers' sums
+// Device blocks of calls that take host buffers (b200exl3_scratch_*).
+struct ScratchBlock { void* ptr; void* host; size_t bytes; int device; };
+constexpr size_t kScratchKeptBytes = size_t(64) << 20;
+// above this a copy through page-locked memory is no faster than the driver's own staging
+constexpr size_t kScratchHostBytes = size_t(1) << 20;
+std::mutex g_scratch_mutex;
+std::vector<ScratchBlock> g_scratch_free, g_scratch_used;
+
+// gives the current device's kept blocks back; the bytes freed
+size_t scratch_trim() {
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess) return 0;
+    std::lock_guard<std::mutex> lock(g_scratch_mutex);
+    size_t freed = 0;
+    for (size_t i = g_scratch_free.size(); i-- > 0;)
+        if (g_scratch_free[i].device == device) {
+            cudaFree(g_scratch_free[i].ptr);
+            cudaFreeHost(g_scratch_free[i].host);
+            freed += g_scratch_free[i].bytes;
+            g_scratch_free.erase(g_scratch_free.begin() + static_cast<long>(i));
+        }
+    return freed;
+}
 constexpr int kMaxBatchRows = kQmvMaxRows;              // rows handled by one launch of the fused kernel
 constexpr size_t kCounterBytes = B200EXL3_WORKSPACE_HEADER_BYTES;   // arrival counters at the head of a workspace
 
@@ -197,7 +220,63 @@ int b200exl3_malloc(size_t bytes, void** out) {
     if (!out) return fail("out pointer is NULL");
     *out = nullptr;
     if (bytes == 0) return 0;
-    return check(cudaMalloc(out, bytes), "cudaMalloc");
+    cudaError_t e = cudaMalloc(out, bytes);
+    if (e == cudaErrorMemoryAllocation && scratch_trim() > 0) {
+        (void)cudaGetLastError();
+        e = cudaMalloc(out, bytes);
+    }
+    return check(e, "cudaMalloc");
+}
+int b200exl3_scratch_acquire(size_t bytes, void** out, void** out_host) {
+    if (!out || !out_host) return fail("out pointer is NULL");
+    *out = *out_host = nullptr;
+    if (bytes == 0) return fail("scratch of no bytes");
+    ScratchBlock block{};
+    B200_TRY(cudaGetDevice(&block.device), "cudaGetDevice");
+    block.bytes = size_t(4) << 10;                            // powers of two: few sizes, so a block is found again
+    while (block.bytes < bytes) block.bytes *= 2;
+    std::unique_lock<std::mutex> lock(g_scratch_mutex);
+    for (size_t i = g_scratch_free.size(); i-- > 0 && !block.ptr;)
+        if (g_scratch_free[i].device == block.device && g_scratch_free[i].bytes == block.bytes) {
+            block = g_scratch_free[i];
+            g_scratch_free.erase(g_scratch_free.begin() + static_cast<long>(i));
+        }
+    if (!block.ptr) {
+        lock.unlock();
+        if (b200exl3_malloc(block.bytes, &block.ptr)) return -1;
+        if (block.bytes <= kScratchHostBytes && check(cudaMallocHost(&block.host, block.bytes), "cudaMallocHost")) {
+            cudaFree(block.ptr);
+            return -1;
+        }
+        lock.lock();
+    }
+    g_scratch_used.push_back(block);
+    *out = block.ptr;
+    *out_host = block.host;
+    return 0;
+}
+int b200exl3_scratch_release(void* p) {
+    if (!p) return 0;
+    ScratchBlock block{};
+    {
+        std::lock_guard<std::mutex> lock(g_scratch_mutex);
+        for (size_t i = 0; i < g_scratch_used.size(); ++i)
+            if (g_scratch_used[i].ptr == p) {
+                block = g_scratch_used[i];
+                g_scratch_used.erase(g_scratch_used.begin() + static_cast<long>(i));
+                break;
+            }
+        if (!block.ptr) return fail("not a scratch block");
+        size_t kept = block.bytes;
+        for (const ScratchBlock& b : g_scratch_free)
+            if (b.device == block.device) kept += b.bytes;
+        if (kept <= kScratchKeptBytes) {
+            g_scratch_free.push_back(block);
+            return 0;
+        }
+    }
+    cudaFreeHost(block.host);
+    return check(cudaFree(block.ptr), "cudaFree");
 }
 int b200exl3_free(void* p) { return p ? check(cudaFree(p), "cudaFree") : 0; }
 int b200exl3_host_alloc(size_t bytes, void** out) {

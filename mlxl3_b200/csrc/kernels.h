@@ -57,7 +57,8 @@ constexpr int kQmvRedStride = 132;   // floats per reduced row: 128 + 4 keeps th
 constexpr int kQmvMaxGroups = 8;     // projections fused in one launch (q/k/v, gate/up)
 constexpr int kQmvMaxRows = 16;      // activation rows one launch can take
 constexpr int kQmvMaxSmemBytes = 200 * 1024;
-constexpr int kQmvXBlocks = 6;       // 128-blocks of rotated activations a warp keeps per row
+constexpr size_t kQmvSharedSmemBytes = 112 * 1024;   // dynamic shared memory of a CTA that leaves room for another one (228 KB per SM)
+constexpr int kQmvXBlocks = 6;       // 128-blocks of rotated activations a warp keeps per row when it rotates them itself
 constexpr int kQmvFusedRows = 2;     // up to this many rows the kernel rotates the activations itself
 
 // The weight stream of a warp: chunks of consecutive rows of a column block (a row is 8 tiles; one bulk copy per chunk),
@@ -86,7 +87,9 @@ struct QmvArgs {
     int in, out, rows, tiles_k, tiles_n, max_pieces;
     int warp_smem;             // bytes of shared memory per warp
     int xs_offset;             // offset of the rotated activations inside a warp's shared memory
-    int stage_offset;          // offset of the staged result tiles inside a warp's shared memory
+    int stage_offset, stage2_offset;   // offsets of the staged result tiles of a warp's first and second block inside its shared memory
+    int tile_stride;           // floats between the rows of a staged tile
+    int x_blocks, xs_stride;   // 128-blocks of rotated activations a warp keeps per row; halves between its rows
     int pdl_early;             // 1: let the next kernel start as soon as this one has started its copies
     // Expert-mapped mode (map_selected != nullptr; rows == 1, raw output): the `out` axis is virtual,
     // [slots, map_proj, map_blocks * 128]; slot s reads the columns of expert map_selected[s] in the bank
@@ -140,7 +143,8 @@ struct QmvPlan {
     int col_blocks;      // out / 128
     int warp_smem;       // bytes of shared memory per warp
     int xs_offset;       // offset of the rotated activations inside a warp's shared memory
-    int stage_offset;    // offset of the staged result tiles inside a warp's shared memory
+    int stage_offset, stage2_offset;   // offsets of the staged result tiles of a warp's first and second block
+    int tile_stride, x_blocks, xs_stride;
     bool fused_rotation; // the kernel rotates the activations itself (rows <= kQmvFusedRows)
     size_t smem_bytes;   // dynamic shared memory per CTA
     bool pdl;            // launch with programmatic stream serialization (overlap with the previous kernel's tail)

@@ -24,6 +24,8 @@ __device__ __forceinline__ int expert_of(const uint32_t* selected, int64_t slot,
 
 __device__ __forceinline__ float silu(float v) { return glu_silu(v); }
 
+// SORTED: slots lie where the route plan put them (slot_row)
+template <bool SORTED>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 glu_down_input_kernel(const float* __restrict__ ygu, const __half* __restrict__ gu_svh, const __half* __restrict__ down_suh,
                       const uint32_t* __restrict__ selected, int experts, int64_t slots, int hidden, int logical_hidden,
@@ -41,7 +43,7 @@ glu_down_input_kernel(const float* __restrict__ ygu, const __half* __restrict__ 
         const int col = static_cast<int>(unit % blocks_per_row) * 128 + lane * 4;
         const int64_t expert = expert_of(selected, slot, experts);
         int64_t grow = slot * 2, up = 1, xrow = slot;           // gate row, distance to the up row, row of the result
-        if (slot_row != nullptr) {
+        if (SORTED) {
             xrow = slot_row[slot];
             grow = (xrow / kQmmSegRows) * 2 * kQmmSegRows + xrow % kQmmSegRows;
             up = kQmmSegRows;
@@ -72,7 +74,7 @@ glu_down_input_kernel(const float* __restrict__ ygu, const __half* __restrict__ 
     }
 }
 
-template <bool F32>
+template <bool F32, bool SORTED>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 finish_and_reduce_kernel(const float* __restrict__ raw, const __half* __restrict__ down_svh,
                          const uint32_t* __restrict__ selected, int experts, const void* __restrict__ scores,
@@ -99,7 +101,7 @@ finish_and_reduce_kernel(const float* __restrict__ raw, const __half* __restrict
             for (int i = 0; i < 4; ++i) {
                 if (t0 + i >= top_k) continue;
                 const int64_t slot = row * top_k + t0 + i;
-                r[i] = *reinterpret_cast<const float4*>(raw + (slot_row ? static_cast<int64_t>(slot_row[slot]) : slot) * out + col);
+                r[i] = *reinterpret_cast<const float4*>(raw + (SORTED ? static_cast<int64_t>(slot_row[slot]) : slot) * out + col);
                 svw[i] = *reinterpret_cast<const uint2*>(down_svh + static_cast<int64_t>(expert_of(selected, slot, experts)) * out + col);
                 if (F32) score32[i] = reinterpret_cast<const float*>(scores)[slot];
                 else score16[i] = reinterpret_cast<const __half*>(scores)[slot];
@@ -141,7 +143,7 @@ cudaError_t launch_glu_down_input(const float* ygu, const __half* gu_svh, const 
                                   int experts, int64_t slots, int hidden, int logical_hidden, __half* xhat,
                                   cudaStream_t stream, const int* count, const uint32_t* slot_row) {
     if (slots == 0) return cudaSuccess;
-    return launch_dependent(glu_down_input_kernel, dim3(grid_for(slots * (hidden / 128))), dim3(kWarpsPerBlock * 32), 0, stream, ygu, gu_svh,
+    return launch_dependent(slot_row ? glu_down_input_kernel<true> : glu_down_input_kernel<false>, dim3(grid_for(slots * (hidden / 128))), dim3(kWarpsPerBlock * 32), 0, stream, ygu, gu_svh,
                             down_suh, selected, experts, slots, hidden, logical_hidden, xhat, count, slot_row);
 }
 
@@ -150,7 +152,9 @@ cudaError_t launch_finish_and_reduce(const float* raw, const __half* down_svh, c
                                      cudaStream_t stream, const uint32_t* slot_row) {
     if (rows == 0) return cudaSuccess;
     const unsigned grid = grid_for(rows * (out / 128));
-    return launch_dependent(score_dtype == kF32 ? finish_and_reduce_kernel<true> : finish_and_reduce_kernel<false>, dim3(grid),
+    const auto kernel = slot_row ? (score_dtype == kF32 ? finish_and_reduce_kernel<true, true> : finish_and_reduce_kernel<false, true>)
+                                 : (score_dtype == kF32 ? finish_and_reduce_kernel<true, false> : finish_and_reduce_kernel<false, false>);
+    return launch_dependent(kernel, dim3(grid),
                             dim3(kWarpsPerBlock * 32), 0, stream, raw, down_svh, selected, experts, scores, rows, top_k, out, y, slot_row);
 }
 

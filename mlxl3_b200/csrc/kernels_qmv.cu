@@ -57,29 +57,48 @@ QmvPlan plan_qmv(int in, int out, int k, int64_t rows) {
     QmvPlan plan{};
     plan.col_blocks = out / 128;
     const int tiles_k = in / 16;
-    const int64_t total = static_cast<int64_t>(tiles_k) * 8 * plan.col_blocks;
     const int r = static_cast<int>(std::min<int64_t>(rows, kQmvMaxRows));
-    // two 8-row blocks need about twice the registers and shared memory: one CTA per SM
-    const int resident = r <= 8 ? g_ctas_per_sm.load() : 1;
     const int forced = g_force_grid.load();
-    int64_t grid = forced > 0 ? forced : static_cast<int64_t>(sm_count()) * resident;
-    // the layer is dealt out in whole rows of 8 tiles: no more warps than rows
     const int64_t rb = tiles_k, rt = rb * plan.col_blocks;
-    grid = std::max<int64_t>(1, std::min(grid, rt / kQmvWarps));
-    // a warp's range must not exceed one column block (it then touches at most two blocks)
-    const int64_t min_warps = (rt + rb - 2) / (rb - 1) + 1;
-    grid = std::max(grid, (min_warps + kQmvWarps - 1) / kQmvWarps);
-    plan.grid = static_cast<int>(grid);
-    plan.max_pieces = static_cast<int>((grid + plan.col_blocks - 1) / plan.col_blocks + 1);
+    // CTAs for `resident` of them per SM
+    auto grid_for = [&](int resident) {
+        int64_t grid = forced > 0 ? forced : static_cast<int64_t>(sm_count()) * resident;
+        // the layer is dealt out in whole rows of 8 tiles: no more warps than rows
+        grid = std::max<int64_t>(1, std::min(grid, rt / kQmvWarps));
+        // a warp's range must not exceed one column block (it then touches at most two blocks)
+        const int64_t min_warps = (rt + rb - 2) / (rb - 1) + 1;
+        return static_cast<int>(std::max(grid, (min_warps + kQmvWarps - 1) / kQmvWarps));
+    };
+    // Per warp: [ring of packed rows | rotated activations | staged result tile of its first block | of its second].  The
+    // second tile is staged when the activations are no longer read, so with rows that come rotated it shares their place.
+    auto layout = [&](int x_blocks, int tile_stride) {
+        const int ring = qmv_chunk_rows(k) * qmv_slots(k) * 64 * k * static_cast<int>(sizeof(uint32_t));
+        const int tile = r * tile_stride * static_cast<int>(sizeof(float));
+        plan.tile_stride = tile_stride;
+        plan.x_blocks = x_blocks;
+        // rows eight words apart modulo 32 banks: the eight rows of a fragment load hit different banks
+        plan.xs_stride = x_blocks * 128 + (plan.fused_rotation ? 0 : 8);
+        const int xs = r * plan.xs_stride * static_cast<int>(sizeof(__half));
+        plan.xs_offset = ring;
+        plan.stage_offset = (ring + (plan.fused_rotation ? xs : std::max(xs, tile)) + 15) / 16 * 16;
+        plan.stage2_offset = plan.fused_rotation ? plan.stage_offset + tile : plan.xs_offset;
+        plan.warp_smem = (plan.stage_offset + (plan.fused_rotation ? 2 : 1) * tile + 15) / 16 * 16;
+        plan.smem_bytes = static_cast<size_t>(plan.warp_smem) * kQmvWarps;
+    };
     plan.fused_rotation = r <= kQmvFusedRows;
-    // per warp: [ring of packed rows | rotated activations | two staged result tiles]
-    const size_t ring = static_cast<size_t>(qmv_chunk_rows(k)) * qmv_slots(k) * 64 * k * sizeof(uint32_t);
-    const size_t xs = plan.fused_rotation ? static_cast<size_t>(r) * kQmvXBlocks * 128 * sizeof(__half) : 0;
-    const size_t stage = 2 * static_cast<size_t>(r) * kQmvRedStride * sizeof(float);   // first and second block of a warp
-    plan.xs_offset = static_cast<int>(ring);
-    plan.stage_offset = static_cast<int>(ring + xs);
-    plan.warp_smem = static_cast<int>((ring + xs + stage + 15) / 16 * 16);
-    plan.smem_bytes = static_cast<size_t>(plan.warp_smem) * kQmvWarps;
+    // Two 8-row blocks need about twice the registers: one CTA per SM.  Up to 8 rows two CTAs share an SM where their shared
+    // memory allows it (all widths up to 6 bits), because twice the warps decode; where it does not, the grid is one wave of
+    // single CTAs (4096 -> 4096, 4 bits, 8 rows: 116 KB per CTA ran a grid for two per SM in two waves, 51 us).
+    int resident = r <= 8 ? g_ctas_per_sm.load() : 1;
+    if (plan.fused_rotation) layout(kQmvXBlocks, kQmvRedStride);
+    else {
+        layout(2, kQmvRedStride);
+        // a tile without the padding costs a few bank conflicts once per warp, the second CTA is worth more
+        if (resident > 1 && plan.smem_bytes > kQmvSharedSmemBytes) layout(1, 128);
+        if (resident > 1 && plan.smem_bytes > kQmvSharedSmemBytes) { resident = 1; layout(2, kQmvRedStride); }
+    }
+    plan.grid = grid_for(resident);
+    plan.max_pieces = static_cast<int>((plan.grid + plan.col_blocks - 1) / plan.col_blocks + 1);
     const int pdl = g_pdl.load();
     plan.pdl = pdl != 0;
     plan.pdl_early = pdl == 2;
@@ -100,6 +119,10 @@ cudaError_t launch_qmv(QmvArgs args, int k, int cb, bool exact, const QmvPlan& p
     args.warp_smem = plan.warp_smem;
     args.xs_offset = plan.xs_offset;
     args.stage_offset = plan.stage_offset;
+    args.stage2_offset = plan.stage2_offset;
+    args.tile_stride = plan.tile_stride;
+    args.x_blocks = plan.x_blocks;
+    args.xs_stride = plan.xs_stride;
     args.pdl_early = plan.pdl_early ? 1 : 0;
     switch (k) {
         case 1: return qmv_dispatch_k1(args, cb, exact, plan, stream);

@@ -105,8 +105,7 @@ __device__ __forceinline__ int qmv_group_of(const QmvArgs& p, int cblock) {
 // memory: xs[row][blk][128] = H128(half(half(x) * suh)).  The loads of the next block are issued before
 // the butterflies of the current one.
 __device__ __forceinline__ void qmv_rotate_chunk(const void* x, int x_dtype, const __half* suh, int in, int rows, int kb0,
-                                                 int nblk, __half* xs, int lane) {
-    constexpr int kXsHalves = kQmvXBlocks * 128;
+                                                 int nblk, __half* xs, int xs_stride, int lane) {
     const int total = rows * nblk;
     auto fetch = [&](int unit, uint2& sv, __half (&xv)[4]) {
         const int row = unit / nblk, blk = unit - row * nblk;
@@ -128,7 +127,7 @@ __device__ __forceinline__ void qmv_rotate_chunk(const void* x, int x_dtype, con
         if (unit + 1 < total) fetch(unit + 1, sv_next, xv_next);
         warp_hadamard128_f16(h, lane);
         const int row = unit / nblk, blk = unit - row * nblk;
-        *reinterpret_cast<uint2*>(xs + row * kXsHalves + blk * 128 + lane * 4) = *reinterpret_cast<uint2*>(h);
+        *reinterpret_cast<uint2*>(xs + row * xs_stride + blk * 128 + lane * 4) = *reinterpret_cast<uint2*>(h);
     }
     __syncwarp();
 }
@@ -202,7 +201,6 @@ __device__ __forceinline__ void qmv_row_inv_rms(const __half* x, const __half* r
 template <int kFused>
 __device__ __forceinline__ void qmv_rotate_chunk_fused(const QmvArgs& p, const __half* suh, const float (&inv)[kQmvFusedRows], int rows, int kb0,
                                                        int nblk, bool store_sum, __half* xs, int lane) {
-    constexpr int kXsHalves = kQmvXBlocks * 128;
     const __half* x = reinterpret_cast<const __half*>(p.x);
 #pragma unroll 1
     for (int row = 0; row < rows; ++row) {
@@ -246,13 +244,185 @@ __device__ __forceinline__ void qmv_rotate_chunk_fused(const QmvArgs& p, const _
             *reinterpret_cast<__half2*>(h) = __hmul2_rn(v[0], sh[0]);
             *reinterpret_cast<__half2*>(h + 2) = __hmul2_rn(v[1], sh[1]);
             warp_hadamard128_f16(h, lane);
-            *reinterpret_cast<uint2*>(xs + row * kXsHalves + blk * 128 + lane * 4) = *reinterpret_cast<uint2*>(h);
+            *reinterpret_cast<uint2*>(xs + row * p.xs_stride + blk * 128 + lane * 4) = *reinterpret_cast<uint2*>(h);
         }
     }
     __syncwarp();
 }
 
-// The last warp of a CTA to stage its tile of column block `cblock`: adds the tiles of the warps that
+// sum of the tiles that the CTA's warps staged for a block, in warp order (lane L: columns 4L..4L+3 of one row)
+__device__ __forceinline__ float4 qmv_sum_tiles(const QmvArgs& p, int row, unsigned int warp_mask, unsigned int second_mask,
+                                                const unsigned char* smem_base, int lane) {
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+    bool any = false;
+#pragma unroll 1
+    for (int w = 0; w < kQmvWarps; ++w) {
+        if (!((warp_mask >> w) & 1u)) continue;
+        // a warp stages the tile of its first block and of its second block in buffers of their own
+        const float4 t4 = *reinterpret_cast<const float4*>(
+            reinterpret_cast<const float*>(smem_base + static_cast<size_t>(w) * p.warp_smem +
+                                           ((second_mask >> w) & 1u ? p.stage2_offset : p.stage_offset)) +
+            row * p.tile_stride + lane * 4);
+        if (!any) { a = t4; any = true; }
+        else { a.x = __fadd_rn(a.x, t4.x); a.y = __fadd_rn(a.y, t4.y); a.z = __fadd_rn(a.z, t4.z); a.w = __fadd_rn(a.w, t4.w); }
+    }
+    return a;
+}
+
+// sum of the pieces that the CTAs of a block left, in piece order
+__device__ __forceinline__ float4 qmv_sum_pieces(const float* src, int tile_floats, int pieces) {
+    float4 a = __ldcg(reinterpret_cast<const float4*>(src));
+#pragma unroll 1
+    for (int s0 = 1; s0 < pieces; s0 += 4) {         // loads of four pieces go out together
+        float4 part[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (s0 + j < pieces) part[j] = __ldcg(reinterpret_cast<const float4*>(src + (s0 + j) * tile_floats));
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (s0 + j < pieces) {
+                a.x = __fadd_rn(a.x, part[j].x); a.y = __fadd_rn(a.y, part[j].y);
+                a.z = __fadd_rn(a.z, part[j].z); a.w = __fadd_rn(a.w, part[j].w);
+            }
+    }
+    return a;
+}
+
+// The complete sum of one row of a column block: raw, or rotated and stored with whatever is fused behind the layer.
+template <int kFused>
+__device__ __forceinline__ void qmv_finish_row(const QmvArgs& p, int cblock, int row, float4 a, int lane) {
+    const int col = cblock * 128 + lane * 4;              // column in the concatenated output space
+    if (p.yhat != nullptr && QMV_EPI(p) == 3) {
+        // Expert-mapped down product, one row per slot: virtual block = (slot, block j of the expert's columns).
+        // The block is rotated, scaled by the expert's output scales and the slot's routing weight and parked in
+        // yhat; the last of a token's top_k slots to arrive adds them in slot order (the arithmetic and the order
+        // of finish_and_reduce_kernel, so the same bits).
+        const int slot = cblock / p.map_blocks, j = cblock - slot * p.map_blocks;
+        const int width = p.map_blocks << 7, top_k = p.map_top_k;
+        const int64_t expert = static_cast<int64_t>(min(p.map_selected[slot], static_cast<uint32_t>(p.map_experts - 1)));
+        __half h[4] = {__float2half_rn(a.x), __float2half_rn(a.y), __float2half_rn(a.z), __float2half_rn(a.w)};
+        warp_hadamard128_f16(h, lane);
+        const uint2 svw = *reinterpret_cast<const uint2*>(p.svh + expert * width + j * 128 + lane * 4);
+        const __half* sv = reinterpret_cast<const __half*>(&svw);
+        float v[4];
+        if (p.epi_score_f32) {
+            const float score = reinterpret_cast<const float*>(p.epi_scores)[slot];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) v[e] = __fmul_rn(__half2float(__hmul_rn(h[e], sv[e])), score);
+        } else {
+            const __half score = reinterpret_cast<const __half*>(p.epi_scores)[slot];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) v[e] = __half2float(__hmul_rn(__hmul_rn(h[e], sv[e]), score));
+        }
+        __stcg(reinterpret_cast<float4*>(p.yhat + col), make_float4(v[0], v[1], v[2], v[3]));
+        __threadfence();                                // the parked block before the arrival
+        __syncwarp();
+        const int token = slot / top_k;
+        unsigned int* arrived = p.counters + p.epi_counter0 + token * p.map_blocks + j;
+        unsigned int before = 0;
+        if (lane == 0) before = atomicAdd(arrived, 1u);
+        before = __shfl_sync(0xffffffffu, before, 0);
+        if (before != static_cast<unsigned int>(top_k - 1)) return;
+        __threadfence();
+        if (lane == 0) *arrived = 0;                    // leave the scratch ready for the next call
+        const float* parked = p.yhat + (static_cast<int64_t>(token) * top_k * p.map_blocks + j) * 128 + lane * 4;
+        float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 1
+        for (int t0 = 0; t0 < top_k; t0 += 4) {         // four loads in flight, added in slot order
+            float4 r[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (t0 + i < top_k) r[i] = __ldcg(reinterpret_cast<const float4*>(parked + static_cast<int64_t>(t0 + i) * width));
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                if (t0 + i >= top_k) continue;
+                const float f[4] = {r[i].x, r[i].y, r[i].z, r[i].w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    if (t0 + i == 0) acc[e] = f[e];
+                    else if (p.epi_score_f32) acc[e] = __fadd_rn(acc[e], f[e]);
+                    else acc[e] = __half2float(__hadd_rn(__float2half_rn(acc[e]), __float2half_rn(f[e])));
+                }
+            }
+        }
+        const int64_t at = static_cast<int64_t>(token) * width + j * 128 + lane * 4;
+        if (p.epi_score_f32) {
+            *reinterpret_cast<float4*>(reinterpret_cast<float*>(p.gy[0]) + at) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+        } else {
+            __align__(8) __half o16[4] = {__float2half_rn(acc[0]), __float2half_rn(acc[1]), __float2half_rn(acc[2]), __float2half_rn(acc[3])};
+            *reinterpret_cast<uint2*>(reinterpret_cast<__half*>(p.gy[0]) + at) = *reinterpret_cast<const uint2*>(o16);
+        }
+    } else if (p.yhat != nullptr) {
+        *reinterpret_cast<float4*>(p.yhat + static_cast<int64_t>(row) * p.out + col) = a;
+    } else {
+        // a row shard of a tensor-parallel layer first adds the other ranks' sums for this block
+        if (p.tp.world > 0) a = tp_exchange_unit(p.tp, (p.tp_row0 + row) * (p.out >> 7) + cblock, a, lane);
+        __half h[4] = {__float2half_rn(a.x), __float2half_rn(a.y), __float2half_rn(a.z), __float2half_rn(a.w)};
+        warp_hadamard128_f16(h, lane);
+        __align__(8) __half sv[4];
+        *reinterpret_cast<uint2*>(sv) = *reinterpret_cast<const uint2*>(p.svh + col);
+        if (QMV_EPI(p) == 1) {
+            // residual add and the block's sum of squares for the next RMSNorm (fixed shuffle order)
+            const int64_t at = static_cast<int64_t>(row) * p.out + col;
+            const uint2 rv = __ldcg(reinterpret_cast<const uint2*>(p.epi_residual + at));
+            const __half* rh = reinterpret_cast<const __half*>(&rv);
+            __align__(8) __half sum[4];
+            float sq = 0.0f;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                __half y = __hmul_rn(h[j], sv[j]);
+                if (p.bias) y = __hadd_rn(y, p.bias[col + j]);
+                sum[j] = __hadd_rn(rh[j], y);
+                const float f = __half2float(sum[j]);
+                sq = fmaf(f, f, sq);
+            }
+            *reinterpret_cast<uint2*>(p.epi_sum + at) = *reinterpret_cast<const uint2*>(sum);
+#pragma unroll
+            for (int d = 16; d >= 1; d >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, d);
+            if (lane == 0) p.epi_sumsq[row * (p.out >> 7) + cblock] = sq;
+            return;
+        }
+        const int grp = qmv_group_of(p, cblock);
+        const int gcol = col - p.gcol0[grp];
+        if (QMV_EPI(p) == 2) {
+            // [q | k | v] with 128-wide heads: this block is one head.  Rotary embedding of q and k heads (pairs
+            // (i, i + 64): lane L holds columns 4L..4L+3, its partner is lane L ^ 16), keys and values go
+            // straight into row `pos` of the caches.
+            int pos = __ldg(p.epi_pos);
+            pos = pos < 0 ? 0 : (pos >= p.epi_max_ctx ? p.epi_max_ctx - 1 : pos);
+            __align__(8) __half y[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                y[j] = __hmul_rn(h[j], sv[j]);
+                if (p.bias) y[j] = __hadd_rn(y[j], p.bias[col + j]);
+            }
+            if (grp < 2) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float mine = __half2float(y[j]);
+                    const float other = __shfl_xor_sync(0xffffffffu, mine, 16);
+                    const int i = (lane & 15) * 4 + j;
+                    const float inv_freq = exp2f(-p.epi_log2_theta * static_cast<float>(2 * i) / 128.0f);
+                    float sn, cs;
+                    sincosf(static_cast<float>(pos) * inv_freq, &sn, &cs);
+                    const float a0 = lane < 16 ? mine : other, b0 = lane < 16 ? other : mine;
+                    y[j] = __float2half_rn(lane < 16 ? a0 * cs - b0 * sn : a0 * sn + b0 * cs);
+                }
+            }
+            __half* dst = grp == 0 ? reinterpret_cast<__half*>(p.gy[0]) + gcol
+                                   : (grp == 1 ? p.epi_k_cache : p.epi_v_cache) +
+                                         (static_cast<int64_t>(gcol >> 7) * p.epi_max_ctx + pos) * 128 + lane * 4;
+            *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(y);
+            return;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            store_from_half(p.gy[grp], p.y_dtype, static_cast<int64_t>(row) * p.gout[grp] + gcol + j,
+                            __hmul_rn(h[j], sv[j]), p.bias ? p.bias + (col - gcol) : nullptr, gcol + j);
+    }
+}
+
+// The last warp of a CTA to stage its tile of column block `cblock` (one or two rows): adds the tiles of the warps that
 // had work in the block (warp_mask) in warp order; if other CTAs share the block, publishes the
 // sum as this CTA's piece and counts arrivals; the last CTA adds the pieces in piece order.  Whoever
 // holds the complete sum applies the output rotation (or stores the raw sum).
@@ -263,7 +433,6 @@ __device__ __forceinline__ void qmv_finish_block(const QmvArgs& p, int cblock, u
     const int tile_floats = rows * 128;
     const float* piece_base = p.partials + static_cast<int64_t>(cblock) * p.max_pieces * tile_floats;
     float* piece_dst = p.partials + (static_cast<int64_t>(cblock) * p.max_pieces + piece) * tile_floats;
-    const int stage_floats = rows * kQmvRedStride;
 #pragma unroll 1
     for (int pass = 0; pass < (pieces > 1 ? 2 : 1); ++pass) {
         if (pass == 1) {
@@ -279,183 +448,58 @@ __device__ __forceinline__ void qmv_finish_block(const QmvArgs& p, int cblock, u
         const bool complete = pass == 1 || pieces == 1;
 #pragma unroll 1
         for (int row = 0; row < rows; ++row) {
-            float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (pass == 0) {
-                bool any = false;
+            const float4 a = pass == 0 ? qmv_sum_tiles(p, row, warp_mask, second_mask, smem_base, lane)
+                                       : qmv_sum_pieces(piece_base + row * 128 + lane * 4, tile_floats, pieces);
+            if (!complete) __stcg(reinterpret_cast<float4*>(piece_dst + row * 128 + lane * 4), a);
+            else qmv_finish_row<kFused>(p, cblock, row, a, lane);
+        }
+    }
+}
+
+// The same for more than two rows, by all warps of the CTA once the last of them has staged its tiles: a warp takes every
+// eighth row.  (One warp for all rows, as above, spends a microsecond or two per row on its chain of loads and shuffles:
+// 8 rows of 4096 -> 4096 took 30 us, 20 of them here.)
+template <int kFused>
+__device__ __noinline__ void qmv_finish_many(const QmvArgs& p, int cblock, unsigned int warp_mask, unsigned int second_mask, int pieces, int piece,
+                                             const unsigned char* smem_base, unsigned int* s_last, int warp, int lane) {
+    const int rows = p.rows;
+    const int tile_floats = rows * 128;
+    float* const block = p.partials + static_cast<int64_t>(cblock) * p.max_pieces * tile_floats;
 #pragma unroll 1
-                for (int w = 0; w < kQmvWarps; ++w) {
-                    if (!((warp_mask >> w) & 1u)) continue;
-                    // a warp stages the tile of its first block in buffer 0 and of its second block in buffer 1
-                    const float4 t4 = *reinterpret_cast<const float4*>(
-                        reinterpret_cast<const float*>(smem_base + static_cast<size_t>(w) * p.warp_smem + p.stage_offset) +
-                        ((second_mask >> w) & 1u) * stage_floats + row * kQmvRedStride + lane * 4);
-                    if (!any) { a = t4; any = true; }
-                    else { a.x = __fadd_rn(a.x, t4.x); a.y = __fadd_rn(a.y, t4.y); a.z = __fadd_rn(a.z, t4.z); a.w = __fadd_rn(a.w, t4.w); }
-                }
-            } else {
-                const float* src = piece_base + row * 128 + lane * 4;
-                a = __ldcg(reinterpret_cast<const float4*>(src));
+    for (int pass = 0; pass < (pieces > 1 ? 2 : 1); ++pass) {
+        if (pass == 1) {
+            __threadfence();
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                const unsigned int prev = atomicAdd(p.counters + cblock, 1u);
+                *s_last = prev == static_cast<unsigned int>(pieces - 1);
+                if (*s_last) p.counters[cblock] = 0;            // leave the scratch ready for the next call
+            }
+            __syncthreads();
+            const bool last = *s_last != 0;
+            __syncthreads();                                    // read by all before the next block's answer
+            if (!last) return;
+            __threadfence();
+        }
 #pragma unroll 1
-                for (int s0 = 1; s0 < pieces; s0 += 4) {         // loads of four pieces go out together
-                    float4 part[4];
-#pragma unroll
-                    for (int j = 0; j < 4; ++j)
-                        if (s0 + j < pieces) part[j] = __ldcg(reinterpret_cast<const float4*>(src + (s0 + j) * tile_floats));
-#pragma unroll
-                    for (int j = 0; j < 4; ++j)
-                        if (s0 + j < pieces) {
-                            a.x = __fadd_rn(a.x, part[j].x); a.y = __fadd_rn(a.y, part[j].y);
-                            a.z = __fadd_rn(a.z, part[j].z); a.w = __fadd_rn(a.w, part[j].w);
-                        }
-                }
-            }
-            if (!complete) {
-                __stcg(reinterpret_cast<float4*>(piece_dst + row * 128 + lane * 4), a);
-                continue;
-            }
-            const int col = cblock * 128 + lane * 4;              // column in the concatenated output space
-            if (p.yhat != nullptr && QMV_EPI(p) == 3) {
-                // Expert-mapped down product, one row per slot: virtual block = (slot, block j of the expert's columns).
-                // The block is rotated, scaled by the expert's output scales and the slot's routing weight and parked in
-                // yhat; the last of a token's top_k slots to arrive adds them in slot order (the arithmetic and the order
-                // of finish_and_reduce_kernel, so the same bits).
-                const int slot = cblock / p.map_blocks, j = cblock - slot * p.map_blocks;
-                const int width = p.map_blocks << 7, top_k = p.map_top_k;
-                const int64_t expert = static_cast<int64_t>(min(p.map_selected[slot], static_cast<uint32_t>(p.map_experts - 1)));
-                __half h[4] = {__float2half_rn(a.x), __float2half_rn(a.y), __float2half_rn(a.z), __float2half_rn(a.w)};
-                warp_hadamard128_f16(h, lane);
-                const uint2 svw = *reinterpret_cast<const uint2*>(p.svh + expert * width + j * 128 + lane * 4);
-                const __half* sv = reinterpret_cast<const __half*>(&svw);
-                float v[4];
-                if (p.epi_score_f32) {
-                    const float score = reinterpret_cast<const float*>(p.epi_scores)[slot];
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) v[e] = __fmul_rn(__half2float(__hmul_rn(h[e], sv[e])), score);
-                } else {
-                    const __half score = reinterpret_cast<const __half*>(p.epi_scores)[slot];
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) v[e] = __half2float(__hmul_rn(__hmul_rn(h[e], sv[e]), score));
-                }
-                __stcg(reinterpret_cast<float4*>(p.yhat + col), make_float4(v[0], v[1], v[2], v[3]));
-                __threadfence();                                // the parked block before the arrival
-                __syncwarp();
-                const int token = slot / top_k;
-                unsigned int* arrived = p.counters + p.epi_counter0 + token * p.map_blocks + j;
-                unsigned int before = 0;
-                if (lane == 0) before = atomicAdd(arrived, 1u);
-                before = __shfl_sync(0xffffffffu, before, 0);
-                if (before != static_cast<unsigned int>(top_k - 1)) continue;
-                __threadfence();
-                if (lane == 0) *arrived = 0;                    // leave the scratch ready for the next call
-                const float* parked = p.yhat + (static_cast<int64_t>(token) * top_k * p.map_blocks + j) * 128 + lane * 4;
-                float acc[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 1
-                for (int t0 = 0; t0 < top_k; t0 += 4) {         // four loads in flight, added in slot order
-                    float4 r[4];
-#pragma unroll
-                    for (int i = 0; i < 4; ++i)
-                        if (t0 + i < top_k) r[i] = __ldcg(reinterpret_cast<const float4*>(parked + static_cast<int64_t>(t0 + i) * width));
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        if (t0 + i >= top_k) continue;
-                        const float f[4] = {r[i].x, r[i].y, r[i].z, r[i].w};
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            if (t0 + i == 0) acc[e] = f[e];
-                            else if (p.epi_score_f32) acc[e] = __fadd_rn(acc[e], f[e]);
-                            else acc[e] = __half2float(__hadd_rn(__float2half_rn(acc[e]), __float2half_rn(f[e])));
-                        }
-                    }
-                }
-                const int64_t at = static_cast<int64_t>(token) * width + j * 128 + lane * 4;
-                if (p.epi_score_f32) {
-                    *reinterpret_cast<float4*>(reinterpret_cast<float*>(p.gy[0]) + at) = make_float4(acc[0], acc[1], acc[2], acc[3]);
-                } else {
-                    __align__(8) __half o16[4] = {__float2half_rn(acc[0]), __float2half_rn(acc[1]), __float2half_rn(acc[2]), __float2half_rn(acc[3])};
-                    *reinterpret_cast<uint2*>(reinterpret_cast<__half*>(p.gy[0]) + at) = *reinterpret_cast<const uint2*>(o16);
-                }
-            } else if (p.yhat != nullptr) {
-                *reinterpret_cast<float4*>(p.yhat + static_cast<int64_t>(row) * p.out + col) = a;
-            } else {
-                // a row shard of a tensor-parallel layer first adds the other ranks' sums for this block
-                if (p.tp.world > 0) a = tp_exchange_unit(p.tp, (p.tp_row0 + row) * (p.out >> 7) + cblock, a, lane);
-                __half h[4] = {__float2half_rn(a.x), __float2half_rn(a.y), __float2half_rn(a.z), __float2half_rn(a.w)};
-                warp_hadamard128_f16(h, lane);
-                __align__(8) __half sv[4];
-                *reinterpret_cast<uint2*>(sv) = *reinterpret_cast<const uint2*>(p.svh + col);
-                if (QMV_EPI(p) == 1) {
-                    // residual add and the block's sum of squares for the next RMSNorm (fixed shuffle order)
-                    const int64_t at = static_cast<int64_t>(row) * p.out + col;
-                    const uint2 rv = __ldcg(reinterpret_cast<const uint2*>(p.epi_residual + at));
-                    const __half* rh = reinterpret_cast<const __half*>(&rv);
-                    __align__(8) __half sum[4];
-                    float sq = 0.0f;
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        __half y = __hmul_rn(h[j], sv[j]);
-                        if (p.bias) y = __hadd_rn(y, p.bias[col + j]);
-                        sum[j] = __hadd_rn(rh[j], y);
-                        const float f = __half2float(sum[j]);
-                        sq = fmaf(f, f, sq);
-                    }
-                    *reinterpret_cast<uint2*>(p.epi_sum + at) = *reinterpret_cast<const uint2*>(sum);
-#pragma unroll
-                    for (int d = 16; d >= 1; d >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, d);
-                    if (lane == 0) p.epi_sumsq[row * (p.out >> 7) + cblock] = sq;
-                    continue;
-                }
-                const int grp = qmv_group_of(p, cblock);
-                const int gcol = col - p.gcol0[grp];
-                if (QMV_EPI(p) == 2) {
-                    // [q | k | v] with 128-wide heads: this block is one head.  Rotary embedding of q and k heads (pairs
-                    // (i, i + 64): lane L holds columns 4L..4L+3, its partner is lane L ^ 16), keys and values go
-                    // straight into row `pos` of the caches.
-                    int pos = __ldg(p.epi_pos);
-                    pos = pos < 0 ? 0 : (pos >= p.epi_max_ctx ? p.epi_max_ctx - 1 : pos);
-                    __align__(8) __half y[4];
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        y[j] = __hmul_rn(h[j], sv[j]);
-                        if (p.bias) y[j] = __hadd_rn(y[j], p.bias[col + j]);
-                    }
-                    if (grp < 2) {
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            const float mine = __half2float(y[j]);
-                            const float other = __shfl_xor_sync(0xffffffffu, mine, 16);
-                            const int i = (lane & 15) * 4 + j;
-                            const float inv_freq = exp2f(-p.epi_log2_theta * static_cast<float>(2 * i) / 128.0f);
-                            float sn, cs;
-                            sincosf(static_cast<float>(pos) * inv_freq, &sn, &cs);
-                            const float a0 = lane < 16 ? mine : other, b0 = lane < 16 ? other : mine;
-                            y[j] = __float2half_rn(lane < 16 ? a0 * cs - b0 * sn : a0 * sn + b0 * cs);
-                        }
-                    }
-                    __half* dst = grp == 0 ? reinterpret_cast<__half*>(p.gy[0]) + gcol
-                                           : (grp == 1 ? p.epi_k_cache : p.epi_v_cache) +
-                                                 (static_cast<int64_t>(gcol >> 7) * p.epi_max_ctx + pos) * 128 + lane * 4;
-                    *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(y);
-                    continue;
-                }
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    store_from_half(p.gy[grp], p.y_dtype, static_cast<int64_t>(row) * p.gout[grp] + gcol + j,
-                                    __hmul_rn(h[j], sv[j]), p.bias ? p.bias + (col - gcol) : nullptr, gcol + j);
-            }
+        for (int row = warp; row < rows; row += kQmvWarps) {
+            const float4 a = pass == 0 ? qmv_sum_tiles(p, row, warp_mask, second_mask, smem_base, lane)
+                                       : qmv_sum_pieces(block + row * 128 + lane * 4, tile_floats, pieces);
+            if (pass == 0 && pieces > 1) __stcg(reinterpret_cast<float4*>(block + piece * tile_floats + row * 128 + lane * 4), a);
+            else qmv_finish_row<kFused>(p, cblock, row, a, lane);
         }
     }
 }
 
 template <int K, int CB, int NB, int MODE, int kFused>
 __global__ void __launch_bounds__(kQmvWarps * 32, NB == 1 ? 2 : 1)
-qmv_kernel(const QmvArgs p) {
+qmv_kernel(const __grid_constant__ QmvArgs p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr int WARPS = kQmvWarps;
     constexpr int R = qmv_chunk_rows(K);                    // rows per bulk copy (the rows of a column block are contiguous)
     constexpr int SLOTS = qmv_slots(K);                     // chunks in flight per warp
     constexpr int kRowWords = 64 * K;                       // 2 quads x 8K words x 4 tiles
     constexpr uint32_t kRowBytes = kRowWords * 4;
-    constexpr int kXsHalves = kQmvXBlocks * 128;            // rotated activations kept per row and warp
     __shared__ __align__(8) uint64_t s_bar[WARPS][SLOTS];
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -497,8 +541,7 @@ qmv_kernel(const QmvArgs p) {
 
     unsigned char* mine = smem_raw + static_cast<size_t>(warp) * p.warp_smem;
     uint32_t* ring = reinterpret_cast<uint32_t*>(mine);                  // SLOTS chunks of R rows of packed words
-    __half* xs = reinterpret_cast<__half*>(mine + p.xs_offset);          // [rows][kXsHalves] (fused rotation only)
-    const int stage_floats = rows * kQmvRedStride;                       // one staged [rows][128] tile
+    __half* xs = reinterpret_cast<__half*>(mine + p.xs_offset);          // [rows][xs_stride] rotated activations
     uint64_t* bars = s_bar[warp];
     constexpr size_t row_stride = 256 * K;                               // consecutive rows of a column block are contiguous
     const LaneGeom<K> geom(lane);
@@ -524,6 +567,29 @@ qmv_kernel(const QmvArgs p) {
         if (threadIdx.x == 0) atomicExch(p.error, 2u);
         return;
     }
+    // warps of this CTA with a tile of block `cblock`, and those of them whose second block it is
+    auto contributors = [&](int cblock, unsigned int& mask, unsigned int& second) {
+        mask = second = 0;
+#pragma unroll 1
+        for (int w = 0; w < WARPS; ++w)
+            if (min(s_begin[w + 1], (cblock + 1) * UB) > max(s_begin[w], cblock * UB)) {
+                mask |= 1u << w;
+                if (s_begin[w] / UB != cblock) second |= 1u << w;
+            }
+    };
+    // first and last CTA with rows of the block: the inverse of unit_begin (warp holding row x: ceil((x+1)*W/RT) - 1)
+    auto sharing_ctas = [&](int cblock, int& i_first, int& i_last) {
+        if (aligned) {
+            i_first = static_cast<int>(static_cast<unsigned int>(cblock) * W / C) / WARPS;
+            i_last = (static_cast<int>(static_cast<unsigned int>(cblock + 1) * W / C) - 1) / WARPS;
+        } else if (narrow) {
+            i_first = static_cast<int>(((static_cast<unsigned int>(cblock * RB + 1) * W - 1u) / RT) / WARPS);
+            i_last = static_cast<int>(((static_cast<unsigned int>((cblock + 1) * RB) * W - 1u) / RT) / WARPS);
+        } else {
+            i_first = static_cast<int>((((static_cast<int64_t>(cblock) * RB + 1) * W - 1) / RT) / WARPS);
+            i_last = static_cast<int>(((static_cast<int64_t>(cblock + 1) * RB * W - 1) / RT) / WARPS);
+        }
+    };
     int slot = 0;
     uint32_t parity = 0;
     bool copy_lost = false;
@@ -535,7 +601,7 @@ qmv_kernel(const QmvArgs p) {
         // ---- this warp's segment [u0, u1) of the block ----------------------------------------------------
         const int u0 = max(w0, cblock * UB) - cblock * UB;
         const int u1 = min(w1, (cblock + 1) * UB) - cblock * UB;
-        float* stage = reinterpret_cast<float*>(mine + p.stage_offset) + (cblock - w0 / UB) * stage_floats;
+        float* const stage = reinterpret_cast<float*>(mine + (cblock == w0 / UB ? p.stage_offset : p.stage2_offset));
         int grp = qmv_group_of(p, cblock);
         int tn0 = cblock * 8;                               // first tile column of the block in the weight array
         bool active = true;
@@ -596,11 +662,11 @@ qmv_kernel(const QmvArgs p) {
                     if (req_tk <= tk_last) refill(slot + i < SLOTS ? slot + i : slot + i - SLOTS);
             }
 
-            // The segment is walked in stretches whose inputs span at most kQmvXBlocks 128-blocks, so that
+            // The segment is walked in stretches whose inputs span at most x_blocks 128-blocks, so that
             // the rotated activations of a stretch fit the warp's shared memory.
             for (int tk0 = tk_first; active && tk0 <= tk_last;) {
                 const int kb0 = tk0 >> 3;
-                const int tk_end = min(tk_last + 1, (kb0 + kQmvXBlocks) * 8);
+                const int tk_end = min(tk_last + 1, (kb0 + p.x_blocks) * 8);
                 const int nrows = tk_end - tk0;
 
                 if (first_chunk) {
@@ -635,8 +701,22 @@ qmv_kernel(const QmvArgs p) {
                         qmv_rotate_chunk_fused<kFused>(p, p.suh + suh_row * p.in, inv_rms, rows, kb0, ((tk_end - 1) >> 3) - kb0 + 1, cblock == 0, xs, lane);
                     } else {
                         qmv_rotate_chunk(x_rows, p.x_dtype, p.suh + suh_row * p.in, p.in, rows, kb0,
-                                         ((tk_end - 1) >> 3) - kb0 + 1, xs, lane);
+                                         ((tk_end - 1) >> 3) - kb0 + 1, xs, p.xs_stride, lane);
                     }
+                } else {
+                    // rows that come rotated: copied without passing through registers (read fragment by fragment from
+                    // global memory, every row of tiles waited for its own loads)
+                    __syncwarp();                           // all lanes have read the stretch before
+                    const int nblk = ((tk_end - 1) >> 3) - kb0 + 1;
+                    const __half* src = p.xhat + grp * p.xhat_group_stride + kb0 * 128 + (lane & 15) * 8;
+                    const uint32_t dst = smem_addr(xs + (lane & 15) * 8);
+#pragma unroll 1
+                    for (int b = 0; b < nblk; ++b)
+#pragma unroll 1
+                        for (int row = lane >> 4; row < rows; row += 2)
+                            copy16_async(dst + (row * p.xs_stride + b * 128) * 2, src + static_cast<int64_t>(row) * p.in + b * 128);
+                    copy_async_wait();
+                    __syncwarp();
                 }
                 if (tracing && tk0 == tk_first) p.trace[blockIdx.x * 8 + 2] = global_ns();
 
@@ -646,10 +726,7 @@ qmv_kernel(const QmvArgs p) {
 #pragma unroll
                 for (int nb = 0; nb < NB; ++nb) {
                     const int row = min(nb * 8 + g, rows - 1);
-                    if (p.xhat == nullptr)
-                        xfrag[nb] = reinterpret_cast<const uint32_t*>(xs + row * kXsHalves + (tk0 * 16 - kb0 * 128)) + q;
-                    else
-                        xfrag[nb] = reinterpret_cast<const uint32_t*>(p.xhat + grp * p.xhat_group_stride + static_cast<int64_t>(row) * p.in + tk0 * 16) + q;
+                    xfrag[nb] = reinterpret_cast<const uint32_t*>(xs + row * p.xs_stride + (tk0 * 16 - kb0 * 128)) + q;
                 }
                 // The rows of the stretch are walked run by run (a run = the part of one chunk inside the stretch): the
                 // barrier wait and the hand-back of the slot happen once per chunk, and the row loop tests nothing per
@@ -703,7 +780,7 @@ qmv_kernel(const QmvArgs p) {
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
                         const int row = nb * 8 + 2 * q + (i & 1), col = t * 16 + g + ((i & 2) ? 8 : 0);
-                        if (row < rows) stage[row * kQmvRedStride + col] = acc[t][nb][i];
+                        if (row < rows) stage[row * p.tile_stride + col] = acc[t][nb][i];
                     }
         }
         if (!p.pdl_early && (cblock + 1) * UB >= w1) pdl_launch_dependents();
@@ -711,13 +788,9 @@ qmv_kernel(const QmvArgs p) {
 
         // ---- phase 4: the last warp of the CTA to arrive at this block adds the CTA's tiles, meets the
         //      other CTAs of the block, rotates and stores ---------------------------------------------------
-        unsigned int mask = 0, second = 0;                      // warps with a tile here; ... as their 2nd block
-#pragma unroll 1
-        for (int w = 0; w < WARPS; ++w)
-            if (min(s_begin[w + 1], (cblock + 1) * UB) > max(s_begin[w], cblock * UB)) {
-                mask |= 1u << w;
-                if (s_begin[w] / UB != cblock) second |= 1u << w;
-            }
+        if (rows > kQmvFusedRows) continue;                     // all warps finish the CTA's blocks together, below
+        unsigned int mask, second;
+        contributors(cblock, mask, second);
         __syncwarp();
         unsigned int prev = 0;
         if (lane == 0) {
@@ -728,22 +801,25 @@ qmv_kernel(const QmvArgs p) {
         if (tracing) p.trace[blockIdx.x * 8 + 4] = global_ns();
         if (prev + 1 == static_cast<unsigned int>(__popc(mask))) {
             __threadfence_block();
-            // first and last CTA with rows of this block: the inverse of unit_begin (warp holding row x: ceil((x+1)*W/RT) - 1)
             int i_first, i_last;
-            if (aligned) {
-                i_first = static_cast<int>(static_cast<unsigned int>(cblock) * W / C) / WARPS;
-                i_last = (static_cast<int>(static_cast<unsigned int>(cblock + 1) * W / C) - 1) / WARPS;
-            } else if (narrow) {
-                i_first = static_cast<int>(((static_cast<unsigned int>(cblock * RB + 1) * W - 1u) / RT) / WARPS);
-                i_last = static_cast<int>(((static_cast<unsigned int>((cblock + 1) * RB) * W - 1u) / RT) / WARPS);
-            } else {
-                i_first = static_cast<int>((((static_cast<int64_t>(cblock) * RB + 1) * W - 1) / RT) / WARPS);
-                i_last = static_cast<int>(((static_cast<int64_t>(cblock + 1) * RB * W - 1) / RT) / WARPS);
-            }
-            qmv_finish_block<kFused>(p, cblock, mask, second, i_last - i_first + 1, static_cast<int>(blockIdx.x) - i_first, smem_raw,
-                             lane);
+            sharing_ctas(cblock, i_first, i_last);
+            qmv_finish_block<kFused>(p, cblock, mask, second, i_last - i_first + 1, static_cast<int>(blockIdx.x) - i_first, smem_raw, lane);
             if (tracing) p.trace[blockIdx.x * 8 + 5] = global_ns();
         }
+    }
+    if (rows > kQmvFusedRows) {
+        __syncthreads();                                        // every tile of the CTA is staged
+        if (tracing) p.trace[blockIdx.x * 8 + 4] = global_ns();
+#pragma unroll 1
+        for (int cblock = cta0 / UB; cblock * UB < s_begin[WARPS]; ++cblock) {
+            unsigned int mask, second;
+            contributors(cblock, mask, second);
+            int i_first, i_last;
+            sharing_ctas(cblock, i_first, i_last);
+            qmv_finish_many<kFused>(p, cblock, mask, second, i_last - i_first + 1, static_cast<int>(blockIdx.x) - i_first, smem_raw, &s_arrived[0],
+                                    warp, lane);
+        }
+        if (tracing) p.trace[blockIdx.x * 8 + 5] = global_ns();
     }
     if (copy_lost && lane == 0) atomicExch(p.error, 1u);
 }

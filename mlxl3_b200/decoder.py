@@ -16,7 +16,7 @@ import numpy as np
 from . import _lib
 from ._lib import F16
 from .linear import Exl3Group, Exl3Linear, Prologue, new_workspace
-from .runtime import DEFAULT_STREAM, DeviceBuffer, Graph, Stream
+from .runtime import DEFAULT_STREAM, DeviceBuffer, Graph, Scratch, Stream
 
 
 def _p(x):
@@ -367,9 +367,11 @@ class DenseMlp:
     def forward(self, x: np.ndarray, stream: Stream = DEFAULT_STREAM) -> np.ndarray:
         x = np.ascontiguousarray(x, np.float16)
         rows = x.shape[0]
-        d_x, d_y = DeviceBuffer.from_numpy(x, stream), DeviceBuffer(rows * self.hidden * 2)
-        self.forward_device(d_x.ptr, rows, d_y.ptr, stream)
-        return d_y.download((rows, self.hidden), np.float16, stream)
+        at_x, at_y, end = Scratch.offsets(x.nbytes, rows * self.hidden * 2)
+        with Scratch(end, stream) as s:
+            s.upload(x, at_x)
+            self.forward_device(s.ptr + at_x, rows, s.ptr + at_y, stream)
+            return s.download((rows, self.hidden), np.float16, at_y)
 
     def flops(self, rows: int) -> int:
         return 3 * 2 * rows * self.hidden * self.ffn

@@ -15,7 +15,7 @@ import numpy as np
 
 from . import _lib
 from ._lib import BF16, F16, F32, B200Exl3Error
-from .runtime import DEFAULT_STREAM, DeviceBuffer, Stream
+from .runtime import DEFAULT_STREAM, DeviceBuffer, Scratch, Stream
 
 DEFAULT, MCG, MUL1 = 0, 1, 2
 
@@ -195,7 +195,7 @@ class Exl3Linear:
 
     def workspace_bytes(self, rows: int) -> int:
         out = c_size_t()
-        _lib.call("b200exl3_linear_workspace_bytes", c_void_p(self.handle), rows, byref(out))
+        _lib.call("b200exl3_linear_workspace_bytes", self.handle, rows, byref(out))
         return out.value
 
     def _ensure_workspace(self, rows: int) -> DeviceBuffer:
@@ -207,15 +207,14 @@ class Exl3Linear:
     # ---- device-pointer entry points (no host copies) ---------------------------------------------
     def forward_device(self, d_x: int, dtype: int, rows: int, d_y: int, workspace: DeviceBuffer,
                        stream: Stream = DEFAULT_STREAM) -> None:
-        _lib.call("b200exl3_linear_forward", c_void_p(self.handle), c_void_p(d_x), dtype, rows, c_void_p(d_y),
-                  c_void_p(workspace.ptr), workspace.nbytes, c_void_p(stream.handle))
+        _lib.call("b200exl3_linear_forward", self.handle, d_x, dtype, rows, d_y, workspace.ptr, workspace.nbytes, stream.handle)
 
     def forward_fused_device(self, prologue: Prologue, d_x: int, rows: int, d_y: int, workspace: DeviceBuffer,
                              stream: Stream = DEFAULT_STREAM, tp=None) -> None:
         """``forward_device`` for fp16 rows with an RMSNorm or SwiGLU prologue fused into the kernel's input rotation;
         ``tp`` (a ``TpContext``) makes it the row-parallel form."""
-        _lib.call("b200exl3_linear_forward_fused", c_void_p(self.handle), byref(prologue), c_void_p(tp.handle) if tp is not None else None,
-                  c_void_p(d_x), rows, c_void_p(d_y), c_void_p(workspace.ptr), workspace.nbytes, c_void_p(stream.handle))
+        _lib.call("b200exl3_linear_forward_fused", self.handle, byref(prologue), tp.handle if tp is not None else None, d_x, rows, d_y,
+                  workspace.ptr, workspace.nbytes, stream.handle)
 
     def forward_static_device(self, d_x: int, dtype: int, rows: int, d_y: int, stream: Stream = DEFAULT_STREAM) -> None:
         """``forward_device`` without a workspace: the scratch is a fixed 4 MiB array inside the library,
@@ -246,11 +245,12 @@ class Exl3Linear:
             raise B200Exl3Error("EXL3 linear input cannot be empty")
         code = dtype_code(x, dtype)
         x2 = np.ascontiguousarray(x).reshape(matrix_rows, self.rows)
-        d_x = DeviceBuffer.from_numpy(x2, stream)
-        d_y = DeviceBuffer(matrix_rows * self.cols * x2.dtype.itemsize)
-        self.forward_device(d_x.ptr, code, matrix_rows, d_y.ptr, self._ensure_workspace(matrix_rows), stream)
-        y = d_y.download((matrix_rows, self.cols), x2.dtype, stream)
-        return y.reshape(*x.shape[:-1], self.cols)
+        workspace = self._ensure_workspace(matrix_rows)
+        at_x, at_y, end = Scratch.offsets(x2.nbytes, matrix_rows * self.cols * x2.dtype.itemsize)
+        with Scratch(end, stream) as s:
+            s.upload(x2, at_x)
+            self.forward_device(s.ptr + at_x, code, matrix_rows, s.ptr + at_y, workspace, stream)
+            return s.download((*x.shape[:-1], self.cols), x2.dtype, at_y)
 
     def forward_raw(self, xhat: np.ndarray, stream: Stream = DEFAULT_STREAM) -> np.ndarray:
         """fp32 ``xhat @ W`` for already rotated fp16 inputs ``[rows, in]`` (no rotations, no scales)."""
@@ -258,12 +258,12 @@ class Exl3Linear:
         if xh.ndim != 2 or xh.shape[1] != self.rows or xh.shape[0] == 0:
             raise B200Exl3Error(f"invalid EXL3 linear input for {self.rows} inputs")
         rows = xh.shape[0]
-        d_x = DeviceBuffer.from_numpy(xh, stream)
-        d_y = DeviceBuffer(rows * self.cols * 4)
         ws = self._ensure_workspace(rows)
-        _lib.call("b200exl3_linear_forward_raw", c_void_p(self.handle), c_void_p(d_x.ptr), rows, c_void_p(d_y.ptr),
-                  c_void_p(ws.ptr), ws.nbytes, c_void_p(stream.handle))
-        return d_y.download((rows, self.cols), np.float32, stream)
+        at_x, at_y, end = Scratch.offsets(xh.nbytes, rows * self.cols * 4)
+        with Scratch(end, stream) as s:
+            s.upload(xh, at_x)
+            _lib.call("b200exl3_linear_forward_raw", self.handle, s.ptr + at_x, rows, s.ptr + at_y, ws.ptr, ws.nbytes, stream.handle)
+            return s.download((rows, self.cols), np.float32, at_y)
 
     def decode(self, stream: Stream = DEFAULT_STREAM) -> np.ndarray:
         """Inner matrix ``W[in, out]`` as fp16 (``codec::reconstruct_inner``, native/src/codec.rs:159-190)."""
@@ -314,8 +314,7 @@ class Exl3Group:
     def forward_device(self, d_x: int, dtype: int, rows: int, d_ys, workspace: DeviceBuffer,
                        stream: Stream = DEFAULT_STREAM) -> None:
         ptrs = (c_void_p * len(self.widths))(*d_ys)
-        _lib.call("b200exl3_group_forward", c_void_p(self.handle), c_void_p(d_x), dtype, rows, ptrs, c_void_p(workspace.ptr),
-                  workspace.nbytes, c_void_p(stream.handle))
+        _lib.call("b200exl3_group_forward", self.handle, d_x, dtype, rows, ptrs, workspace.ptr, workspace.nbytes, stream.handle)
 
     def forward_fused_device(self, prologue: Prologue, d_x: int, rows: int, d_ys, workspace: DeviceBuffer,
                              stream: Stream = DEFAULT_STREAM) -> None:
@@ -330,13 +329,14 @@ class Exl3Group:
         matrix_rows = x.size // self.rows
         code = dtype_code(x, dtype)
         x2 = np.ascontiguousarray(x).reshape(matrix_rows, self.rows)
-        d_x = DeviceBuffer.from_numpy(x2, stream)
-        d_ys = [DeviceBuffer(matrix_rows * w * x2.dtype.itemsize) for w in self.widths]
         need = self.workspace_bytes(matrix_rows)
         if self._workspace is None or self._workspace.nbytes < need:
             self._workspace = new_workspace(need)
-        self.forward_device(d_x.ptr, code, matrix_rows, [d.ptr for d in d_ys], self._workspace, stream)
-        return [d.download((matrix_rows, w), x2.dtype, stream).reshape(*x.shape[:-1], w) for d, w in zip(d_ys, self.widths)]
+        at_x, *at_ys, end = Scratch.offsets(x2.nbytes, *(matrix_rows * w * x2.dtype.itemsize for w in self.widths))
+        with Scratch(end, stream) as s:
+            s.upload(x2, at_x)
+            self.forward_device(s.ptr + at_x, code, matrix_rows, [s.ptr + at for at in at_ys], self._workspace, stream)
+            return [s.download((*x.shape[:-1], w), x2.dtype, at) for at, w in zip(at_ys, self.widths)]
 
     def close(self) -> None:
         if getattr(self, "handle", None):

@@ -9,7 +9,7 @@ import numpy as np
 from . import _lib
 from ._lib import B200Exl3Error, F16, F32
 from .linear import DEFAULT, MCG, MUL1, dtype_code, _np_dtype, new_workspace
-from .runtime import DEFAULT_STREAM, DeviceBuffer, Stream
+from .runtime import DEFAULT_STREAM, DeviceBuffer, Scratch, Stream
 
 
 class Exl3SwitchGlu:
@@ -114,9 +114,8 @@ class Exl3SwitchGlu:
 
     def forward_device(self, d_x: int, x_dtype: int, rows: int, d_selected: int, d_scores: int, score_dtype: int, d_y: int,
                        workspace: DeviceBuffer, stream: Stream = DEFAULT_STREAM) -> None:
-        _lib.call("b200exl3_moe_forward", c_void_p(self.handle), c_void_p(d_x), x_dtype, rows, c_void_p(d_selected),
-                  c_void_p(d_scores), score_dtype, c_void_p(d_y), c_void_p(workspace.ptr), workspace.nbytes,
-                  c_void_p(stream.handle))
+        _lib.call("b200exl3_moe_forward", self.handle, d_x, x_dtype, rows, d_selected, d_scores, score_dtype, d_y, workspace.ptr,
+                  workspace.nbytes, stream.handle)
 
     def forward(self, x: np.ndarray, selected: np.ndarray, scores: np.ndarray, dtype: int | None = None,
                 stream: Stream = DEFAULT_STREAM) -> np.ndarray:
@@ -131,16 +130,18 @@ class Exl3SwitchGlu:
         if scores.dtype not in (np.float16, np.float32):
             raise B200Exl3Error("routing weights must be float16 or float32")
         score_code = F16 if scores.dtype == np.float16 else F32
-        d_x = DeviceBuffer.from_numpy(x, stream)
-        d_sel = DeviceBuffer.from_numpy(selected.astype(np.uint32, copy=False), stream)
-        d_scores = DeviceBuffer.from_numpy(scores, stream)
-        d_y = DeviceBuffer(rows * self.input * scores.dtype.itemsize)
         need = self.workspace_bytes(rows)
         if self._workspace is None or self._workspace.nbytes < need:
             self._workspace = new_workspace(need)
-        self.forward_device(d_x.ptr, dtype_code(x, dtype), rows, d_sel.ptr, d_scores.ptr, score_code, d_y.ptr,
-                            self._workspace, stream)
-        return d_y.download((rows, self.input), scores.dtype, stream)
+        code = dtype_code(x, dtype)
+        arrays = [np.ascontiguousarray(x), np.ascontiguousarray(selected.astype(np.uint32, copy=False)), np.ascontiguousarray(scores)]
+        *at, at_y, end = Scratch.offsets(*(a.nbytes for a in arrays), rows * self.input * scores.dtype.itemsize)
+        with Scratch(end, stream) as s:
+            for a, offset in zip(arrays, at):
+                s.upload(a, offset)
+            d_x, d_sel, d_scores = (s.ptr + offset for offset in at)
+            self.forward_device(d_x, code, rows, d_sel, d_scores, score_code, s.ptr + at_y, self._workspace, stream)
+            return s.download((rows, self.input), scores.dtype, at_y)
 
     def close(self) -> None:
         if getattr(self, "handle", None):

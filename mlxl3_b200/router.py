@@ -7,7 +7,7 @@ import numpy as np
 
 from . import _lib
 from ._lib import B200Exl3Error, F16, F32
-from .runtime import DEFAULT_STREAM, DeviceBuffer, Stream
+from .runtime import DEFAULT_STREAM, Scratch, Stream
 
 
 def topk_device(d_values: int, dtype: int, rows: int, experts: int, top_k: int, normalize: bool, d_indices: int,
@@ -26,12 +26,12 @@ def topk(values: np.ndarray, top_k: int, normalize: bool, stream: Stream = DEFAU
     if values.dtype not in (np.float16, np.float32):
         raise B200Exl3Error("native router expects FP16 or FP32 values")
     rows, experts = values.shape
-    d_values = DeviceBuffer.from_numpy(values, stream)
-    d_indices = DeviceBuffer(max(rows * top_k, 1) * 4)
-    d_scores = DeviceBuffer(max(rows * top_k, 1) * values.dtype.itemsize)
-    topk_device(d_values.ptr, F16 if values.dtype == np.float16 else F32, rows, experts, top_k, normalize, d_indices.ptr,
-                d_scores.ptr, stream)
-    return (d_indices.download((rows, top_k), np.uint32, stream), d_scores.download((rows, top_k), values.dtype, stream))
+    slots = max(rows * top_k, 1)
+    at_v, at_i, at_s, end = Scratch.offsets(values.nbytes, slots * 4, slots * values.dtype.itemsize)
+    with Scratch(end, stream) as s:
+        s.upload(values, at_v)
+        topk_device(s.ptr + at_v, F16 if values.dtype == np.float16 else F32, rows, experts, top_k, normalize, s.ptr + at_i, s.ptr + at_s, stream)
+        return s.download((rows, top_k), np.uint32, at_i), s.download((rows, top_k), values.dtype, at_s)
 
 
 def softmax_topk(logits: np.ndarray, top_k: int, normalize: bool = True, stream: Stream = DEFAULT_STREAM):
@@ -43,14 +43,14 @@ def softmax_topk(logits: np.ndarray, top_k: int, normalize: bool = True, stream:
     if logits.dtype not in (np.float16, np.float32):
         raise B200Exl3Error("native router expects FP16 or FP32 values")
     rows, experts = logits.shape
-    d_logits = DeviceBuffer.from_numpy(logits, stream)
-    d_indices = DeviceBuffer(max(rows * top_k, 1) * 4)
-    d_scores = DeviceBuffer(max(rows * top_k, 1) * logits.dtype.itemsize)
-    d_probs = DeviceBuffer(max(logits.nbytes, 1))
-    _lib.call("b200exl3_router_softmax_topk", c_void_p(d_logits.ptr), F16 if logits.dtype == np.float16 else F32, rows, experts,
-              top_k, int(normalize), c_void_p(d_indices.ptr), c_void_p(d_scores.ptr), c_void_p(d_probs.ptr), c_void_p(stream.handle))
-    return (d_indices.download((rows, top_k), np.uint32, stream), d_scores.download((rows, top_k), logits.dtype, stream),
-            d_probs.download((rows, experts), logits.dtype, stream))
+    slots = max(rows * top_k, 1)
+    at_l, at_i, at_s, at_p, end = Scratch.offsets(logits.nbytes, slots * 4, slots * logits.dtype.itemsize, logits.nbytes)
+    with Scratch(end, stream) as s:
+        s.upload(logits, at_l)
+        _lib.call("b200exl3_router_softmax_topk", s.ptr + at_l, F16 if logits.dtype == np.float16 else F32, rows, experts, top_k,
+                  int(normalize), s.ptr + at_i, s.ptr + at_s, s.ptr + at_p, stream.handle)
+        return (s.download((rows, top_k), np.uint32, at_i), s.download((rows, top_k), logits.dtype, at_s),
+                s.download((rows, experts), logits.dtype, at_p))
 
 
 def gate(x: np.ndarray, weight: np.ndarray, stream: Stream = DEFAULT_STREAM) -> np.ndarray:
@@ -60,8 +60,9 @@ def gate(x: np.ndarray, weight: np.ndarray, stream: Stream = DEFAULT_STREAM) -> 
         raise B200Exl3Error("invalid router gate dimensions")
     rows, n_in = x.shape
     experts = weight.shape[0]
-    d_x, d_w = DeviceBuffer.from_numpy(x, stream), DeviceBuffer.from_numpy(weight, stream)
-    d_logits = DeviceBuffer(rows * experts * 2)
-    _lib.call("b200exl3_router_gate", c_void_p(d_x.ptr), F16, c_void_p(d_w.ptr), rows, n_in, experts, c_void_p(d_logits.ptr),
-              c_void_p(stream.handle))
-    return d_logits.download((rows, experts), np.float16, stream)
+    at_x, at_w, at_l, end = Scratch.offsets(x.nbytes, weight.nbytes, rows * experts * 2)
+    with Scratch(end, stream) as s:
+        s.upload(x, at_x)
+        s.upload(weight, at_w)
+        _lib.call("b200exl3_router_gate", s.ptr + at_x, F16, s.ptr + at_w, rows, n_in, experts, s.ptr + at_l, stream.handle)
+        return s.download((rows, experts), np.float16, at_l)

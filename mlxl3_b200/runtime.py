@@ -35,7 +35,7 @@ class Stream:
         self.handle = handle
 
     def sync(self) -> None:
-        _lib.call("b200exl3_stream_sync", c_void_p(self.handle))
+        _lib.call("b200exl3_stream_sync", self.handle)
 
     def close(self) -> None:
         if self._own and self.handle:
@@ -97,15 +97,13 @@ class DeviceBuffer:
         a = np.ascontiguousarray(array)
         if offset + a.nbytes > self.nbytes:
             raise ValueError("upload exceeds the device buffer")
-        _lib.call("b200exl3_memcpy_h2d", c_void_p(self.ptr + offset), a.ctypes.data_as(c_void_p), a.nbytes,
-                  c_void_p(stream.handle))
+        _lib.call("b200exl3_memcpy_h2d", self.ptr + offset, a.ctypes.data, a.nbytes, stream.handle)
 
     def download(self, shape, dtype, stream: Stream = DEFAULT_STREAM, offset: int = 0) -> np.ndarray:
         out = np.empty(shape, dtype)
         if offset + out.nbytes > self.nbytes:
             raise ValueError("download exceeds the device buffer")
-        _lib.call("b200exl3_memcpy_d2h", out.ctypes.data_as(c_void_p), c_void_p(self.ptr + offset), out.nbytes,
-                  c_void_p(stream.handle))
+        _lib.call("b200exl3_memcpy_d2h", out.ctypes.data, self.ptr + offset, out.nbytes, stream.handle)
         stream.sync()
         return out
 
@@ -122,6 +120,62 @@ class DeviceBuffer:
             self.free()
         except Exception:
             pass
+
+
+class Scratch:
+    """Device memory for one call with host arrays in and out: ``with Scratch(nbytes, stream) as s``.  The block comes from
+    the library's bounded pool and goes back to it at the end of the block, when the stream has been waited for (the last
+    ``download`` did that; after an exception it is done here), so a call allocates nothing once its sizes were seen."""
+
+    __slots__ = ("ptr", "host", "nbytes", "stream")
+
+    def __init__(self, nbytes: int, stream: "Stream" = DEFAULT_STREAM):
+        p, host = c_void_p(), c_void_p()
+        _lib.call("b200exl3_scratch_acquire", max(int(nbytes), 1), byref(p), byref(host))
+        self.ptr, self.host, self.nbytes, self.stream = p.value, host.value, int(nbytes), stream
+
+    @staticmethod
+    def offsets(*sizes: int) -> list[int]:
+        """Places of arrays of these sizes one after the other, each on a 256-byte boundary, and the end of the last."""
+        at, out = 0, []
+        for n in sizes:
+            out.append(at)
+            at += (int(n) + 255) // 256 * 256
+        return out + [at]
+
+    def upload(self, array: np.ndarray, offset: int = 0) -> None:
+        """Queues the copy; the array has to stay as it is until the stream has been waited for."""
+        a = np.ascontiguousarray(array)
+        if offset + a.nbytes > self.nbytes:
+            raise ValueError("upload exceeds the scratch block")
+        source = a.ctypes.data
+        if self.host:                           # through page-locked memory: nothing for the driver to stage
+            ctypes.memmove(self.host + offset, source, a.nbytes)
+            source = self.host + offset
+        _lib.call("b200exl3_memcpy_h2d", self.ptr + offset, source, a.nbytes, self.stream.handle)
+        if a is not array and not self.host:
+            self.stream.sync()                  # the copy made here goes away
+
+    def download(self, shape, dtype, offset: int = 0) -> np.ndarray:
+        out = np.empty(shape, dtype)
+        if offset + out.nbytes > self.nbytes:
+            raise ValueError("download exceeds the scratch block")
+        target = self.host + offset if self.host else out.ctypes.data
+        _lib.call("b200exl3_memcpy_d2h", target, self.ptr + offset, out.nbytes, self.stream.handle)
+        self.stream.sync()
+        if self.host:
+            ctypes.memmove(out.ctypes.data, target, out.nbytes)
+        return out
+
+    def __enter__(self) -> "Scratch":
+        return self
+
+    def __exit__(self, exc_type, exc, tb) -> None:
+        try:
+            if exc_type is not None:
+                self.stream.sync()
+        finally:
+            _lib.call("b200exl3_scratch_release", self.ptr)
 
 
 class PinnedBuffer:
@@ -179,7 +233,7 @@ class Graph:
             self.handle = h.value
 
     def launch(self, stream: Stream) -> None:
-        _lib.call("b200exl3_graph_launch", c_void_p(self.handle), c_void_p(stream.handle))
+        _lib.call("b200exl3_graph_launch", self.handle, stream.handle)
 
     def __del__(self):
         try:

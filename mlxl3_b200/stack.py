@@ -57,7 +57,7 @@ class Exl3Stack:
         self.count, self.rows = len(ops), rows
 
     def forward(self, stream: Stream = DEFAULT_STREAM) -> None:
-        _lib.call("b200exl3_stack_forward", c_void_p(self.handle), c_void_p(stream.handle))
+        _lib.call("b200exl3_stack_forward", self.handle, stream.handle)
 
     def status(self) -> int:
         out = c_int()
