@@ -197,8 +197,10 @@ int b200exl3_plan_query(const char* kind, int in, int out, int k, int64_t rows, 
         return 0;
     }
     if (!strcmp(kind, "qmm")) {
-        const QmmPlan p = plan_qmm(in, out, rows);   // rows of a pass in tiles of 512, each in halves of up to 256
-        out_values[0] = p.splits; out_values[1] = p.token_tiles; out_values[2] = p.small ? 1 : 0; out_values[3] = in / 64;
+        // tiles of 512 rows are a unit of the report only: the launch takes smaller ones where that is faster
+        out_values[0] = 1; out_values[1] = rows <= 64 ? 1 : (rows + 511) / 512; out_values[2] = rows <= 64 ? 1 : 0; out_values[3] = in / 64;
+        const QmmPlan p = plan_qmm(in, out, rows);
+        out_values[4] = p.tile_tokens; out_values[5] = p.splits; out_values[6] = p.pass_rows; out_values[7] = static_cast<int64_t>(p.piece_bytes);
         return 0;
     }
     if (!strcmp(kind, "stack")) {

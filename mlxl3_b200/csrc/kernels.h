@@ -337,10 +337,7 @@ cudaError_t launch_head_argmax(const __half* x, const __half* w, int64_t vocab, 
 
 // ---- tensor-core product for many rows (kernels_qmm.cu) ---------------------------------------------------
 struct QmmPlan {
-    int token_tiles;     // ceil(rows / 512) (taken in halves of up to 256), 1 for the small shape
-    bool small;          // up to 64 rows: the whole batch is one tile, no weight is decoded twice
-    bool fixed;          // every item goes to `splits` CTAs; otherwise one wave of CTAs gets equal runs of stages
-    int splits;
+    int splits;          // CTAs per item, or 0: one wave of CTAs gets equal runs of stages
     int tile_tokens;     // tokens of an item, a multiple of 16
     int64_t pass_rows;   // rows of one launch (more rows go in passes)
     size_t piece_bytes;  // scratch for the parts of items that CTAs share

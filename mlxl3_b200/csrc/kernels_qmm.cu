@@ -607,37 +607,66 @@ std::atomic<unsigned long long*> g_qmm_trace{nullptr};
 static std::atomic<int> g_qmm_splits{0};                              // 0 = one wave of CTAs with equal runs of stages
 void qmm_set_tuning(int splits) { g_qmm_splits = splits > 0 ? splits : 0; }
 
-constexpr int64_t kQmmSmallMaxRows = 64;     // one token tile: a second one would decode every weight twice
-
-// CTAs of a launch over `items` items: one wave of equal runs, at least one stage each (below that a CTA would only add a
-// piece to be summed), or as many per item as asked for.
+// CTAs of a launch over `items` items of `stages` stages: the same number for every item, or one wave of equal runs.
 static int64_t qmm_grid(const QmmPlan& plan, int64_t items, int64_t stages) {
-    return plan.fixed ? items * plan.splits : std::max<int64_t>(1, std::min<int64_t>(sm_count(), items * stages));
+    return plan.splits > 0 ? items * plan.splits : std::min<int64_t>(sm_count(), items * stages);
 }
-
 static size_t qmm_piece_count(int64_t items, int64_t grid) { return static_cast<size_t>(items < grid ? grid + items : 2 * grid); }
 
-QmmPlan plan_qmm(int in, int out, int64_t rows, bool whole_items) {
+// How a batch is cut up: tokens per item and CTAs per item (or one wave of equal runs).  The estimate below is fitted to 474
+// measured launches (512 to 25600 inputs or outputs, 10 to 2000 rows; 10 % rms, its choice 4 % above the best measured one
+// on average): a fixed part; a stage, mostly decode, with a share that grows with the tokens; the epilogue of
+// every item or part of one; parts that are written, counted and read again by the last CTA; and a run that starts in one
+// item and ends in another.  So small tiles (every tile decodes the weights again) win where the layer alone gives the SMs
+// too little to do: 256 rows of 2048 -> 2048 take 15.7 us as 4 tiles of 64 rows and 39 as one tile in 148 equal runs.
+static double qmm_cost_us(int64_t sms, int64_t items, int64_t stages, int tile, int64_t splits) {
+    const int64_t grid = splits > 0 ? items * splits : std::min(sms, items * stages);
+    const int64_t waves = (grid + sms - 1) / sms, run = splits > 0 ? (stages + splits - 1) / splits : (items * stages + grid - 1) / grid;
+    const double parts = splits > 0 ? static_cast<double>(splits) : static_cast<double>(items < grid ? (grid + items - 1) / items + 1 : 2);
+    const double ends = splits > 0 ? 1.0 : static_cast<double>((run + stages - 1) / stages + 1);
+    return 4.6 + waves * (run * (0.548 + 0.0017 * tile) + ends * 0.03 * tile) + (parts > 1 ? 2.0 + 0.15 * parts + 0.0064 * tile * parts : 0.0) +
+           (splits > 0 ? 0.0 : 3.0);
+}
+
+static QmmPlan make_qmm_plan(int in, int out, int64_t rows, bool whole_items, int forced, int64_t sms) {
     QmmPlan plan{};
-    plan.small = rows <= kQmmSmallMaxRows;
-    plan.token_tiles = static_cast<int>(plan.small ? 1 : (rows + 511) / 512);
-    const int nt = plan.small ? 64 : 256;
-    const int col_blocks = out / 128, stages = in / kStageIn;
+    const int64_t col_blocks = out / 128, stages = in / kStageIn;
     // the items of one launch need an arrival counter each, and stages x CTAs must fit 32 bits: more rows go in passes
-    const int64_t max_items = std::min<int64_t>(4000, (int64_t{1} << 31) / (static_cast<int64_t>(stages) * 1024));
+    const int64_t max_items = std::min<int64_t>(4000, (int64_t{1} << 31) / (stages * 1024));
     const int64_t max_tiles = std::max<int64_t>(1, max_items / col_blocks);
-    const int64_t tiles = (rows + nt - 1) / nt;
-    const int64_t passes = (tiles + max_tiles - 1) / max_tiles;
-    plan.pass_rows = passes == 1 ? rows : max_tiles * nt;
-    const int64_t pass_tiles = std::min(tiles, max_tiles);
-    // equal tiles of whole sixteens: N of the MMA is a multiple of 16
-    plan.tile_tokens = static_cast<int>(((std::min(rows, plan.pass_rows) + pass_tiles - 1) / pass_tiles + 15) / 16 * 16);
-    const int64_t items = pass_tiles * col_blocks;
-    const int forced = g_qmm_splits.load();
-    plan.fixed = whole_items || forced > 0;
-    plan.splits = whole_items || !forced ? 1 : std::max(1, std::min(forced, stages / 4));
-    plan.piece_bytes = plan.fixed && plan.splits == 1 ? 256 : qmm_piece_count(items, qmm_grid(plan, items, stages)) * plan.tile_tokens * 128 * sizeof(float);
+    plan.pass_rows = std::min(rows, max_tiles * 256);
+    double best = 0;
+    for (const int target : {16, 32, 64, 96, 128, 192, 256}) {
+        const int64_t tiles = (plan.pass_rows + target - 1) / target;
+        if (tiles > max_tiles) continue;
+        // equal tiles of whole sixteens: N of the MMA is a multiple of 16
+        const int tile = static_cast<int>(((plan.pass_rows + tiles - 1) / tiles + 15) / 16 * 16);
+        const int64_t items = tiles * col_blocks;
+        auto consider = [&](int64_t splits) {
+            const double t = qmm_cost_us(sms, items, stages, tile, splits);
+            if (best == 0 || t < best) { best = t; plan.tile_tokens = tile; plan.splits = static_cast<int>(splits); }
+        };
+        if (whole_items) consider(1);
+        else if (forced) consider(std::max<int64_t>(1, std::min<int64_t>(forced, stages)));
+        else {
+            for (int64_t splits = 1; splits <= stages && items * splits <= sms; ++splits) consider(splits);
+            consider(0);
+        }
+    }
+    const int64_t items = (plan.pass_rows + plan.tile_tokens - 1) / plan.tile_tokens * col_blocks;
+    plan.piece_bytes = plan.splits == 1 ? 256 : qmm_piece_count(items, qmm_grid(plan, items, stages)) * plan.tile_tokens * 128 * sizeof(float);
     return plan;
+}
+
+// Weighing the choices takes a few microseconds of the host and a call asks twice: a thread remembers its last plans.
+QmmPlan plan_qmm(int in, int out, int64_t rows, bool whole_items) {
+    struct Entry { int in, out, forced, sms; int64_t rows; bool whole; QmmPlan plan; };
+    thread_local Entry cache[64] = {};
+    const int forced = g_qmm_splits.load(), sms = sm_count();
+    Entry& e = cache[(static_cast<unsigned>(in) / 128 * 7 + static_cast<unsigned>(out) / 128 * 3 + static_cast<unsigned>(rows)) % 64];
+    if (e.in != in || e.out != out || e.rows != rows || e.whole != whole_items || e.forced != forced || e.sms != sms)
+        e = {in, out, forced, sms, rows, whole_items, make_qmm_plan(in, out, rows, whole_items, forced, sms)};
+    return e.plan;
 }
 
 cudaError_t launch_qmm(QmmArgs p, const __half* xhat, int k, int cb, const QmmPlan& plan, cudaStream_t stream) {
@@ -650,7 +679,7 @@ cudaError_t launch_qmm(QmmArgs p, const __half* xhat, int k, int cb, const QmmPl
     p.trace = g_qmm_trace.load();
     const int64_t stages = p.in / kStageIn, grid = qmm_grid(plan, p.items, stages);
     if (p.items * stages * grid >= (int64_t{1} << 32)) return cudaErrorInvalidValue;
-    return qmm_dispatch(k, cb, map, p, static_cast<int>(grid), plan.small, stream);
+    return qmm_dispatch(k, cb, map, p, static_cast<int>(grid), plan.tile_tokens <= 64, stream);
 }
 
 size_t qmm_mapped_piece_bytes() { return static_cast<size_t>(sm_count()) * 2 * kQmmSegRows * 128 * sizeof(float); }
