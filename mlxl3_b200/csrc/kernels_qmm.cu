@@ -138,7 +138,13 @@ __device__ __noinline__ bool qmm_wait_slow(uint64_t* bar, uint32_t parity, volat
 __device__ __forceinline__ bool qmm_wait(uint64_t* bar, uint32_t parity, volatile int* cta_failed) {
     return mbar_try_wait(bar, parity) || qmm_wait_slow(bar, parity, cta_failed);
 }
-__device__ __forceinline__ void group_sync(int id, int threads) { asm volatile("barrier.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+// Barrier of some warps.  Lanes may come from, and leave, the barrier one by one; the tcgen05 instructions around it want
+// the warp as one, which the warp barriers state.
+__device__ __forceinline__ void group_sync(int id, int threads) {
+    __syncwarp();
+    asm volatile("barrier.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+    __syncwarp();
+}
 
 // What an item is: where its weights, its activation rows and its outputs are.
 struct QmmItem {
@@ -289,6 +295,7 @@ qmm_kernel(const __grid_constant__ CUtensorMap xmap, const QmmArgs p) {
         s_failed = 0;
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
+    __syncwarp();                                                // thread 0 comes from a branch of its own
     if (warp == kMmaWarp) tmem_alloc(&tmem_base_slot, 512);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -386,6 +393,7 @@ qmm_kernel(const __grid_constant__ CUtensorMap xmap, const QmmArgs p) {
             // chunks of 16 tokens: four warps hold 32 columns each of the same tokens
             for (int c = quad * kChunk; c < info.n; c += S::kDecoders / 4 * kChunk) {
                 uint32_t r[16];
+                __syncwarp();
                 tmem_ld16(lanes + c, r);
                 if (!complete || p.yhat != nullptr) {
                     float* dst = complete ? p.yhat + static_cast<int64_t>(info.tok0 + c) * p.yhat_ld + info.cblock * 128 + quarter * 32 + lane
@@ -400,7 +408,6 @@ qmm_kernel(const __grid_constant__ CUtensorMap xmap, const QmmArgs p) {
                     __half* stage = stage_base + (quad * 2 + buf) * (kChunk * 128);
 #pragma unroll
                     for (int i = 0; i < kChunk; ++i) stage[i * 128 + stage_col(quarter * 32 + lane)] = __float2half_rn(__uint_as_float(r[i]));
-                    __syncwarp();
                     group_sync(1 + quad, 128);
                     if (c + quarter * 4 < info.n)
                         qmm_finish4(stage + quarter * 512, p, store, info.tok0 + c + quarter * 4, info.n - c - quarter * 4, lane);
@@ -422,7 +429,6 @@ qmm_kernel(const __grid_constant__ CUtensorMap xmap, const QmmArgs p) {
                     s_last = before == c_last - c_first;
                     if (s_last) p.counters[item] = 0;            // leave the scratch ready for the next call
                 }
-                __syncwarp();
                 group_sync(8, S::kDecoders * 32);
                 if (s_last) {
                     __threadfence();
@@ -488,7 +494,6 @@ qmm_kernel(const __grid_constant__ CUtensorMap xmap, const QmmArgs p) {
                                 qmm_finish4(mine, p, store, info.tok0 + t0, info.n - t0, lane);
                             }
                         }
-                        __syncwarp();
                         group_sync(8, S::kDecoders * 32);        // the next item stages in other warps' rows
                     }
                 }
@@ -615,6 +620,7 @@ qmm_kernel(const __grid_constant__ CUtensorMap xmap, const QmmArgs p) {
         const unsigned long long t0 = global_ns();
         while (global_ns() - t0 < 2000000ull) __nanosleep(1000);
     }
+    __syncwarp();
     if (warp == kMmaWarp) tmem_dealloc(tmem, 512);
     if (threadIdx.x == 0 && s_failed) {
         pdl_wait();
