@@ -86,3 +86,19 @@ def test_array_calls_from_several_threads_share_the_pool(gpu):
     for t in threads:
         t.join()
     assert not failures, failures
+
+
+@pytest.mark.parametrize("k", [5, 7, 8])
+@pytest.mark.parametrize("rows", [48, 260])
+def test_long_runs_of_wide_weights(gpu, k, rows):
+    """Every CTA's run goes round the ring of packed stages many times and through several items."""
+    rng = np.random.default_rng(k * rows)
+    trellis, suh, svh = random_layer(rng, 2048, 3200, k)
+    layer = gpu.Exl3Linear(trellis, suh, svh, None, k, 0)
+    x = rng.standard_normal((rows, 2048)).astype(np.float16)
+    got = layer.forward(x)
+    for _ in range(10):
+        assert np.array_equal(bits(layer.forward(x)), bits(got))
+    pick = np.unique([0, rows // 2, rows - 1])
+    _close(got[pick], oracle.linear_forward(trellis, k, 0, suh, svh, None, x[pick]))
+    layer.close()
