@@ -483,7 +483,7 @@ static QmmLayout qmm_layout(const LayerCore& c, int64_t rows, bool whole_items =
 static int core_workspace_bytes(const LayerCore& c, int64_t rows, size_t* out_bytes) {
     if (!out_bytes) return fail("NULL argument");
     if (rows <= 0) return fail("EXL3 linear input cannot be empty");
-    QmvPlan plan = plan_qmv(c.in, c.out, c.k, rows);
+    const QmvPlan plan = plan_qmv(c.in, c.out, c.k, rows, true);             // the larger of the two grids
     size_t bytes = kCounterBytes + qmv_partial_bytes(plan, c.out, rows) + xhat_bytes(c, rows);
     if (rows >= kQmmMinRows) bytes = std::max(bytes, qmm_layout(c, rows).total);
     *out_bytes = bytes;
@@ -561,7 +561,7 @@ static int forward_common(const LayerCore& c, const void* d_x, int x_dtype, cons
     }
     for (int64_t r0 = 0; r0 < rows; r0 += kMaxBatchRows) {
         const int64_t n = rows - r0 < kMaxBatchRows ? rows - r0 : kMaxBatchRows;
-        const QmvPlan plan = plan_qmv(c.in, c.out, c.k, n);
+        const QmvPlan plan = plan_qmv(c.in, c.out, c.k, n, pro != nullptr);
         QmvArgs a{};
         a.wq = c.wq;
         a.x = !xhat ? static_cast<const char*>(d_x) + static_cast<size_t>(r0) * c.in * x_size : nullptr;
@@ -1039,8 +1039,8 @@ struct MoeLayout {
 static MoeLayout moe_layout(const b200exl3_moe* h, int64_t rows) {
     MoeLayout l{};
     const int64_t slots = std::min(rows, moe_chunk_rows(h)) * h->top_k;
-    l.gu_plan = plan_qmv(h->in, static_cast<int>(slots * 2 * h->hidden), h->k, 1);
-    l.down_plan = plan_qmv(h->hidden, static_cast<int>(slots * h->in), h->k, 1);
+    l.gu_plan = plan_qmv(h->in, static_cast<int>(slots * 2 * h->hidden), h->k, 1, true);
+    l.down_plan = plan_qmv(h->hidden, static_cast<int>(slots * h->in), h->k, 1, true);
     size_t at = kCounterBytes;
     l.xgu = at; at += round256(static_cast<size_t>(slots) * 2 * h->in * sizeof(__half));
     l.ygu = at; at += round256(static_cast<size_t>(slots) * 2 * h->hidden * sizeof(float));
@@ -1262,7 +1262,7 @@ int b200exl3_moe_forward(const b200exl3_moe* h, const void* d_x, int x_dtype, in
             a.tiles_n = h->experts * proj * width / 16;
             a.map_selected = sel; a.map_blocks = width / 128; a.map_proj = proj; a.map_stride_blocks = stride_blocks;
             a.map_experts = h->experts;
-            return launch_qmv(a, h->k, h->cb, exact, plan_qmv(in, out, h->k, 1), stream);
+            return launch_qmv(a, h->k, h->cb, exact, plan_qmv(in, out, h->k, 1, true), stream);
         };
         // gate/up: the kernel rotates each slot's token row itself, with the input scales of the slot's expert
         B200_TRY(mapped(h->gu_wq, nullptr, h->in, h->hidden, 2, h->experts * (h->hidden / 128), ygu), "expert gate/up kernel");
@@ -1288,7 +1288,7 @@ int b200exl3_moe_forward(const b200exl3_moe* h, const void* d_x, int x_dtype, in
             a.in = h->hidden; a.out = out; a.rows = 1;
             a.tiles_n = h->experts * h->in / 16;
             a.map_selected = sel; a.map_blocks = h->in / 128; a.map_proj = 1; a.map_stride_blocks = 0; a.map_experts = h->experts;
-            B200_TRY(launch_qmv(a, h->k, h->cb, exact, plan_qmv(h->hidden, out, h->k, 1), stream), "expert down kernel");
+            B200_TRY(launch_qmv(a, h->k, h->cb, exact, plan_qmv(h->hidden, out, h->k, 1, true), stream), "expert down kernel");
             continue;
         }
         B200_TRY(launch_glu_down_input(ygu, h->gu_svh, h->down_suh, sel, h->experts, slots, h->hidden, h->hidden, xdown, stream),
@@ -1333,7 +1333,7 @@ int b200exl3_expert_mapped(const void* d_x, int x_dtype, const uint16_t* d_trell
     float* raw = nullptr;
     char* ws = nullptr;
     const size_t bank_bytes = static_cast<size_t>(in / 16) * source_tiles * 16 * k * sizeof(uint16_t);
-    const QmvPlan plan = plan_qmv(in, static_cast<int>(std::min(pass_slots, slots) * projections * out), k, 1);
+    const QmvPlan plan = plan_qmv(in, static_cast<int>(std::min(pass_slots, slots) * projections * out), k, 1, true);
     const size_t ws_bytes = kCounterBytes + qmv_partial_bytes(plan, static_cast<int>(std::min(pass_slots, slots) * projections * out), 1);
     int rc = check(cudaMalloc(&wq, bank_bytes), "cudaMalloc(bank)");
     if (!rc) rc = check(cudaMalloc(&xhat, static_cast<size_t>(rows) * in * sizeof(__half)), "cudaMalloc(rows)");
@@ -1362,7 +1362,7 @@ int b200exl3_expert_mapped(const void* d_x, int x_dtype, const uint16_t* d_trell
         a.tiles_n = static_cast<int>(source_tiles);
         a.map_selected = d_selected + s0; a.map_blocks = out / 128; a.map_proj = projections;
         a.map_stride_blocks = static_cast<int>(projection_stride_tiles / 8); a.map_experts = static_cast<int>(experts);
-        rc = check(launch_qmv(a, k, cb, true, plan_qmv(in, vout, k, 1), stream), "expert-mapped kernel");
+        rc = check(launch_qmv(a, k, cb, true, plan_qmv(in, vout, k, 1, true), stream), "expert-mapped kernel");
     }
     if (!rc && !return_raw)
         rc = check(launch_finish(raw, 1, rows * out, reinterpret_cast<const __half*>(d_svh), rows, nullptr, rows, out, x_dtype, d_out, stream), "finish");
@@ -1500,8 +1500,8 @@ struct MoeEpLayout {
 
 static MoeEpLayout moe_ep_layout(const b200exl3_moe* h, int64_t slots) {
     MoeEpLayout l{};
-    l.gu_plan = plan_qmv(h->in, static_cast<int>(slots * 2 * h->hidden), h->k, 1);
-    l.down_plan = plan_qmv(h->hidden, static_cast<int>(slots * h->in), h->k, 1);
+    l.gu_plan = plan_qmv(h->in, static_cast<int>(slots * 2 * h->hidden), h->k, 1, true);
+    l.down_plan = plan_qmv(h->hidden, static_cast<int>(slots * h->in), h->k, 1, true);
     size_t at = kCounterBytes;
     l.local_count = at; at += 256;
     l.local_slot = at; at += round256(static_cast<size_t>(slots) * sizeof(uint32_t));
@@ -1574,7 +1574,7 @@ int b200exl3_moe_forward_ep(const b200exl3_moe* h, b200exl3_ep* ep, int first_ex
             a.tiles_n = h->experts * proj * width / 16;
             a.map_selected = local_expert; a.map_count = local_count;
             a.map_blocks = width / 128; a.map_proj = proj; a.map_stride_blocks = stride_blocks; a.map_experts = h->experts;
-            return launch_qmv(a, h->k, h->cb, exact, plan_qmv(in, out, h->k, 1), stream);
+            return launch_qmv(a, h->k, h->cb, exact, plan_qmv(in, out, h->k, 1, true), stream);
         };
         B200_TRY(launch_ep_plan(sel, slots, first_expert, h->experts, local_count, local_slot, local_expert, stream), "expert plan");
         B200_TRY(launch_ep_dispatch(static_cast<const char*>(d_x) + static_cast<size_t>(r0) * h->in * x_size, x_dtype, h->gu_suh, local_count,

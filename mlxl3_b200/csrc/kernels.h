@@ -150,7 +150,7 @@ struct QmvPlan {
     bool pdl;            // launch with programmatic stream serialization (overlap with the previous kernel's tail)
     bool pdl_early;      // trigger the dependent launch before the main loop instead of after it
 };
-QmvPlan plan_qmv(int in, int out, int k, int64_t rows);
+QmvPlan plan_qmv(int in, int out, int k, int64_t rows, bool full_grid = false);
 // Scratch a launch needs: counters first (zero-initialised once by the owner), then the partial sums.
 size_t qmv_partial_bytes(const QmvPlan& plan, int out, int64_t rows);
 // exact: decode the reference's fp16 weight bit for bit before multiplying (codebooks 0/1 default to

@@ -53,21 +53,45 @@ void qmv_set_tuning(int ctas_per_sm, int force_grid, int pdl) {
 static std::atomic<unsigned long long*> g_trace{nullptr};
 void qmv_set_trace(unsigned long long* device_buffer) { g_trace = device_buffer; }
 
-QmvPlan plan_qmv(int in, int out, int k, int64_t rows) {
+QmvPlan plan_qmv(int in, int out, int k, int64_t rows, bool full_grid) {
     QmvPlan plan{};
     plan.col_blocks = out / 128;
     const int tiles_k = in / 16;
     const int r = static_cast<int>(std::min<int64_t>(rows, kQmvMaxRows));
     const int forced = g_force_grid.load();
     const int64_t rb = tiles_k, rt = rb * plan.col_blocks;
-    // CTAs for `resident` of them per SM
+    // CTAs of a layer, for `resident` of them per SM
     auto grid_for = [&](int resident) {
-        int64_t grid = forced > 0 ? forced : static_cast<int64_t>(sm_count()) * resident;
+        const int64_t sms = sm_count();
+        int64_t grid = forced > 0 ? forced : sms * resident;
         // the layer is dealt out in whole rows of 8 tiles: no more warps than rows
         grid = std::max<int64_t>(1, std::min(grid, rt / kQmvWarps));
         // a warp's range must not exceed one column block (it then touches at most two blocks)
         const int64_t min_warps = (rt + rb - 2) / (rb - 1) + 1;
-        return static_cast<int>(std::max(grid, (min_warps + kQmvWarps - 1) / kQmvWarps));
+        grid = std::max(grid, (min_warps + kQmvWarps - 1) / kQmvWarps);
+        if (forced > 0 || full_grid) return static_cast<int>(grid);
+        // Against that full grid: m whole CTAs for every column block.  Fewer CTAs share a block, none works on two, and a
+        // warp that holds more rows rotates fewer 128-input blocks twice -- worth more than the last few idle SMs while a
+        // layer is small.  Nanoseconds fitted to 168 sweeps (512..14336 inputs, 512..14336 outputs, 1, 2, 4 and 8 rows, 3, 4
+        // and 6 bits; the choice is 1.5 % above the best grid measured, never more than 1.2 % above the full one): a
+        // row of a warp, a row of an SM, a part of a block, a second CTA on an SM, a 128-input block a warp rotates.  The
+        // row count is left out so that a row's sums are added in the same order in every batch of up to 8.
+        // 4096->4096, 4 bits, 1 row: 12.4 -> 11.4 us; 4096->1024, 2 rows: 15.5 -> 12.5.
+        // `full_grid`: the layers of a decode step and the expert block, whose prologues and neighbours fill the SMs that
+        // this would leave idle (one token of the expert block 31.1 us with the full grid, 31.9 without).
+        auto cost = [&](int64_t ctas, int64_t warp_rows, int64_t sm_rows, int64_t parts, int64_t spans) {
+            return 181 * warp_rows + 42 * sm_rows + 149 * parts + (ctas > sms ? 407 : 0) + 628 * spans;
+        };
+        const int64_t full = grid, rows_w = (rt + full * kQmvWarps - 1) / (full * kQmvWarps);
+        int64_t best = 59 + cost(full, rows_w, (full + sms - 1) / sms * rt / full, (full + plan.col_blocks - 1) / plan.col_blocks + 1, (rows_w + 6) / 8 + 1);
+        for (int64_t m = 1; m <= 64 && m * plan.col_blocks <= sms * resident && m * kQmvWarps <= rb; ++m) {
+            const int64_t ctas = m * plan.col_blocks, warps = m * kQmvWarps, n = (rb + warps - 1) / warps;
+            // a warp's rows start at a 128-input block (8 rows) or divide one, or lie anywhere
+            const int64_t spans = rb % warps == 0 && n % 8 == 0 ? n / 8 : rb % warps == 0 && 8 % n == 0 ? 1 : (n + 6) / 8 + 1;
+            const int64_t t = cost(ctas, n, (ctas + sms - 1) / sms * rb / m, m, spans);
+            if (t < best) { best = t; grid = ctas; }
+        }
+        return static_cast<int>(grid);
     };
     // Per warp: [ring of packed rows | rotated activations | staged result tile of its first block | of its second].  The
     // second tile is staged when the activations are no longer read, so with rows that come rotated it shares their place.
