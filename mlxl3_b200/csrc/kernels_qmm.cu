@@ -708,19 +708,22 @@ static int64_t qmm_grid(const QmmPlan& plan, int64_t items, int64_t stages) {
 }
 static size_t qmm_piece_count(int64_t items, int64_t grid) { return static_cast<size_t>(items < grid ? grid + items : 2 * grid); }
 
-// How a batch is cut up: tokens per item and CTAs per item (or one wave of equal runs).  The estimate below is fitted to 474
-// measured launches (512 to 25600 inputs or outputs, 10 to 2000 rows; 10 % rms, its choice 4 % above the best measured one
-// on average): a fixed part; a stage, mostly decode, with a share that grows with the tokens; the epilogue of
-// every item or part of one; parts that are written, counted and read again by the last CTA; and a run that starts in one
-// item and ends in another.  So small tiles (every tile decodes the weights again) win where the layer alone gives the SMs
-// too little to do: 256 rows of 2048 -> 2048 take 15.7 us as 4 tiles of 64 rows and 39 as one tile in 148 equal runs.
+// How a batch is cut up: tokens per item and CTAs per item (or one wave of equal runs).  The estimate below is fitted to 1160
+// measured launches (512 to 14336 inputs, 512 to 25600 outputs, 16 to 2000 rows, 3, 4 and 6 bits; its choice is 1.2 % above
+// the best measured one on average): a fixed part; a stage, mostly decode, with a share that grows with the tokens and more of
+// both the more SMs are busy (they share the second-level cache and the power); the epilogue of every item or part of one;
+// parts that are written, counted and read again by the last CTA; and a run that starts in one item and ends in another.  So
+// small tiles (every tile decodes the weights again) win where the layer alone gives the SMs too little to do: 256 rows of
+// 2048 -> 2048 take 15.7 us as 4 tiles of 64 rows and 39 as one tile in 148 equal runs.
 static double qmm_cost_us(int64_t sms, int64_t items, int64_t stages, int tile, int64_t splits) {
     const int64_t grid = splits > 0 ? items * splits : std::min(sms, items * stages);
     const int64_t waves = (grid + sms - 1) / sms, run = splits > 0 ? (stages + splits - 1) / splits : (items * stages + grid - 1) / grid;
-    const double parts = splits > 0 ? static_cast<double>(splits) : static_cast<double>(items < grid ? (grid + items - 1) / items + 1 : 2);
-    const double ends = splits > 0 ? 1.0 : static_cast<double>((run + stages - 1) / stages + 1);
-    return 4.6 + waves * (run * (0.548 + 0.0017 * tile) + ends * 0.03 * tile) + (parts > 1 ? 2.0 + 0.15 * parts + 0.0064 * tile * parts : 0.0) +
-           (splits > 0 ? 0.0 : 3.0);
+    const bool whole = splits == 0 && items % grid == 0;                     // equal runs of whole items
+    const double parts = splits > 0 ? static_cast<double>(splits) : whole ? 1.0 : static_cast<double>(items < grid ? (grid + items - 1) / items + 1 : 2);
+    const double ends = splits > 0 ? 1.0 : static_cast<double>(whole ? items / grid : (run + stages - 1) / stages + 1);
+    const double load = static_cast<double>(grid) / static_cast<double>(sms * waves);
+    return 4.4 + 2.24 * load + waves * (run * (0.414 + 0.001 * tile) * (1 + 0.48 * load) + ends * (0.38 + 0.0306 * tile)) +
+           (parts > 1 ? 1.8 + 0.1 * parts + 0.003 * tile * parts : 0.0) + (splits > 0 ? 0.0 : 1.27);
 }
 
 static QmmPlan make_qmm_plan(int in, int out, int64_t rows, bool whole_items, int forced, int64_t sms) {
