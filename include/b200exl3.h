@@ -58,13 +58,13 @@ int b200exl3_version(void);
  * (device address of a uint64 [grid, 8] array that receives nanosecond stamps of each CTA's phases:
  * start, activations visible, rotated, main loop done, warps joined, reduced, finished; 0 = off), "qmm" (0 = batches
  * of more than 8 rows also go through the small-batch kernel (16 rows per launch) instead of the tensor-core product; default 1),
- * "qmm_splits" (input splits of the tensor-core product, 0 = chosen by a cost model; set it before asking for
+ * "qmm_splits" (CTAs per tile of the tensor-core product, 0 = chosen by a cost model; set it before asking for
  * workspace sizes), "moe_sorted" (0 = the expert block runs one row per slot for any batch instead of grouping
  * slots by expert for larger batches; set it before asking for workspace sizes), "moe_fused" (1 = a small batch of the
  * expert block runs its SwiGLU glue and its weighted reduction as the prologue and the epilogue of the down product, two
  * launches instead of four; same bits either way, measured no faster; default 0), "qmm_trace_buffer" (device address of a uint64 [CTAs, 8] array that receives nanosecond
- * stamps of the tensor-core kernel's phases: start, set up, decoders done, MMAs issued, accumulator ready,
- * epilogue done, end, activation copies issued; 0 = off), "tp_wait_ms" (how long a rank waits for the other ranks'
+ * stamps of the tensor-core kernel's phases: start, set up, first epilogue begins, products issued, (unused),
+ * epilogues done, end, activation copies issued; 0 = off), "tp_wait_ms" (how long a rank waits for the other ranks'
  * words inside a tensor- or expert-parallel kernel before it gives up with status 4; default 4000), "stack_wait_ms"
  * (the same bound for every wait inside the decode-step kernel: status 5 = a layer never completed, 6 = a piece of
  * a column block never arrived; default 2000), "stack_trace_buffer" (device address of a uint64
@@ -247,8 +247,7 @@ int b200exl3_moe_workspace_bytes(const b200exl3_moe* handle, int64_t rows, size_
  * fp32 = 10); y [rows, in] in score_dtype (the reference's result dtype: fp16 products promoted by the scores).
  * Small batches run one activation row per (token, choice) slot against the slot's expert's columns.  From 33
  * slots and two slots per expert on, the slots are grouped by expert on the device (the reference's route_plan, native/src/moe.rs:66-182) into
- * segments of 8 rows (fused kernel) or, from 12 slots per expert on, of 64 rows (tensor cores), so that an expert's
- * columns are decoded once per segment; rows are
+ * segments of up to 64 rows (tensor cores), so that an expert's columns are decoded once per segment; rows are
  * processed in passes of at most 16384 slots.  No host synchronisation either way.
  * The workspace follows the rules of the linear layer's workspace. */
 int b200exl3_moe_forward(const b200exl3_moe* handle, const void* d_x, int x_dtype, int64_t rows,
