@@ -271,7 +271,7 @@ qmm_kernel(const __grid_constant__ CUtensorMap xmap, const QmmArgs p) {
     constexpr int kRawWords = 512 * K;                       // a packed stage: 8 tile rows x 2 quads x 32K words
     constexpr uint32_t kRawBytes = kRawWords * 4;
     constexpr int kRaw = raw_slots<K, NT>();
-    __shared__ __align__(8) uint64_t full[S::kSlots], done[S::kSlots], raw_full[kRaw], raw_empty[kRaw];
+    __shared__ __align__(8) uint64_t full[S::kSlots], done[S::kSlots], full2[S::kSlots], half[S::kSlots], raw_full[kRaw], raw_empty[kRaw];
     __shared__ __align__(8) uint64_t accum_full, accum_free;
     __shared__ uint32_t tmem_base_slot, s_last;
     __shared__ volatile int s_failed;
@@ -294,8 +294,9 @@ qmm_kernel(const __grid_constant__ CUtensorMap xmap, const QmmArgs p) {
     __half* stage_base = reinterpret_cast<__half*>(raw_base + kRaw * kRawWords);
 
     if (threadIdx.x == 0) {
-        // a stage is full when its eight decoder warps and its activation copies have arrived
-        for (int s = 0; s < S::kSlots; ++s) { mbar_init(&full[s], 9); mbar_init(&done[s], 1); }
+        // a stage is full when its eight decoder warps and its activation copies have arrived (of a large tile the first half;
+        // the second has a barrier of its own, and so has the end of the first half's products)
+        for (int s = 0; s < S::kSlots; ++s) { mbar_init(&full[s], 9); mbar_init(&done[s], 1); mbar_init(&full2[s], 1); mbar_init(&half[s], 1); }
         for (int s = 0; s < kRaw; ++s) { mbar_init(&raw_full[s], 1); mbar_init(&raw_empty[s], 8); }
         mbar_init(&accum_full, 1);
         mbar_init(&accum_free, S::kDecoders);
@@ -552,14 +553,27 @@ qmm_kernel(const __grid_constant__ CUtensorMap xmap, const QmmArgs p) {
                     // the slot is free once the MMAs of the stage that used it last (kBSlots stages ago) are done
                     constexpr int kB = S::kBSlots;
                     const int before = (s + S::kSlots - kB) % S::kSlots;
-                    if (!qmm_wait(&done[before], s >= kB ? par : par ^ 1u, &s_failed)) { running = false; break; }
                     unsigned char* dst = b_base + (s % kB) * S::kBSlotBytes;
-                    mbar_expect_tx(&full[s], box_bytes);
-                    tma_load_2d(dst, &xmap, x, info.brow, &full[s]);
-                    tma_load_2d(dst + S::kBHalfBytes, &xmap, x + 64, info.brow, &full[s]);
-                    for (int b = 1; b < boxes; ++b) {
-                        tma_load_2d(dst + b * 2048, &xmap, x, info.brow + b * 16, &full[s]);
-                        tma_load_2d(dst + S::kBHalfBytes + b * 2048, &xmap, x + 64, info.brow + b * 16, &full[s]);
+                    const uint32_t before_par = s >= kB ? par : par ^ 1u;
+                    if constexpr (NT > 64) {
+                        // Only two slots fit beside 256 tokens, and a stage of products is shorter than a copy takes: each
+                        // half of a slot is asked for as soon as its own products are done, and multiplied as soon as it
+                        // lands (2000 rows 14336->4096, 3 bits: 283 -> 269 us).
+                        if (!qmm_wait(&half[before], before_par, &s_failed)) { running = false; break; }
+                        mbar_expect_tx(&full[s], box_bytes / 2);
+                        tma_load_2d(dst, &xmap, x, info.brow, &full[s]);
+                        if (!qmm_wait(&done[before], before_par, &s_failed)) { running = false; break; }
+                        mbar_expect_tx(&full2[s], box_bytes / 2);
+                        tma_load_2d(dst + S::kBHalfBytes, &xmap, x + 64, info.brow, &full2[s]);
+                    } else {
+                        if (!qmm_wait(&done[before], before_par, &s_failed)) { running = false; break; }
+                        mbar_expect_tx(&full[s], box_bytes);
+                        tma_load_2d(dst, &xmap, x, info.brow, &full[s]);
+                        tma_load_2d(dst + S::kBHalfBytes, &xmap, x + 64, info.brow, &full[s]);
+                        for (int b = 1; b < boxes; ++b) {
+                            tma_load_2d(dst + b * 2048, &xmap, x, info.brow + b * 16, &full[s]);
+                            tma_load_2d(dst + S::kBHalfBytes + b * 2048, &xmap, x + 64, info.brow + b * 16, &full[s]);
+                        }
                     }
                     x += kStageIn;
                     if (--rem == 0) {
@@ -604,9 +618,16 @@ qmm_kernel(const __grid_constant__ CUtensorMap xmap, const QmmArgs p) {
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint64_t bd = b_desc0 + (s % S::kBSlots) * (S::kBSlotBytes >> 4);
 #pragma unroll
-                    for (int kk = 0; kk < 8; ++kk)                               // 8 x 16 inputs: two halves of 64
+                    for (int kk = 0; kk < 8; ++kk) {                             // 8 x 16 inputs: two halves of 64
+                        if (NT > 64 && kk == 4) {
+                            umma_commit(&half[s]);
+                            if (!qmm_wait(&full2[s], par, &s_failed)) { running = false; break; }
+                            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                        }
                         umma_f16_ts(tmem, tmem + NT + s * kStageCols + kk * 8, bd + (kk >> 2) * (S::kBHalfBytes >> 4) + (kk & 3) * 2, idesc,
                                     kk > 0 ? 1u : accumulate);
+                    }
+                    if (NT > 64 && !running) break;
                     accumulate = 1;
                     umma_commit(&done[s]);                                       // A stage and activation slot free once these MMAs have read them
                     --rem;
