@@ -345,6 +345,9 @@ qmm_kernel(const __grid_constant__ CUtensorMap xmap, const QmmArgs p) {
                     if (!__all_sync(0xffffffffu, ready)) break;
                 }
                 __syncwarp();
+                // the products that read this A stage last are done (two lanes saw it, the warp barrier passed it on): the
+                // stores below come after them
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t* rw = words + rslot * kRawWords;
                 const uint32_t dst = lanes + NT + rows4 * 32 + slot * kStageCols;
                 uint64_t* stage_full = &full[slot];
@@ -642,6 +645,7 @@ qmm_kernel(const __grid_constant__ CUtensorMap xmap, const QmmArgs p) {
     __syncwarp();
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");   // every warp's last access before the memory is given back
     if (tr && threadIdx.x == 0) tr[6] = global_ns();
     if (s_failed) {
         // copies that were still in flight when a wait gave up must land before the CTA's shared memory is released
