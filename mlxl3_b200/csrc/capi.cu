@@ -468,15 +468,24 @@ static size_t xhat_bytes(const LayerCore& c, int64_t rows) {
 // output rotation in its epilogue) instead of the fused kernel, whose two-block form takes twice its one-block form's time.
 constexpr int64_t kQmmMinRows = 9;
 
+// Rows of a row shard that one pass of the tensor-core path takes: their fp32 sums lie in the workspace until the exchange
+// with the other ranks has added them, at most 32 MiB of them (or 256 rows' worth).  It depends on the width alone, so that
+// all ranks cut a call alike, and is a multiple of the 256 tokens a tile holds, so that a pass decodes no weight more often.
+constexpr size_t kShardSumBytes = size_t(32) << 20;
+static int64_t shard_pass_rows(int out) {
+    return std::max<int64_t>(256, static_cast<int64_t>(kShardSumBytes / (static_cast<size_t>(out) * sizeof(float))) / 256 * 256);
+}
+
 // tensor-core path: [counters | rotated rows of a pass, once per member | pieces of shared items | fp32 sums of a row shard]
 struct QmmLayout { QmmPlan plan; size_t xhat, pieces, sums, total; };
-static QmmLayout qmm_layout(const LayerCore& c, int64_t rows, bool whole_items = false) {
+static QmmLayout qmm_layout(const LayerCore& c, int64_t rows, bool whole_items = false, bool row_shard = false) {
     QmmLayout l;
+    if (row_shard) rows = std::min(rows, shard_pass_rows(c.out));
     l.plan = plan_qmm(c.in, c.out, rows, whole_items);
     l.xhat = kCounterBytes;
     l.pieces = l.xhat + xhat_bytes(c, std::min(rows, l.plan.pass_rows));
     l.sums = l.pieces + round256(l.plan.piece_bytes);
-    l.total = l.sums + (whole_items ? 0 : round256(static_cast<size_t>(std::min(rows, l.plan.pass_rows)) * c.out * sizeof(float)));
+    l.total = l.sums + (row_shard ? round256(static_cast<size_t>(std::min(rows, l.plan.pass_rows)) * c.out * sizeof(float)) : 0);
     return l;
 }
 
@@ -485,7 +494,10 @@ static int core_workspace_bytes(const LayerCore& c, int64_t rows, size_t* out_by
     if (rows <= 0) return fail("EXL3 linear input cannot be empty");
     const QmvPlan plan = plan_qmv(c.in, c.out, c.k, rows, true);             // the larger of the two grids
     size_t bytes = kCounterBytes + qmv_partial_bytes(plan, c.out, rows) + xhat_bytes(c, rows);
-    if (rows >= kQmmMinRows) bytes = std::max(bytes, qmm_layout(c, rows).total);
+    if (rows >= kQmmMinRows) {
+        bytes = std::max(bytes, qmm_layout(c, rows).total);
+        if (c.groups == 1) bytes = std::max(bytes, qmm_layout(c, rows, false, true).total);      // the layer may be a row shard
+    }
     *out_bytes = bytes;
     return 0;
 }
@@ -523,7 +535,7 @@ static int forward_common(const LayerCore& c, const void* d_x, int x_dtype, cons
         // many rows: input rotation (once per member of a group, each has its own input scales) -> tensor-core product
         // over all members with the output rotation in its epilogue; of a row shard of a tensor-parallel layer the sums
         // over the inputs are kept, and the sum over ranks and the rotation follow as one kernel
-        const QmmLayout l = qmm_layout(c, rows, whole_items);
+        const QmmLayout l = qmm_layout(c, rows, whole_items, tp != nullptr);
         for (int64_t r0 = 0; r0 < rows; r0 += l.plan.pass_rows) {
             const int64_t n = std::min(l.plan.pass_rows, rows - r0);
             __half* buf = reinterpret_cast<__half*>(base + l.xhat);
