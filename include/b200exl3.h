@@ -177,8 +177,10 @@ int b200exl3_linear_forward(const b200exl3_linear* handle, const void* d_x, int 
  * ever see input and output pointers: the scratch memory is a fixed 4 MiB array inside the library's
  * device image (held by every GPU that loads the library, until the process exits), and the call
  * itself allocates and frees nothing.  x and y are as in b200exl3_linear_forward.
- *   - A call whose scratch need (b200exl3_linear_workspace_bytes) exceeds 4 MiB is rejected with an
- *     error; decode-sized calls (a few rows) of any layer of the supported models fit.
+ *   - A call whose scratch need exceeds 4 MiB is rejected with an error; decode-sized calls (a few rows) of any
+ *     layer of the supported models fit.  Up to 8 rows the need is b200exl3_linear_workspace_bytes; with more it is
+ *     the rotated rows [rows, in] in fp16 and one fp32 copy of the result [rows, out], or the parts of column
+ *     blocks that the path in use keeps, whichever is more.
  *   - The first call on each device looks up the array's device address; make that first call
  *     outside any stream capture.
  *   - All calls share the one array: every call clears the counters at its head on `stream` first,

@@ -489,11 +489,16 @@ static QmmLayout qmm_layout(const LayerCore& c, int64_t rows, bool whole_items =
     return l;
 }
 
+// few-row path: [counters | parts of shared column blocks | rotated rows, when the kernel does not rotate]
+static size_t qmv_workspace_bytes(const LayerCore& c, int64_t rows) {
+    const QmvPlan plan = plan_qmv(c.in, c.out, c.k, rows, true);             // the larger of the two grids
+    return kCounterBytes + qmv_partial_bytes(plan, c.out, rows) + xhat_bytes(c, rows);
+}
+
 static int core_workspace_bytes(const LayerCore& c, int64_t rows, size_t* out_bytes) {
     if (!out_bytes) return fail("NULL argument");
     if (rows <= 0) return fail("EXL3 linear input cannot be empty");
-    const QmvPlan plan = plan_qmv(c.in, c.out, c.k, rows, true);             // the larger of the two grids
-    size_t bytes = kCounterBytes + qmv_partial_bytes(plan, c.out, rows) + xhat_bytes(c, rows);
+    size_t bytes = qmv_workspace_bytes(c, rows);
     if (rows >= kQmmMinRows) {
         bytes = std::max(bytes, qmm_layout(c, rows).total);
         if (c.groups == 1) bytes = std::max(bytes, qmm_layout(c, rows, false, true).total);      // the layer may be a row shard
@@ -507,19 +512,14 @@ int b200exl3_linear_workspace_bytes(const b200exl3_linear* h, int64_t rows, size
     return core_workspace_bytes(h->c, rows, out_bytes);
 }
 
-// One fused launch per batch of up to kMaxBatchRows rows.  Exactly one of d_x / d_xhat is given;
-// ys (one pointer per group) selects the rotated output, otherwise the summed fp32 product goes to d_yhat.
 static TpPeers tp_peers(const b200exl3_tp* tp);
 
-static int forward_common(const LayerCore& c, const void* d_x, int x_dtype, const uint16_t* d_xhat, int64_t rows,
-                          void* const* ys, float* d_yhat, void* ws, size_t ws_bytes, cudaStream_t stream,
-                          const b200exl3_tp* tp = nullptr, const b200exl3_prologue* pro = nullptr, bool whole_items = false) {
-    if (rows <= 0) return fail("EXL3 linear input cannot be empty");
-    size_t need = 0;
-    if (whole_items) need = qmm_layout(c, rows, true).total;
-    else if (core_workspace_bytes(c, rows, &need)) return -1;
-    if (!ws || ws_bytes < need) return fail("workspace too small: %zu bytes given, %zu needed", ws_bytes, need);
-    if (!aligned16(ws)) return fail("device pointers must be 16-byte aligned");
+// Exactly one of d_x / d_xhat is given; ys (one pointer per group) selects the rotated output, otherwise the summed fp32
+// product goes to d_yhat.  With a `layout` (rows that are to be rotated and stored rotated) the many-row product, without one
+// a fused launch per batch of up to kMaxBatchRows rows.  The caller has checked that `ws` holds what that path needs.
+static int run_forward(const LayerCore& c, const void* d_x, int x_dtype, const uint16_t* d_xhat, int64_t rows, void* const* ys,
+                       float* d_yhat, void* ws, cudaStream_t stream, const b200exl3_tp* tp, const b200exl3_prologue* pro,
+                       const QmmLayout* layout) {
     char* base = static_cast<char*>(ws);
     const bool exact = (c.flags & B200EXL3_EXACT_WEIGHTS) != 0;
     const size_t x_size = dtype_size(x_dtype);
@@ -531,11 +531,11 @@ static int forward_common(const LayerCore& c, const void* d_x, int x_dtype, cons
         glu_up = reinterpret_cast<const __half*>(pro->d_aux);
         pro = nullptr;
     }
-    if (rows >= kQmmMinRows && ys && !d_xhat && g_qmm_enabled) {
+    if (layout) {
         // many rows: input rotation (once per member of a group, each has its own input scales) -> tensor-core product
         // over all members with the output rotation in its epilogue; of a row shard of a tensor-parallel layer the sums
         // over the inputs are kept, and the sum over ranks and the rotation follow as one kernel
-        const QmmLayout l = qmm_layout(c, rows, whole_items, tp != nullptr);
+        const QmmLayout& l = *layout;
         for (int64_t r0 = 0; r0 < rows; r0 += l.plan.pass_rows) {
             const int64_t n = std::min(l.plan.pass_rows, rows - r0);
             __half* buf = reinterpret_cast<__half*>(base + l.xhat);
@@ -621,6 +621,22 @@ static int forward_common(const LayerCore& c, const void* d_x, int x_dtype, cons
         B200_TRY(launch_qmv(a, c.k, c.cb, exact, plan, stream), "fused linear kernel");
     }
     return 0;
+}
+
+static int forward_common(const LayerCore& c, const void* d_x, int x_dtype, const uint16_t* d_xhat, int64_t rows,
+                          void* const* ys, float* d_yhat, void* ws, size_t ws_bytes, cudaStream_t stream,
+                          const b200exl3_tp* tp = nullptr, const b200exl3_prologue* pro = nullptr) {
+    size_t need = 0;
+    if (core_workspace_bytes(c, rows, &need)) return -1;
+    QmmLayout layout{};                                       // planned once: what is checked is what runs
+    const bool tensor_cores = rows >= kQmmMinRows && ys && !d_xhat && g_qmm_enabled;
+    if (tensor_cores) {
+        layout = qmm_layout(c, rows, false, tp != nullptr);
+        need = std::max(need, layout.total);
+    }
+    if (!ws || ws_bytes < need) return fail("workspace too small: %zu bytes given, %zu needed", ws_bytes, need);
+    if (!aligned16(ws)) return fail("device pointers must be 16-byte aligned");
+    return run_forward(c, d_x, x_dtype, d_xhat, rows, ys, d_yhat, ws, stream, tp, pro, tensor_cores ? &layout : nullptr);
 }
 
 int b200exl3_workspace_status(const void* ws, int* out_status) {
@@ -749,14 +765,18 @@ int b200exl3_linear_forward_static(const b200exl3_linear* h, const void* d_x, in
     if (!h) return fail("NULL handle");
     if (!dtype_is_float(x_dtype)) return fail("unsupported input dtype %d", x_dtype);
     if (!d_x || !d_y) return fail("NULL buffer");
-    size_t need = 0;
-    if (core_workspace_bytes(h->c, rows, &need)) return -1;
-    bool whole_items = false;
-    if (need > kStaticScratchBytes && rows >= kQmmMinRows) {
-        // many rows: without parts of items shared by CTAs the call needs less (what counts against the array is the
-        // rotated rows and one fp32 copy of the result, as it always did)
-        const size_t smallest = qmm_layout(h->c, rows, true).total + static_cast<size_t>(rows) * h->c.out * sizeof(float);
-        if (smallest <= kStaticScratchBytes) { whole_items = true; need = smallest; }
+    if (rows <= 0) return fail("EXL3 linear input cannot be empty");
+    const LayerCore& c = h->c;
+    QmmLayout layout{};                                       // planned once: what is checked is what runs
+    const bool tensor_cores = rows >= kQmmMinRows && g_qmm_enabled;
+    if (tensor_cores) {
+        layout = qmm_layout(c, rows);
+        if (layout.total > kStaticScratchBytes) layout = qmm_layout(c, rows, true);       // without parts the call needs less
+    }
+    size_t need = tensor_cores ? layout.total : qmv_workspace_bytes(c, rows);
+    if (rows >= kQmmMinRows) {
+        // the limit as it is promised to callers, whatever the path keeps where: the rotated rows and one fp32 copy of the result
+        need = std::max(need, qmm_layout(c, rows, true).total + static_cast<size_t>(rows) * c.out * sizeof(float));
     }
     if (need > kStaticScratchBytes)
         return fail("this call needs %zu bytes of scratch but the allocation-free entry point owns %zu; "
@@ -769,7 +789,7 @@ int b200exl3_linear_forward_static(const b200exl3_linear* h, const void* d_x, in
     // until that call clears it, as it does in a caller's workspace.
     B200_TRY(cudaMemsetAsync(scratch, 0, kCounterBytes - sizeof(unsigned int), as_stream(s)), "clear static scratch");
     void* ys[1] = {d_y};
-    return forward_common(h->c, d_x, x_dtype, nullptr, rows, ys, nullptr, scratch, kStaticScratchBytes, as_stream(s), nullptr, nullptr, whole_items);
+    return run_forward(c, d_x, x_dtype, nullptr, rows, ys, nullptr, scratch, as_stream(s), nullptr, nullptr, tensor_cores ? &layout : nullptr);
 }
 
 int b200exl3_static_status(int* out_status, int clear) {
