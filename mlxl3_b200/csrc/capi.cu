@@ -1101,14 +1101,14 @@ static int64_t moe_sorted_chunk_rows(const b200exl3_moe* h, int64_t rows) {
 }
 
 struct MoeSortedLayout {
-    size_t counters, counter_bytes, seg_count, seg_expert, seg_rows, slot_row, xgu, ygu, xdown, ydown, pieces, total;
+    size_t counters, counter_bytes, seg_count, seg_expert, seg_rows, seg_row0, slot_row, xgu, ygu, xdown, ydown, pieces, total;
     int max_segments;
 };
 
 static MoeSortedLayout moe_sorted_layout(const b200exl3_moe* h, int64_t rows) {
     MoeSortedLayout l{};
     const int64_t slots = moe_sorted_chunk_rows(h, rows) * h->top_k;
-    const size_t segs = static_cast<size_t>(moe_max_segments(h, slots)), padded = segs * kQmmSegRows;
+    const size_t segs = static_cast<size_t>(moe_max_segments(h, slots)), n = static_cast<size_t>(slots);
     l.max_segments = static_cast<int>(segs);
     size_t at = kCounterBytes;
     // arrival counters of its own (one per virtual column block; the header's 16 KiB would cap a pass at 4093 blocks),
@@ -1118,11 +1118,12 @@ static MoeSortedLayout moe_sorted_layout(const b200exl3_moe* h, int64_t rows) {
     l.seg_count = at; at += 256;
     l.seg_expert = at; at += round256(segs * sizeof(uint32_t));
     l.seg_rows = at; at += round256(segs * sizeof(int));
-    l.slot_row = at; at += round256(static_cast<size_t>(slots) * sizeof(uint32_t));
-    l.xgu = at; at += round256(padded * 2 * h->in * sizeof(__half));
-    l.ygu = at; at += round256(padded * 2 * h->hidden * sizeof(float));
-    l.xdown = at; at += round256(padded * h->hidden * sizeof(__half));
-    l.ydown = at; at += round256(padded * h->in * sizeof(float));
+    l.seg_row0 = at; at += round256(segs * sizeof(int));
+    l.slot_row = at; at += round256(n * sizeof(uint32_t));
+    l.xgu = at; at += round256(n * 2 * h->in * sizeof(__half));
+    l.ygu = at; at += round256(n * 2 * h->hidden * sizeof(float));
+    l.xdown = at; at += round256(n * h->hidden * sizeof(__half));
+    l.ydown = at; at += round256(n * h->in * sizeof(float));
     l.pieces = at; at += round256(qmm_mapped_piece_bytes());
     l.total = at;
     return l;
@@ -1225,6 +1226,7 @@ int b200exl3_moe_forward(const b200exl3_moe* h, const void* d_x, int x_dtype, in
         int* seg_count = reinterpret_cast<int*>(base + l.seg_count);
         uint32_t* seg_expert = reinterpret_cast<uint32_t*>(base + l.seg_expert);
         int* seg_rows = reinterpret_cast<int*>(base + l.seg_rows);
+        int* seg_row0 = reinterpret_cast<int*>(base + l.seg_row0);
         uint32_t* slot_row = reinterpret_cast<uint32_t*>(base + l.slot_row);
         __half* xgu = reinterpret_cast<__half*>(base + l.xgu);
         float* ygu = reinterpret_cast<float*>(base + l.ygu);
@@ -1245,13 +1247,14 @@ int b200exl3_moe_forward(const b200exl3_moe* h, const void* d_x, int x_dtype, in
                 a.error = reinterpret_cast<unsigned int*>(base + kCounterBytes - sizeof(unsigned int));
                 a.yhat = yhat; a.yhat_ld = width;
                 a.in = in;
-                a.map_expert = seg_expert; a.map_rows = seg_rows; a.map_count = seg_count;
+                a.map_expert = seg_expert; a.map_rows = seg_rows; a.map_row0 = seg_row0; a.map_count = seg_count;
+                a.map_slots = static_cast<int>(slots);
                 a.map_blocks = width / 128; a.map_proj = proj; a.map_stride_blocks = stride_blocks; a.map_experts = h->experts;
                 return launch_qmm_mapped(a, xhat, segs, h->k, h->cb, stream);
             };
-            B200_TRY(launch_route_plan(sel, slots, h->experts, segs, seg_count, seg_expert, seg_rows, slot_row, stream), "route plan");
+            B200_TRY(launch_route_plan(sel, slots, h->experts, segs, seg_count, seg_expert, seg_rows, seg_row0, slot_row, stream), "route plan");
             B200_TRY(launch_routed_prepare(static_cast<const char*>(d_x) + static_cast<size_t>(r0) * h->in * x_size, x_dtype, h->gu_suh, sel,
-                                           slot_row, h->experts, slots, h->top_k, 2, segs, h->in, xgu, stream), "routed prepare");
+                                           slot_row, h->experts, slots, h->top_k, 2, h->in, xgu, stream), "routed prepare");
             B200_TRY(mapped(h->gu_wq, xgu, h->in, h->hidden, 2, h->experts * (h->hidden / 128), ygu), "expert gate/up kernel");
             B200_TRY(launch_glu_down_input(ygu, h->gu_svh, h->down_suh, sel, h->experts, slots, h->hidden, h->hidden, xdown, stream, nullptr,
                                            slot_row), "SwiGLU glue");

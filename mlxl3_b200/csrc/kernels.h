@@ -254,7 +254,7 @@ cudaError_t launch_stack(const StackArgs& args, int k, int cb, bool exact, const
 // ---- grouped experts (kernels_moe.cu) ------------------------------------------------------------------
 // SwiGLU glue between the expert projections (native/src/moe.rs:438-533, SiLU): raw gate/up sums
 // ygu[slot * 2 + {0,1}, :] -> rotated input of the down projection xhat[slot, :].  With slot_row (the expert-sorted form)
-// slot s is row r = slot_row[s] % 64 of segment g = slot_row[s] / 64: sums ygu[(g * 2 + {0,1}) * 64 + r, :], result xhat[g * 64 + r, :].
+// slot s is row r = slot_row[s]: sums ygu[{0,1} * slots + r, :], result xhat[r, :].
 // `count` (optional, device): only slots below *count are computed
 cudaError_t launch_glu_down_input(const float* ygu, const __half* gu_svh, const __half* down_suh, const uint32_t* selected,
                                   int experts, int64_t slots, int hidden, int logical_hidden, __half* xhat,
@@ -294,17 +294,19 @@ struct TpArgs {
 cudaError_t launch_tp_finish(const TpArgs& args, cudaStream_t stream);
 
 // Expert-sorted form for many slots (native/src/moe.rs:66-182 route_plan, 1001-1085): slots are grouped by expert
-// into segments of up to kQmmSegRows rows, so that an expert's columns are decoded once per 64 rows that use them.
+// into segments of up to kQmmSegRows rows, so that an expert's columns are decoded once per 64 rows that use them.  The rows
+// lie one after the other, without gaps between experts.
 //   seg_count[0]     number of segments
 //   seg_expert[s]    expert of segment s
 //   seg_rows[s]      slots in segment s
-//   slot_row[slot]   padded row 64 * segment + r that holds the slot
+//   seg_row0[s]      first row of segment s
+//   slot_row[slot]   row that holds the slot
 // max_segments bounds the arrays (min(experts, slots) + slots / 64 always suffices).
 cudaError_t launch_route_plan(const uint32_t* selected, int64_t slots, int experts, int max_segments, int* seg_count,
-                              uint32_t* seg_expert, int* seg_rows, uint32_t* slot_row, cudaStream_t stream);
-// every slot's token row rotated with its expert's input scales: xhat[(g * proj + p) * 64 + r, :]
+                              uint32_t* seg_expert, int* seg_rows, int* seg_row0, uint32_t* slot_row, cudaStream_t stream);
+// every slot's token row rotated with its expert's input scales: xhat[p * slots + slot_row[slot], :]
 cudaError_t launch_routed_prepare(const void* x, int x_dtype, const __half* suh, const uint32_t* selected, const uint32_t* slot_row,
-                                  int experts, int64_t slots, int top_k, int proj, int max_segments, int in, __half* xhat, cudaStream_t stream);
+                                  int experts, int64_t slots, int top_k, int proj, int in, __half* xhat, cudaStream_t stream);
 
 // ---- router (kernels_router.cu) --------------------------------------------------------------------------
 // stable top-k per row with index tie-break; values and scores fp16 or fp32; experts <= 1024.  With `softmax` the
@@ -365,9 +367,11 @@ struct QmmArgs {
     // Expert-mapped mode (map_expert != nullptr; yhat): an item is (segment, projection, 128 columns); segment s holds
     // map_rows[s] of up to 64 rows that all use expert map_expert[s], whose columns start at column block
     // projection * map_stride_blocks + expert * map_blocks of the bank.  Row r of (segment, projection) is row
-    // (s * map_proj + p) * 64 + r of both xhat and yhat.
+    // p * map_slots + map_row0[s] + r of both xhat and yhat.
     const uint32_t* map_expert;
     const int* map_rows;
+    const int* map_row0;
+    int map_slots;             // rows of a projection
     const int* map_count;      // segments in use (device)
     int map_blocks, map_proj, map_stride_blocks, map_experts;
 };

@@ -44,9 +44,8 @@ glu_down_input_kernel(const float* __restrict__ ygu, const __half* __restrict__ 
         const int64_t expert = expert_of(selected, slot, experts);
         int64_t grow = slot * 2, up = 1, xrow = slot;           // gate row, distance to the up row, row of the result
         if (SORTED) {
-            xrow = slot_row[slot];
-            grow = (xrow / kQmmSegRows) * 2 * kQmmSegRows + xrow % kQmmSegRows;
-            up = kQmmSegRows;
+            grow = xrow = slot_row[slot];
+            up = slots;
         }
         const float4 graw = *reinterpret_cast<const float4*>(ygu + grow * hidden + col);
         const float4 uraw = *reinterpret_cast<const float4*>(ygu + (grow + up) * hidden + col);
@@ -165,16 +164,48 @@ namespace b200exl3 {
 
 namespace {
 
-// One CTA plans the whole batch: counts per expert, segments of 64 rows per expert in expert order, and the padded row of
-// every slot.
+// First row and first segment of every expert, as row << 16 | segment: one running sum over the experts' counts, 32 experts per
+// step of one warp.  Neither half overflows: the expert ids of a pass fit 48 KiB of shared memory, so it has at most 24576 slots.
+__device__ __forceinline__ void plan_bases(const int* count, uint32_t* base, int experts, int max_segments, int* seg_count, int lane) {
+    uint32_t carry = 0;
+    for (int e0 = 0; e0 < experts; e0 += 32) {
+        const int e = e0 + lane;
+        const uint32_t n = e < experts ? static_cast<uint32_t>(count[e]) : 0u;
+        const uint32_t own = n << 16 | (n + kQmmSegRows - 1) / kQmmSegRows;
+        uint32_t incl = own;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t up = __shfl_up_sync(0xffffffffu, incl, d);
+            if (lane >= d) incl += up;
+        }
+        if (e < experts) base[e] = carry + incl - own;
+        carry += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    if (lane == 0) {
+        base[experts] = carry;
+        seg_count[0] = min(static_cast<int>(carry & 0xffffu), max_segments);
+    }
+}
+
+// the segments of expert e: `n` rows from row base >> 16 on
+__device__ __forceinline__ void plan_segments(int e, int n, uint32_t base, int max_segments, uint32_t* seg_expert, int* seg_rows, int* seg_row0) {
+    for (int s = static_cast<int>(base & 0xffffu), row = 0; row < n && s < max_segments; ++s, row += kQmmSegRows) {
+        seg_expert[s] = static_cast<uint32_t>(e);
+        seg_rows[s] = min(kQmmSegRows, n - row);
+        seg_row0[s] = static_cast<int>(base >> 16) + row;
+    }
+}
+
+// One CTA plans the whole batch: counts per expert, the rows of the experts one expert after the other, segments of up to 64
+// of an expert's rows, and the row of every slot.
 __global__ void __launch_bounds__(1024)
 route_plan_kernel(const uint32_t* __restrict__ selected, int64_t slots, int experts, int max_segments, int* __restrict__ seg_count,
-                  uint32_t* __restrict__ seg_expert, int* __restrict__ seg_rows, uint32_t* __restrict__ slot_row) {
+                  uint32_t* __restrict__ seg_expert, int* __restrict__ seg_rows, int* __restrict__ seg_row0, uint32_t* __restrict__ slot_row) {
     pdl_launch_dependents();                    // the kernel after this one may start; it waits for our memory itself
     pdl_wait();                                 // what the kernel before this one wrote is visible from here on
     extern __shared__ int s_mem[];
     int* count = s_mem;                 // [experts] rows per expert, then running position
-    int* base = s_mem + experts;        // [experts + 1] first segment of each expert
+    uint32_t* base = reinterpret_cast<uint32_t*>(s_mem) + experts;   // [experts + 1] first row << 16 | first segment of each expert
     // expert of every slot, staged once (the walk below reads each of them once per expert)
     unsigned short* ids = reinterpret_cast<unsigned short*>(s_mem + 2 * experts + 1);
     for (int64_t s = threadIdx.x; s < slots; s += blockDim.x)
@@ -199,36 +230,11 @@ route_plan_kernel(const uint32_t* __restrict__ selected, int64_t slots, int expe
         }
     }
     __syncthreads();
-    if (warp == 0) {
-        // first segment of every expert: a running sum of the experts' segment counts, 32 experts per step of one warp
-        int carry = 0;
-        for (int e0 = 0; e0 < experts; e0 += 32) {
-            const int e = e0 + lane;
-            const int segs = e < experts ? (count[e] + kQmmSegRows - 1) / kQmmSegRows : 0;
-            int incl = segs;
-#pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                const int up = __shfl_up_sync(0xffffffffu, incl, d);
-                if (lane >= d) incl += up;
-            }
-            if (e < experts) base[e] = carry + incl - segs;
-            carry += __shfl_sync(0xffffffffu, incl, 31);
-        }
-        if (lane == 0) {
-            base[experts] = carry;
-            seg_count[0] = min(carry, max_segments);
-        }
-    }
+    if (warp == 0) plan_bases(count, base, experts, max_segments, seg_count, lane);
     __syncthreads();
-    for (int e = threadIdx.x; e < experts; e += blockDim.x)
-        for (int s = base[e]; s < base[e + 1] && s < max_segments; ++s) {
-            seg_expert[s] = static_cast<uint32_t>(e);
-            seg_rows[s] = min(kQmmSegRows, count[e] - (s - base[e]) * kQmmSegRows);
-        }
+    for (int e = threadIdx.x; e < experts; e += blockDim.x) plan_segments(e, count[e], base[e], max_segments, seg_expert, seg_rows, seg_row0);
     for (int64_t s = threadIdx.x; s < slots; s += blockDim.x) {
-        const int e = ids[s];
-        const int pos = static_cast<int>(slot_row[s]);
-        slot_row[s] = static_cast<uint32_t>(base[e] * kQmmSegRows + pos);      // an expert's segments follow one another
+        slot_row[s] += base[ids[s]] >> 16;
     }
 }
 
@@ -240,12 +246,12 @@ route_plan_kernel(const uint32_t* __restrict__ selected, int64_t slots, int expe
 // costs slots / 32 + groups steps.  Same plan, bit for bit: position = number of earlier slots with the same expert.
 __global__ void __launch_bounds__(1024)
 route_plan_grouped_kernel(const uint32_t* __restrict__ selected, int64_t slots, int experts, int max_segments, int* __restrict__ seg_count,
-                          uint32_t* __restrict__ seg_expert, int* __restrict__ seg_rows, uint32_t* __restrict__ slot_row) {
+                          uint32_t* __restrict__ seg_expert, int* __restrict__ seg_rows, int* __restrict__ seg_row0, uint32_t* __restrict__ slot_row) {
     pdl_launch_dependents();                    // the kernel after this one may start; it waits for our memory itself
     pdl_wait();                                 // what the kernel before this one wrote is visible from here on
     extern __shared__ int s_mem[];
     int* count = s_mem;                 // [experts] rows per expert
-    int* base = s_mem + experts;        // [experts + 1] first segment of each expert
+    uint32_t* base = reinterpret_cast<uint32_t*>(s_mem) + experts;   // [experts + 1] first row << 16 | first segment of each expert
     unsigned short* table = reinterpret_cast<unsigned short*>(s_mem + 2 * experts + 1);   // [groups][experts]: counts, then positions
     const int groups = static_cast<int>((slots + 31) / 32);
     // every slot's expert and its rank inside its group stay in shared memory between the passes
@@ -276,44 +282,19 @@ route_plan_grouped_kernel(const uint32_t* __restrict__ selected, int64_t slots, 
         count[e] = running;
     }
     __syncthreads();
-    if (warp == 0) {
-        // first segment of every expert: a running sum of the experts' segment counts, 32 experts per step of one warp
-        int carry = 0;
-        for (int e0 = 0; e0 < experts; e0 += 32) {
-            const int e = e0 + lane;
-            const int segs = e < experts ? (count[e] + kQmmSegRows - 1) / kQmmSegRows : 0;
-            int incl = segs;
-#pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                const int up = __shfl_up_sync(0xffffffffu, incl, d);
-                if (lane >= d) incl += up;
-            }
-            if (e < experts) base[e] = carry + incl - segs;
-            carry += __shfl_sync(0xffffffffu, incl, 31);
-        }
-        if (lane == 0) {
-            base[experts] = carry;
-            seg_count[0] = min(carry, max_segments);
-        }
-    }
+    if (warp == 0) plan_bases(count, base, experts, max_segments, seg_count, lane);
     __syncthreads();
-    for (int e = threadIdx.x; e < experts; e += blockDim.x)
-        for (int s = base[e]; s < base[e + 1] && s < max_segments; ++s) {
-            seg_expert[s] = static_cast<uint32_t>(e);
-            seg_rows[s] = min(kQmmSegRows, count[e] - (s - base[e]) * kQmmSegRows);
-        }
+    for (int e = threadIdx.x; e < experts; e += blockDim.x) plan_segments(e, count[e], base[e], max_segments, seg_expert, seg_rows, seg_row0);
     for (int64_t s = threadIdx.x; s < slots; s += blockDim.x) {
         const int e = slot_expert[s];
-        const int pos = table[(s >> 5) * experts + e] + static_cast<int>(slot_rank[s]);
-        slot_row[s] = static_cast<uint32_t>(base[e] * kQmmSegRows + pos);      // an expert's segments follow one another
+        slot_row[s] = (base[e] >> 16) + table[(s >> 5) * experts + e] + slot_rank[s];
     }
 }
 
-// One warp per (slot, 128-block), every projection of the slot's expert: only rows that hold a slot are written.  Padding
-// rows are left as they are: every activation row is multiplied on its own, and the product stores no padding row.
+// One warp per (slot, 128-block), every projection of the slot's expert: row slot_row of each projection's `slots` rows.
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 routed_prepare_kernel(const void* __restrict__ x, int x_dtype, const __half* __restrict__ suh, const uint32_t* __restrict__ selected,
-                      const uint32_t* __restrict__ slot_row, int experts, int64_t slots, int max_segments, int top_k, int proj, int in,
+                      const uint32_t* __restrict__ slot_row, int experts, int64_t slots, int top_k, int proj, int in,
                       __half* __restrict__ xhat) {
     pdl_launch_dependents();                    // the kernel after this one may start; it waits for our memory itself
     pdl_wait();                                 // what the kernel before this one wrote is visible from here on
@@ -324,8 +305,7 @@ routed_prepare_kernel(const void* __restrict__ x, int x_dtype, const __half* __r
          unit += static_cast<int64_t>(gridDim.x) * kWarpsPerBlock) {
         const int64_t slot = unit / blocks_per_row;
         const int col = static_cast<int>(unit - slot * blocks_per_row) * 128 + lane * 4;
-        const int64_t prow = slot_row[slot], seg = prow / kQmmSegRows, r = prow % kQmmSegRows;
-        if (seg >= max_segments) continue;
+        const int64_t row = slot_row[slot];
         __half v[4];
         load4_as_half(x, x_dtype, slot / top_k * in + col, v);
         const __half* s = suh + static_cast<int64_t>(expert_of(selected, slot, experts)) * proj * in + col;
@@ -335,7 +315,7 @@ routed_prepare_kernel(const void* __restrict__ x, int x_dtype, const __half* __r
 #pragma unroll
             for (int j = 0; j < 4; ++j) h[j] = __hmul_rn(v[j], reinterpret_cast<const __half*>(&sw)[j]);
             warp_hadamard128_f16(h, lane);
-            *reinterpret_cast<uint2*>(xhat + ((seg * proj + p) * kQmmSegRows + r) * in + col) = *reinterpret_cast<uint2*>(h);
+            *reinterpret_cast<uint2*>(xhat + (p * slots + row) * in + col) = *reinterpret_cast<uint2*>(h);
         }
     }
 }
@@ -343,7 +323,7 @@ routed_prepare_kernel(const void* __restrict__ x, int x_dtype, const __half* __r
 }  // namespace
 
 cudaError_t launch_route_plan(const uint32_t* selected, int64_t slots, int experts, int max_segments, int* seg_count,
-                              uint32_t* seg_expert, int* seg_rows, uint32_t* slot_row, cudaStream_t stream) {
+                              uint32_t* seg_expert, int* seg_rows, int* seg_row0, uint32_t* slot_row, cudaStream_t stream) {
     if (experts > 65535 || slots >= 65535) return cudaErrorInvalidValue;              // positions are kept in 16 bits
     const size_t groups = static_cast<size_t>((slots + 31) / 32);
     const size_t grouped = (2 * static_cast<size_t>(experts) + 1) * sizeof(int) + groups * experts * sizeof(unsigned short) +
@@ -352,13 +332,13 @@ cudaError_t launch_route_plan(const uint32_t* selected, int64_t slots, int exper
     const size_t smem = fits ? grouped : (2 * static_cast<size_t>(experts) + 1) * sizeof(int) + static_cast<size_t>(slots) * sizeof(unsigned short);
     if (smem > 48 * 1024) return cudaErrorInvalidValue;
     return launch_dependent(fits ? route_plan_grouped_kernel : route_plan_kernel, dim3(1), dim3(1024), smem, stream, selected, slots, experts,
-                            max_segments, seg_count, seg_expert, seg_rows, slot_row);
+                            max_segments, seg_count, seg_expert, seg_rows, seg_row0, slot_row);
 }
 
 cudaError_t launch_routed_prepare(const void* x, int x_dtype, const __half* suh, const uint32_t* selected, const uint32_t* slot_row,
-                                  int experts, int64_t slots, int top_k, int proj, int max_segments, int in, __half* xhat, cudaStream_t stream) {
+                                  int experts, int64_t slots, int top_k, int proj, int in, __half* xhat, cudaStream_t stream) {
     return launch_dependent(routed_prepare_kernel, dim3(grid_for(slots * (in / 128))), dim3(kWarpsPerBlock * 32), 0, stream, x, x_dtype, suh,
-                            selected, slot_row, experts, slots, max_segments, top_k, proj, in, xhat);
+                            selected, slot_row, experts, slots, top_k, proj, in, xhat);
 }
 
 }  // namespace b200exl3

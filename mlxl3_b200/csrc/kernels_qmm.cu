@@ -170,7 +170,7 @@ __device__ __forceinline__ QmmItem qmm_item(const QmmArgs& p, uint32_t item) {
         const int expert = static_cast<int>(min(p.map_expert[seg], static_cast<uint32_t>(p.map_experts - 1)));
         it.wblock = proj * p.map_stride_blocks + expert * p.map_blocks + j;
         it.cblock = j;
-        it.brow = it.tok0 = sp * kQmmSegRows;
+        it.brow = it.tok0 = proj * p.map_slots + p.map_row0[seg];
         it.n = p.map_rows[seg];
     } else {
         const int cb = static_cast<int>(item) / p.tiles, t = static_cast<int>(item) - cb * p.tiles;
@@ -808,12 +808,12 @@ cudaError_t launch_qmm(QmmArgs p, const __half* xhat, int k, int cb, const QmmPl
 size_t qmm_mapped_piece_bytes() { return static_cast<size_t>(sm_count()) * 2 * kQmmSegRows * 128 * sizeof(float); }
 
 cudaError_t launch_qmm_mapped(QmmArgs p, const __half* xhat, int max_segments, int k, int cb, cudaStream_t stream) {
-    if (p.in % 128 || p.map_blocks <= 0 || max_segments <= 0 || p.map_proj <= 0 || p.yhat == nullptr) return cudaErrorInvalidValue;
+    if (p.in % 128 || p.map_blocks <= 0 || max_segments <= 0 || p.map_proj <= 0 || p.map_slots <= 0 || p.yhat == nullptr) return cudaErrorInvalidValue;
     const int64_t stages = static_cast<int64_t>(max_segments) * p.map_proj * p.map_blocks * (p.in / kStageIn);
     if (stages * sm_count() >= (int64_t{1} << 32)) return cudaErrorInvalidValue;
     CUtensorMap map;
-    constexpr int box = 16;                                   // segments are short: only the boxes that hold rows are fetched
-    if (!encode_rows(&map, xhat, p.in, static_cast<int64_t>(max_segments) * p.map_proj * kQmmSegRows, box)) return cudaErrorInvalidValue;
+    constexpr int box = 16;      // segments are short: only the boxes that hold rows are fetched (the last may reach into the next segment's)
+    if (!encode_rows(&map, xhat, p.in, static_cast<int64_t>(p.map_proj) * p.map_slots, box)) return cudaErrorInvalidValue;
     p.groups = 1; p.gcol0[0] = 0;
     p.tile_tokens = kQmmSegRows; p.box_rows = box;
     p.trace = nullptr;

@@ -1,0 +1,65 @@
+"""Expert segments lie one after the other in the workspace: rows around the 64 a segment holds, batches whose plan does not
+fit the grouped planner, ids past the bank, and the room the rows take."""
+import numpy as np
+import pytest
+
+import oracle
+from tests.gpu_util import gpu  # noqa: F401
+from tests.test_gpu_moe import check, make_bank, routes
+
+pytestmark = pytest.mark.gpu
+
+
+def counts_to_routes(rng, counts):
+    """One slot per token, expert e chosen counts[e] times, tokens in random order."""
+    selected = np.repeat(np.arange(len(counts), dtype=np.uint32), counts)
+    return rng.permutation(selected)[:, None]
+
+
+@pytest.mark.parametrize("counts", [[64, 64], [65, 1, 63], [1, 130, 0, 2], [0, 0, 35], [15, 16, 17, 33], [128, 0, 64, 129]])
+def test_rows_around_a_segment(gpu, counts):
+    rng = np.random.default_rng(sum(counts))
+    n_in, hidden, k = 384, 128, 3
+    bank = make_bank(rng, len(counts), n_in, hidden, k)
+    moe = gpu.Exl3SwitchGlu(*bank, 1, k, 1, exact_weights=True)
+    selected = counts_to_routes(rng, counts)
+    x = rng.standard_normal((len(selected), n_in)).astype(np.float16)
+    scores = rng.uniform(0.5, 1.0, selected.shape).astype(np.float32)
+    got = moe.forward(x, selected, scores)
+    check(got, oracle.switch_glu_forward(*bank, 1, k, 1, x, selected, scores), rms=3e-3)
+    assert gpu.workspace_status(moe._workspace) == 0
+    moe.close()
+
+
+@pytest.mark.parametrize("experts,top_k,rows", [(1000, 2, 1000), (24, 8, 200)])
+def test_sorted_rows_equal_one_row_per_slot(gpu, experts, top_k, rows):
+    """1000 experts: the planner that walks the slots per expert; ids past the bank count as the last expert's."""
+    rng = np.random.default_rng(experts)
+    n_in, hidden, k = 128, 256, 2
+    bank = make_bank(rng, experts, n_in, hidden, k)
+    moe = gpu.Exl3SwitchGlu(*bank, top_k, k, 0, exact_weights=True)
+    x = rng.standard_normal((rows, n_in)).astype(np.float16)
+    selected, scores = routes(rng, rows, experts, top_k)
+    selected[::7, 0] = np.uint32(2 ** 31 + 5)
+    got = moe.forward(x, selected, scores)
+    assert np.array_equal(got.view(np.uint16), moe.forward(x, selected, scores).view(np.uint16))
+    gpu.set_option("moe_sorted", 0)
+    try:
+        plain = moe.forward(x, selected, scores)
+    finally:
+        gpu.set_option("moe_sorted", 1)
+    check(got, plain)
+    assert gpu.workspace_status(moe._workspace) == 0
+    moe.close()
+
+
+@pytest.mark.parametrize("rows", [37, 256])
+def test_workspace_holds_the_slots_and_no_padding(gpu, rows):
+    rng = np.random.default_rng(rows)
+    experts, top_k, n_in, hidden, k = 128, 8, 1024, 256, 1
+    moe = gpu.Exl3SwitchGlu(*make_bank(rng, experts, n_in, hidden, k), top_k, k, 0)
+    slots = rows * top_k
+    per_slot = 2 * n_in * 2 + 2 * hidden * 4 + hidden * 2 + n_in * 4
+    shared = 148 * 2 * 64 * 128 * 4                          # parts of items that CTAs share, two per CTA
+    assert moe.workspace_bytes(rows) <= slots * (per_slot + 64) + shared + (1 << 16)
+    moe.close()
