@@ -236,7 +236,8 @@ int b200exl3_scratch_acquire(size_t bytes, void** out, void** out_host) {
     ScratchBlock block{};
     B200_TRY(cudaGetDevice(&block.device), "cudaGetDevice");
     block.bytes = size_t(4) << 10;                            // powers of two: few sizes, so a block is found again
-    while (block.bytes < bytes) block.bytes *= 2;
+    while (block.bytes < bytes && block.bytes <= kScratchKeptBytes) block.bytes *= 2;
+    if (block.bytes > kScratchKeptBytes) block.bytes = bytes; // never kept: no more than was asked for
     std::unique_lock<std::mutex> lock(g_scratch_mutex);
     for (size_t i = g_scratch_free.size(); i-- > 0 && !block.ptr;)
         if (g_scratch_free[i].device == block.device && g_scratch_free[i].bytes == block.bytes) {

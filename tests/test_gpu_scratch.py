@@ -1,0 +1,36 @@
+"""The pool behind calls with host arrays (b200exl3_scratch_*)."""
+from ctypes import byref, c_void_p
+
+import pytest
+
+from mlxl3_b200 import _lib
+from tests.gpu_util import gpu  # noqa: F401
+
+pytestmark = pytest.mark.gpu
+
+MIB = 1 << 20
+
+
+def acquire(nbytes):
+    p, host = c_void_p(), c_void_p()
+    _lib.call("b200exl3_scratch_acquire", nbytes, byref(p), byref(host))
+    return p.value, host.value
+
+
+def release(ptr):
+    _lib.call("b200exl3_scratch_release", ptr)
+
+
+def free_bytes():
+    import torch
+    return torch.cuda.mem_get_info(0)[0]
+
+
+@pytest.mark.parametrize("mib", [65, 300, 1100])
+def test_a_block_too_large_to_keep_is_as_large_as_asked(gpu, mib):
+    before = free_bytes()
+    ptr, host = acquire(mib * MIB + 1)
+    taken = before - free_bytes()
+    release(ptr)
+    assert host is None and mib * MIB < taken <= (mib + 8) * MIB      # the driver hands out steps of 2 MiB
+    assert before - free_bytes() <= 2 * MIB                           # and it is given back
