@@ -235,16 +235,22 @@ int b200exl3_scratch_acquire(size_t bytes, void** out, void** out_host) {
     if (bytes == 0) return fail("scratch of no bytes");
     ScratchBlock block{};
     B200_TRY(cudaGetDevice(&block.device), "cudaGetDevice");
-    block.bytes = size_t(4) << 10;                            // powers of two: few sizes, so a block is found again
+    // Powers of two: few sizes, so a block is found again.  Every block with a page-locked half has the same size: the first
+    // call of a new size then finds one, where page-locking another half took 2.7 to 3 ms inside the call (64 KiB and more).
+    block.bytes = kScratchHostBytes;
     while (block.bytes < bytes && block.bytes <= kScratchKeptBytes) block.bytes *= 2;
     if (block.bytes > kScratchKeptBytes) block.bytes = bytes; // never kept: no more than was asked for
     std::unique_lock<std::mutex> lock(g_scratch_mutex);
-    for (size_t i = g_scratch_free.size(); i-- > 0 && !block.ptr;)
-        if (g_scratch_free[i].device == block.device && g_scratch_free[i].bytes == block.bytes) {
-            block = g_scratch_free[i];
-            g_scratch_free.erase(g_scratch_free.begin() + static_cast<long>(i));
-        }
-    if (!block.ptr) {
+    size_t found = g_scratch_free.size();                     // the smallest that is large enough, last released; a small call wants a page-locked half
+    for (size_t i = 0; i < g_scratch_free.size(); ++i) {
+        const ScratchBlock& b = g_scratch_free[i];
+        if (b.device != block.device || b.bytes < block.bytes || (block.bytes <= kScratchHostBytes && !b.host)) continue;
+        if (found == g_scratch_free.size() || b.bytes <= g_scratch_free[found].bytes) found = i;
+    }
+    if (found < g_scratch_free.size()) {
+        block = g_scratch_free[found];
+        g_scratch_free.erase(g_scratch_free.begin() + static_cast<long>(found));
+    } else {
         lock.unlock();
         if (b200exl3_malloc(block.bytes, &block.ptr)) return -1;
         if (block.bytes <= kScratchHostBytes && check(cudaMallocHost(&block.host, block.bytes), "cudaMallocHost")) {

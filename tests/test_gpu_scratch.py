@@ -34,3 +34,29 @@ def test_a_block_too_large_to_keep_is_as_large_as_asked(gpu, mib):
     release(ptr)
     assert host is None and mib * MIB < taken <= (mib + 8) * MIB      # the driver hands out steps of 2 MiB
     assert before - free_bytes() <= 2 * MIB                           # and it is given back
+
+
+def test_a_new_size_finds_a_kept_block(gpu):
+    """What a call of one size left serves the first call of another: nothing is allocated or page-locked again."""
+    first, first_host = acquire(300)
+    release(first)
+    assert first_host
+    for nbytes in (1, 4096, 70_000, MIB // 2 + 1, MIB):
+        ptr, host = acquire(nbytes)
+        release(ptr)
+        assert (ptr, host) == (first, first_host)
+    release(acquire(9 * MIB)[0])
+    for nbytes in (5 * MIB, 2 * MIB + 1, 16 * MIB):
+        before = free_bytes()
+        ptr, host = acquire(nbytes)
+        assert host is None and free_bytes() == before
+        release(ptr)
+
+
+def test_blocks_in_use_are_never_handed_out_twice(gpu):
+    held = [acquire(n)[0] for n in (100, 100, MIB, MIB + 1, 3 * MIB)]
+    assert len(set(held)) == len(held)
+    for ptr in held:
+        release(ptr)
+    with pytest.raises(gpu.B200Exl3Error, match="not a scratch block"):
+        release(held[0])
