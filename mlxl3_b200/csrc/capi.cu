@@ -266,26 +266,35 @@ int b200exl3_scratch_acquire(size_t bytes, void** out, void** out_host) {
 }
 int b200exl3_scratch_release(void* p) {
     if (!p) return 0;
-    ScratchBlock block{};
+    std::vector<ScratchBlock> drop;                           // freed outside the lock
     {
         std::lock_guard<std::mutex> lock(g_scratch_mutex);
-        for (size_t i = 0; i < g_scratch_used.size(); ++i)
-            if (g_scratch_used[i].ptr == p) {
-                block = g_scratch_used[i];
-                g_scratch_used.erase(g_scratch_used.begin() + static_cast<long>(i));
-                break;
-            }
-        if (!block.ptr) return fail("not a scratch block");
-        size_t kept = block.bytes;
-        for (const ScratchBlock& b : g_scratch_free)
-            if (b.device == block.device) kept += b.bytes;
-        if (kept <= kScratchKeptBytes) {
-            g_scratch_free.push_back(block);
-            return 0;
+        size_t at = 0;
+        while (at < g_scratch_used.size() && g_scratch_used[at].ptr != p) ++at;
+        if (at == g_scratch_used.size()) return fail("not a scratch block");
+        const int device = g_scratch_used[at].device;
+        g_scratch_free.push_back(g_scratch_used[at]);
+        g_scratch_used.erase(g_scratch_used.begin() + static_cast<long>(at));
+        size_t kept = 0;
+        for (const ScratchBlock& b : g_scratch_free) kept += b.device == device ? b.bytes : 0;
+        // The largest go first: a call that needs one copies megabytes and hardly notices, while a small call that found none
+        // would page-lock memory each time.
+        while (kept > kScratchKeptBytes) {
+            size_t largest = g_scratch_free.size();
+            for (size_t i = 0; i < g_scratch_free.size(); ++i)
+                if (g_scratch_free[i].device == device && (largest == g_scratch_free.size() || g_scratch_free[i].bytes >= g_scratch_free[largest].bytes)) largest = i;
+            kept -= g_scratch_free[largest].bytes;
+            drop.push_back(g_scratch_free[largest]);
+            g_scratch_free.erase(g_scratch_free.begin() + static_cast<long>(largest));
         }
     }
-    cudaFreeHost(block.host);
-    return check(cudaFree(block.ptr), "cudaFree");
+    cudaError_t e = cudaSuccess;
+    for (const ScratchBlock& b : drop) {
+        cudaFreeHost(b.host);
+        const cudaError_t freed = cudaFree(b.ptr);
+        if (e == cudaSuccess) e = freed;
+    }
+    return check(e, "cudaFree");
 }
 int b200exl3_free(void* p) { return p ? check(cudaFree(p), "cudaFree") : 0; }
 int b200exl3_host_alloc(size_t bytes, void** out) {

@@ -60,3 +60,16 @@ def test_blocks_in_use_are_never_handed_out_twice(gpu):
         release(ptr)
     with pytest.raises(gpu.B200Exl3Error, match="not a scratch block"):
         release(held[0])
+
+
+def test_a_kept_large_block_does_not_push_small_ones_out(gpu):
+    """64 MiB kept, then a small call: the large block makes room, the small one is there for the next call."""
+    small = acquire(300)[0]
+    before = free_bytes()
+    large = acquire(60 * MIB)[0]
+    release(large)
+    release(small)
+    assert before - free_bytes() < 32 * MIB
+    again = acquire(300)[0]
+    release(again)
+    assert again == small
