@@ -13,9 +13,12 @@
  * (the reference passes opaque lazy MLX arrays), every launch takes a cudaStream_t (passed as
  * void*), and forward calls allocate nothing: scratch memory is a caller-provided workspace whose
  * first B200EXL3_WORKSPACE_HEADER_BYTES bytes were zeroed once.  All device pointers must be
- * 16-byte aligned.  Handles are immutable after creation, so one handle may be used from several
- * threads and streams at once, each with its own workspace; calls that share a workspace must be
- * ordered on one stream.
+ * 16-byte aligned, with one exception: the rows x and y of the linear, group and rotation calls, the
+ * rows x of the expert block and the scales and bias of the rotation calls may start at any element
+ * of a larger buffer (input rows are then read element by element, and 9 or more output rows that do
+ * not start on a multiple of four elements go through the few-row kernel).  Handles are immutable
+ * after creation, so one handle may be used from several threads and streams at once, each with its
+ * own workspace; calls that share a workspace must be ordered on one stream.
  */
 #ifndef B200EXL3_H
 #define B200EXL3_H

@@ -47,6 +47,12 @@ cudaStream_t as_stream(b200exl3_stream s) { return static_cast<cudaStream_t>(s);
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
+// Rows of activations may start at any element of a larger buffer, but at an element.
+int check_rows(const void* p, int dtype) {
+    const size_t size = dtype == kU32 ? sizeof(uint32_t) : dtype_size(dtype);
+    return reinterpret_cast<uintptr_t>(p) % size == 0 ? 0 : fail("device pointers must be aligned to their elements");
+}
+
 __global__ void to_half_kernel(const void* src, int dtype, int64_t n, __half* dst) {
     int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i < n) dst[i] = load_as_half(src, dtype, i);
@@ -405,6 +411,7 @@ int b200exl3_prepare(const void* d_x, int x_dtype, const uint16_t* d_suh, int64_
     if (rows == 0) return 0;
     if (!d_x || !d_suh || !d_xhat) return fail("NULL buffer");
     if (!aligned16(d_xhat)) return fail("device pointers must be 16-byte aligned");
+    if (check_rows(d_x, x_dtype) || check_rows(d_suh, kF16)) return -1;
     return check(launch_prepare(d_x, x_dtype, reinterpret_cast<const __half*>(d_suh), scale_rows, rows, in,
                                 reinterpret_cast<__half*>(d_xhat), as_stream(s)), "prepare");
 }
@@ -418,6 +425,7 @@ int b200exl3_finish(const float* d_partials, int splits, const uint16_t* d_svh, 
     if (rows == 0) return 0;
     if (!d_partials || !d_svh || !d_y) return fail("NULL buffer");
     if (!aligned16(d_partials)) return fail("device pointers must be 16-byte aligned");
+    if (check_rows(d_svh, kF16) || check_rows(d_bias, kF16) || check_rows(d_y, y_dtype)) return -1;
     return check(launch_finish(d_partials, splits, rows * out, reinterpret_cast<const __half*>(d_svh), scale_rows,
                                reinterpret_cast<const __half*>(d_bias), rows, out, y_dtype, d_y, as_stream(s)), "finish");
 }
@@ -639,13 +647,21 @@ static int run_forward(const LayerCore& c, const void* d_x, int x_dtype, const u
     return 0;
 }
 
+// The many-row kernel stores four outputs at a time; outputs that do not allow it go through the fused kernel, which stores
+// them one by one (a row shard's are stored by the exchange kernel, one by one as well).
+static bool takes_tensor_cores(const LayerCore& c, int y_dtype, void* const* ys, const b200exl3_tp* tp) {
+    bool wide = g_qmm_enabled;
+    for (int g = 0; g < c.groups; ++g) wide = wide && (tp || four_at_once(ys[g], y_dtype));
+    return wide;
+}
+
 static int forward_common(const LayerCore& c, const void* d_x, int x_dtype, const uint16_t* d_xhat, int64_t rows,
                           void* const* ys, float* d_yhat, void* ws, size_t ws_bytes, cudaStream_t stream,
                           const b200exl3_tp* tp = nullptr, const b200exl3_prologue* pro = nullptr) {
     size_t need = 0;
     if (core_workspace_bytes(c, rows, &need)) return -1;
     QmmLayout layout{};                                       // planned once: what is checked is what runs
-    const bool tensor_cores = rows >= kQmmMinRows && ys && !d_xhat && g_qmm_enabled;
+    const bool tensor_cores = rows >= kQmmMinRows && ys && !d_xhat && takes_tensor_cores(c, x_dtype, ys, tp);
     if (tensor_cores) {
         layout = qmm_layout(c, rows, false, tp != nullptr);
         need = std::max(need, layout.total);
@@ -669,6 +685,7 @@ int b200exl3_linear_forward(const b200exl3_linear* h, const void* d_x, int x_dty
     if (!h) return fail("NULL handle");
     if (!dtype_is_float(x_dtype)) return fail("unsupported input dtype %d", x_dtype);
     if (!d_x || !d_y) return fail("NULL buffer");
+    if (check_rows(d_x, x_dtype) || check_rows(d_y, x_dtype)) return -1;
     void* ys[1] = {d_y};
     return forward_common(h->c, d_x, x_dtype, nullptr, rows, ys, nullptr, ws, ws_bytes, as_stream(s));
 }
@@ -686,6 +703,7 @@ int b200exl3_linear_forward_partial(const b200exl3_linear* h, const void* d_x, i
     if (!h) return fail("NULL handle");
     if (!dtype_is_float(x_dtype)) return fail("unsupported input dtype %d", x_dtype);
     if (!d_x || !d_yhat) return fail("NULL buffer");
+    if (check_rows(d_x, x_dtype)) return -1;
     return forward_common(h->c, d_x, x_dtype, nullptr, rows, nullptr, d_yhat, ws, ws_bytes, as_stream(s));
 }
 
@@ -696,6 +714,7 @@ int b200exl3_linear_finish(const b200exl3_linear* h, const float* d_yhat, int64_
     if (!dtype_is_float(y_dtype)) return fail("unsupported output dtype %d", y_dtype);
     if (!d_yhat || !d_y) return fail("NULL buffer");
     if (!aligned16(d_yhat)) return fail("device pointers must be 16-byte aligned");
+    if (check_rows(d_y, y_dtype)) return -1;
     return check(launch_finish(d_yhat, 1, rows * h->c.out, h->c.svh, 1, h->c.bias, rows, h->c.out, y_dtype, d_y, as_stream(s)),
                  "finish");
 }
@@ -781,10 +800,12 @@ int b200exl3_linear_forward_static(const b200exl3_linear* h, const void* d_x, in
     if (!h) return fail("NULL handle");
     if (!dtype_is_float(x_dtype)) return fail("unsupported input dtype %d", x_dtype);
     if (!d_x || !d_y) return fail("NULL buffer");
+    if (check_rows(d_x, x_dtype) || check_rows(d_y, x_dtype)) return -1;
     if (rows <= 0) return fail("EXL3 linear input cannot be empty");
     const LayerCore& c = h->c;
     QmmLayout layout{};                                       // planned once: what is checked is what runs
-    const bool tensor_cores = rows >= kQmmMinRows && g_qmm_enabled;
+    void* ys[1] = {d_y};
+    const bool tensor_cores = rows >= kQmmMinRows && takes_tensor_cores(c, x_dtype, ys, nullptr);
     if (tensor_cores) {
         layout = qmm_layout(c, rows);
         if (layout.total > kStaticScratchBytes) layout = qmm_layout(c, rows, true);       // without parts the call needs less
@@ -804,7 +825,6 @@ int b200exl3_linear_forward_static(const b200exl3_linear* h, const void* d_x, in
     // last word of the header) is left alone, so a failure stays visible to b200exl3_static_status
     // until that call clears it, as it does in a caller's workspace.
     B200_TRY(cudaMemsetAsync(scratch, 0, kCounterBytes - sizeof(unsigned int), as_stream(s)), "clear static scratch");
-    void* ys[1] = {d_y};
     return run_forward(c, d_x, x_dtype, nullptr, rows, ys, nullptr, scratch, as_stream(s), nullptr, nullptr, tensor_cores ? &layout : nullptr);
 }
 
@@ -899,6 +919,8 @@ int b200exl3_group_forward(const b200exl3_group* h, const void* d_x, int x_dtype
     if (!d_x || !d_ys) return fail("NULL buffer");
     for (int g = 0; g < h->c.groups; ++g)
         if (!d_ys[g]) return fail("NULL buffer");
+        else if (check_rows(d_ys[g], x_dtype)) return -1;
+    if (check_rows(d_x, x_dtype)) return -1;
     return forward_common(h->c, d_x, x_dtype, nullptr, rows, d_ys, nullptr, ws, ws_bytes, as_stream(s));
 }
 
@@ -1232,6 +1254,7 @@ int b200exl3_moe_forward(const b200exl3_moe* h, const void* d_x, int x_dtype, in
     if (score_dtype != kF16 && score_dtype != kF32) return fail("unsupported score dtype %d", score_dtype);
     if (!d_x || !d_selected || !d_scores || !d_y) return fail("NULL buffer");
     if (!aligned16(ws) || !aligned16(d_y)) return fail("device pointers must be 16-byte aligned");
+    if (check_rows(d_x, x_dtype) || check_rows(d_selected, kU32) || check_rows(d_scores, score_dtype)) return -1;
     cudaStream_t stream = as_stream(s);
     char* base = static_cast<char*>(ws);
     const bool exact = (h->flags & B200EXL3_EXACT_WEIGHTS) != 0;
@@ -1370,6 +1393,8 @@ int b200exl3_expert_mapped(const void* d_x, int x_dtype, const uint16_t* d_trell
     if (!dtype_is_float(x_dtype)) return fail("unsupported input dtype %d", x_dtype);
     if (!d_x || !d_trellis || !d_selected || !d_out || (!input_pretransformed && !d_suh) || (!return_raw && !d_svh)) return fail("NULL buffer");
     if (input_pretransformed && x_dtype != kF16) return fail("pretransformed expert input must be fp16");
+    if (check_rows(d_x, x_dtype) || check_rows(d_suh, kF16) || check_rows(d_svh, kF16) || check_rows(d_selected, kU32) ||
+        check_rows(d_out, return_raw ? kF32 : x_dtype)) return -1;
     const int width_tiles = out / 16;
     const int64_t experts = projection_stride_tiles > 0 ? projection_stride_tiles / width_tiles : source_tiles / width_tiles;
     if (experts <= 0 || (projections - 1) * projection_stride_tiles + experts * width_tiles > source_tiles)
@@ -1584,6 +1609,7 @@ int b200exl3_moe_forward_ep(const b200exl3_moe* h, b200exl3_ep* ep, int first_ex
     if (score_dtype != kF16 && score_dtype != kF32) return fail("unsupported score dtype %d", score_dtype);
     if (!d_x || !d_selected || !d_scores || !d_y) return fail("NULL buffer");
     if (!aligned16(ws) || !aligned16(d_y)) return fail("device pointers must be 16-byte aligned");
+    if (check_rows(d_x, x_dtype) || check_rows(d_selected, kU32) || check_rows(d_scores, score_dtype)) return -1;
     if (first_expert < 0) return fail("invalid first expert");
     if (ep->out != h->in) return fail("the exchange buffers were made for rows of %d values, the block produces %d", ep->out, h->in);
     const int64_t chunk = moe_chunk_rows(h);
@@ -1818,6 +1844,7 @@ int b200exl3_linear_forward_tp(const b200exl3_linear* h, b200exl3_tp* tp, const 
     if (!h || !tp) return fail("NULL handle");
     if (!dtype_is_float(x_dtype)) return fail("unsupported input dtype %d", x_dtype);
     if (!d_x || !d_y) return fail("NULL buffer");
+    if (check_rows(d_x, x_dtype) || check_rows(d_y, x_dtype)) return -1;
     if (rows > 0 && rows * (h->c.out / 128) > tp->max_units)
         return fail("%lld units exceed the exchange buffers' %d", static_cast<long long>(rows * (h->c.out / 128)), tp->max_units);
     void* ys[1] = {d_y};
@@ -1831,6 +1858,7 @@ int b200exl3_linear_finish_tp(const b200exl3_linear* h, b200exl3_tp* tp, const f
     if (!dtype_is_float(y_dtype)) return fail("unsupported output dtype %d", y_dtype);
     if (!d_yhat || !d_y) return fail("NULL buffer");
     if (!aligned16(d_yhat)) return fail("device pointers must be 16-byte aligned");
+    if (check_rows(d_y, y_dtype)) return -1;
     const int64_t units = rows * (h->c.out / 128);
     if (units > tp->max_units) return fail("%lld units exceed the exchange buffers' %d", static_cast<long long>(units), tp->max_units);
     TpArgs a{};

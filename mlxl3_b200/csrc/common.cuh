@@ -49,9 +49,19 @@ __device__ __forceinline__ void store_from_half(void* p, int dtype, int64_t i, _
     }
 }
 
-// four consecutive elements (i a multiple of 4) in one load
+// Whether four consecutive elements from a multiple of 4 on may be one access: rows that a caller cut out of a larger buffer
+// need not lie on 8 (16-bit types) or 16 bytes.
+__host__ __device__ __forceinline__ bool four_at_once(const void* p, int dtype) {
+    return (reinterpret_cast<uintptr_t>(p) & (dtype == kF32 ? 15u : 7u)) == 0;
+}
+
+// four consecutive elements (i a multiple of 4): WIDE, in one load, which needs four_at_once(p)
+template <bool WIDE>
 __device__ __forceinline__ void load4_as_half(const void* p, int dtype, int64_t i, __half (&h)[4]) {
-    if (dtype == kF32) {
+    if constexpr (!WIDE) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) h[j] = load_as_half(p, dtype, i + j);
+    } else if (dtype == kF32) {
         const float4 v = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p) + i);
         h[0] = __float2half_rn(v.x); h[1] = __float2half_rn(v.y); h[2] = __float2half_rn(v.z); h[3] = __float2half_rn(v.w);
     } else {
@@ -68,8 +78,15 @@ __device__ __forceinline__ void load4_as_half(const void* p, int dtype, int64_t 
     }
 }
 
-// store_from_half for four consecutive elements (i a multiple of 4) in one store; `bias` points at the first one's bias
+// store_from_half for four consecutive elements (i a multiple of 4); `bias` points at the first one's bias.  WIDE: in one
+// store, which needs four_at_once of both
+template <bool WIDE = true>
 __device__ __forceinline__ void store4_from_half(void* p, int dtype, int64_t i, const __half (&v)[4], const __half* bias) {
+    if constexpr (!WIDE) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) store_from_half(p, dtype, i + j, v[j], bias, j);
+        return;
+    }
     __half b[4];
     if (bias) {
         const uint2 w = *reinterpret_cast<const uint2*>(bias);

@@ -292,6 +292,8 @@ route_plan_grouped_kernel(const uint32_t* __restrict__ selected, int64_t slots, 
 }
 
 // One warp per (slot, 128-block), every projection of the slot's expert: row slot_row of each projection's `slots` rows.
+// WIDE: x lies so that four elements are one access.
+template <bool WIDE>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 routed_prepare_kernel(const void* __restrict__ x, int x_dtype, const __half* __restrict__ suh, const uint32_t* __restrict__ selected,
                       const uint32_t* __restrict__ slot_row, int experts, int64_t slots, int top_k, int proj, int in,
@@ -307,7 +309,7 @@ routed_prepare_kernel(const void* __restrict__ x, int x_dtype, const __half* __r
         const int col = static_cast<int>(unit - slot * blocks_per_row) * 128 + lane * 4;
         const int64_t row = slot_row[slot];
         __half v[4];
-        load4_as_half(x, x_dtype, slot / top_k * in + col, v);
+        load4_as_half<WIDE>(x, x_dtype, slot / top_k * in + col, v);
         const __half* s = suh + static_cast<int64_t>(expert_of(selected, slot, experts)) * proj * in + col;
         for (int p = 0; p < proj; ++p) {
             const uint2 sw = *reinterpret_cast<const uint2*>(s + p * in);
@@ -337,7 +339,7 @@ cudaError_t launch_route_plan(const uint32_t* selected, int64_t slots, int exper
 
 cudaError_t launch_routed_prepare(const void* x, int x_dtype, const __half* suh, const uint32_t* selected, const uint32_t* slot_row,
                                   int experts, int64_t slots, int top_k, int proj, int in, __half* xhat, cudaStream_t stream) {
-    return launch_dependent(routed_prepare_kernel, dim3(grid_for(slots * (in / 128))), dim3(kWarpsPerBlock * 32), 0, stream, x, x_dtype, suh,
+    return launch_dependent(four_at_once(x, x_dtype) ? routed_prepare_kernel<true> : routed_prepare_kernel<false>, dim3(grid_for(slots * (in / 128))), dim3(kWarpsPerBlock * 32), 0, stream, x, x_dtype, suh,
                             selected, slot_row, experts, slots, top_k, proj, in, xhat);
 }
 
