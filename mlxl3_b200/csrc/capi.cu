@@ -7,6 +7,7 @@
 #include <cstdio>
 #include <algorithm>
 #include <cstring>
+#include <initializer_list>
 #include <mutex>
 #include <new>
 #include <string>
@@ -46,6 +47,14 @@ int check(cudaError_t e, const char* what) {
 cudaStream_t as_stream(b200exl3_stream s) { return static_cast<cudaStream_t>(s); }
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+
+// What a kernel reads or writes several elements at a time has to lie on that many bytes.
+struct Place { const void* p; size_t bytes; };
+int check_places(std::initializer_list<Place> places) {
+    for (const Place& at : places)
+        if (reinterpret_cast<uintptr_t>(at.p) % at.bytes != 0) return fail("device pointers must be %zu-byte aligned", at.bytes);
+    return 0;
+}
 
 // Rows of activations may start at any element of a larger buffer, but at an element.
 int check_rows(const void* p, int dtype) {
@@ -381,6 +390,7 @@ int b200exl3_unpack_states(const uint16_t* d_packed, int64_t tiles, int k, int c
     if (valid_format(k, cb)) return -1;
     if (tiles < 0) return fail("packed length is not a whole tile");
     if (tiles > 0 && (!d_packed || (!d_states && !d_values))) return fail("NULL buffer");
+    if (check_places({{d_packed, sizeof(uint16_t)}, {d_states, sizeof(uint16_t)}, {d_values, sizeof(uint16_t)}})) return -1;
     return check(launch_unpack_states(d_packed, tiles, k, cb, d_states, reinterpret_cast<__half*>(d_values), as_stream(s)),
                  "unpack_states");
 }
@@ -388,6 +398,7 @@ int b200exl3_unpack_states(const uint16_t* d_packed, int64_t tiles, int k, int c
 int b200exl3_codebook(const uint16_t* d_states, int64_t n, int cb, uint16_t* d_values, b200exl3_stream s) {
     if (valid_format(1, cb)) return -1;
     if (n < 0 || (n > 0 && !d_values)) return fail("invalid codebook request");
+    if (check_places({{d_states, sizeof(uint16_t)}, {d_values, sizeof(uint16_t)}})) return -1;
     return check(launch_codebook(d_states, n, cb, reinterpret_cast<__half*>(d_values), as_stream(s)), "codebook");
 }
 
@@ -443,6 +454,7 @@ int b200exl3_linear_create(const uint16_t* d_trellis, const void* d_suh, const v
     if (!d_suh || !d_svh) return fail("EXL3 scales have wrong dimensions");
     if (!dtype_is_float(scale_dtype)) return fail("unsupported scale dtype %d", scale_dtype);
     if (!aligned16(d_trellis)) return fail("device pointers must be 16-byte aligned");
+    if (check_rows(d_suh, scale_dtype) || check_rows(d_svh, scale_dtype) || check_rows(d_bias, scale_dtype)) return -1;
     if (out / 128 >= static_cast<int>(kCounterBytes / sizeof(unsigned int))) return fail("output dimension %d is too large", out);
     b200exl3_linear* handle = new (std::nothrow) b200exl3_linear{};
     if (!handle) return fail("out of host memory");
@@ -694,7 +706,7 @@ int b200exl3_linear_forward_raw(const b200exl3_linear* h, const uint16_t* d_xhat
                                 size_t ws_bytes, b200exl3_stream s) {
     if (!h) return fail("NULL handle");
     if (!d_xhat || !d_yhat) return fail("NULL buffer");
-    if (!aligned16(d_xhat)) return fail("device pointers must be 16-byte aligned");
+    if (!aligned16(d_xhat) || !aligned16(d_yhat)) return fail("device pointers must be 16-byte aligned");
     return forward_common(h->c, nullptr, kF16, d_xhat, rows, nullptr, d_yhat, ws, ws_bytes, as_stream(s));
 }
 
@@ -703,7 +715,7 @@ int b200exl3_linear_forward_partial(const b200exl3_linear* h, const void* d_x, i
     if (!h) return fail("NULL handle");
     if (!dtype_is_float(x_dtype)) return fail("unsupported input dtype %d", x_dtype);
     if (!d_x || !d_yhat) return fail("NULL buffer");
-    if (check_rows(d_x, x_dtype)) return -1;
+    if (check_rows(d_x, x_dtype) || check_places({{d_yhat, 16}})) return -1;
     return forward_common(h->c, d_x, x_dtype, nullptr, rows, nullptr, d_yhat, ws, ws_bytes, as_stream(s));
 }
 
@@ -748,7 +760,9 @@ static int check_prologue(const b200exl3_prologue* pro, const void* d_x, int64_t
     if (pro->kind == 1 && pro->d_sum == d_x) return fail("the RMSNorm prologue cannot store the sum over its own input");
     if (pro->kind == 2 && !pro->d_aux) return fail("the SwiGLU prologue needs the up rows");
     if (!aligned16(pro->d_aux) || !aligned16(pro->d_weight) || !aligned16(pro->d_sum)) return fail("device pointers must be 16-byte aligned");
-    return 0;
+    // the sum over a row reads eight values at a time, the other prologues four, a plain rotation one
+    return check_places({{d_x, pro->kind == 1 ? size_t(16) : pro->kind != 0 ? size_t(8) : sizeof(__half)}, {pro->d_sumsq, sizeof(float)},
+                         {pro->d_sumsq_out, sizeof(float)}, {pro->d_pos, sizeof(int32_t)}});
 }
 
 int b200exl3_linear_forward_fused(const b200exl3_linear* h, const b200exl3_prologue* pro, b200exl3_tp* tp, const void* d_x, int64_t rows,
@@ -757,6 +771,7 @@ int b200exl3_linear_forward_fused(const b200exl3_linear* h, const b200exl3_prolo
     if (!d_x || (!d_y && !(pro && pro->epilogue == 1))) return fail("NULL buffer");
     if (check_prologue(pro, d_x, rows)) return -1;
     if (pro->epilogue == 2) return fail("the rotary epilogue belongs to a [q | k | v] group");
+    if (check_rows(d_y, kF16)) return -1;
     if (tp && rows * (h->c.out / 128) > tp->max_units) return fail("units exceed the exchange buffers' %d", tp->max_units);
     void* ys[1] = {d_y};
     return forward_common(h->c, d_x, kF16, nullptr, rows, ys, nullptr, ws, ws_bytes, as_stream(s), tp, pro);
@@ -931,6 +946,9 @@ int b200exl3_group_forward_fused(const b200exl3_group* h, const b200exl3_prologu
     if (check_prologue(pro, d_x, rows)) return -1;
     for (int g = 0; g < h->c.groups; ++g)
         if (!d_ys[g] && !(pro->epilogue == 2 && g > 0)) return fail("NULL buffer");       // the rotary epilogue writes k and v to the caches
+    for (int g = 0; g < h->c.groups; ++g)
+        if (check_rows(d_ys[g], kF16)) return -1;
+    if (pro->epilogue == 2 && check_places({{d_ys[0], 8}})) return -1;                    // rotated heads are stored four values at a time
     if (pro->epilogue == 1) return fail("the residual epilogue belongs to plain layers");
     if (pro->epilogue == 2) {
         const LayerCore& c = h->c;
@@ -1192,6 +1210,8 @@ int b200exl3_moe_create(const uint16_t* d_gu_trellis, const void* d_gu_suh, cons
         return fail("SwitchGLU trellis/scales disagree");
     if (!dtype_is_float(scale_dtype)) return fail("unsupported scale dtype %d", scale_dtype);
     if (!aligned16(d_gu_trellis) || !aligned16(d_down_trellis)) return fail("device pointers must be 16-byte aligned");
+    for (const void* p : {d_gu_suh, d_gu_svh, d_down_suh, d_down_svh})
+        if (check_rows(p, scale_dtype)) return -1;
     b200exl3_moe* h = new (std::nothrow) b200exl3_moe{};
     if (!h) return fail("out of host memory");
     h->experts = experts; h->in = in; h->hidden = hidden; h->top_k = top_k; h->k = k; h->cb = cb; h->flags = flags;
@@ -1394,7 +1414,7 @@ int b200exl3_expert_mapped(const void* d_x, int x_dtype, const uint16_t* d_trell
     if (!d_x || !d_trellis || !d_selected || !d_out || (!input_pretransformed && !d_suh) || (!return_raw && !d_svh)) return fail("NULL buffer");
     if (input_pretransformed && x_dtype != kF16) return fail("pretransformed expert input must be fp16");
     if (check_rows(d_x, x_dtype) || check_rows(d_suh, kF16) || check_rows(d_svh, kF16) || check_rows(d_selected, kU32) ||
-        check_rows(d_out, return_raw ? kF32 : x_dtype)) return -1;
+        check_rows(d_out, x_dtype) || check_places({{d_trellis, sizeof(uint32_t)}, {d_out, return_raw ? size_t(16) : size_t(1)}})) return -1;
     const int width_tiles = out / 16;
     const int64_t experts = projection_stride_tiles > 0 ? projection_stride_tiles / width_tiles : source_tiles / width_tiles;
     if (experts <= 0 || (projections - 1) * projection_stride_tiles + experts * width_tiles > source_tiles)
@@ -1452,6 +1472,7 @@ int b200exl3_swiglu_down_input(const float* d_gate_up_raw, const uint16_t* d_gu_
     if (experts <= 0 || slots <= 0 || hidden <= 0 || hidden % 128) return fail("invalid SwiGLU glue dimensions");
     if (!d_gate_up_raw || !d_gu_svh || !d_down_suh || !d_selected || !d_xhat) return fail("NULL buffer");
     if (!aligned16(d_gate_up_raw) || !aligned16(d_xhat)) return fail("device pointers must be 16-byte aligned");
+    if (check_places({{d_gu_svh, sizeof(__half)}, {d_down_suh, sizeof(__half)}, {d_selected, sizeof(uint32_t)}})) return -1;
     return check(launch_glu_down_input(d_gate_up_raw, reinterpret_cast<const __half*>(d_gu_svh), reinterpret_cast<const __half*>(d_down_suh),
                                        d_selected, experts, slots, hidden, hidden, reinterpret_cast<__half*>(d_xhat), as_stream(s)), "SwiGLU glue");
 }
@@ -1462,6 +1483,7 @@ int b200exl3_finish_and_reduce(const float* d_raw, const uint16_t* d_svh, const 
     if (score_dtype != kF16 && score_dtype != kF32) return fail("unsupported score dtype %d", score_dtype);
     if (!d_raw || !d_svh || !d_selected || !d_scores || !d_y) return fail("NULL buffer");
     if (!aligned16(d_raw) || !aligned16(d_y)) return fail("device pointers must be 16-byte aligned");
+    if (check_places({{d_svh, 8}, {d_selected, sizeof(uint32_t)}, {d_scores, dtype_size(score_dtype)}})) return -1;
     return check(launch_finish_and_reduce(d_raw, reinterpret_cast<const __half*>(d_svh), d_selected, experts, d_scores, score_dtype, rows, top_k,
                                           out, d_y, as_stream(s)), "expert reduction");
 }
@@ -1480,6 +1502,7 @@ int b200exl3_router_topk(const void* d_values, int dtype, int64_t rows, int expe
                          uint32_t* d_indices, void* d_scores, b200exl3_stream s) {
     if (router_check(rows, experts, top_k, dtype)) return -1;
     if (!d_values || !d_indices || !d_scores) return fail("NULL buffer");
+    if (check_places({{d_values, dtype_size(dtype)}, {d_indices, sizeof(uint32_t)}, {d_scores, dtype_size(dtype)}})) return -1;
     return check(launch_router_topk(d_values, dtype, rows, experts, top_k, normalize != 0, false, d_indices, d_scores, nullptr,
                                     as_stream(s)), "router kernel");
 }
@@ -1488,6 +1511,8 @@ int b200exl3_router_softmax_topk(const void* d_logits, int dtype, int64_t rows, 
                                  uint32_t* d_indices, void* d_scores, void* d_probabilities, b200exl3_stream s) {
     if (router_check(rows, experts, top_k, dtype)) return -1;
     if (!d_logits || !d_indices || !d_scores) return fail("NULL buffer");
+    if (check_places({{d_logits, dtype_size(dtype)}, {d_indices, sizeof(uint32_t)}, {d_scores, dtype_size(dtype)}, {d_probabilities, dtype_size(dtype)}}))
+        return -1;
     return check(launch_router_topk(d_logits, dtype, rows, experts, top_k, normalize != 0, true, d_indices, d_scores,
                                     d_probabilities, as_stream(s)), "router kernel");
 }
@@ -1497,6 +1522,7 @@ int b200exl3_router_gate(const void* d_x, int x_dtype, const uint16_t* d_weight_
     if (rows <= 0 || rows > 8 * 65535ll || in <= 0 || in % 2 || experts <= 0) return fail("invalid router gate dimensions");
     if (!dtype_is_float(x_dtype)) return fail("unsupported input dtype %d", x_dtype);
     if (!d_x || !d_weight_f16 || !d_logits_f16) return fail("NULL buffer");
+    if (check_places({{d_x, dtype_size(x_dtype)}, {d_weight_f16, sizeof(__half2)}, {d_logits_f16, sizeof(__half)}})) return -1;
     return check(launch_router_gate(d_x, x_dtype, reinterpret_cast<const __half*>(d_weight_f16), rows, in, experts,
                                     reinterpret_cast<__half*>(d_logits_f16), as_stream(s)), "router gate kernel");
 }
@@ -1675,6 +1701,7 @@ int b200exl3_embed(const uint16_t* d_table, const int32_t* d_tokens, int64_t row
     if (rows <= 0 || rows > INT32_MAX || vocab <= 0 || hidden <= 0 || hidden % 8) return fail("invalid embedding dimensions");
     if (!d_table || !d_tokens || !d_out) return fail("NULL buffer");
     if (!aligned16(d_table) || !aligned16(d_out)) return fail("device pointers must be 16-byte aligned");
+    if (check_places({{d_tokens, sizeof(int32_t)}})) return -1;
     return check(launch_embed(reinterpret_cast<const __half*>(d_table), d_tokens, rows, vocab, hidden, reinterpret_cast<__half*>(d_out),
                               as_stream(s)), "embedding kernel");
 }
@@ -1684,6 +1711,8 @@ int b200exl3_rms_norm(const uint16_t* d_x, const uint16_t* d_residual, const uin
     if (rows <= 0 || rows > INT32_MAX || n <= 0 || n % 2 || n > 48 * 1024) return fail("invalid RMSNorm dimensions");
     if (!(eps >= 0.0f)) return fail("invalid RMSNorm epsilon");
     if (!d_x || !d_weight || !d_y) return fail("NULL buffer");
+    if (check_places({{d_x, sizeof(__half2)}, {d_residual, sizeof(__half2)}, {d_weight, sizeof(__half2)}, {d_sum, sizeof(__half2)},
+                      {d_y, sizeof(__half2)}})) return -1;
     return check(launch_rms_norm(reinterpret_cast<const __half*>(d_x), reinterpret_cast<const __half*>(d_residual),
                                  reinterpret_cast<const __half*>(d_weight), rows, n, eps, reinterpret_cast<__half*>(d_sum),
                                  reinterpret_cast<__half*>(d_y), as_stream(s)), "RMSNorm kernel");
@@ -1692,6 +1721,7 @@ int b200exl3_rms_norm(const uint16_t* d_x, const uint16_t* d_residual, const uin
 int b200exl3_swiglu(const uint16_t* d_gate, const uint16_t* d_up, int64_t n, uint16_t* d_out, b200exl3_stream s) {
     if (n <= 0 || n % 2) return fail("invalid SwiGLU length");
     if (!d_gate || !d_up || !d_out) return fail("NULL buffer");
+    if (check_places({{d_gate, sizeof(__half2)}, {d_up, sizeof(__half2)}, {d_out, sizeof(__half2)}})) return -1;
     return check(launch_swiglu(reinterpret_cast<const __half*>(d_gate), reinterpret_cast<const __half*>(d_up), n,
                                reinterpret_cast<__half*>(d_out), as_stream(s)), "SwiGLU kernel");
 }
@@ -1707,6 +1737,8 @@ int b200exl3_rope_append(uint16_t* d_q, const uint16_t* d_k, const uint16_t* d_v
     if (attention_shape(heads, kv_heads, head_dim, max_ctx)) return -1;
     if (!(theta > 1.0f)) return fail("invalid RoPE base");
     if (!d_q || !d_k || !d_v || !d_pos || !d_k_cache || !d_v_cache) return fail("NULL buffer");
+    if (check_places({{d_q, sizeof(__half)}, {d_k, sizeof(__half)}, {d_v, sizeof(__half2)}, {d_pos, sizeof(int32_t)},
+                      {d_k_cache, sizeof(__half)}, {d_v_cache, sizeof(__half2)}})) return -1;
     return check(launch_rope_append(reinterpret_cast<__half*>(d_q), reinterpret_cast<const __half*>(d_k), reinterpret_cast<const __half*>(d_v),
                                     heads, kv_heads, head_dim, d_pos, theta, max_ctx, reinterpret_cast<__half*>(d_k_cache),
                                     reinterpret_cast<__half*>(d_v_cache), as_stream(s)), "RoPE kernel");
@@ -1725,6 +1757,7 @@ int b200exl3_attention_decode(const uint16_t* d_q, const uint16_t* d_k_cache, co
     if (attention_shape(heads, kv_heads, head_dim, max_ctx)) return -1;
     if (!d_q || !d_k_cache || !d_v_cache || !d_pos || !d_out) return fail("NULL buffer");
     if (!aligned16(d_q) || !aligned16(d_k_cache) || !aligned16(d_v_cache) || !aligned16(ws)) return fail("device pointers must be 16-byte aligned");
+    if (check_places({{d_pos, sizeof(int32_t)}, {d_out, 8}})) return -1;
     const size_t need = round256(attention_workspace_bytes(heads, kv_heads));
     if (!ws || ws_bytes < need) return fail("workspace too small: %zu bytes given, %zu needed", ws_bytes, need);
     return check(launch_attention_decode(reinterpret_cast<const __half*>(d_q), reinterpret_cast<const __half*>(d_k_cache),
@@ -1743,6 +1776,7 @@ int b200exl3_head_argmax(const uint16_t* d_x, const uint16_t* d_weight, int64_t 
     if (vocab <= 0 || hidden <= 0 || hidden % 8 || hidden > 48 * 1024) return fail("invalid head dimensions");
     if (!d_x || !d_weight || !d_best_value || !d_best_index) return fail("NULL buffer");
     if (!aligned16(d_x) || !aligned16(d_weight) || !aligned16(ws)) return fail("device pointers must be 16-byte aligned");
+    if (check_places({{d_logits, sizeof(__half)}, {d_best_value, sizeof(float)}, {d_best_index, sizeof(int64_t)}})) return -1;
     size_t need = 0;
     b200exl3_head_workspace_bytes(&need);
     if (!ws || ws_bytes < need) return fail("workspace too small: %zu bytes given, %zu needed", ws_bytes, need);

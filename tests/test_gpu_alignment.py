@@ -114,3 +114,35 @@ def test_expert_block_input_at_any_element(gpu, rows):
         with pytest.raises(gpu.B200Exl3Error, match="aligned to their elements"):
             moe.forward_device(args[0], gpu.F32, rows, args[1], args[2], gpu.F16, d_y.ptr, ws)
     moe.close()
+
+
+def test_calls_that_need_wider_places_say_so(gpu):
+    """Raw products are stored four floats at a time; fused operators read four or eight values at a time."""
+    from ctypes import c_void_p
+
+    from mlxl3_b200 import _lib
+    from mlxl3_b200.linear import Prologue
+    rng = np.random.default_rng(2)
+    n, k = 256, 4
+    t, suh, svh = random_layer(rng, n, n, k)
+    layer = gpu.Exl3Linear(t, suh, svh, None, k, 0)
+    x = rng.standard_normal((1, n)).astype(np.float16)
+    keep, d_x = at(gpu, x, 0)
+    ws = gpu.new_workspace(layer.workspace_bytes(1))
+    y, d_y, read = out(gpu, (2, n), np.float32, 0)
+    w, d_w = at(gpu, np.ones(n, np.float16), 0)
+    with pytest.raises(gpu.B200Exl3Error, match="must be 16-byte aligned"):
+        _lib.call("b200exl3_linear_forward_raw", c_void_p(layer.handle), c_void_p(d_x), 1, c_void_p(d_y + 8), c_void_p(ws.ptr), ws.nbytes, None)
+    with pytest.raises(gpu.B200Exl3Error, match="must be 16-byte aligned"):
+        layer.forward_partial_device(d_x, gpu.F16, 1, d_y + 4, ws)
+    with pytest.raises(gpu.B200Exl3Error, match="must be 16-byte aligned"):
+        layer.forward_fused_device(Prologue.rms_norm(d_w, 1e-5), d_x + 8, 1, d_y, ws)
+    with pytest.raises(gpu.B200Exl3Error, match="must be 8-byte aligned"):
+        layer.forward_fused_device(Prologue.swiglu(d_w), d_x + 4, 1, d_y, ws)
+    # rows on 8 bytes are enough for the SwiGLU prologue, as before
+    k8, d_x8 = at(gpu, x, 4)
+    layer.forward_fused_device(Prologue.swiglu(d_w), d_x8, 1, d_y, ws)
+    got = read().reshape(-1).view(np.float16)[:n].copy()
+    layer.forward_fused_device(Prologue.swiglu(d_w), d_x, 1, d_y, ws)
+    assert np.array_equal(bits(got), bits(read().reshape(-1).view(np.float16)[:n]))
+    layer.close()
