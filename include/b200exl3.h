@@ -80,10 +80,11 @@ int b200exl3_set_option(const char* name, int64_t value);
 /* The launch policy as data, for tests and reports (replaces the Kani proofs beside exl3_projection_splits and
  * qmv_batch_layout, native/src/contracts.rs:1995-2012, 1051-1069, by values an exhaustive test can check; needs no GPU:
  * without one the planners assume 148 multiprocessors).  kind "qmv": {CTAs, bound on CTAs sharing a column block,
- * column blocks, warps per CTA, shared memory per CTA, kernel rotates the rows itself}; "qmm": {1, blocks
- * of 512 rows (1 up to 64 rows), up to 64 rows, 64-input stages, tokens per tile, CTAs per tile and 128 columns (0 = one wave
- * of CTAs with equal runs of stages), rows per launch, bytes for parts of shared tiles}; "stack": {CTAs, bound on CTAs per block, column blocks, warps per CTA, shared
- * memory, warps that share the layer, 32-bit partition arithmetic, layer accepted}. */
+ * column blocks, warps per CTA, shared memory per CTA, kernel rotates the rows itself}; "qmm": {CTAs, token tiles
+ * of a launch, items of a launch (tile x 128 columns), 128-input stages of an item, tokens per tile, CTAs per item
+ * (0 = one wave of CTAs with equal runs of stages), rows per launch, bytes for parts of shared items}; "stack":
+ * {CTAs, bound on CTAs per block, column blocks, warps per CTA, shared memory, warps that share the layer, 32-bit
+ * partition arithmetic, layer accepted}. */
 int b200exl3_plan_query(const char* kind, int in, int out, int k, int64_t rows, int64_t* out_values, int capacity);
 
 /* Plain device-memory plumbing for hosts that have no CUDA binding of their own (replaces

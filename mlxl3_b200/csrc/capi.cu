@@ -212,9 +212,9 @@ int b200exl3_plan_query(const char* kind, int in, int out, int k, int64_t rows, 
         return 0;
     }
     if (!strcmp(kind, "qmm")) {
-        // tiles of 512 rows are a unit of the report only: the launch takes smaller ones where that is faster
-        out_values[0] = 1; out_values[1] = rows <= 64 ? 1 : (rows + 511) / 512; out_values[2] = rows <= 64 ? 1 : 0; out_values[3] = in / 64;
         const QmmPlan p = plan_qmm(in, out, rows);
+        const int64_t tiles = (p.pass_rows + p.tile_tokens - 1) / p.tile_tokens, items = tiles * (out / 128), stages = in / kQmmStageIn;
+        out_values[0] = qmm_grid(p, items, stages); out_values[1] = tiles; out_values[2] = items; out_values[3] = stages;
         out_values[4] = p.tile_tokens; out_values[5] = p.splits; out_values[6] = p.pass_rows; out_values[7] = static_cast<int64_t>(p.piece_bytes);
         return 0;
     }

@@ -346,6 +346,9 @@ struct QmmPlan {
 };
 // `out` counts all members of a group; `whole_items`: no item is shared, so no scratch for pieces
 QmmPlan plan_qmm(int in, int out, int64_t rows, bool whole_items = false);
+constexpr int kQmmStageIn = 128;     // inputs of a stage
+// CTAs of a launch over `items` items of `stages` stages
+int64_t qmm_grid(const QmmPlan& plan, int64_t items, int64_t stages);
 constexpr int kQmmSegRows = 64;      // rows of an expert segment
 struct QmmArgs {
     const uint32_t* wq;        // quad layout

@@ -42,7 +42,6 @@ namespace {
 
 // The single-thread roles take the lowest warp numbers: the scheduler favours older warps.
 constexpr int kMmaWarp = 0, kWeightWarp = 1, kActWarp = 2, kFirstDecoder = 4;
-constexpr int kStageIn = 128;                          // inputs of a stage
 constexpr int kStageCols = 64;                         // tensor-memory columns of an A stage: two fp16 inputs each
 constexpr int kChunk = 16;                             // tokens four warps finish at a time
 
@@ -277,7 +276,7 @@ qmm_kernel(const __grid_constant__ CUtensorMap xmap, const QmmArgs p) {
     __shared__ volatile int s_failed;
 
     const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;   // warp: uniform
-    const uint32_t spi = static_cast<uint32_t>(p.in) / kStageIn;                       // stages of an item
+    const uint32_t spi = static_cast<uint32_t>(p.in) / kQmmStageIn;                       // stages of an item
     const uint32_t items = p.map_expert != nullptr ? static_cast<uint32_t>(*p.map_count * p.map_proj * p.map_blocks) : static_cast<uint32_t>(p.items);
     // one run per CTA, at least one stage each; the launch keeps total * CTAs below 2^32
     const uint32_t total = items * spi, G = min(gridDim.x, total);
@@ -544,7 +543,7 @@ qmm_kernel(const __grid_constant__ CUtensorMap xmap, const QmmArgs p) {
         if (elect_one()) {
             pdl_wait();
             uint32_t item = first_item, par = 0;
-            int done_before = 0, rem = min(count, static_cast<int>(spi - k0)), x = static_cast<int>(k0) * kStageIn;
+            int done_before = 0, rem = min(count, static_cast<int>(spi - k0)), x = static_cast<int>(k0) * kQmmStageIn;
             int run = rem;                                                       // stages of the current item here
             QmmItem info = qmm_item<NT>(p, item);
             int boxes = p.map_expert != nullptr ? (info.n + 15) >> 4 : 1;        // expert segments come in boxes of 16 rows
@@ -578,7 +577,7 @@ qmm_kernel(const __grid_constant__ CUtensorMap xmap, const QmmArgs p) {
                             tma_load_2d(dst + S::kBHalfBytes + b * 2048, &xmap, x + 64, info.brow + b * 16, &full[s]);
                         }
                     }
-                    x += kStageIn;
+                    x += kQmmStageIn;
                     if (--rem == 0) {
                         done_before += run;
                         if (done_before == count) { running = false; break; }
@@ -728,7 +727,7 @@ static std::atomic<int> g_qmm_splits{0};                              // 0 = one
 void qmm_set_tuning(int splits) { g_qmm_splits = splits > 0 ? splits : 0; }
 
 // CTAs of a launch over `items` items of `stages` stages: the same number for every item, or one wave of equal runs.
-static int64_t qmm_grid(const QmmPlan& plan, int64_t items, int64_t stages) {
+int64_t qmm_grid(const QmmPlan& plan, int64_t items, int64_t stages) {
     return plan.splits > 0 ? items * plan.splits : std::min<int64_t>(sm_count(), items * stages);
 }
 static size_t qmm_piece_count(int64_t items, int64_t grid) { return static_cast<size_t>(items < grid ? grid + items : 2 * grid); }
@@ -753,7 +752,7 @@ static double qmm_cost_us(int64_t sms, int64_t items, int64_t stages, int tile, 
 
 static QmmPlan make_qmm_plan(int in, int out, int64_t rows, bool whole_items, int forced, int64_t sms) {
     QmmPlan plan{};
-    const int64_t col_blocks = out / 128, stages = in / kStageIn;
+    const int64_t col_blocks = out / 128, stages = in / kQmmStageIn;
     // the items of one launch need an arrival counter each, and stages x CTAs must fit 32 bits: more rows go in passes
     const int64_t max_items = std::min<int64_t>(4000, (int64_t{1} << 31) / (stages * 1024));
     const int64_t max_tiles = std::max<int64_t>(1, max_items / col_blocks);
@@ -800,7 +799,7 @@ cudaError_t launch_qmm(QmmArgs p, const __half* xhat, int k, int cb, const QmmPl
     p.tiles = (p.rows + plan.tile_tokens - 1) / plan.tile_tokens;
     p.items = p.tiles * (p.out / 128);
     p.trace = g_qmm_trace.load();
-    const int64_t stages = p.in / kStageIn, grid = qmm_grid(plan, p.items, stages);
+    const int64_t stages = p.in / kQmmStageIn, grid = qmm_grid(plan, p.items, stages);
     if (p.items * stages * grid >= (int64_t{1} << 32)) return cudaErrorInvalidValue;
     return qmm_dispatch(k, cb, map, p, static_cast<int>(grid), plan.tile_tokens <= 64, stream);
 }
@@ -809,7 +808,7 @@ size_t qmm_mapped_piece_bytes() { return static_cast<size_t>(sm_count()) * 2 * k
 
 cudaError_t launch_qmm_mapped(QmmArgs p, const __half* xhat, int max_segments, int k, int cb, cudaStream_t stream) {
     if (p.in % 128 || p.map_blocks <= 0 || max_segments <= 0 || p.map_proj <= 0 || p.map_slots <= 0 || p.yhat == nullptr) return cudaErrorInvalidValue;
-    const int64_t stages = static_cast<int64_t>(max_segments) * p.map_proj * p.map_blocks * (p.in / kStageIn);
+    const int64_t stages = static_cast<int64_t>(max_segments) * p.map_proj * p.map_blocks * (p.in / kQmmStageIn);
     if (stages * sm_count() >= (int64_t{1} << 32)) return cudaErrorInvalidValue;
     CUtensorMap map;
     constexpr int box = 16;      // segments are short: only the boxes that hold rows are fetched (the last may reach into the next segment's)

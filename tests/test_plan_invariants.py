@@ -7,8 +7,8 @@ Invariants:
   never exceeds one 128-column block's worth (so it touches at most two blocks and owns two staging buffers), the
   stated bound on the CTAs that share a column block holds for every block, every tile belongs to exactly one warp;
   where every block goes to a whole number of warps, no warp works on two blocks and the largest share did not grow;
-* tensor-core product: every input split keeps at least 8 stages of 64 inputs (or there is one split), the token
-  tiles cover the rows, the small shape is used up to 64 rows.
+* tensor-core product: the token tiles cover a pass, every CTA's run has a stage at least, CTAs per item are the same for
+  all items or the runs are equal, and every part of a shared item has a place of its own inside the room for parts.
 """
 import ctypes
 
@@ -90,16 +90,43 @@ def test_decode_step_partition(k):
     assert query("stack", 128, 128 * 4000, k, 1)[7] == 0
 
 
+def qmm_runs(items, stages, grid):
+    """First and last stage of every CTA's run, as the kernel deals the stages of all items out."""
+    total = items * stages
+    bounds = (np.arange(grid + 1, dtype=np.uint64) * total) // grid
+    assert total * grid < 2 ** 32                                                       # the kernel's products are 32 bits wide
+    return bounds[:-1].astype(np.int64), bounds[1:].astype(np.int64)
+
+
 def test_tensor_core_splits():
+    seen = set()
     for n_in in DIMS_IN:
         for n_out in DIMS_OUT:
-            for rows in (9, 16, 64, 65, 256, 512, 513, 2048):
-                splits, token_tiles, small, stages = query("qmm", n_in, n_out, 4, rows)[:4]
-                assert stages == n_in // 64 and splits >= 1
-                assert splits == 1 or stages // splits >= 8
-                assert small == (1 if rows <= 64 else 0)
-                tile = 64 if small else 512
-                assert token_tiles == -(-rows // tile)
+            for rows in (9, 16, 64, 65, 256, 512, 513, 2048, 40000):
+                grid, tiles, items, stages, tile, splits, pass_rows, part_bytes = query("qmm", n_in, n_out, 4, rows)
+                assert stages == n_in // 128 and items == tiles * n_out // 128
+                assert (tiles - 1) * tile < pass_rows <= tiles * tile and pass_rows <= rows
+                assert grid == (items * splits if splits else min(148, items * stages))
+                first, last = qmm_runs(items, stages, grid)
+                assert (last > first).all()                                             # no CTA without work
+                item0, item1 = first // stages, (last - 1) // stages
+                if splits:
+                    # every item belongs to `splits` CTAs of its own, so no run crosses an item's end
+                    assert (item0 == item1).all() and (np.bincount(item0, minlength=items) == splits).all()
+                # parts: (CTA, item) pairs that do not hold the whole item, each in a place of its own inside the room
+                places = []
+                for cta in range(grid):
+                    for item in range(item0[cta], item1[cta] + 1):
+                        if first[cta] <= item * stages and last[cta] >= (item + 1) * stages:
+                            continue
+                        # a run has such a part at its two ends only: with more items than CTAs two places per CTA are enough
+                        assert item in (item0[cta], item1[cta])
+                        places.append(cta + item if items < grid else 2 * cta + (1 if item > item0[cta] else 0))
+                assert len(set(places)) == len(places)
+                assert not places or (max(places) + 1) * tile * 128 * 4 <= part_bytes
+                seen.add("shared" if places else "whole")
+                seen.add("equal runs" if splits == 0 else "per item")
+    assert seen == {"shared", "whole", "equal runs", "per item"}
 
 
 def test_query_validation():
