@@ -17,14 +17,19 @@
 //  * packed words: one bulk copy per stage (8 tile rows x 8 tiles are contiguous in the quad layout);
 //  * one thread issues the stage's eight products and one commit, which frees the A stage and the activation slot.
 //
-// What bounds it: the decode (60 to 70 cycles per tile and scheduler with everything else running; 49 at 4 bits, 53 at 3
-// bits alone), at NT = 256 nearly the products as well (1024 cycles of a stage's 1400).  Stages of 128 inputs and a single
-// barrier per stage are there because the single-thread roles share the schedulers with decoders that keep the integer
-// pipes full: an instruction of theirs takes about eight cycles, a stage of any of them 400 to 600.  For the same reason
-// the issuing loop is unrolled over the ring and its thread picked by elect.sync, so that addresses and descriptors are
-// constants in uniform registers; the producers' loops stay rolled (all three unrolled: instruction fetch stalls, 714 ns
-// per 64 inputs against 523).  Measured: 64 rows 4096->14336, 4 bits, 42 -> 29.7 us with the input rotation; 16 rows
-// 5120->25600, 3 bits, 74 -> 48.2 us (A in shared memory, one CTA per item and 64-token tile before).
+// What bounds it: up to 64 rows the decode.  Cycles per 16x16 tile and scheduler with sixteen decoder warps: the decode loop
+// alone (words resident in shared memory, tensor-memory stores and nothing else) 47 at 4 bits, 51 at 3, 52 at 1 and 2, 54 at 5
+// and 6; in the kernel 59 at 4 bits and 68 at 3, and another 5 to 8 of waits for packed words and for the products.  A stage
+// takes 1060 to 1230 cycles (16 rows, 5120 inputs), 0.58 to 0.66 us at the 1845 MHz that the cycle counter shows against the
+// global timer while tensor-core instructions run (nvidia-smi reports 1965).  That depends neither on how many SMs work (3 bits:
+// 1180 cycles with 37, 1181 with 74, 1199 with 148) nor on where the weights come from (1167 when all stages read the same
+// ones).  At NT = 256 a stage takes 1320 cycles, 1024 of them products, and back to back the power cap holds the clock at 1560.
+// Stages of 128 inputs and a single barrier per stage are there because the single-thread roles share the schedulers with
+// decoders that keep the integer pipes full: an instruction of theirs takes about eight cycles, a stage of any of them 400 to
+// 600.  For the same reason the issuing loop is unrolled over the ring and its thread picked by elect.sync; the producers'
+// loops stay rolled (all three unrolled: 714 ns per 64 inputs against 523).  Measured: 64 rows 4096->14336, 4 bits, 42 -> 29.7 us
+// with the input rotation; 16 rows 5120->25600, 3 bits, 74 -> 48.2 us (A in shared memory, one CTA per item and 64-token tile
+// before).
 // Every wait is bounded in time; a wait that gives up sets the status word and the kernel still releases its tensor memory.
 #include <cuda.h>
 
@@ -96,9 +101,8 @@ __device__ __forceinline__ void umma_f16_ts(uint32_t d, uint32_t a, uint64_t bde
         "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}"
         ::"r"(d), "r"(a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
-// One lane of a converged warp, chosen so that the compiler knows the branch is warp-uniform: the descriptors then live
-// in uniform registers.  Under `if (lane == 0)` every product was wrapped in a loop that moves them there one lane at a
-// time: 68 cycles per issued product against 30 (128 x 16..64 tile, measured back to back).
+// One lane of a converged warp.  Products issued under `if (elect_one())` take 30 cycles each, under `if (lane == 0)` 68
+// (128 x 16..64 tile, back to back): the first branch is known to be uniform, as the descriptors' registers want it.
 __device__ __forceinline__ bool elect_one() {
     uint32_t p;
     asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(p));
@@ -144,8 +148,11 @@ __device__ __noinline__ bool qmm_wait_slow(uint64_t* bar, uint32_t parity, volat
 __device__ __forceinline__ bool qmm_wait(uint64_t* bar, uint32_t parity, volatile int* cta_failed) {
     return mbar_try_wait(bar, parity) || qmm_wait_slow(bar, parity, cta_failed);
 }
-// Barrier of some warps.  Lanes may come from, and leave, the barrier one by one; the tcgen05 instructions around it want
-// the warp as one, which the warp barriers state.
+// Barrier of some warps.  Not the aligned form (`bar.sync`), which all lanes of a warp have to execute as one: lanes come here
+// from branches of their own (lane 0 from an atomic or an arrival), where nothing but a warp barrier brings them together again.
+// The same holds for the instructions marked .sync.aligned -- allocation and release of tensor memory, its loads and stores and
+// the waits for them: each has a warp barrier before it with no branch on the lane, no elected lane and no polling loop in
+// between, and the branches around it are on values that all lanes share (warp, item, token counts).
 __device__ __forceinline__ void group_sync(int id, int threads) {
     __syncwarp();
     asm volatile("barrier.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
@@ -734,11 +741,14 @@ static size_t qmm_piece_count(int64_t items, int64_t grid) { return static_cast<
 
 // How a batch is cut up: tokens per item and CTAs per item (or one wave of equal runs).  The estimate below is fitted to 1160
 // measured launches (512 to 14336 inputs, 512 to 25600 outputs, 16 to 2000 rows, 3, 4 and 6 bits; its choice is 1.2 % above
-// the best measured one on average): a fixed part; a stage, mostly decode, with a share that grows with the tokens and more of
-// both the more SMs are busy (they share the second-level cache and the power); the epilogue of every item or part of one;
-// parts that are written, counted and read again by the last CTA; and a run that starts in one item and ends in another.  So
-// small tiles (every tile decodes the weights again) win where the layer alone gives the SMs too little to do: 256 rows of
-// 2048 -> 2048 take 15.7 us as 4 tiles of 64 rows and 39 as one tile in 148 equal runs.
+// the best measured one on average): a fixed part; a stage, mostly decode, with a share that grows with the tokens; the epilogue
+// of every item or part of one; parts that are written, counted and read again by the last CTA; and a run that starts in one item
+// and ends in another.  So small tiles (every tile decodes the weights again) win where the layer alone gives the SMs too little
+// to do: 256 rows of 2048 -> 2048 take 15.7 us as 4 tiles of 64 rows and 39 as one tile in 148 equal runs.
+// What it does not say: the bits are no term (64 rows 4096 -> 14336 at 4 bits come out at 29 us, measured 24.4; 1, 2, 5, 7 and 8
+// bits were not in the fit), so it ranks the ways to cut one layer and predicts no times.  `load` makes a launch dearer the more
+// SMs it takes although a stage takes the same cycles on 37 SMs as on 148: the launches were timed back to back with dependent
+// launch, where the next call starts on the SMs that are left (37 CTAs 29.0 us, 148 CTAs 33.4; without dependent launch 33.3, 34.4).
 static double qmm_cost_us(int64_t sms, int64_t items, int64_t stages, int tile, int64_t splits) {
     const int64_t grid = splits > 0 ? items * splits : std::min(sms, items * stages);
     const int64_t waves = (grid + sms - 1) / sms, run = splits > 0 ? (stages + splits - 1) / splits : (items * stages + grid - 1) / grid;

@@ -17,8 +17,8 @@ __device__ __forceinline__ constexpr uint32_t hash_mul() { return CB == 0 ? 8922
 template <int CB>
 __device__ __forceinline__ constexpr uint32_t hash_add() { return CB == 0 ? 64248484u : 0u; }
 
-// bits [O, O + 16) of v, O at most 16.  The left shift is spelled in PTX so that it stays one (folded with the right shift
-// it becomes a shift and a mask, both on the logic pipe).
+// bits [O, O + 16) of v, O at most 16.  The left shift is spelled in PTX: written in C++, the pair of shifts takes as long as a
+// shift and a mask (cycles per tile at 3 bits: the few-row loop 56.6 both, 49.8 like this; the many-row decoder's 58.7 and 51.0).
 template <int O>
 __device__ __forceinline__ uint32_t window(uint32_t v) {
     if constexpr (O == 0) return v & 0xffffu;
@@ -62,11 +62,12 @@ __device__ __forceinline__ void lane_hashes(uint32_t w2, uint32_t w1, uint32_t w
         }
     } else {
         // The states are 16-bit windows at bit offsets 0, K, .., 7K from the lane's end.  A few registers are funnelled out
-        // of the stream words so that every window lies at an offset 0..16 of one of them; there it costs ONE logic-pipe
-        // instruction: nothing but a shift at offset 16, a mask at 0, and in between a left shift, which the integer
-        // multiply-add pipe takes, followed by the right shift that drops what lies below (shifting right and masking,
-        // two logic-pipe instructions per state, made the decode of a tile 53 cycles at K = 3; now 41, the multiply-add
-        // pipe being busy as long as the logic pipe).
+        // of the stream words so that every window lies at an offset 0..16 of one of them; there it costs ONE instruction of
+        // the logic pipe, the one that bounds the decode: nothing but a shift at offset 16, a mask at 0, and in between a left
+        // shift, which the integer multiply-add pipe can take, followed by the right shift that drops what lies below.
+        // Cycles per tile and scheduler against a shift and a mask per state, 16 warps, words in shared memory: the few-row
+        // loop (two mma.sync a tile) 54.8 -> 47.5 at 2 bits, 56.6 -> 49.8 at 3, 59.9 -> 50.9 at 5, 59.1 -> 50.9 at 6; the
+        // many-row decoder's loop (stores to tensor memory) 59.0 -> 52.1, 58.7 -> 51.0, 61.5 -> 54.1, 62.1 -> 53.6.
         uint32_t v[8];
         const uint32_t n = __funnelshift_r(w2, w1, slack);                       // offsets 0..31
         if constexpr (K <= 2) {

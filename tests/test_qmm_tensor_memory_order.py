@@ -41,3 +41,29 @@ def test_the_check_sees_a_missing_fence():
     body = kernel_body()
     without = body.replace(FENCE, "removed")
     assert len(unordered(without)) >= 4
+
+
+# instructions that all lanes of a warp execute as one (.sync.aligned), and what lets lanes go ways of their own before them
+ALIGNED = ("tmem_alloc(", "tmem_st_tile<", "tcgen05.wait::st.sync.aligned", "tmem_ld16(", "tmem_dealloc(")
+TOGETHER = ("__syncwarp(", "group_sync(")
+APART = ("qmm_wait(", "if (lane", "lane == 0) {", "threadIdx.x == 0) {", "elect_one()", "while (global_ns()")
+
+
+def not_converged(body):
+    tokens = re.finditer("|".join(re.escape(t) for t in (*ALIGNED, *TOGETHER, *APART)), body)
+    together, out = True, []
+    for m in tokens:
+        if m.group() in TOGETHER:
+            together = True
+        elif m.group() in APART:
+            together = False
+        elif not together:
+            out.append(body[m.start():m.start() + 60])
+    return out
+
+
+def test_a_warp_barrier_lies_before_every_warp_wide_instruction():
+    body = kernel_body()
+    assert all(t in body for t in (*ALIGNED, *TOGETHER, *APART))
+    assert not_converged(body) == []
+    assert len(not_converged(body.replace("__syncwarp(", "removed(").replace("group_sync(", "removed("))) >= 4
