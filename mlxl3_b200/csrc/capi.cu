@@ -86,6 +86,7 @@ constexpr size_t kScratchKeptBytes = size_t(64) << 20;
 constexpr size_t kScratchHostBytes = size_t(1) << 20;
 std::mutex g_scratch_mutex;
 std::vector<ScratchBlock> g_scratch_free, g_scratch_used;
+size_t g_scratch_acquiring = 0;                          // calls that are allocating a block for the second list
 
 // gives the current device's kept blocks back; the bytes freed
 size_t scratch_trim() {
@@ -256,6 +257,13 @@ int b200exl3_scratch_acquire(size_t bytes, void** out, void** out_host) {
     while (block.bytes < bytes && block.bytes <= kScratchKeptBytes) block.bytes *= 2;
     if (block.bytes > kScratchKeptBytes) block.bytes = bytes; // never kept: no more than was asked for
     std::unique_lock<std::mutex> lock(g_scratch_mutex);
+    // room for this block in both lists, so that neither this call nor its release has to allocate with the block in hand
+    try {
+        g_scratch_used.reserve(g_scratch_used.size() + g_scratch_acquiring + 1);
+        g_scratch_free.reserve(g_scratch_free.size() + g_scratch_used.size() + g_scratch_acquiring + 1);
+    } catch (const std::bad_alloc&) {
+        return fail("out of host memory");
+    }
     size_t found = g_scratch_free.size();                     // the smallest that is large enough, last released; a small call wants a page-locked half
     for (size_t i = 0; i < g_scratch_free.size(); ++i) {
         const ScratchBlock& b = g_scratch_free[i];
@@ -266,13 +274,16 @@ int b200exl3_scratch_acquire(size_t bytes, void** out, void** out_host) {
         block = g_scratch_free[found];
         g_scratch_free.erase(g_scratch_free.begin() + static_cast<long>(found));
     } else {
+        ++g_scratch_acquiring;
         lock.unlock();
-        if (b200exl3_malloc(block.bytes, &block.ptr)) return -1;
-        if (block.bytes <= kScratchHostBytes && check(cudaMallocHost(&block.host, block.bytes), "cudaMallocHost")) {
+        int rc = b200exl3_malloc(block.bytes, &block.ptr);
+        if (!rc && block.bytes <= kScratchHostBytes && check(cudaMallocHost(&block.host, block.bytes), "cudaMallocHost")) {
             cudaFree(block.ptr);
-            return -1;
+            rc = -1;
         }
         lock.lock();
+        --g_scratch_acquiring;
+        if (rc) return -1;
     }
     g_scratch_used.push_back(block);
     *out = block.ptr;
@@ -281,33 +292,31 @@ int b200exl3_scratch_acquire(size_t bytes, void** out, void** out_host) {
 }
 int b200exl3_scratch_release(void* p) {
     if (!p) return 0;
-    std::vector<ScratchBlock> drop;                           // freed outside the lock
-    {
-        std::lock_guard<std::mutex> lock(g_scratch_mutex);
-        size_t at = 0;
-        while (at < g_scratch_used.size() && g_scratch_used[at].ptr != p) ++at;
-        if (at == g_scratch_used.size()) return fail("not a scratch block");
-        const int device = g_scratch_used[at].device;
-        g_scratch_free.push_back(g_scratch_used[at]);
-        g_scratch_used.erase(g_scratch_used.begin() + static_cast<long>(at));
-        size_t kept = 0;
-        for (const ScratchBlock& b : g_scratch_free) kept += b.device == device ? b.bytes : 0;
-        // The largest go first: a call that needs one copies megabytes and hardly notices, while a small call that found none
-        // would page-lock memory each time.
-        while (kept > kScratchKeptBytes) {
-            size_t largest = g_scratch_free.size();
-            for (size_t i = 0; i < g_scratch_free.size(); ++i)
-                if (g_scratch_free[i].device == device && (largest == g_scratch_free.size() || g_scratch_free[i].bytes >= g_scratch_free[largest].bytes)) largest = i;
-            kept -= g_scratch_free[largest].bytes;
-            drop.push_back(g_scratch_free[largest]);
-            g_scratch_free.erase(g_scratch_free.begin() + static_cast<long>(largest));
-        }
-    }
+    std::unique_lock<std::mutex> lock(g_scratch_mutex);
+    size_t at = 0;
+    while (at < g_scratch_used.size() && g_scratch_used[at].ptr != p) ++at;
+    if (at == g_scratch_used.size()) return fail("not a scratch block");
+    const int device = g_scratch_used[at].device;
+    g_scratch_free.push_back(g_scratch_used[at]);             // acquire made room for it
+    g_scratch_used.erase(g_scratch_used.begin() + static_cast<long>(at));
+    // Kept are 64 MiB per device.  The largest go first: a call that needs one copies megabytes and hardly notices, while a
+    // small call that found none would page-lock memory each time.
     cudaError_t e = cudaSuccess;
-    for (const ScratchBlock& b : drop) {
-        cudaFreeHost(b.host);
-        const cudaError_t freed = cudaFree(b.ptr);
+    for (;;) {
+        size_t kept = 0, largest = g_scratch_free.size();
+        for (size_t i = 0; i < g_scratch_free.size(); ++i) {
+            if (g_scratch_free[i].device != device) continue;
+            kept += g_scratch_free[i].bytes;
+            if (largest == g_scratch_free.size() || g_scratch_free[i].bytes >= g_scratch_free[largest].bytes) largest = i;
+        }
+        if (kept <= kScratchKeptBytes) break;
+        const ScratchBlock drop = g_scratch_free[largest];
+        g_scratch_free.erase(g_scratch_free.begin() + static_cast<long>(largest));
+        lock.unlock();                                        // freeing waits for the device
+        cudaFreeHost(drop.host);
+        const cudaError_t freed = cudaFree(drop.ptr);
         if (e == cudaSuccess) e = freed;
+        lock.lock();
     }
     return check(e, "cudaFree");
 }
