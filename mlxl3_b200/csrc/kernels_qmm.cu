@@ -16,6 +16,7 @@
 //  * B operand: rotated activations, two TMA tensor copies of [tile tokens, 64 in] fp16 per stage, 128-byte swizzle;
 //  * packed words: one bulk copy per stage (8 tile rows x 8 tiles are contiguous in the quad layout);
 //  * one thread issues the stage's eight products and one commit, which frees the A stage and the activation slot.
+//  * tiles of up to 64 tokens: two accumulators, so that four more warps finish an item while the next one is multiplied.
 //
 // What bounds it: up to 64 rows the decode.  Cycles per 16x16 tile and scheduler with sixteen decoder warps: the decode loop
 // alone (words resident in shared memory, tensor-memory stores and nothing else) 47 at 4 bits, 51 at 3, 52 at 1 and 2, 54 at 5
@@ -54,13 +55,19 @@ template <int NT>
 struct QmmShape {
     static constexpr int kGroups = 2;                  // groups of eight decoder warps that take alternate stages
     static constexpr int kDecoders = 8 * kGroups;
-    static constexpr int kThreads = 32 * (kFirstDecoder + kDecoders);
-    static constexpr int kSlots = NT == 64 ? 6 : 4;    // A stages in tensor memory beside NT accumulator columns
+    // Small tiles: two accumulators, and four warps that finish an item while the next one is decoded and multiplied; the decoders
+    // finish only the CTA's last item.  Before, the pipeline drained at every item (5000 cycles, 2000 of them waiting for the last
+    // products): 16 rows 5120->2x25600, 3 bits, 84.8 -> 80.1 us; expert block 37 / 256 tokens 176 -> 165 / 250 -> 230.  Large tiles
+    // leave no tensor memory for a second accumulator: their decoders finish every item.
+    static constexpr uint32_t kAccums = NT == 64 ? 2 : 1;
+    static constexpr int kFinishers = NT == 64 ? 4 : kDecoders;
+    static constexpr int kThreads = 32 * (kFirstDecoder + kDecoders + (NT == 64 ? kFinishers : 0));
+    static constexpr int kSlots = NT == 64 ? 6 : 4;    // A stages in tensor memory beside the accumulators
     static constexpr int kBSlots = NT == 64 ? 6 : 2;   // activation stages in shared memory; divides kSlots
     static constexpr uint32_t kBHalfBytes = NT * 128;  // NT tokens x 64 fp16
     static constexpr uint32_t kBSlotBytes = 2 * kBHalfBytes;
-    static constexpr uint32_t kEpilogueBytes = kDecoders / 4 * 2 * kChunk * 128 * sizeof(__half);
-    static_assert(NT + kSlots * kStageCols <= 512 && kSlots % kGroups == 0 && kSlots % kBSlots == 0, "tensor memory");
+    static constexpr uint32_t kEpilogueBytes = (kDecoders / 4 + (NT == 64 ? 1 : 0)) * 2 * kChunk * 128 * sizeof(__half);
+    static_assert(kAccums * NT + kSlots * kStageCols <= 512 && kSlots % kGroups == 0 && kSlots % kBSlots == 0, "tensor memory");
 };
 // Packed stages (2048 * K bytes) in flight.  A multiple of the decoder groups, so that a slot always belongs to one group:
 // parity alone does not tell a phase from the one after the next, and a group that met a slot only every other time could
@@ -278,8 +285,8 @@ qmm_kernel(const __grid_constant__ CUtensorMap xmap, const QmmArgs p) {
     constexpr uint32_t kRawBytes = kRawWords * 4;
     constexpr int kRaw = raw_slots<K, NT>();
     __shared__ __align__(8) uint64_t full[S::kSlots], done[S::kSlots], full2[S::kSlots], half[S::kSlots], raw_full[kRaw], raw_empty[kRaw];
-    __shared__ __align__(8) uint64_t accum_full, accum_free;
-    __shared__ uint32_t tmem_base_slot, s_last;
+    __shared__ __align__(8) uint64_t accum_full[S::kAccums], accum_free[S::kAccums], last_full;
+    __shared__ uint32_t tmem_base_slot, s_last[2];
     __shared__ volatile int s_failed;
 
     const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;   // warp: uniform
@@ -304,8 +311,8 @@ qmm_kernel(const __grid_constant__ CUtensorMap xmap, const QmmArgs p) {
         // the second has a barrier of its own, and so has the end of the first half's products)
         for (int s = 0; s < S::kSlots; ++s) { mbar_init(&full[s], 9); mbar_init(&done[s], 1); mbar_init(&full2[s], 1); mbar_init(&half[s], 1); }
         for (int s = 0; s < kRaw; ++s) { mbar_init(&raw_full[s], 1); mbar_init(&raw_empty[s], 8); }
-        mbar_init(&accum_full, 1);
-        mbar_init(&accum_free, S::kDecoders);
+        mbar_init(&last_full, 1);
+        for (uint32_t s = 0; s < S::kAccums; ++s) { mbar_init(&accum_full[s], 1); mbar_init(&accum_free[s], S::kFinishers); }
         s_failed = 0;
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
@@ -316,12 +323,152 @@ qmm_kernel(const __grid_constant__ CUtensorMap xmap, const QmmArgs p) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_base_slot;
     const uint32_t first_item = s0 / spi, k0 = s0 - first_item * spi;            // first item and its first stage here
+    const uint32_t last_item = (s1 - 1) / spi;
+    const int last_stages = static_cast<int>(s1 - max(s0, last_item * spi));     // stages of the last item here
     if (tr && threadIdx.x == 0) tr[1] = global_ns();
 
-    if (warp >= kFirstDecoder) {
+    int buf = 0;                                                 // half of the staging rows that the next sixteen tokens go through
+    // Epilogue of an item (or of this CTA's part of it) by W warps, of which this is the one numbered w: the sixteen decoders, or
+    // the four warps that finish items while the next one is decoded.
+    auto finish_item = [&](auto warps, const int w, const uint32_t item, const uint32_t seg, const int stages, const uint32_t quarter_lanes,
+                           __half* staging, uint32_t* last, const int quad_bar, const int all_bar) {
+        constexpr int W = decltype(warps)::value;
+        const int quad = w >> 2, quarter = w & 3;
+        const uint32_t acc = quarter_lanes + (seg % S::kAccums) * NT;
+        const QmmItem info = qmm_item<NT>(p, item);
+        QmmStore store{};
+        if (p.yhat == nullptr) store = qmm_store_of(p, info, lane);
+        // The decoders that take only the last item have a barrier of their own for it: they may come several items early, when the
+        // parity of a barrier that completes once every two items does not tell their phase from an older one.
+        const bool single = W > S::kFinishers;
+        qmm_wait(single ? &last_full : &accum_full[seg % S::kAccums], single ? 0u : (seg / S::kAccums) & 1u, &s_failed);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        __syncwarp();
+        const bool complete = stages == static_cast<int>(spi);
+        // parts of shared items in order of (CTA, item): CTA + item numbers them; with more items than CTAs, two per CTA
+        const size_t piece_floats = static_cast<size_t>(p.tile_tokens) * 128;
+        float* piece = p.pieces + (items < G ? blockIdx.x + item : 2 * blockIdx.x + (seg > 0 ? 1 : 0)) * piece_floats;
+        // chunks of 16 tokens: four warps hold 32 columns each of the same tokens
+        for (int c = quad * kChunk; c < info.n; c += W / 4 * kChunk) {
+            uint32_t r[16];
+            __syncwarp();
+            tmem_ld16(acc + c, r);
+            if (!complete || p.yhat != nullptr) {
+                float* dst = complete ? p.yhat + static_cast<int64_t>(info.tok0 + c) * p.yhat_ld + info.cblock * 128 + quarter * 32 + lane
+                                      : piece + c * 128 + quarter * 32 + lane;
+                const int64_t ld = complete ? p.yhat_ld : 128;
+#pragma unroll
+                for (int i = 0; i < kChunk; ++i)
+                    if (c + i < info.n) dst[i * ld] = __uint_as_float(r[i]);
+            } else {
+                // the output rotation runs over the 128 columns of a token: transposed through shared memory, then
+                // every warp rotates four tokens
+                __half* stage = staging + (quad * 2 + buf) * (kChunk * 128);
+#pragma unroll
+                for (int i = 0; i < kChunk; ++i) stage[i * 128 + stage_col(quarter * 32 + lane)] = __float2half_rn(__uint_as_float(r[i]));
+                group_sync(quad_bar, 128);
+                if (c + quarter * 4 < info.n)
+                    qmm_finish4(stage + quarter * 512, p, store, info.tok0 + c + quarter * 4, info.n - c - quarter * 4, lane);
+                buf ^= 1;
+            }
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0 && W == S::kFinishers) mbar_arrive(&accum_free[seg % S::kAccums]);   // the accumulator may be overwritten
+        __syncwarp();
+        if (!complete) {
+            // CTAs share the item: this one's part is a piece; the last to arrive adds the pieces in input order
+            const uint32_t x0 = item * spi;
+            const uint32_t c_first = ((x0 + 1) * G - 1) / total, c_last = ((x0 + spi) * G - 1) / total;
+            __threadfence();
+            group_sync(all_bar, W * 32);
+            if (w == 0 && lane == 0) {
+                const unsigned int before = atomicAdd(p.counters + item, 1u);
+                *last = before == c_last - c_first;
+                if (*last) p.counters[item] = 0;            // leave the scratch ready for the next call
+            }
+            group_sync(all_bar, W * 32);
+            if (*last) {
+                __threadfence();
+                // the first CTA's part is its last one if it starts before the item, the others' their first
+                const size_t stride = items < G ? piece_floats : 2 * piece_floats;
+                const float* base = p.pieces + (items < G ? c_first + item : 2 * c_first) * piece_floats + lane * 4;
+                const float* base0 = base + (items >= G && total * c_first / G < x0 ? piece_floats : 0);
+                const int pieces = static_cast<int>(c_last - c_first) + 1;
+                auto store_sum = [&](int t, const float4& a) {
+                    *reinterpret_cast<float4*>(p.yhat + static_cast<int64_t>(info.tok0 + t) * p.yhat_ld + info.cblock * 128 + lane * 4) = a;
+                };
+                if (info.n <= W) {
+                    // few rows: one per warp, up to four parts in flight
+                    if (w < info.n) {
+                        float4 a = __ldcg(reinterpret_cast<const float4*>(base0 + w * 128));
+                        const float* src = base + stride + w * 128;
+#pragma unroll 4
+                        for (int q = 1; q < pieces; ++q, src += stride) {
+                            const float4 part = __ldcg(reinterpret_cast<const float4*>(src));
+                            a.x = __fadd_rn(a.x, part.x); a.y = __fadd_rn(a.y, part.y); a.z = __fadd_rn(a.z, part.z); a.w = __fadd_rn(a.w, part.w);
+                        }
+                        if (p.yhat != nullptr) {
+                            store_sum(w, a);
+                        } else {
+                            __half h[4] = {__float2half_rn(a.x), __float2half_rn(a.y), __float2half_rn(a.z), __float2half_rn(a.w)};
+                            warp_hadamard128_f16(h, lane);
+                            qmm_store4(p, store, info.tok0 + w, h);
+                        }
+                    }
+                } else {
+                    __half* mine = staging + w * 512;
+                    for (int t0 = w * 4; t0 < info.n; t0 += 4 * W) {
+                        int row[4];
+                        float4 a[4];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            row[i] = min(t0 + i, info.n - 1) * 128;
+                            a[i] = __ldcg(reinterpret_cast<const float4*>(base0 + row[i]));
+                        }
+                        const float* src = base + stride;
+#pragma unroll 1
+                        for (int q = 1; q < pieces; ++q, src += stride) {
+                            float4 part[4];
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) part[i] = __ldcg(reinterpret_cast<const float4*>(src + row[i]));
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) {
+                                a[i].x = __fadd_rn(a[i].x, part[i].x); a[i].y = __fadd_rn(a[i].y, part[i].y);
+                                a[i].z = __fadd_rn(a[i].z, part[i].z); a[i].w = __fadd_rn(a[i].w, part[i].w);
+                            }
+                        }
+                        if (p.yhat != nullptr) {
+#pragma unroll
+                            for (int i = 0; i < 4; ++i)
+                                if (t0 + i < info.n) store_sum(t0 + i, a[i]);
+                        } else {
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) {
+                                __align__(8) const __half2 h[2] = {__floats2half2_rn(a[i].x, a[i].y), __floats2half2_rn(a[i].z, a[i].w)};
+                                *reinterpret_cast<uint2*>(mine + i * 128 + stage_col(lane * 4)) = *reinterpret_cast<const uint2*>(h);
+                            }
+                            __syncwarp();
+                            qmm_finish4(mine, p, store, info.tok0 + t0, info.n - t0, lane);
+                        }
+                    }
+                    group_sync(all_bar, W * 32);        // the next item stages in other warps' rows
+                }
+            }
+        }
+    };
+
+    if (warp >= kFirstDecoder + S::kDecoders) {
+        // ================= finishing warps: every item of the CTA but its last, while the next one is decoded =================
+        pdl_wait();
+        const int w = warp - kFirstDecoder - S::kDecoders;
+        const uint32_t quarter_lanes = tmem + (static_cast<uint32_t>((w & 3) * 32) << 16);
+        for (uint32_t item = first_item; item < last_item; ++item)
+            finish_item(std::integral_constant<int, 4>{}, w, item, item - first_item, static_cast<int>(item == first_item ? spi - k0 : spi), quarter_lanes,
+                        stage_base + S::kDecoders / 4 * 2 * kChunk * 128, &s_last[1], 5, 6);
+    } else if (warp >= kFirstDecoder) {
         // ================= decoders: packed words -> A stages in tensor memory; then the epilogue of each item =================
         const int dec = warp - kFirstDecoder, group = dec >> 3, rows4 = (dec >> 2) & 1, quarter = dec & 3;   // quarter == warp & 3: the lanes it may access
-        const int quad = dec >> 2;                               // four warps that hold all lanes
         const LaneGeom<K> geom(lane);
         // this warp's two tiles of each row: half of a quad of four interleaved tiles
         const uint32_t* words = raw_base + rows4 * (256 * K) + (quarter >> 1) * (32 * K) + (quarter & 1) * 2;
@@ -339,12 +486,9 @@ qmm_kernel(const __grid_constant__ CUtensorMap xmap, const QmmArgs p) {
         };
         bool ready = group < count && stage_ready();
         int it = group;
-        int seg_begin = 0, buf = 0;
-        uint32_t item = first_item, k_first = k0, seg = 0;
-        while (seg_begin < count) {
-            const int seg_end = min(count, seg_begin + static_cast<int>(spi - k_first));
+        auto decode_until = [&](const int end) {
 #pragma unroll 1
-            for (; it < seg_end; it += S::kGroups) {
+            for (; it < end; it += S::kGroups) {
                 if (!__all_sync(0xffffffffu, ready)) {
                     // the packed stage has landed, and the MMAs that read this A stage last time are done
                     ready = qmm_wait(&raw_full[rslot], rpar, &s_failed) && qmm_wait(&done[slot], par ^ 1u, &s_failed);
@@ -355,7 +499,7 @@ qmm_kernel(const __grid_constant__ CUtensorMap xmap, const QmmArgs p) {
                 // stores below come after them
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t* rw = words + rslot * kRawWords;
-                const uint32_t dst = lanes + NT + rows4 * 32 + slot * kStageCols;
+                const uint32_t dst = lanes + S::kAccums * NT + rows4 * 32 + slot * kStageCols;
                 uint64_t* stage_full = &full[slot];
                 uint64_t* empty = &raw_empty[rslot];
                 slot += S::kGroups;
@@ -392,133 +536,26 @@ qmm_kernel(const __grid_constant__ CUtensorMap xmap, const QmmArgs p) {
                     mbar_arrive(empty);                          // the packed words were consumed: slot free for this warp
                 }
             }
-            // ---- epilogue of the item (or of this CTA's part of it) ----
-            if (seg == 0) {
+        };
+        auto finish = [&](uint32_t item, uint32_t seg, int stages) {
+            if (seg == 0 || S::kFinishers < S::kDecoders) {
                 pdl_wait();                                      // returns at once: the kernel before ended long ago
                 if (tr && dec == 0 && lane == 0) tr[2] = global_ns();
             }
-            const QmmItem info = qmm_item<NT>(p, item);
-            QmmStore store{};
-            if (p.yhat == nullptr) store = qmm_store_of(p, info, lane);
-            qmm_wait(&accum_full, seg & 1u, &s_failed);
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            __syncwarp();
-            const bool complete = seg_end - seg_begin == static_cast<int>(spi);
-            // parts of shared items in order of (CTA, item): CTA + item numbers them; with more items than CTAs, two per CTA
-            const size_t piece_floats = static_cast<size_t>(p.tile_tokens) * 128;
-            float* piece = p.pieces + (items < G ? blockIdx.x + item : 2 * blockIdx.x + (seg > 0 ? 1 : 0)) * piece_floats;
-            // chunks of 16 tokens: four warps hold 32 columns each of the same tokens
-            for (int c = quad * kChunk; c < info.n; c += S::kDecoders / 4 * kChunk) {
-                uint32_t r[16];
-                __syncwarp();
-                tmem_ld16(lanes + c, r);
-                if (!complete || p.yhat != nullptr) {
-                    float* dst = complete ? p.yhat + static_cast<int64_t>(info.tok0 + c) * p.yhat_ld + info.cblock * 128 + quarter * 32 + lane
-                                          : piece + c * 128 + quarter * 32 + lane;
-                    const int64_t ld = complete ? p.yhat_ld : 128;
-#pragma unroll
-                    for (int i = 0; i < kChunk; ++i)
-                        if (c + i < info.n) dst[i * ld] = __uint_as_float(r[i]);
-                } else {
-                    // the output rotation runs over the 128 columns of a token: transposed through shared memory, then
-                    // every warp rotates four tokens
-                    __half* stage = stage_base + (quad * 2 + buf) * (kChunk * 128);
-#pragma unroll
-                    for (int i = 0; i < kChunk; ++i) stage[i * 128 + stage_col(quarter * 32 + lane)] = __float2half_rn(__uint_as_float(r[i]));
-                    group_sync(1 + quad, 128);
-                    if (c + quarter * 4 < info.n)
-                        qmm_finish4(stage + quarter * 512, p, store, info.tok0 + c + quarter * 4, info.n - c - quarter * 4, lane);
-                    buf ^= 1;
-                }
+            finish_item(std::integral_constant<int, S::kDecoders>{}, dec, item, seg, stages, lanes, stage_base, &s_last[0], 1 + (dec >> 2), 8);
+        };
+        if constexpr (S::kFinishers < S::kDecoders) {
+            // the finishing warps take every item but the last, which nothing is decoded behind
+            decode_until(count);
+            finish(last_item, last_item - first_item, last_stages);
+        } else {
+            int seg_begin = 0;
+            for (uint32_t item = first_item, k_first = k0; seg_begin < count; ++item, k_first = 0) {
+                const int seg_end = min(count, seg_begin + static_cast<int>(spi - k_first));
+                decode_until(seg_end);
+                finish(item, item - first_item, seg_end - seg_begin);
+                seg_begin = seg_end;
             }
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&accum_free);             // the accumulator may be overwritten
-            __syncwarp();
-            if (!complete) {
-                // CTAs share the item: this one's part is a piece; the last to arrive adds the pieces in input order
-                const uint32_t x0 = item * spi;
-                const uint32_t c_first = ((x0 + 1) * G - 1) / total, c_last = ((x0 + spi) * G - 1) / total;
-                __threadfence();
-                group_sync(8, S::kDecoders * 32);
-                if (dec == 0 && lane == 0) {
-                    const unsigned int before = atomicAdd(p.counters + item, 1u);
-                    s_last = before == c_last - c_first;
-                    if (s_last) p.counters[item] = 0;            // leave the scratch ready for the next call
-                }
-                group_sync(8, S::kDecoders * 32);
-                if (s_last) {
-                    __threadfence();
-                    // the first CTA's part is its last one if it starts before the item, the others' their first
-                    const size_t stride = items < G ? piece_floats : 2 * piece_floats;
-                    const float* base = p.pieces + (items < G ? c_first + item : 2 * c_first) * piece_floats + lane * 4;
-                    const float* base0 = base + (items >= G && total * c_first / G < x0 ? piece_floats : 0);
-                    const int pieces = static_cast<int>(c_last - c_first) + 1;
-                    auto store_sum = [&](int t, const float4& a) {
-                        *reinterpret_cast<float4*>(p.yhat + static_cast<int64_t>(info.tok0 + t) * p.yhat_ld + info.cblock * 128 + lane * 4) = a;
-                    };
-                    if (info.n <= S::kDecoders) {
-                        // few rows: one per warp, up to four parts in flight
-                        if (dec < info.n) {
-                            float4 a = __ldcg(reinterpret_cast<const float4*>(base0 + dec * 128));
-                            const float* src = base + stride + dec * 128;
-#pragma unroll 4
-                            for (int q = 1; q < pieces; ++q, src += stride) {
-                                const float4 part = __ldcg(reinterpret_cast<const float4*>(src));
-                                a.x = __fadd_rn(a.x, part.x); a.y = __fadd_rn(a.y, part.y); a.z = __fadd_rn(a.z, part.z); a.w = __fadd_rn(a.w, part.w);
-                            }
-                            if (p.yhat != nullptr) {
-                                store_sum(dec, a);
-                            } else {
-                                __half h[4] = {__float2half_rn(a.x), __float2half_rn(a.y), __float2half_rn(a.z), __float2half_rn(a.w)};
-                                warp_hadamard128_f16(h, lane);
-                                qmm_store4(p, store, info.tok0 + dec, h);
-                            }
-                        }
-                    } else {
-                        __half* mine = stage_base + dec * 512;
-                        for (int t0 = dec * 4; t0 < info.n; t0 += 4 * S::kDecoders) {
-                            int row[4];
-                            float4 a[4];
-#pragma unroll
-                            for (int i = 0; i < 4; ++i) {
-                                row[i] = min(t0 + i, info.n - 1) * 128;
-                                a[i] = __ldcg(reinterpret_cast<const float4*>(base0 + row[i]));
-                            }
-                            const float* src = base + stride;
-#pragma unroll 1
-                            for (int q = 1; q < pieces; ++q, src += stride) {
-                                float4 part[4];
-#pragma unroll
-                                for (int i = 0; i < 4; ++i) part[i] = __ldcg(reinterpret_cast<const float4*>(src + row[i]));
-#pragma unroll
-                                for (int i = 0; i < 4; ++i) {
-                                    a[i].x = __fadd_rn(a[i].x, part[i].x); a[i].y = __fadd_rn(a[i].y, part[i].y);
-                                    a[i].z = __fadd_rn(a[i].z, part[i].z); a[i].w = __fadd_rn(a[i].w, part[i].w);
-                                }
-                            }
-                            if (p.yhat != nullptr) {
-#pragma unroll
-                                for (int i = 0; i < 4; ++i)
-                                    if (t0 + i < info.n) store_sum(t0 + i, a[i]);
-                            } else {
-#pragma unroll
-                                for (int i = 0; i < 4; ++i) {
-                                    __align__(8) const __half2 h[2] = {__floats2half2_rn(a[i].x, a[i].y), __floats2half2_rn(a[i].z, a[i].w)};
-                                    *reinterpret_cast<uint2*>(mine + i * 128 + stage_col(lane * 4)) = *reinterpret_cast<const uint2*>(h);
-                                }
-                                __syncwarp();
-                                qmm_finish4(mine, p, store, info.tok0 + t0, info.n - t0, lane);
-                            }
-                        }
-                        group_sync(8, S::kDecoders * 32);        // the next item stages in other warps' rows
-                    }
-                }
-            }
-            seg_begin = seg_end;
-            k_first = 0;
-            ++item;
-            ++seg;
         }
         if (tr && dec == 0 && lane == 0) tr[5] = global_ns();
     } else if (warp == kWeightWarp) {
@@ -601,7 +638,7 @@ qmm_kernel(const __grid_constant__ CUtensorMap xmap, const QmmArgs p) {
     } else if (warp == kMmaWarp) {
         // ================= MMA issuer =================
         if (elect_one()) {
-            uint32_t item = first_item, par = 0, seg = 0, accumulate = 0;
+            uint32_t item = first_item, par = 0, seg = 0, accumulate = 0, d = tmem;
             int left = count, rem = min(count, static_cast<int>(spi - k0));
             auto instr_desc = [&](uint32_t i) -> uint32_t {
                 const int n16 = (qmm_item<NT>(p, i).n + 15) >> 4;
@@ -614,10 +651,12 @@ qmm_kernel(const __grid_constant__ CUtensorMap xmap, const QmmArgs p) {
 #pragma unroll
                 for (int s = 0; s < S::kSlots; ++s) {
                     if (rem == 0) {
-                        umma_commit(&accum_full);                                // accumulator of this item complete
+                        umma_commit(S::kFinishers < S::kDecoders && left == 0 ? &last_full : &accum_full[seg % S::kAccums]);   // accumulator of this item complete
                         if (left == 0) { running = false; break; }
-                        if (!qmm_wait(&accum_free, seg & 1u, &s_failed)) { running = false; break; }
                         ++seg;
+                        // the accumulator of kAccums items ago has been read
+                        if (seg >= S::kAccums && !qmm_wait(&accum_free[seg % S::kAccums], (seg / S::kAccums - 1) & 1u, &s_failed)) { running = false; break; }
+                        d = tmem + (seg % S::kAccums) * NT;
                         idesc = instr_desc(++item);
                         rem = min(left, static_cast<int>(spi));
                         accumulate = 0;
@@ -633,7 +672,7 @@ qmm_kernel(const __grid_constant__ CUtensorMap xmap, const QmmArgs p) {
                             if (!qmm_wait(&full2[s], par, &s_failed)) { running = false; break; }
                             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                         }
-                        umma_f16_ts(tmem, tmem + NT + s * kStageCols + kk * 8, bd + (kk >> 2) * (S::kBHalfBytes >> 4) + (kk & 3) * 2, idesc,
+                        umma_f16_ts(d, tmem + S::kAccums * NT + s * kStageCols + kk * 8, bd + (kk >> 2) * (S::kBHalfBytes >> 4) + (kk & 3) * 2, idesc,
                                     kk > 0 ? 1u : accumulate);
                     }
                     if (NT > 64 && !running) break;
@@ -644,7 +683,10 @@ qmm_kernel(const __grid_constant__ CUtensorMap xmap, const QmmArgs p) {
                 }
                 par ^= 1u;
             }
-            if (s_failed) umma_commit(&accum_full);
+            if (s_failed) {
+                umma_commit(&last_full);
+                for (uint32_t a = 0; a < S::kAccums; ++a) umma_commit(&accum_full[a]);
+            }
             if (tr) tr[3] = global_ns();
         }
     }

@@ -102,3 +102,20 @@ def test_long_runs_of_wide_weights(gpu, k, rows):
     pick = np.unique([0, rows // 2, rows - 1])
     _close(got[pick], oracle.linear_forward(trellis, k, 0, suh, svh, None, x[pick]))
     layer.close()
+
+
+@pytest.mark.parametrize("n_in,n_out,k,rows", [(128, 81920, 3, 16), (256, 51200, 4, 48), (384, 30720, 6, 33), (640, 2176, 4, 64)])
+def test_many_items_on_a_cta(gpu, n_in, n_out, k, rows):
+    """Tiles of up to 64 tokens: a CTA's items follow each other while the one before is still being finished; items of one to
+    five stages, fewer than are in flight."""
+    rng = np.random.default_rng(n_in + rows)
+    trellis, suh, svh = random_layer(rng, n_in, n_out, k)
+    layer = gpu.Exl3Linear(trellis, suh, svh, None, k, 0)
+    x = rng.standard_normal((rows, n_in)).astype(np.float16)
+    got = layer.forward(x)
+    for _ in range(5):
+        assert np.array_equal(bits(layer.forward(x)), bits(got))
+    assert gpu.workspace_status(layer._workspace) == 0
+    pick = np.unique([0, 15, rows // 2, rows - 1])
+    _close(got[pick], oracle.linear_forward(trellis, k, 0, suh, svh, None, x[pick]))
+    layer.close()
