@@ -51,7 +51,7 @@ constexpr int kMmaWarp = 0, kWeightWarp = 1, kActWarp = 2, kFirstDecoder = 4;
 constexpr int kStageCols = 64;                         // tensor-memory columns of an A stage: two fp16 inputs each
 constexpr int kChunk = 16;                             // tokens four warps finish at a time
 
-template <int NT>
+template <int K, int NT>
 struct QmmShape {
     static constexpr int kGroups = 2;                  // groups of eight decoder warps that take alternate stages
     static constexpr int kDecoders = 8 * kGroups;
@@ -62,26 +62,22 @@ struct QmmShape {
     static constexpr uint32_t kAccums = NT == 64 ? 2 : 1;
     static constexpr int kFinishers = NT == 64 ? 4 : kDecoders;
     static constexpr int kThreads = 32 * (kFirstDecoder + kDecoders + (NT == 64 ? kFinishers : 0));
-    static constexpr int kSlots = NT == 64 ? 6 : 4;    // A stages in tensor memory beside the accumulators
-    static constexpr int kBSlots = NT == 64 ? 6 : 2;   // activation stages in shared memory; divides kSlots
+    // Stages in flight, packed (2048 * K bytes of shared memory each) and decoded (64 columns of tensor memory beside the
+    // accumulators), so that one slot number serves both.  A multiple of the decoder groups: a slot always belongs to one group,
+    // since parity alone does not tell a phase from the one after the next, and a group that met a slot only every other time
+    // could take a copy that has not landed for its own.  With two packed slots above 4 bits the decoders waited for the copies:
+    // 1969 rows 7936->1408, 6 bits, 98 -> 83 us; 128 rows 4096->14336, 8 bits, 37.9 -> 31.
+    static constexpr int kSlots = NT == 64 && K <= 4 ? 6 : 4;
+    static constexpr int kBSlots = NT == 64 ? kSlots : 2;   // activation stages in shared memory; divides kSlots
     static constexpr uint32_t kBHalfBytes = NT * 128;  // NT tokens x 64 fp16
     static constexpr uint32_t kBSlotBytes = 2 * kBHalfBytes;
     static constexpr uint32_t kEpilogueBytes = (kDecoders / 4 + (NT == 64 ? 1 : 0)) * 2 * kChunk * 128 * sizeof(__half);
     static_assert(kAccums * NT + kSlots * kStageCols <= 512 && kSlots % kGroups == 0 && kSlots % kBSlots == 0, "tensor memory");
 };
-// Packed stages (2048 * K bytes) in flight.  A multiple of the decoder groups, so that a slot always belongs to one group:
-// parity alone does not tell a phase from the one after the next, and a group that met a slot only every other time could
-// take a copy that has not landed for its own.  With two slots above 4 bits the decoders waited for the copies: 1969 rows
-// 7936->1408, 6 bits, 98 -> 83 us; 128 rows 4096->14336, 8 bits, 37.9 -> 31.
-template <int K, int NT>
-constexpr int raw_slots() {
-    constexpr int slots = NT == 64 && K <= 4 ? 6 : 4;
-    static_assert(slots % QmmShape<NT>::kGroups == 0, "a slot belongs to one group");
-    return slots;
-}
 template <int K, int NT>
 constexpr size_t qmm_smem_bytes() {
-    return 1024 + QmmShape<NT>::kBSlots * QmmShape<NT>::kBSlotBytes + static_cast<size_t>(raw_slots<K, NT>()) * 2048 * K + QmmShape<NT>::kEpilogueBytes;
+    using S = QmmShape<K, NT>;
+    return 1024 + S::kBSlots * S::kBSlotBytes + static_cast<size_t>(S::kSlots) * 2048 * K + S::kEpilogueBytes;
 }
 
 __device__ __forceinline__ uint64_t umma_desc(uint32_t smem_byte_addr) {
@@ -121,6 +117,11 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar) {
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
 }
+// The same by the lanes for which `arrive` holds, without a branch; bar is a shared-memory address.
+__device__ __forceinline__ void mbar_arrive(bool arrive, uint32_t bar) {
+    asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %1, 0;\n@p mbarrier.arrive.shared::cta.b64 _, [%0];\n}"
+                 ::"r"(bar), "r"(static_cast<uint32_t>(arrive)) : "memory");
+}
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int c0, int c1, uint64_t* bar) {
     asm volatile(
         "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
@@ -143,13 +144,12 @@ __device__ __forceinline__ void tmem_st_tile(uint32_t taddr, uint32_t a0, uint32
 // Wait that gives up after about a quarter of a second, or at once when another role of the CTA has
 // already given up, so that a lost copy or a miscounted barrier ends the kernel instead of hanging it.
 __device__ __noinline__ bool qmm_wait_slow(uint64_t* bar, uint32_t parity, volatile int* cta_failed) {
-    // Reading the global timer costs about 0.2 us, so the clock only starts after many plain polls.
-    for (int i = 0; i < 4096; ++i)
-        if (mbar_try_wait(bar, parity)) return true;
+    constexpr uint32_t kNap = 20000;                             // the hardware wakes the thread when the phase completes
+    if (mbar_try_wait_for(bar, parity, kNap)) return true;
     const unsigned long long t0 = global_ns();
-    for (int i = 1;; ++i) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if ((i & 255) == 0 && (*cta_failed || global_ns() - t0 > 250000000ull)) { *cta_failed = 1; return false; }
+    while (true) {
+        if (mbar_try_wait_for(bar, parity, kNap)) return true;
+        if (*cta_failed || global_ns() - t0 > 250000000ull) { *cta_failed = 1; return false; }
     }
 }
 __device__ __forceinline__ bool qmm_wait(uint64_t* bar, uint32_t parity, volatile int* cta_failed) {
@@ -269,9 +269,9 @@ __device__ __forceinline__ void qmm_finish4(__half* rows, const QmmArgs& p, cons
 }
 
 template <int K, int CB, int NT>
-__global__ void __launch_bounds__(QmmShape<NT>::kThreads, 1)
+__global__ void __launch_bounds__(QmmShape<K, NT>::kThreads, 1)
 qmm_kernel(const __grid_constant__ CUtensorMap xmap, const QmmArgs p) {
-    using S = QmmShape<NT>;
+    using S = QmmShape<K, NT>;
     // Dependent launch: this kernel may be scheduled under the tail of the kernel before it (the input rotation, the
     // glue of the expert block).  The packed weights are nobody's output, so the barriers, the tensor memory and the
     // first weight copies do not wait; what that kernel wrote -- the rotated rows, the segment table -- is read only
@@ -283,8 +283,7 @@ qmm_kernel(const __grid_constant__ CUtensorMap xmap, const QmmArgs p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr int kRawWords = 512 * K;                       // a packed stage: 8 tile rows x 2 quads x 32K words
     constexpr uint32_t kRawBytes = kRawWords * 4;
-    constexpr int kRaw = raw_slots<K, NT>();
-    __shared__ __align__(8) uint64_t full[S::kSlots], done[S::kSlots], full2[S::kSlots], half[S::kSlots], raw_full[kRaw], raw_empty[kRaw];
+    __shared__ __align__(8) uint64_t full[S::kSlots], done[S::kSlots], full2[S::kSlots], half[S::kSlots], raw_full[S::kSlots], raw_empty[S::kSlots];
     __shared__ __align__(8) uint64_t accum_full[S::kAccums], accum_free[S::kAccums], last_full;
     __shared__ uint32_t tmem_base_slot, s_last[2];
     __shared__ volatile int s_failed;
@@ -304,13 +303,13 @@ qmm_kernel(const __grid_constant__ CUtensorMap xmap, const QmmArgs p) {
     // shared memory: activation ring | packed ring | epilogue staging; the swizzled operand needs 1024-byte alignment
     unsigned char* b_base = smem_raw + ((1024u - (smem_addr(smem_raw) & 1023u)) & 1023u);
     uint32_t* raw_base = reinterpret_cast<uint32_t*>(b_base + S::kBSlots * S::kBSlotBytes);
-    __half* stage_base = reinterpret_cast<__half*>(raw_base + kRaw * kRawWords);
+    __half* stage_base = reinterpret_cast<__half*>(raw_base + S::kSlots * kRawWords);
 
     if (threadIdx.x == 0) {
         // a stage is full when its eight decoder warps and its activation copies have arrived (of a large tile the first half;
         // the second has a barrier of its own, and so has the end of the first half's products)
         for (int s = 0; s < S::kSlots; ++s) { mbar_init(&full[s], 9); mbar_init(&done[s], 1); mbar_init(&full2[s], 1); mbar_init(&half[s], 1); }
-        for (int s = 0; s < kRaw; ++s) { mbar_init(&raw_full[s], 1); mbar_init(&raw_empty[s], 8); }
+        for (int s = 0; s < S::kSlots; ++s) { mbar_init(&raw_full[s], 1); mbar_init(&raw_empty[s], 8); }
         mbar_init(&last_full, 1);
         for (uint32_t s = 0; s < S::kAccums; ++s) { mbar_init(&accum_full[s], 1); mbar_init(&accum_free[s], S::kFinishers); }
         s_failed = 0;
@@ -474,40 +473,30 @@ qmm_kernel(const __grid_constant__ CUtensorMap xmap, const QmmArgs p) {
         const uint32_t* words = raw_base + rows4 * (256 * K) + (quarter >> 1) * (32 * K) + (quarter & 1) * 2;
         const int j2 = geom.i2 * 4, j1 = geom.i1 * 4, j0 = geom.i0 * 4;
         const uint32_t lanes = tmem + (static_cast<uint32_t>(quarter * 32) << 16);
-        int slot = group, rslot = group % kRaw;
-        uint32_t par = 0, rpar = (group / kRaw) & 1;
-        // A barrier test takes a few hundred cycles to answer beside busy decoders, so the tests for the warp's next stage
-        // are issued before the current stage is decoded: lane 0 tests the packed words and lane 1 the A stage in ONE
-        // instruction (the warp barrier orders the other lanes' reads after the two observations).
-        auto stage_ready = [&]() -> bool {
-            bool ok = true;
-            if (lane < 2) ok = mbar_test_wait(lane == 0 ? &raw_full[rslot] : &done[slot], lane == 0 ? rpar : par ^ 1u);
-            return ok;
-        };
-        bool ready = group < count && stage_ready();
+        // What a stage costs a warp beside its eight tiles is kept to few instructions, since the integer pipe is what bounds the
+        // loop: lane 0 waits for the packed words and the others for the A stage in ONE instruction, lanes 0 and 1 arrive at two
+        // barriers in one, and what depends on the slot is stepped instead of computed.  Instructions per tile in all roles, 4 bits:
+        // 54.9 -> 51.2 (43.1 are the decode); 16 rows 5120->2x25600, 3 bits, 80.1 -> 72.0 us; 64 rows 4096->14336, 4 bits,
+        // 24.1 -> 21.7; expert block 37 / 256 tokens 165 -> 143 / 230 -> 213.  The loop unrolled over the ring of slots executes 49.6
+        // but misses the instruction cache twice as often (78.8 us); two rows at a time, rolled: 53.0 and 74.9 us.
+        const uint32_t wait_bar = smem_addr(lane == 0 ? raw_full : done), arrive_bar = smem_addr(lane == 0 ? full : raw_empty);
+        const bool arrives = lane < 2;
+        const uint32_t a_stages = lanes + S::kAccums * NT + rows4 * 32;
+        uint32_t at = group * 8, par = lane == 0 ? 0u : 1u;      // byte offset of the slot's barriers; parity this lane waits for
         int it = group;
         auto decode_until = [&](const int end) {
 #pragma unroll 1
             for (; it < end; it += S::kGroups) {
-                if (!__all_sync(0xffffffffu, ready)) {
-                    // the packed stage has landed, and the MMAs that read this A stage last time are done
-                    ready = qmm_wait(&raw_full[rslot], rpar, &s_failed) && qmm_wait(&done[slot], par ^ 1u, &s_failed);
+                // the packed stage has landed, and the MMAs that read this A stage last time are done
+                if (!__all_sync(0xffffffffu, mbar_try_wait(wait_bar + at, par))) {
+                    const bool ready = qmm_wait(lane == 0 ? &raw_full[at / 8] : &done[at / 8], par, &s_failed);
                     if (!__all_sync(0xffffffffu, ready)) break;
                 }
                 __syncwarp();
-                // the products that read this A stage last are done (two lanes saw it, the warp barrier passed it on): the
-                // stores below come after them
+                // the stores below come after the products that read this A stage last
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t* rw = words + rslot * kRawWords;
-                const uint32_t dst = lanes + S::kAccums * NT + rows4 * 32 + slot * kStageCols;
-                uint64_t* stage_full = &full[slot];
-                uint64_t* empty = &raw_empty[rslot];
-                slot += S::kGroups;
-                if (slot >= S::kSlots) { slot -= S::kSlots; par ^= 1u; }
-                rslot += S::kGroups;
-                if (rslot >= kRaw) { rslot -= kRaw; rpar ^= 1u; }
-                ready = it + S::kGroups < count && stage_ready();
-                __syncwarp();                                    // the two testing lanes are back: what follows is warp-wide
+                const uint32_t* rw = words + at * (kRawWords / 8);
+                const uint32_t dst = a_stages + at * (kStageCols / 8);
                 uint2 w2[4], w1[4], w0[4];
 #pragma unroll
                 for (int r = 0; r < 4; ++r) {
@@ -531,10 +520,9 @@ qmm_kernel(const __grid_constant__ CUtensorMap xmap, const QmmArgs p) {
                 tile_pair(std::integral_constant<int, 3>{});
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                if (lane == 0) {
-                    mbar_arrive(stage_full);
-                    mbar_arrive(empty);                          // the packed words were consumed: slot free for this warp
-                }
+                mbar_arrive(arrives, arrive_bar + at);           // decoded; the packed words were consumed
+                at += S::kGroups * 8;
+                if (at >= S::kSlots * 8) { at -= S::kSlots * 8; par ^= 1u; }
             }
         };
         auto finish = [&](uint32_t item, uint32_t seg, int stages) {
@@ -567,7 +555,7 @@ qmm_kernel(const __grid_constant__ CUtensorMap xmap, const QmmArgs p) {
             bool running = true;
             while (running) {
 #pragma unroll 1
-                for (int s = 0; s < kRaw; ++s) {
+                for (int s = 0; s < S::kSlots; ++s) {
                     if (!qmm_wait(&raw_empty[s], par ^ 1u, &s_failed)) { running = false; break; }
                     mbar_expect_tx(&raw_full[s], kRawBytes);
                     bulk_copy_g2s(raw_base + s * kRawWords, src, kRawBytes, &raw_full[s]);
@@ -745,7 +733,7 @@ cudaError_t qmm_launch_shape(const CUtensorMap& map, const QmmArgs& p, int grid,
         if (e != cudaSuccess) return e;
         attribute.mark();
     }
-    return launch_dependent(kernel, dim3(static_cast<unsigned>(grid)), dim3(QmmShape<NT>::kThreads), smem, stream, map, p);
+    return launch_dependent(kernel, dim3(static_cast<unsigned>(grid)), dim3(QmmShape<K, NT>::kThreads), smem, stream, map, p);
 }
 
 template <int K>
