@@ -57,15 +57,16 @@ int b200exl3_version(void);
 /* Process-wide knobs: "qmv_ctas_per_sm" (CTAs per SM the grids are sized for), "qmv_force_grid"
  * (CTAs per launch, 0 = heuristic), "pdl" (1 or 2 = launch layer kernels with programmatic stream serialization, so the
  * weight prefetch of a layer overlaps the tail of the previous kernel in the stream; 1 releases the
- * next kernel after the main loop, 2 as soon as the first copies are in flight), "qmv_trace_buffer"
+ * next kernel once this one's inputs are there or after its main loop, 2 as soon as the first copies are in flight), "qmv_trace_buffer"
  * (device address of a uint64 [grid, 8] array that receives nanosecond stamps of each CTA's phases:
  * start, activations visible, rotated, main loop done, warps joined, reduced, finished; 0 = off), "qmm" (0 = batches
  * of more than 8 rows also go through the small-batch kernel (16 rows per launch) instead of the tensor-core product; default 1),
  * "qmm_splits" (CTAs per tile of the tensor-core product, 0 = chosen by a cost model; set it before asking for
  * workspace sizes), "moe_sorted" (0 = the expert block runs one row per slot for any batch instead of grouping
- * slots by expert for larger batches; set it before asking for workspace sizes), "moe_fused" (1 = a small batch of the
- * expert block runs its SwiGLU glue and its weighted reduction as the prologue and the epilogue of the down product, two
- * launches instead of four; same bits either way, measured no faster; default 0), "qmm_trace_buffer" (device address of a uint64 [CTAs, 8] array that receives nanosecond
+ * slots by expert for larger batches; set it before asking for workspace sizes), "moe_fused" (0 = a small batch of the
+ * expert block keeps its SwiGLU glue and its weighted reduction in launches of their own instead of behind the gate and up
+ * products and the down product; same bits either way; default 1), "block_cluster" (few-row kernel with a cluster of CTAs per
+ * column block: CTAs of a cluster, 0 = chosen by a cost model, -1 = never), "qmm_trace_buffer" (device address of a uint64 [CTAs, 8] array that receives nanosecond
  * stamps of the tensor-core kernel's phases: start, set up, first epilogue begins, products issued, (unused),
  * epilogues done, end, activation copies issued; 0 = off), "tp_wait_ms" (how long a rank waits for the other ranks'
  * words inside a tensor- or expert-parallel kernel before it gives up with status 4; default 4000), "stack_wait_ms"

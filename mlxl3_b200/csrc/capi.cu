@@ -74,7 +74,7 @@ int valid_format(int k, int cb) {
 }
 
 std::atomic<bool> g_moe_sorted{true};                    // "moe_sorted" option: 0 keeps one row per slot for any batch
-std::atomic<bool> g_moe_fused{false};                    // "moe_fused" option: 1 folds the glue of a small batch into the down product (measured: no faster)
+std::atomic<bool> g_moe_fused{true};                     // "moe_fused" option: 0 keeps the glue of a small batch in launches of its own
 std::atomic<bool> g_qmm_enabled{true};                   // "qmm" option: 0 sends every batch through the fused kernel
 std::atomic<long long> g_tp_wait_ms{4000};
 std::atomic<long long> g_stack_wait_ms{2000};            // "stack_wait_ms" option: bound of a layer-boundary wait inside a step
@@ -190,6 +190,7 @@ int b200exl3_set_option(const char* name, int64_t value) {
     else if (!strcmp(name, "qmm_trace_buffer")) { b200exl3::g_qmm_trace = reinterpret_cast<unsigned long long*>(value); return 0; }
     else if (!strcmp(name, "moe_sorted")) { g_moe_sorted = value != 0; return 0; }
     else if (!strcmp(name, "moe_fused")) { g_moe_fused = value != 0; return 0; }
+    else if (!strcmp(name, "block_cluster")) { block_set_tuning(static_cast<int>(value)); return 0; }
     else if (!strcmp(name, "qmm_splits")) { qmm_set_tuning(static_cast<int>(value)); return 0; }
     else if (!strcmp(name, "qmv_trace_buffer")) {
         qmv_set_trace(reinterpret_cast<unsigned long long*>(static_cast<uintptr_t>(value)));
@@ -210,6 +211,14 @@ int b200exl3_plan_query(const char* kind, int in, int out, int k, int64_t rows, 
         const QmvPlan p = plan_qmv(in, out, k, rows);
         out_values[0] = p.grid; out_values[1] = p.max_pieces; out_values[2] = p.col_blocks; out_values[3] = kQmvWarps;
         out_values[4] = static_cast<int64_t>(p.smem_bytes); out_values[5] = p.fused_rotation ? 1 : 0;
+        return 0;
+    }
+    if (!strcmp(kind, "block")) {
+        const BlockPlan p = plan_block(in, out, k, rows);
+        out_values[0] = p.use ? 1 : 0;
+        if (!p.use) return 0;
+        out_values[1] = p.cluster; out_values[2] = p.grid; out_values[3] = kBlockWarps; out_values[4] = static_cast<int64_t>(p.smem_bytes);
+        out_values[5] = p.warp_smem; out_values[6] = p.xs_stride; out_values[7] = p.stage_offset;
         return 0;
     }
     if (!strcmp(kind, "qmm")) {
@@ -569,10 +578,12 @@ static int run_forward(const LayerCore& c, const void* d_x, int x_dtype, const u
     const bool exact = (c.flags & B200EXL3_EXACT_WEIGHTS) != 0;
     const size_t x_size = dtype_size(x_dtype);
     const __half* xhat = reinterpret_cast<const __half*>(d_xhat);
-    // more rows than the fused kernel rotates itself: the input rotation is a kernel of its own, and the SwiGLU
+    // up to 8 rows of a layer that fills one wave of clusters or less: one launch with a cluster of CTAs per column block.  Else,
+    // with more rows than the fused kernel rotates itself, the input rotation is a kernel of its own, and the SwiGLU
     // prologue (the only one taken with that many rows) is applied there
+    const BlockPlan block = tp ? BlockPlan{} : plan_block(c.in, c.out, c.k, rows);
     const __half* glu_up = nullptr;
-    if (pro && pro->kind == 2 && rows > kQmvFusedRows) {
+    if (pro && pro->kind == 2 && rows > kQmvFusedRows && !block.use) {
         glu_up = reinterpret_cast<const __half*>(pro->d_aux);
         pro = nullptr;
     }
@@ -609,7 +620,7 @@ static int run_forward(const LayerCore& c, const void* d_x, int x_dtype, const u
         }
         return 0;
     }
-    if (!xhat && rows > kQmvFusedRows) {
+    if (!xhat && rows > kQmvFusedRows && !block.use) {
         // more than two rows: rotate all of them once per group, the product kernel reads the rotated rows
         const QmvPlan first = plan_qmv(c.in, c.out, c.k, rows);
         __half* buf = reinterpret_cast<__half*>(base + kCounterBytes + qmv_partial_bytes(first, c.out, rows));
@@ -618,7 +629,6 @@ static int run_forward(const LayerCore& c, const void* d_x, int x_dtype, const u
     }
     for (int64_t r0 = 0; r0 < rows; r0 += kMaxBatchRows) {
         const int64_t n = rows - r0 < kMaxBatchRows ? rows - r0 : kMaxBatchRows;
-        const QmvPlan plan = plan_qmv(c.in, c.out, c.k, n, pro != nullptr);
         QmvArgs a{};
         a.wq = c.wq;
         a.x = !xhat ? static_cast<const char*>(d_x) + static_cast<size_t>(r0) * c.in * x_size : nullptr;
@@ -663,7 +673,8 @@ static int run_forward(const LayerCore& c, const void* d_x, int x_dtype, const u
             a.epi_sum = reinterpret_cast<__half*>(pro->d_residual_out);
             a.epi_sumsq = pro->d_sumsq_out;
         }
-        B200_TRY(launch_qmv(a, c.k, c.cb, exact, plan, stream), "fused linear kernel");
+        if (block.use) B200_TRY(launch_block(a, c.k, c.cb, exact, block, stream), "fused linear kernel");
+        else B200_TRY(launch_qmv(a, c.k, c.cb, exact, plan_qmv(c.in, c.out, c.k, n, pro != nullptr), stream), "fused linear kernel");
     }
     return 0;
 }
@@ -1273,10 +1284,6 @@ int b200exl3_moe_workspace_bytes(const b200exl3_moe* h, int64_t rows, size_t* ou
 // Measured on 128 experts, top-8, 2048 <-> 768, 3 bits, one token: 39.5 us against 39.1 us for the four launches with
 // dependent launch on (42.1 against 40.2 without): the launch gaps were already hidden, and every warp of the down
 // product now redoes the glue of its own input blocks.  Same bits either way; off unless the option asks for it.
-static bool moe_fused_fits(const b200exl3_moe* h, int64_t rows) {
-    const int64_t blocks = h->in / 128;
-    return g_moe_fused.load() != 0 && (rows * h->top_k + rows) * blocks + 1 <= static_cast<int64_t>(kCounterBytes / sizeof(unsigned int)) - 1;
-}
 
 int b200exl3_moe_forward(const b200exl3_moe* h, const void* d_x, int x_dtype, int64_t rows, const uint32_t* d_selected,
                          const void* d_scores, int score_dtype, void* d_y, void* ws, size_t ws_bytes, b200exl3_stream s) {
@@ -1348,8 +1355,13 @@ int b200exl3_moe_forward(const b200exl3_moe* h, const void* d_x, int x_dtype, in
     for (int64_t r0 = 0; r0 < rows; r0 += chunk) {
         const int64_t n = std::min(chunk, rows - r0), slots = n * h->top_k;
         const uint32_t* sel = d_selected + r0 * h->top_k;
+        // Where one wave of clusters holds it, the SwiGLU glue runs behind the gate and up products of a block, and the weighted
+        // sum over a token's slots behind the down product: two launches instead of four.
+        const bool fuse = g_moe_fused.load();
+        const BlockPlan gate_up = plan_block(h->in, static_cast<int>(slots * 2 * h->hidden), h->k, 1, BlockUse::kGateUp);
+        const BlockPlan down = plan_block(h->hidden, static_cast<int>(slots * h->in), h->k, 1, BlockUse::kDown, h->top_k);
         // every slot is one activation row against the columns of its own expert
-        auto mapped = [&](const uint32_t* wq, const __half* xhat, int in, int width, int proj, int stride_blocks, float* yhat) {
+        auto mapped = [&](const uint32_t* wq, const __half* xhat, int in, int width, int proj, int stride_blocks, float* yhat, BlockPlan block) {
             const int out = static_cast<int>(slots * proj * width);
             QmvArgs a{};
             a.wq = wq; a.xhat = xhat; a.xhat_group_stride = in;
@@ -1368,43 +1380,33 @@ int b200exl3_moe_forward(const b200exl3_moe* h, const void* d_x, int x_dtype, in
             a.tiles_n = h->experts * proj * width / 16;
             a.map_selected = sel; a.map_blocks = width / 128; a.map_proj = proj; a.map_stride_blocks = stride_blocks;
             a.map_experts = h->experts;
+            const bool fused = fuse && block.use;
+            // the same partition, and so the same sums, with the glue in launches of its own
+            if (!fused) block = plan_block(in, out, h->k, 1, BlockUse::kMapped, block.use ? block.parts : 0);
+            if (fused && proj == 1) {
+                a.epilogue = 3; a.svh = h->down_svh; a.yhat = nullptr;
+                a.epi_scores = static_cast<const char*>(d_scores) + static_cast<size_t>(r0) * h->top_k * score_size;
+                a.epi_score_f32 = score_dtype == kF32 ? 1 : 0;
+                a.gy[0] = static_cast<char*>(d_y) + static_cast<size_t>(r0) * h->in * score_size;
+                a.map_early = block.pdl_early ? 0 : 1;        // the launches before this one start it after their own wait for the routes
+            } else if (fused) {
+                a.epilogue = 4; a.glu_svh = h->gu_svh; a.glu_down_suh = h->down_suh; a.glu_out = xdown; a.yhat = nullptr;
+            }
+            if (block.use) return launch_block(a, h->k, h->cb, exact, block, stream);
             return launch_qmv(a, h->k, h->cb, exact, plan_qmv(in, out, h->k, 1, true), stream);
         };
         // gate/up: the kernel rotates each slot's token row itself, with the input scales of the slot's expert
-        B200_TRY(mapped(h->gu_wq, nullptr, h->in, h->hidden, 2, h->experts * (h->hidden / 128), ygu), "expert gate/up kernel");
-        if (moe_fused_fits(h, n)) {
-            const int out = static_cast<int>(slots * h->in);
-            QmvArgs a{};
-            a.wq = h->down_wq; a.xhat = nullptr; a.xhat_group_stride = h->hidden;
-            a.x = ygu;                                        // read through the prologue only
-            a.suh = h->down_suh;
-            a.prologue = 4; a.pro_ygu = ygu; a.pro_gu_svh = h->gu_svh; a.pro_logical = h->hidden;
-            a.map_top_k = h->top_k;
-            a.counters = reinterpret_cast<unsigned int*>(base);
-            a.error = reinterpret_cast<unsigned int*>(base + kCounterBytes - sizeof(unsigned int));
-            a.partials = reinterpret_cast<float*>(base + l.partials);
-            a.yhat = ydown;
-            a.epilogue = 3; a.svh = h->down_svh;
-            a.epi_scores = static_cast<const char*>(d_scores) + static_cast<size_t>(r0) * h->top_k * score_size;
-            a.epi_score_f32 = score_dtype == kF32 ? 1 : 0;
-            a.epi_counter0 = static_cast<int>(slots * (h->in / 128));
-            a.groups = 1; a.gcol0[0] = 0; a.gout[0] = out;
-            a.gy[0] = static_cast<char*>(d_y) + static_cast<size_t>(r0) * h->in * score_size;
-            a.x_dtype = kF16; a.y_dtype = kF16;
-            a.in = h->hidden; a.out = out; a.rows = 1;
-            a.tiles_n = h->experts * h->in / 16;
-            a.map_selected = sel; a.map_blocks = h->in / 128; a.map_proj = 1; a.map_stride_blocks = 0; a.map_experts = h->experts;
-            B200_TRY(launch_qmv(a, h->k, h->cb, exact, plan_qmv(h->hidden, out, h->k, 1, true), stream), "expert down kernel");
-            continue;
-        }
-        B200_TRY(launch_glu_down_input(ygu, h->gu_svh, h->down_suh, sel, h->experts, slots, h->hidden, h->hidden, xdown, stream),
-                 "SwiGLU glue");
-        B200_TRY(mapped(h->down_wq, xdown, h->hidden, h->in, 1, 0, ydown), "expert down kernel");
-        B200_TRY(launch_finish_and_reduce(ydown, h->down_svh, sel, h->experts,
-                                          static_cast<const char*>(d_scores) + static_cast<size_t>(r0) * h->top_k * score_size,
-                                          score_dtype, n, h->top_k, h->in,
-                                          static_cast<char*>(d_y) + static_cast<size_t>(r0) * h->in * score_size, stream),
-                 "expert reduction");
+        B200_TRY(mapped(h->gu_wq, nullptr, h->in, h->hidden, 2, h->experts * (h->hidden / 128), ygu, gate_up), "expert gate/up kernel");
+        if (!gate_up.use || !fuse)
+            B200_TRY(launch_glu_down_input(ygu, h->gu_svh, h->down_suh, sel, h->experts, slots, h->hidden, h->hidden, xdown, stream),
+                     "SwiGLU glue");
+        B200_TRY(mapped(h->down_wq, xdown, h->hidden, h->in, 1, 0, ydown, down), "expert down kernel");
+        if (!down.use || !fuse)
+            B200_TRY(launch_finish_and_reduce(ydown, h->down_svh, sel, h->experts,
+                                              static_cast<const char*>(d_scores) + static_cast<size_t>(r0) * h->top_k * score_size,
+                                              score_dtype, n, h->top_k, h->in,
+                                              static_cast<char*>(d_y) + static_cast<size_t>(r0) * h->in * score_size, stream),
+                     "expert reduction");
     }
     return 0;
 }

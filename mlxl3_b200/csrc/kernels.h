@@ -117,16 +117,16 @@ struct QmvArgs {
     int epi_max_ctx;           // ... rows per head of the caches ...
     __half* epi_k_cache;       // ... [k heads, max_ctx, 128]: rotated keys go to row *epi_pos
     __half* epi_v_cache;       // ... values are copied there
-    // expert-mapped down product of a small batch (one row per slot) with the glue around it in the same launch:
-    // prologue 4 = the SwiGLU glue (native/src/moe.rs:438-533) from the raw gate/up products of the launch before,
-    const float* pro_ygu;      // [slots * 2, in] raw gate and up products (in = the experts' width)
-    const __half* pro_gu_svh;  // [experts, 2, in] output scales of gate and up; suh = [experts, in] input scales of down
-    int pro_logical;           // columns at and past this one are padding: their activation is zero
-    // epilogue 3 = finish_and_reduce (moe.rs:586-609): every slot's block is rotated, scaled by svh[expert] and its score
-    // and parked in yhat; the last slot of a token to arrive adds the token's top_k blocks in slot order into gy[0]
+    // The expert block of a small batch, expert-mapped, one row per slot (cluster-per-column-block kernel only).
+    // Epilogue 4 (gate and up products): the SwiGLU glue (native/src/moe.rs:438-533) behind them, its result = the rotated input
+    // of the down product.
+    const __half* glu_svh;     // [experts, 2, width] output scales of gate and up
+    const __half* glu_down_suh;// [experts, width] input scales of down
+    __half* glu_out;           // [slots, width]
+    // Epilogue 3 (down product) = finish_and_reduce (moe.rs:586-609): every slot's block is rotated, scaled by svh[expert] and its
+    // score, and the cluster's first CTA adds the token's top_k blocks in slot order into gy[0]
     const void* epi_scores;    // [slots] routing weights, fp16 or fp32 (the output has their type)
     int epi_score_f32;
-    int epi_counter0;          // first of the (token, block) arrival counters inside `counters`
     int epilogue;
     const __half* epi_residual;
     __half* epi_sum;
@@ -135,6 +135,10 @@ struct QmvArgs {
     // exchanged with the other ranks (unit = (tp_row0 + row) * out/128 + block) before the output rotation.
     TpPeers tp;
     int tp_row0;
+    // cluster-per-column-block kernel only
+    int cluster;               // CTAs of a cluster: they share the block's inputs, or (prologue 4) are the slots of one token
+    int x_wide;                // four elements of x are one access
+    int map_early;             // the routes may be read before the wait for the kernel before this one
 };
 
 struct QmvPlan {
@@ -158,6 +162,27 @@ size_t qmv_partial_bytes(const QmvPlan& plan, int out, int64_t rows);
 cudaError_t launch_qmv(QmvArgs args, int k, int cb, bool exact, const QmvPlan& plan, cudaStream_t stream);
 void qmv_set_tuning(int ctas_per_sm, int force_grid, int pdl);
 void qmv_set_trace(unsigned long long* device_buffer);
+
+// ---- the same for up to 8 rows with a cluster of CTAs per column block (kernels_block*.cu) -----------------------
+// Warps of a CTA, one CTA per SM; they share the CTA's rows of 16 inputs.  4096->4096, 4 bits, one row: 16 warps 7.8 us, 12 warps 8.2,
+// 16 warps at 64 registers (two CTAs per SM, the spare one for the next launch) 8.6.
+constexpr int kBlockWarps = 16;
+constexpr int kBlockRows = 8;        // activation rows
+constexpr int kBlockCluster = 8;     // CTAs of a cluster (the portable limit)
+struct BlockPlan {
+    bool use;            // false: the layer goes to the kernel that deals it out over the whole grid
+    int cluster, parts, grid;            // CTAs of a cluster, of them those that share a column block's inputs
+    int warp_smem, xs_offset, xs_stride, stage_offset;
+    size_t smem_bytes;
+    bool pdl, pdl_early;
+};
+// The expert-mapped products of the expert block, one row each, have an `out` axis that is virtual (slots x projections x columns):
+// on their own, with the SwiGLU glue behind gate and up, with the weighted sum over a token's `top_k` slots behind down.
+enum class BlockUse { kLayer, kMapped, kGateUp, kDown };
+// `top_k`: of kMapped the parts that a column block's inputs are cut into (0: one, if a wave holds all blocks).
+BlockPlan plan_block(int in, int out, int k, int64_t rows, BlockUse use = BlockUse::kLayer, int top_k = 0);
+cudaError_t launch_block(QmvArgs args, int k, int cb, bool exact, const BlockPlan& plan, cudaStream_t stream);
+void block_set_tuning(int cluster);  // 0 automatic, -1 never, else the CTAs of a cluster
 
 // ---- a whole decode step in one persistent launch (kernels_stack*.cu) ------------------------------------------
 // The kernel streams weights in chunks of consecutive rows of a column block (one bulk copy each; a row is 8 tiles)

@@ -134,6 +134,105 @@ size_t qmv_partial_bytes(const QmvPlan& plan, int out, int64_t rows) {
     return (static_cast<size_t>(plan.col_blocks) * plan.max_pieces * r * 128 * sizeof(float) + 255) / 256 * 256;
 }
 
+cudaError_t block_dispatch_k1(const QmvArgs&, int, bool, const BlockPlan&, cudaStream_t);
+cudaError_t block_dispatch_k2(const QmvArgs&, int, bool, const BlockPlan&, cudaStream_t);
+cudaError_t block_dispatch_k3(const QmvArgs&, int, bool, const BlockPlan&, cudaStream_t);
+cudaError_t block_dispatch_k4(const QmvArgs&, int, bool, const BlockPlan&, cudaStream_t);
+cudaError_t block_dispatch_k5(const QmvArgs&, int, bool, const BlockPlan&, cudaStream_t);
+cudaError_t block_dispatch_k6(const QmvArgs&, int, bool, const BlockPlan&, cudaStream_t);
+cudaError_t block_dispatch_k7(const QmvArgs&, int, bool, const BlockPlan&, cudaStream_t);
+cudaError_t block_dispatch_k8(const QmvArgs&, int, bool, const BlockPlan&, cudaStream_t);
+
+static std::atomic<int> g_block_cluster{0};
+void block_set_tuning(int cluster) { g_block_cluster = cluster < -1 ? 0 : std::min(cluster, kBlockCluster); }
+
+BlockPlan plan_block(int in, int out, int k, int64_t rows, BlockUse use, int top_k) {
+    BlockPlan plan{};
+    const int forced = g_block_cluster.load();
+    const int64_t rb = in / 16, blocks = out / 128;
+    if (rows > kBlockRows || forced < 0 || g_force_grid.load() > 0) return plan;
+    const int ring = qmv_chunk_rows(k) * qmv_slots(k) * 64 * k * static_cast<int>(sizeof(uint32_t));
+    auto lay_out = [&](int cluster, int parts, int64_t r) {
+        // a part's rows may begin and end inside a block of 128 inputs
+        const int nblk = static_cast<int>(std::min<int64_t>(in / 128, (rb + parts - 1) / parts / 8 + 2));
+        plan.cluster = cluster;
+        plan.parts = parts;
+        plan.warp_smem = (std::max(ring, static_cast<int>(r) * kQmvRedStride * static_cast<int>(sizeof(float))) + 15) / 16 * 16;
+        plan.xs_offset = plan.warp_smem * kBlockWarps;
+        plan.xs_stride = nblk * 128 + 8;                     // rows four words apart modulo 32 banks
+        plan.stage_offset = plan.xs_offset + (static_cast<int>(r) * plan.xs_stride * static_cast<int>(sizeof(__half)) + 15) / 16 * 16;
+        // the parts of the rows that a CTA finishes (down product: its own sum, and the slots')
+        plan.smem_bytes = static_cast<size_t>(plan.stage_offset) + ((r + cluster - 1) / cluster * cluster + 1) * 128 * sizeof(float);
+        // One CTA per SM: where two fit, the hardware puts the CTAs of the next launch in pairs on the SMs that are free first, and the
+        // launch takes as long as such a pair (4096->4096, 4 bits, clusters of 4: 9.5 us instead of 8.2).
+        plan.smem_bytes = std::max(plan.smem_bytes, kQmvSharedSmemBytes + 4096);
+        return plan.smem_bytes <= static_cast<size_t>(kQmvMaxSmemBytes);
+    };
+    // Clusters of 1..8 CTAs that a B200 holds at one CTA per SM (a cluster lies inside one processing cluster of SMs); a constant, so
+    // that a layer's sums are added in the same order on every GPU.
+    constexpr int kResident[kBlockCluster] = {148, 74, 45, 33, 26, 22, 15, 15};
+    int cluster = 1, parts = 1;
+    int64_t clusters = blocks;
+    if (use == BlockUse::kMapped) {
+        plan.use = top_k > 0 || blocks <= kResident[0];
+        cluster = parts = std::max(1, top_k);
+    } else if (use == BlockUse::kDown) {
+        if (top_k < 1 || top_k > kBlockCluster) return plan;
+        cluster = top_k;
+        clusters = blocks / top_k;
+        plan.use = lay_out(cluster, 1, rows) && clusters <= kResident[top_k - 1];
+    } else {
+        // Microseconds fitted to sweeps of 1..8 CTAs over 22 shapes (512..14336 inputs, 128..28672 outputs, 2, 3, 4 and 6 bits, one
+        // row; the choice is 1 % above the best measured on average): a row of 16 inputs per warp, the sum over a cluster, a second
+        // wave of single CTAs; against the other kernel's launch, its decode over all SMs and the parts of its blocks.  The row
+        // count is left out, so that a row's sums are added in the same order in every batch of up to 8 (with 8 rows the other
+        // kernel is further behind where the inputs are few, because its input rotation is a launch of its own).
+        const int projections = use == BlockUse::kGateUp ? 2 : 1;
+        const bool even = k == 4 || k == 8;                  // the cheapest widths to decode
+        double best = forced > 0 || projections > 1 ? 1e30 : 7.5 + (even ? 0.00044 : 0.0005) * static_cast<double>(rb * blocks) + 0.004 * rb;
+        for (int n = 1; n * projections <= kBlockCluster && n <= rb; ++n) {
+            const int m = n * projections;
+            const int64_t waves = m == 1 && blocks > kResident[0] ? 2 : 1;
+            if (forced > 0 && projections == 1 ? m != forced : blocks / projections > waves * kResident[m - 1]) continue;
+            if (!lay_out(m, n, projections > 1 ? 1 : kBlockRows)) continue;
+            const double warp_rows = 0.5 * (static_cast<double>(((rb + n - 1) / n + kBlockWarps - 1) / kBlockWarps) + static_cast<double>(rb) / (n * kBlockWarps));
+            const double t = 0.7 + waves * (2.7 + (even ? 0.89 : 1.04) * warp_rows) + (m > 1 ? 1.0 + 0.04 * m : 0.0);
+            if (t < best) { best = t; cluster = m; parts = n; plan.use = true; }
+        }
+        clusters = blocks / projections;
+    }
+    plan.use = plan.use && lay_out(cluster, parts, rows);
+    plan.grid = static_cast<int>(clusters) * cluster;
+    const int pdl = g_pdl.load();
+    plan.pdl = pdl != 0;
+    plan.pdl_early = pdl == 2;
+    return plan;
+}
+
+cudaError_t launch_block(QmvArgs args, int k, int cb, bool exact, const BlockPlan& plan, cudaStream_t stream) {
+    if (!plan.use || args.rows <= 0 || args.rows > kBlockRows || args.tp.world > 0 || args.map_count != nullptr) return cudaErrorInvalidValue;
+    args.tiles_k = args.in / 16;
+    args.trace = g_trace.load();
+    args.cluster = plan.cluster;
+    args.warp_smem = plan.warp_smem;
+    args.xs_offset = plan.xs_offset;
+    args.xs_stride = plan.xs_stride;
+    args.stage_offset = plan.stage_offset;
+    args.x_wide = args.x != nullptr && four_at_once(args.x, args.x_dtype) ? 1 : 0;
+    args.pdl_early = plan.pdl_early ? 1 : 0;
+    switch (k) {
+        case 1: return block_dispatch_k1(args, cb, exact, plan, stream);
+        case 2: return block_dispatch_k2(args, cb, exact, plan, stream);
+        case 3: return block_dispatch_k3(args, cb, exact, plan, stream);
+        case 4: return block_dispatch_k4(args, cb, exact, plan, stream);
+        case 5: return block_dispatch_k5(args, cb, exact, plan, stream);
+        case 6: return block_dispatch_k6(args, cb, exact, plan, stream);
+        case 7: return block_dispatch_k7(args, cb, exact, plan, stream);
+        case 8: return block_dispatch_k8(args, cb, exact, plan, stream);
+        default: return cudaErrorInvalidValue;
+    }
+}
+
 cudaError_t launch_qmv(QmvArgs args, int k, int cb, bool exact, const QmvPlan& plan, cudaStream_t stream) {
     if (args.rows <= 0 || args.rows > kQmvMaxRows) return cudaErrorInvalidValue;
     args.tiles_k = args.in / 16;
