@@ -78,6 +78,46 @@ __device__ __forceinline__ void load4_as_half(const void* p, int dtype, int64_t 
     }
 }
 
+// Whether sixteen consecutive elements from a multiple of 16 on may be read 16 bytes at a time.
+__host__ __device__ __forceinline__ bool sixteen_bytes_at_once(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+
+// sixteen consecutive elements (i a multiple of 16): WIDE, 16 bytes at a time, which needs sixteen_bytes_at_once(p)
+template <bool WIDE>
+__device__ __forceinline__ void load16_as_half(const void* p, int dtype, int64_t i, __half2 (&h)[8]) {
+    if constexpr (!WIDE) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) h[j] = __halves2half2(load_as_half(p, dtype, i + 2 * j), load_as_half(p, dtype, i + 2 * j + 1));
+    } else if (dtype == kF32) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float4 v = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p) + i + 4 * j);
+            h[2 * j] = __floats2half2_rn(v.x, v.y); h[2 * j + 1] = __floats2half2_rn(v.z, v.w);
+        }
+    } else {
+        __align__(16) uint4 w[2];
+        w[0] = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(p) + i);
+        w[1] = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(p) + i + 8);
+        if (dtype == kF16) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) h[j] = reinterpret_cast<const __half2*>(w)[j];
+        } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const float2 f = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(w)[j]);
+                h[j] = __floats2half2_rn(f.x, f.y);
+            }
+        }
+    }
+}
+// ... and stored, at a multiple of 16 bytes
+__device__ __forceinline__ void store16_half(__half* p, const __half2 (&h)[8]) {
+    __align__(16) __half2 o[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) o[j] = h[j];
+    reinterpret_cast<uint4*>(p)[0] = reinterpret_cast<const uint4*>(o)[0];
+    reinterpret_cast<uint4*>(p)[1] = reinterpret_cast<const uint4*>(o)[1];
+}
+
 // store_from_half for four consecutive elements (i a multiple of 4); `bias` points at the first one's bias.  WIDE: in one
 // store, which needs four_at_once of both
 template <bool WIDE = true>
