@@ -189,7 +189,7 @@ BlockPlan plan_block(int in, int out, int k, int64_t rows, BlockUse use, int top
         // kernel is further behind where the inputs are few, because its input rotation is a launch of its own).
         const int projections = use == BlockUse::kGateUp ? 2 : 1;
         const bool even = k == 4 || k == 8;                  // the cheapest widths to decode
-        double best = forced > 0 || projections > 1 ? 1e30 : 7.5 + (even ? 0.00044 : 0.0005) * static_cast<double>(rb * blocks) + 0.004 * rb;
+        double best = forced > 0 || projections > 1 ? 1e30 : 7.0 + (even ? 0.00042 : 0.00048) * static_cast<double>(rb * blocks) + 0.004 * rb;
         for (int n = 1; n * projections <= kBlockCluster && n <= rb; ++n) {
             const int m = n * projections;
             const int64_t waves = m == 1 && blocks > kResident[0] ? 2 : 1;

@@ -335,6 +335,7 @@ __device__ __forceinline__ void qmv_finish_block(const QmvArgs& p, int cblock, u
     const int tile_floats = rows * 128;
     const float* piece_base = p.partials + static_cast<int64_t>(cblock) * p.max_pieces * tile_floats;
     float* piece_dst = p.partials + (static_cast<int64_t>(cblock) * p.max_pieces + piece) * tile_floats;
+    if (p.yhat == nullptr) asm volatile("prefetch.global.L1 [%0];" ::"l"(p.svh + cblock * 128 + lane * 4));   // read last
 #pragma unroll 1
     for (int pass = 0; pass < (pieces > 1 ? 2 : 1); ++pass) {
         if (pass == 1) {
@@ -469,16 +470,6 @@ qmv_kernel(const __grid_constant__ QmvArgs p) {
         if (threadIdx.x == 0) atomicExch(p.error, 2u);
         return;
     }
-    // warps of this CTA with a tile of block `cblock`, and those of them whose second block it is
-    auto contributors = [&](int cblock, unsigned int& mask, unsigned int& second) {
-        mask = second = 0;
-#pragma unroll 1
-        for (int w = 0; w < WARPS; ++w)
-            if (min(s_begin[w + 1], (cblock + 1) * UB) > max(s_begin[w], cblock * UB)) {
-                mask |= 1u << w;
-                if (s_begin[w] / UB != cblock) second |= 1u << w;
-            }
-    };
     // first and last CTA with rows of the block: the inverse of unit_begin (warp holding row x: ceil((x+1)*W/RT) - 1)
     auto sharing_ctas = [&](int cblock, int& i_first, int& i_last) {
         if (aligned) {
@@ -492,6 +483,28 @@ qmv_kernel(const __grid_constant__ QmvArgs p) {
             i_last = static_cast<int>(((static_cast<int64_t>(cblock + 1) * RB * W - 1) / RT) / WARPS);
         }
     };
+    // Of every block that the CTA's warps work on, worked out before anything is waited for (by every arriving warp for itself it
+    // took 1.3 us of a layer): the warps with a tile of it, those of them whose second block it is, and its CTAs.
+    __shared__ unsigned int s_mask[WARPS + 1], s_second[WARPS + 1];
+    __shared__ int s_first[WARPS + 1], s_pieces[WARPS + 1];
+    const int block0 = cta0 / UB;
+    if (threadIdx.x <= WARPS && (block0 + static_cast<int>(threadIdx.x)) * UB < s_begin[WARPS]) {
+        const int b = block0 + static_cast<int>(threadIdx.x);
+        unsigned int mask = 0, second = 0;
+#pragma unroll 1
+        for (int w = 0; w < WARPS; ++w)
+            if (min(s_begin[w + 1], (b + 1) * UB) > max(s_begin[w], b * UB)) {
+                mask |= 1u << w;
+                if (s_begin[w] < b * UB) second |= 1u << w;
+            }
+        int i_first, i_last;
+        sharing_ctas(b, i_first, i_last);
+        s_mask[threadIdx.x] = mask;
+        s_second[threadIdx.x] = second;
+        s_first[threadIdx.x] = i_first;
+        s_pieces[threadIdx.x] = i_last - i_first + 1;
+    }
+    __syncthreads();
     int slot = 0;
     uint32_t parity = 0;
     bool copy_lost = false;
@@ -687,21 +700,19 @@ qmv_kernel(const __grid_constant__ QmvArgs p) {
         // ---- phase 4: the last warp of the CTA to arrive at this block adds the CTA's tiles, meets the
         //      other CTAs of the block, rotates and stores ---------------------------------------------------
         if (rows > kQmvFusedRows) continue;                     // all warps finish the CTA's blocks together, below
-        unsigned int mask, second;
-        contributors(cblock, mask, second);
+        const int local = cblock - block0;
+        const unsigned int mask = s_mask[local];
         __syncwarp();
         unsigned int prev = 0;
         if (lane == 0) {
             __threadfence_block();                              // the staged tile before the arrival
-            prev = atomicAdd(&s_arrived[cblock - cta0 / UB], 1u);
+            prev = atomicAdd(&s_arrived[local], 1u);
         }
         prev = __shfl_sync(0xffffffffu, prev, 0);
         if (tracing) p.trace[blockIdx.x * 8 + 4] = global_ns();
         if (prev + 1 == static_cast<unsigned int>(__popc(mask))) {
             __threadfence_block();
-            int i_first, i_last;
-            sharing_ctas(cblock, i_first, i_last);
-            qmv_finish_block<kFused>(p, cblock, mask, second, i_last - i_first + 1, static_cast<int>(blockIdx.x) - i_first, smem_raw, lane);
+            qmv_finish_block<kFused>(p, cblock, mask, s_second[local], s_pieces[local], static_cast<int>(blockIdx.x) - s_first[local], smem_raw, lane);
             if (tracing) p.trace[blockIdx.x * 8 + 5] = global_ns();
         }
     }
@@ -709,13 +720,10 @@ qmv_kernel(const __grid_constant__ QmvArgs p) {
         __syncthreads();                                        // every tile of the CTA is staged
         if (tracing) p.trace[blockIdx.x * 8 + 4] = global_ns();
 #pragma unroll 1
-        for (int cblock = cta0 / UB; cblock * UB < s_begin[WARPS]; ++cblock) {
-            unsigned int mask, second;
-            contributors(cblock, mask, second);
-            int i_first, i_last;
-            sharing_ctas(cblock, i_first, i_last);
-            qmv_finish_many<kFused>(p, cblock, mask, second, i_last - i_first + 1, static_cast<int>(blockIdx.x) - i_first, smem_raw, &s_arrived[0],
-                                    warp, lane);
+        for (int cblock = block0; cblock * UB < s_begin[WARPS]; ++cblock) {
+            const int local = cblock - block0;
+            qmv_finish_many<kFused>(p, cblock, s_mask[local], s_second[local], s_pieces[local], static_cast<int>(blockIdx.x) - s_first[local], smem_raw,
+                                    &s_arrived[0], warp, lane);
         }
         if (tracing) p.trace[blockIdx.x * 8 + 5] = global_ns();
     }
