@@ -42,6 +42,8 @@ cudaError_t launch_reconstruct(const uint16_t* trellis, int tiles_k, int tiles_n
                                cudaStream_t stream);
 
 // ---- rotations (kernels_rotate.cu) ----------------------------------------------------------------
+// From this many 128-blocks on the input rotations take four blocks per warp: about one block for every warp the GPU holds.
+constexpr int64_t kQuadRotationUnits = 8192;
 // xhat[r, :] = H128(half(half(x[r, :]) * suh[(r % scale_rows), :])); scale_rows is 1 or rows.  With groups > 1 (scale_rows
 // 1) the rows are rotated once per member: suh [groups, in], xhat [groups, rows, in].
 cudaError_t launch_prepare(const void* x, int x_dtype, const __half* suh, int64_t scale_rows, int64_t rows, int in,

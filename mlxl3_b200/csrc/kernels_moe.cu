@@ -291,11 +291,41 @@ route_plan_grouped_kernel(const uint32_t* __restrict__ selected, int64_t slots, 
     }
 }
 
-// Four (slot, 128-block) pairs per warp (see quad_hadamard128_f16), every projection of the slot's expert: row slot_row of each
-// projection's `slots` rows.  WIDE: x starts at a multiple of 16 bytes.
+// One warp per (slot, 128-block), every projection of the slot's expert: row slot_row of each projection's `slots` rows.
+// WIDE: x lies so that four elements are one access.
 template <bool WIDE>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 routed_prepare_kernel(const void* __restrict__ x, int x_dtype, const __half* __restrict__ suh, const uint32_t* __restrict__ selected,
+                      const uint32_t* __restrict__ slot_row, int experts, int64_t slots, int top_k, int proj, int in,
+                      __half* __restrict__ xhat) {
+    pdl_launch_dependents();                    // the kernel after this one may start; it waits for our memory itself
+    pdl_wait();                                 // what the kernel before this one wrote is visible from here on
+    const int lane = threadIdx.x & 31;
+    const int blocks_per_row = in >> 7;
+    const int64_t total = slots * blocks_per_row;
+    for (int64_t unit = static_cast<int64_t>(blockIdx.x) * kWarpsPerBlock + (threadIdx.x >> 5); unit < total;
+         unit += static_cast<int64_t>(gridDim.x) * kWarpsPerBlock) {
+        const int64_t slot = unit / blocks_per_row;
+        const int col = static_cast<int>(unit - slot * blocks_per_row) * 128 + lane * 4;
+        const int64_t row = slot_row[slot];
+        __half v[4];
+        load4_as_half<WIDE>(x, x_dtype, slot / top_k * in + col, v);
+        const __half* s = suh + static_cast<int64_t>(expert_of(selected, slot, experts)) * proj * in + col;
+        for (int p = 0; p < proj; ++p) {
+            const uint2 sw = *reinterpret_cast<const uint2*>(s + p * in);
+            __align__(8) __half h[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) h[j] = __hmul_rn(v[j], reinterpret_cast<const __half*>(&sw)[j]);
+            warp_hadamard128_f16(h, lane);
+            *reinterpret_cast<uint2*>(xhat + (p * slots + row) * in + col) = *reinterpret_cast<uint2*>(h);
+        }
+    }
+}
+
+// The same for many slots, four (slot, 128-block) pairs per warp (see quad_hadamard128_f16 and the plain input rotation).  WIDE: x starts at a multiple of 16 bytes.
+template <bool WIDE>
+__global__ void __launch_bounds__(kWarpsPerBlock * 32)
+routed_prepare_quads_kernel(const void* __restrict__ x, int x_dtype, const __half* __restrict__ suh, const uint32_t* __restrict__ selected,
                       const uint32_t* __restrict__ slot_row, int experts, int64_t slots, int top_k, int proj, int in,
                       __half* __restrict__ xhat) {
     pdl_launch_dependents();                    // the kernel after this one may start; it waits for our memory itself
@@ -341,7 +371,11 @@ cudaError_t launch_route_plan(const uint32_t* selected, int64_t slots, int exper
 
 cudaError_t launch_routed_prepare(const void* x, int x_dtype, const __half* suh, const uint32_t* selected, const uint32_t* slot_row,
                                   int experts, int64_t slots, int top_k, int proj, int in, __half* xhat, cudaStream_t stream) {
-    return launch_dependent(sixteen_bytes_at_once(x) ? routed_prepare_kernel<true> : routed_prepare_kernel<false>, dim3(grid_for((slots * (in / 128) + 3) / 4)), dim3(kWarpsPerBlock * 32), 0, stream, x, x_dtype, suh,
+    const int64_t units = slots * (in / 128);
+    const bool quads = units > kQuadRotationUnits;
+    auto kernel = quads ? (sixteen_bytes_at_once(x) ? routed_prepare_quads_kernel<true> : routed_prepare_quads_kernel<false>)
+                        : (four_at_once(x, x_dtype) ? routed_prepare_kernel<true> : routed_prepare_kernel<false>);
+    return launch_dependent(kernel, dim3(grid_for(quads ? (units + 3) / 4 : units)), dim3(kWarpsPerBlock * 32), 0, stream, x, x_dtype, suh,
                             selected, slot_row, experts, slots, top_k, proj, in, xhat);
 }
 

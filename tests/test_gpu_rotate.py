@@ -67,3 +67,14 @@ def test_rotation_edge_cases(gpu):
     once = gpu.codec.prepare(x, np.ones(128, np.float16))
     twice = gpu.codec.prepare(once, np.ones(128, np.float16))
     assert np.allclose(twice.astype(np.float32), x.astype(np.float32), atol=2e-3)
+
+
+@pytest.mark.parametrize("rows,n_in", [(2049, 512), (8193, 128), (75, 14080)])
+def test_many_rows_take_four_blocks_a_warp(gpu, rows, n_in):
+    """Past the line where a warp rotates four blocks, with a last warp that has all, one or two of them."""
+    rng = np.random.default_rng(rows)
+    x = rng.standard_normal((rows, n_in)).astype(np.float32)
+    suh = rng.uniform(0.5, 1.5, n_in).astype(np.float16)
+    assert rows * n_in // 128 > 8192
+    for code, data in ((gpu.F16, x.astype(np.float16)), (gpu.F32, x)):
+        assert np.array_equal(bits(gpu.codec.prepare(data, suh, code)), bits(oracle.prepare(data, suh)))
