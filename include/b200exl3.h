@@ -63,7 +63,7 @@ int b200exl3_version(void);
  * of more than 8 rows also go through the small-batch kernel (16 rows per launch) instead of the tensor-core product; default 1),
  * "qmm_splits" (CTAs per tile of the tensor-core product, 0 = chosen by a cost model; set it before asking for
  * workspace sizes), "moe_sorted" (0 = the expert block runs one row per slot for any batch instead of grouping
- * slots by expert for larger batches; set it before asking for workspace sizes), "moe_fused" (0 = a small batch of the
+ * slots by expert where that is faster, 2 = it groups them in any batch; set it before asking for workspace sizes), "moe_fused" (0 = a small batch of the
  * expert block keeps its SwiGLU glue and its weighted reduction in launches of their own instead of behind the gate and up
  * products and the down product; same bits either way; default 1), "block_cluster" (few-row kernel with a cluster of CTAs per
  * column block: CTAs of a cluster, 0 = chosen by a cost model, -1 = never), "qmm_trace_buffer" (device address of a uint64 [CTAs, 8] array that receives nanosecond

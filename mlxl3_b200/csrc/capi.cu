@@ -73,7 +73,7 @@ int valid_format(int k, int cb) {
     return 0;
 }
 
-std::atomic<bool> g_moe_sorted{true};                    // "moe_sorted" option: 0 keeps one row per slot for any batch
+std::atomic<int> g_moe_sorted{1};                       // "moe_sorted" option: 0 keeps one row per slot for any batch, 2 sorts any batch
 std::atomic<bool> g_moe_fused{true};                     // "moe_fused" option: 0 keeps the glue of a small batch in launches of its own
 std::atomic<bool> g_qmm_enabled{true};                   // "qmm" option: 0 sends every batch through the fused kernel
 std::atomic<long long> g_tp_wait_ms{4000};
@@ -188,7 +188,7 @@ int b200exl3_set_option(const char* name, int64_t value) {
         return 0;
     }
     else if (!strcmp(name, "qmm_trace_buffer")) { b200exl3::g_qmm_trace = reinterpret_cast<unsigned long long*>(value); return 0; }
-    else if (!strcmp(name, "moe_sorted")) { g_moe_sorted = value != 0; return 0; }
+    else if (!strcmp(name, "moe_sorted")) { g_moe_sorted = static_cast<int>(value); return 0; }
     else if (!strcmp(name, "moe_fused")) { g_moe_fused = value != 0; return 0; }
     else if (!strcmp(name, "block_cluster")) { block_set_tuning(static_cast<int>(value)); return 0; }
     else if (!strcmp(name, "qmm_splits")) { qmm_set_tuning(static_cast<int>(value)); return 0; }
@@ -1206,11 +1206,19 @@ static MoeSortedLayout moe_sorted_layout(const b200exl3_moe* h, int64_t rows) {
 }
 
 static bool moe_sorted(const b200exl3_moe* h, int64_t rows) {
-    // Worth it once experts see several rows each.  Two slots per expert is on the safe side: with the kernels as they are the
-    // sorted form is the faster one from about 24 slots of 8 experts, 40 of 32, 64 of 64 and 100 of 128 on (2048 <-> 768, 3 bits;
-    // slots / sorted in us: 8 experts, 24 slots 46 / 43; 32, 48 slots 75 / 66; 64, 96 slots 133 / 112; 128, 64 slots 97 / 105,
-    // 128 slots 169 / 160, 248 slots 367 / 195).
-    if (!g_moe_sorted || !g_qmm_enabled || rows * h->top_k < std::max<int64_t>(kMoeSortedMinSlots, 2 * static_cast<int64_t>(h->experts))) return false;
+    const int mode = g_moe_sorted.load();
+    const int64_t slots = rows * h->top_k;
+    if (mode == 0 || !g_qmm_enabled) return false;
+    // One row per slot decodes an expert's columns for every slot, the sorted form once per expert asked for (at most min(slots,
+    // experts) of them), at the price of two more launches and the tensor-core kernel's start.  In units of the columns of a
+    // 2048 <-> 768 expert a slot costs 1.4 us and an expert of the sorted form 0.9; small experts cost a slot more than their columns.
+    // One row per slot / sorted in us: 128 experts, top 8, 2048 <-> 768, 3 bits, 40 slots 66 / 71, 64 94 / 84, 248 359 / 139; 64,
+    // top 6, 2048 <-> 1408, 4 bits, 24 slots 65 / 70, 36 87 / 80; 60, 1024 <-> 512, 2 bits, 48 slots 37 / 41, 100 53 / 44; 32,
+    // 1024 <-> 256, 3 bits, 64 slots 33 / 39, 96 39 / 40; 8, 512 <-> 256, 4 bits, 100 slots 29 / 32, 200 37 / 32.
+    const double expert = static_cast<double>(h->in) * h->hidden / (2048.0 * 768.0);
+    const double gain = expert * (1.4 * slots - 0.9 * std::min<int64_t>(slots, h->experts));
+    const bool worth = gain > (slots >= std::max<int64_t>(kMoeSortedMinSlots, 2 * static_cast<int64_t>(h->experts)) ? 17.0 : 24.0);
+    if (!worth && mode != 2) return false;
     // the route plan keeps 2 * experts + 1 counters and one 16-bit expert id per slot of a pass in 48 KiB of shared
     // memory; shapes beyond that keep one row per slot
     const size_t plan_smem = (2 * static_cast<size_t>(h->experts) + 1) * sizeof(int) +

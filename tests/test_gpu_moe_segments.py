@@ -63,3 +63,22 @@ def test_workspace_holds_the_slots_and_no_padding(gpu, rows):
     shared = 148 * 2 * 64 * 128 * 4                          # parts of items that CTAs share, two per CTA
     assert moe.workspace_bytes(rows) <= slots * (per_slot + 64) + shared + (1 << 16)
     moe.close()
+
+
+@pytest.mark.parametrize("experts,top_k,rows", [(64, 8, 1), (128, 4, 9), (5, 1, 3)])
+def test_sorted_form_with_few_slots(gpu, experts, top_k, rows):
+    """The sorted form is taken from far fewer than a row per expert on: experts without rows, segments of one row."""
+    rng = np.random.default_rng(experts + rows)
+    n_in, hidden, k = 256, 384, 3
+    bank = make_bank(rng, experts, n_in, hidden, k)
+    moe = gpu.Exl3SwitchGlu(*bank, top_k, k, 0, exact_weights=True)
+    x = rng.standard_normal((rows, n_in)).astype(np.float16)
+    selected, scores = routes(rng, rows, experts, top_k)
+    gpu.set_option("moe_sorted", 2)
+    try:
+        got = moe.forward(x, selected, scores)
+    finally:
+        gpu.set_option("moe_sorted", 1)
+    check(got, oracle.switch_glu_forward(*bank, top_k, k, 0, x, selected, scores), rms=3e-3)
+    assert gpu.workspace_status(moe._workspace) == 0
+    moe.close()
