@@ -138,7 +138,7 @@ struct QmvArgs {
     TpPeers tp;
     int tp_row0;
     // cluster-per-column-block kernel only
-    int cluster;               // CTAs of a cluster: they share the block's inputs, or (prologue 4) are the slots of one token
+    int cluster;               // CTAs of a cluster: they share the block's inputs (epilogue 4: of two blocks), or (epilogue 3) are the slots of one token
     int x_wide;                // four elements of x are one access
     int map_early;             // the routes may be read before the wait for the kernel before this one
 };

@@ -18,19 +18,17 @@
 //  * one thread issues the stage's eight products and one commit, which frees the A stage and the activation slot.
 //  * tiles of up to 64 tokens: two accumulators, so that four more warps finish an item while the next one is multiplied.
 //
-// What bounds it: up to 64 rows the decode.  Cycles per 16x16 tile and scheduler with sixteen decoder warps: the decode loop
-// alone (words resident in shared memory, tensor-memory stores and nothing else) 47 at 4 bits, 51 at 3, 52 at 1 and 2, 54 at 5
-// and 6; in the kernel 59 at 4 bits and 68 at 3, and another 5 to 8 of waits for packed words and for the products.  A stage
-// takes 1060 to 1230 cycles (16 rows, 5120 inputs), 0.58 to 0.66 us at the 1845 MHz that the cycle counter shows against the
-// global timer while tensor-core instructions run (nvidia-smi reports 1965).  That depends neither on how many SMs work (3 bits:
-// 1180 cycles with 37, 1181 with 74, 1199 with 148) nor on where the weights come from (1167 when all stages read the same
-// ones).  At NT = 256 a stage takes 1320 cycles, 1024 of them products, and back to back the power cap holds the clock at 1560.
+// What bounds it: up to 64 rows the decode, and of it the issue slots: the decode loop alone (words resident in shared memory,
+// tensor-memory stores and nothing else) executes 43 warp instructions per 16x16 tile at 4 bits and 48 at 3, in 47 to 49 and 51 to 53
+// cycles per tile and scheduler; in the kernel all roles together execute 51 (4 bits), at 0.80 per cycle (instruction cache
+// misses, the single-thread roles), 64 cycles per tile from the first stage to the last.  The clock is 1845 MHz by the cycle counter
+// while tensor-core instructions run (nvidia-smi reports 1965).  A stage takes the same time however many SMs work and wherever the
+// weights come from (measured with 37, 74 and 148 SMs, and with all stages reading the same ones).  At NT = 256 a stage takes 1320 cycles, 1024 of them products, and back to back the power cap holds the clock at 1560.
 // Stages of 128 inputs and a single barrier per stage are there because the single-thread roles share the schedulers with
 // decoders that keep the integer pipes full: an instruction of theirs takes about eight cycles, a stage of any of them 400 to
 // 600.  For the same reason the issuing loop is unrolled over the ring and its thread picked by elect.sync; the producers'
-// loops stay rolled (all three unrolled: 714 ns per 64 inputs against 523).  Measured: 64 rows 4096->14336, 4 bits, 42 -> 29.7 us
-// with the input rotation; 16 rows 5120->25600, 3 bits, 74 -> 48.2 us (A in shared memory, one CTA per item and 64-token tile
-// before).
+// loops stay rolled (all three unrolled: 714 ns per 64 inputs against 523).  Us per call with the input rotation: 64 rows
+// 4096->14336, 4 bits, 21.7; 16 rows 5120->2x25600, 3 bits, 72.0.
 // Every wait is bounded in time; a wait that gives up sets the status word and the kernel still releases its tensor memory.
 #include <cuda.h>
 
