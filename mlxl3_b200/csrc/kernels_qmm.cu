@@ -60,12 +60,13 @@ struct QmmShape {
     static constexpr uint32_t kAccums = NT == 64 ? 2 : 1;
     static constexpr int kFinishers = NT == 64 ? 4 : kDecoders;
     static constexpr int kThreads = 32 * (kFirstDecoder + kDecoders + (NT == 64 ? kFinishers : 0));
-    // Stages in flight, packed (2048 * K bytes of shared memory each) and decoded (64 columns of tensor memory beside the
-    // accumulators), so that one slot number serves both.  A multiple of the decoder groups: a slot always belongs to one group,
-    // since parity alone does not tell a phase from the one after the next, and a group that met a slot only every other time
-    // could take a copy that has not landed for its own.  With two packed slots above 4 bits the decoders waited for the copies:
-    // 1969 rows 7936->1408, 6 bits, 98 -> 83 us; 128 rows 4096->14336, 8 bits, 37.9 -> 31.
-    static constexpr int kSlots = NT == 64 && K <= 4 ? 6 : 4;
+    static constexpr int kSlots = NT == 64 ? 6 : 4;    // A stages in tensor memory beside the accumulators
+    // Packed stages (2048 * K bytes) in flight.  A multiple of the decoder groups, so that a slot always belongs to one group:
+    // parity alone does not tell a phase from the one after the next, and a group that met a slot only every other time could
+    // take a copy that has not landed for its own.  With two slots above 4 bits the decoders waited for the copies: 1969 rows
+    // 7936->1408, 6 bits, 98 -> 83 us; 128 rows 4096->14336, 8 bits, 37.9 -> 31.
+    static constexpr int kRaw = NT == 64 && K <= 4 ? 6 : 4;
+    static_assert(kRaw % kGroups == 0, "a slot belongs to one group");
     static constexpr int kBSlots = NT == 64 ? kSlots : 2;   // activation stages in shared memory; divides kSlots
     static constexpr uint32_t kBHalfBytes = NT * 128;  // NT tokens x 64 fp16
     static constexpr uint32_t kBSlotBytes = 2 * kBHalfBytes;
@@ -75,7 +76,7 @@ struct QmmShape {
 template <int K, int NT>
 constexpr size_t qmm_smem_bytes() {
     using S = QmmShape<K, NT>;
-    return 1024 + S::kBSlots * S::kBSlotBytes + static_cast<size_t>(S::kSlots) * 2048 * K + S::kEpilogueBytes;
+    return 1024 + S::kBSlots * S::kBSlotBytes + static_cast<size_t>(S::kRaw) * 2048 * K + S::kEpilogueBytes;
 }
 
 __device__ __forceinline__ uint64_t umma_desc(uint32_t smem_byte_addr) {
@@ -142,8 +143,9 @@ __device__ __forceinline__ void tmem_st_tile(uint32_t taddr, uint32_t a0, uint32
 // Wait that gives up after about a quarter of a second, or at once when another role of the CTA has
 // already given up, so that a lost copy or a miscounted barrier ends the kernel instead of hanging it.
 __device__ __noinline__ bool qmm_wait_slow(uint64_t* bar, uint32_t parity, volatile int* cta_failed) {
+    for (int i = 0; i < 64; ++i)
+        if (mbar_try_wait(bar, parity)) return true;
     constexpr uint32_t kNap = 20000;                             // the hardware wakes the thread when the phase completes
-    if (mbar_try_wait_for(bar, parity, kNap)) return true;
     const unsigned long long t0 = global_ns();
     while (true) {
         if (mbar_try_wait_for(bar, parity, kNap)) return true;
@@ -281,7 +283,7 @@ qmm_kernel(const __grid_constant__ CUtensorMap xmap, const QmmArgs p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr int kRawWords = 512 * K;                       // a packed stage: 8 tile rows x 2 quads x 32K words
     constexpr uint32_t kRawBytes = kRawWords * 4;
-    __shared__ __align__(8) uint64_t full[S::kSlots], done[S::kSlots], full2[S::kSlots], half[S::kSlots], raw_full[S::kSlots], raw_empty[S::kSlots];
+    __shared__ __align__(8) uint64_t full[S::kSlots], done[S::kSlots], full2[S::kSlots], half[S::kSlots], raw_full[S::kRaw], raw_empty[S::kRaw];
     __shared__ __align__(8) uint64_t accum_full[S::kAccums], accum_free[S::kAccums], last_full;
     __shared__ uint32_t tmem_base_slot, s_last[2];
     __shared__ volatile int s_failed;
@@ -301,13 +303,13 @@ qmm_kernel(const __grid_constant__ CUtensorMap xmap, const QmmArgs p) {
     // shared memory: activation ring | packed ring | epilogue staging; the swizzled operand needs 1024-byte alignment
     unsigned char* b_base = smem_raw + ((1024u - (smem_addr(smem_raw) & 1023u)) & 1023u);
     uint32_t* raw_base = reinterpret_cast<uint32_t*>(b_base + S::kBSlots * S::kBSlotBytes);
-    __half* stage_base = reinterpret_cast<__half*>(raw_base + S::kSlots * kRawWords);
+    __half* stage_base = reinterpret_cast<__half*>(raw_base + S::kRaw * kRawWords);
 
     if (threadIdx.x == 0) {
         // a stage is full when its eight decoder warps and its activation copies have arrived (of a large tile the first half;
         // the second has a barrier of its own, and so has the end of the first half's products)
         for (int s = 0; s < S::kSlots; ++s) { mbar_init(&full[s], 9); mbar_init(&done[s], 1); mbar_init(&full2[s], 1); mbar_init(&half[s], 1); }
-        for (int s = 0; s < S::kSlots; ++s) { mbar_init(&raw_full[s], 1); mbar_init(&raw_empty[s], 8); }
+        for (int s = 0; s < S::kRaw; ++s) { mbar_init(&raw_full[s], 1); mbar_init(&raw_empty[s], 8); }
         mbar_init(&last_full, 1);
         for (uint32_t s = 0; s < S::kAccums; ++s) { mbar_init(&accum_full[s], 1); mbar_init(&accum_free[s], S::kFinishers); }
         s_failed = 0;
@@ -477,23 +479,25 @@ qmm_kernel(const __grid_constant__ CUtensorMap xmap, const QmmArgs p) {
         // 54.9 -> 51.2 (43.1 are the decode); 16 rows 5120->2x25600, 3 bits, 80.1 -> 72.0 us; 64 rows 4096->14336, 4 bits,
         // 24.1 -> 21.7; expert block 37 / 256 tokens 165 -> 143 / 230 -> 213.  The loop unrolled over the ring of slots executes 49.6
         // but misses the instruction cache twice as often (78.8 us); two rows at a time, rolled: 53.0 and 74.9 us.
-        const uint32_t wait_bar = smem_addr(lane == 0 ? raw_full : done), arrive_bar = smem_addr(lane == 0 ? full : raw_empty);
+        const uint32_t wait_bar = smem_addr(lane == 0 ? raw_full : done), arrive_bar = smem_addr(lane == 0 ? raw_empty : full);
         const bool arrives = lane < 2;
         const uint32_t a_stages = lanes + S::kAccums * NT + rows4 * 32;
-        uint32_t at = group * 8, par = lane == 0 ? 0u : 1u;      // byte offset of the slot's barriers; parity this lane waits for
+        // byte offsets of the slots' barriers (A stage, packed stage, the one this lane waits and arrives for); parity it waits for
+        uint32_t at = group * 8, raw_at = group * 8, my_at = group * 8, par = lane == 0 ? 0u : 1u;
+        const uint32_t my_end = lane == 0 ? S::kRaw * 8 : S::kSlots * 8;
         int it = group;
         auto decode_until = [&](const int end) {
 #pragma unroll 1
             for (; it < end; it += S::kGroups) {
                 // the packed stage has landed, and the MMAs that read this A stage last time are done
-                if (!__all_sync(0xffffffffu, mbar_try_wait(wait_bar + at, par))) {
-                    const bool ready = qmm_wait(lane == 0 ? &raw_full[at / 8] : &done[at / 8], par, &s_failed);
+                if (!__all_sync(0xffffffffu, mbar_try_wait(wait_bar + my_at, par))) {
+                    const bool ready = qmm_wait(lane == 0 ? &raw_full[my_at / 8] : &done[my_at / 8], par, &s_failed);
                     if (!__all_sync(0xffffffffu, ready)) break;
                 }
                 __syncwarp();
                 // the stores below come after the products that read this A stage last
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t* rw = words + at * (kRawWords / 8);
+                const uint32_t* rw = words + (S::kRaw == S::kSlots ? at : raw_at) * (kRawWords / 8);
                 const uint32_t dst = a_stages + at * (kStageCols / 8);
                 uint2 w2[4], w1[4], w0[4];
 #pragma unroll
@@ -518,9 +522,18 @@ qmm_kernel(const __grid_constant__ CUtensorMap xmap, const QmmArgs p) {
                 tile_pair(std::integral_constant<int, 3>{});
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                mbar_arrive(arrives, arrive_bar + at);           // decoded; the packed words were consumed
+                mbar_arrive(arrives, arrive_bar + (S::kRaw == S::kSlots ? at : my_at));   // decoded; the packed words were consumed
                 at += S::kGroups * 8;
-                if (at >= S::kSlots * 8) { at -= S::kSlots * 8; par ^= 1u; }
+                if constexpr (S::kRaw == S::kSlots) {
+                    if (at >= S::kSlots * 8) { at -= S::kSlots * 8; par ^= 1u; }
+                    my_at = at;
+                } else {
+                    if (at >= S::kSlots * 8) at -= S::kSlots * 8;
+                    raw_at += S::kGroups * 8;
+                    if (raw_at >= S::kRaw * 8) raw_at -= S::kRaw * 8;
+                    my_at += S::kGroups * 8;
+                    if (my_at >= my_end) { my_at -= my_end; par ^= 1u; }
+                }
             }
         };
         auto finish = [&](uint32_t item, uint32_t seg, int stages) {
@@ -553,7 +566,7 @@ qmm_kernel(const __grid_constant__ CUtensorMap xmap, const QmmArgs p) {
             bool running = true;
             while (running) {
 #pragma unroll 1
-                for (int s = 0; s < S::kSlots; ++s) {
+                for (int s = 0; s < S::kRaw; ++s) {
                     if (!qmm_wait(&raw_empty[s], par ^ 1u, &s_failed)) { running = false; break; }
                     mbar_expect_tx(&raw_full[s], kRawBytes);
                     bulk_copy_g2s(raw_base + s * kRawWords, src, kRawBytes, &raw_full[s]);
