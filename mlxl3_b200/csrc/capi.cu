@@ -581,7 +581,8 @@ static int run_forward(const LayerCore& c, const void* d_x, int x_dtype, const u
     // up to 8 rows of a layer that fills one wave of clusters or less: one launch with a cluster of CTAs per column block.  Else,
     // with more rows than the fused kernel rotates itself, the input rotation is a kernel of its own, and the SwiGLU
     // prologue (the only one taken with that many rows) is applied there
-    const BlockPlan block = tp ? BlockPlan{} : plan_block(c.in, c.out, c.k, rows);
+    // -- of a row shard too: a rank's sums are the same with the exchange inside the kernel and without one
+    const BlockPlan block = plan_block(c.in, c.out, c.k, rows);
     const __half* glu_up = nullptr;
     if (pro && pro->kind == 2 && rows > kQmvFusedRows && !block.use) {
         glu_up = reinterpret_cast<const __half*>(pro->d_aux);

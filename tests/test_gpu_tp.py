@@ -12,7 +12,7 @@ import numpy as np
 import pytest
 
 import oracle
-from tests.gpu_util import gpu  # noqa: F401
+from tests.gpu_util import bits, gpu, random_layer  # noqa: F401
 
 pytestmark = pytest.mark.gpu
 
@@ -62,6 +62,34 @@ def test_world_of_one_equals_plain_finish(gpu):
     with pytest.raises(gpu.B200Exl3Error, match="exceed the exchange buffers"):
         small = TpContext(0, 1, 2, lambda raw: [raw])
         small.finish(layer, d_yhat.ptr, rows, gpu.F16, d_y.ptr, stream)
+    ctx.close()
+    layer.close()
+
+
+@pytest.mark.parametrize("n_in,n_out,rows", [(4096, 1408, 1), (2176, 4096, 3), (4096, 256, 8), (14336, 512, 2), (4096, 28672, 2)])
+def test_the_fused_exchange_adds_in_the_order_of_the_plain_product(gpu, n_in, n_out, rows):
+    """One rank's sums are the same bits with the exchange inside the kernel, without one, and as a raw product: layers cut into
+    clusters of several CTAs, where another order of the fp32 sums shows in the outputs, and one that is dealt out over the grid."""
+    from mlxl3_b200.runtime import DeviceBuffer, Stream
+    from mlxl3_b200.tp import TpContext
+    rng = np.random.default_rng(n_in + n_out)
+    trellis, suh, svh = random_layer(rng, n_in, n_out, 3, signs=False)
+    x = rng.standard_normal((rows, n_in)).astype(np.float16)
+    layer = gpu.Exl3Linear(trellis, suh, svh, None, 3, 0)
+    stream = Stream()
+    ctx = TpContext(0, 1, rows * n_out // 128, lambda raw: [raw])
+    d_x, d_y, d_yhat = DeviceBuffer.from_numpy(x), DeviceBuffer(rows * n_out * 2), DeviceBuffer(rows * n_out * 4)
+    ws = gpu.new_workspace(layer.workspace_bytes(rows))
+    layer.forward_device(d_x.ptr, gpu.F16, rows, d_y.ptr, ws, stream)
+    plain = d_y.download((rows, n_out), np.float16, stream)
+    layer.forward_partial_device(d_x.ptr, gpu.F16, rows, d_yhat.ptr, ws, stream)
+    partial = d_yhat.download((rows, n_out), np.float32, stream)
+    for _ in range(3):                                   # both slots of every unit get used
+        d_y.fill(0, stream)
+        ctx.forward(layer, d_x.ptr, gpu.F16, rows, d_y.ptr, ws, stream)
+        assert np.array_equal(bits(d_y.download((rows, n_out), np.float16, stream)), bits(plain))
+    assert np.array_equal(bits(oracle.finish(partial, svh, None)), bits(plain))
+    assert gpu.workspace_status(ws) == 0 and ctx.status() == 0
     ctx.close()
     layer.close()
 
