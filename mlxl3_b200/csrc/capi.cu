@@ -1287,12 +1287,11 @@ int b200exl3_moe_workspace_bytes(const b200exl3_moe* h, int64_t rows, size_t* ou
     return 0;
 }
 
-// Two launches instead of four for a small batch (one row per slot): the down product takes the SwiGLU glue as its
-// prologue and finish_and_reduce as its epilogue.  The (token, block) arrival counters of the epilogue sit behind the
-// column-block counters in the workspace header; batches whose counters do not fit take the four-launch form.
-// Measured on 128 experts, top-8, 2048 <-> 768, 3 bits, one token: 39.5 us against 39.1 us for the four launches with
-// dependent launch on (42.1 against 40.2 without): the launch gaps were already hidden, and every warp of the down
-// product now redoes the glue of its own input blocks.  Same bits either way; off unless the option asks for it.
+// The partition of a product whose plan with the glue behind it is `fused`, with the glue in launches of its own: the same one, and
+// so the same sums.  The expert-parallel block takes it too: a column block's sums do not depend on how many slots are local.
+static BlockPlan moe_plain_plan(const BlockPlan& fused, int in, int out, int k) {
+    return plan_block(in, out, k, 1, BlockUse::kMapped, fused.use ? fused.parts : 0);
+}
 
 int b200exl3_moe_forward(const b200exl3_moe* h, const void* d_x, int x_dtype, int64_t rows, const uint32_t* d_selected,
                          const void* d_scores, int score_dtype, void* d_y, void* ws, size_t ws_bytes, b200exl3_stream s) {
@@ -1390,8 +1389,7 @@ int b200exl3_moe_forward(const b200exl3_moe* h, const void* d_x, int x_dtype, in
             a.map_selected = sel; a.map_blocks = width / 128; a.map_proj = proj; a.map_stride_blocks = stride_blocks;
             a.map_experts = h->experts;
             const bool fused = fuse && block.use;
-            // the same partition, and so the same sums, with the glue in launches of its own
-            if (!fused) block = plan_block(in, out, h->k, 1, BlockUse::kMapped, block.use ? block.parts : 0);
+            if (!fused) block = moe_plain_plan(block, in, out, h->k);
             if (fused && proj == 1) {
                 a.epilogue = 3; a.svh = h->down_svh; a.yhat = nullptr;
                 a.epi_scores = static_cast<const char*>(d_scores) + static_cast<size_t>(r0) * h->top_k * score_size;
@@ -1686,7 +1684,9 @@ int b200exl3_moe_forward_ep(const b200exl3_moe* h, b200exl3_ep* ep, int first_ex
         const int64_t n = std::min(chunk, rows - r0), slots = n * h->top_k;
         const uint32_t* sel = d_selected + r0 * h->top_k;
         // one activation row per local slot against the columns of its (local) expert; slots past the count are skipped
-        auto mapped = [&](const uint32_t* wq, const __half* xhat, int in, int width, int proj, int stride_blocks, float* yhat) {
+        const BlockPlan gate_up = plan_block(h->in, static_cast<int>(slots * 2 * h->hidden), h->k, 1, BlockUse::kGateUp);
+        const BlockPlan down = plan_block(h->hidden, static_cast<int>(slots * h->in), h->k, 1, BlockUse::kDown, h->top_k);
+        auto mapped = [&](const uint32_t* wq, const __half* xhat, int in, int width, int proj, int stride_blocks, float* yhat, const BlockPlan& fused) {
             const int out = static_cast<int>(slots * proj * width);
             QmvArgs a{};
             a.wq = wq; a.xhat = xhat; a.xhat_group_stride = in;
@@ -1700,15 +1700,17 @@ int b200exl3_moe_forward_ep(const b200exl3_moe* h, b200exl3_ep* ep, int first_ex
             a.tiles_n = h->experts * proj * width / 16;
             a.map_selected = local_expert; a.map_count = local_count;
             a.map_blocks = width / 128; a.map_proj = proj; a.map_stride_blocks = stride_blocks; a.map_experts = h->experts;
+            const BlockPlan block = moe_plain_plan(fused, in, out, h->k);
+            if (block.use) return launch_block(a, h->k, h->cb, exact, block, stream);
             return launch_qmv(a, h->k, h->cb, exact, plan_qmv(in, out, h->k, 1, true), stream);
         };
         B200_TRY(launch_ep_plan(sel, slots, first_expert, h->experts, local_count, local_slot, local_expert, stream), "expert plan");
         B200_TRY(launch_ep_dispatch(static_cast<const char*>(d_x) + static_cast<size_t>(r0) * h->in * x_size, x_dtype, h->gu_suh, local_count,
                                     local_slot, local_expert, h->top_k, h->in, slots, xgu, stream), "expert dispatch");
-        B200_TRY(mapped(h->gu_wq, xgu, h->in, h->hidden, 2, h->experts * (h->hidden / 128), ygu), "expert gate/up kernel");
+        B200_TRY(mapped(h->gu_wq, xgu, h->in, h->hidden, 2, h->experts * (h->hidden / 128), ygu, gate_up), "expert gate/up kernel");
         B200_TRY(launch_glu_down_input(ygu, h->gu_svh, h->down_suh, local_expert, h->experts, slots, h->hidden, h->hidden, xdown, stream,
                                        local_count), "SwiGLU glue");
-        B200_TRY(mapped(h->down_wq, xdown, h->hidden, h->in, 1, 0, ydown), "expert down kernel");
+        B200_TRY(mapped(h->down_wq, xdown, h->hidden, h->in, 1, 0, ydown, down), "expert down kernel");
         B200_TRY(launch_ep_publish(ydown, h->down_svh, local_count, local_slot, local_expert, h->in, slots, peers, stream), "expert publish");
         B200_TRY(launch_ep_combine(static_cast<const char*>(d_scores) + static_cast<size_t>(r0) * h->top_k * score_size, score_dtype, n,
                                    h->top_k, h->in, static_cast<char*>(d_y) + static_cast<size_t>(r0) * h->in * score_size, peers, stream),

@@ -218,6 +218,10 @@ block_kernel(const __grid_constant__ QmvArgs p) {
         const int sp = cblock / p.map_blocks;
         slot = sp / p.map_proj;
         const int proj = sp - slot * p.map_proj;
+        if (kFused == 0 && p.map_count != nullptr && slot >= *p.map_count) {      // no such slot: the whole cluster is done
+            if (m > 1) cluster_wait();
+            return;
+        }
         expert = static_cast<int>(min(p.map_selected[slot], static_cast<uint32_t>(p.map_experts - 1)));   // unsigned: an id of 2^31 or more is clamped too
         wblock = proj * p.map_stride_blocks + expert * p.map_blocks + (cblock - sp * p.map_blocks);
         suh += (static_cast<int64_t>(expert) * p.map_proj + proj) * p.in;

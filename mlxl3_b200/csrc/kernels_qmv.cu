@@ -210,7 +210,7 @@ BlockPlan plan_block(int in, int out, int k, int64_t rows, BlockUse use, int top
 }
 
 cudaError_t launch_block(QmvArgs args, int k, int cb, bool exact, const BlockPlan& plan, cudaStream_t stream) {
-    if (!plan.use || args.rows <= 0 || args.rows > kBlockRows || args.map_count != nullptr) return cudaErrorInvalidValue;
+    if (!plan.use || args.rows <= 0 || args.rows > kBlockRows || (args.map_count != nullptr && args.map_early)) return cudaErrorInvalidValue;
     args.tiles_k = args.in / 16;
     args.trace = g_trace.load();
     args.cluster = plan.cluster;

@@ -49,6 +49,25 @@ def test_world_of_one_matches_the_block(gpu, rows, experts, top_k, k, cb):
     sharded.close(), whole.close(), ctx.close()
 
 
+@pytest.mark.parametrize("rows,experts,top_k,n_in,hidden,k", [(1, 16, 8, 2048, 768, 3), (2, 8, 2, 1024, 384, 4), (3, 6, 3, 512, 1152, 6),
+                                                              (1, 4, 1, 4096, 256, 2)])
+def test_few_slots_give_the_bytes_of_the_block(gpu, rows, experts, top_k, n_in, hidden, k):
+    """A batch small enough for clusters: the sums of a column block are cut as in the one-device block, wherever the slot lies
+    among the local ones, so a rank that owns all experts ends with the same bytes."""
+    from mlxl3_b200 import ep
+    rng = np.random.default_rng(rows + n_in)
+    bank = make_bank(rng, experts, n_in, hidden, k)
+    ctx = ep.EpContext(0, 1, 64, n_in, lambda raw: [raw])
+    sharded = ep.Exl3SwitchGluEp(*bank, top_k, k, 0, ctx)
+    whole = gpu.Exl3SwitchGlu(*bank, top_k, k, 0)
+    for call in range(3):
+        x = rng.standard_normal((rows, n_in)).astype(np.float16)
+        selected, scores = routes(rng, rows, experts, top_k)
+        assert np.array_equal(bits(sharded.forward(x, selected, scores)), bits(whole.forward(x, selected, scores)))
+    assert ctx.status() == 0 and gpu.workspace_status(sharded._workspace) == 0
+    sharded.close(), whole.close(), ctx.close()
+
+
 def _rank(rank, world, port, out):
     import torch.distributed as dist
     os.environ.update(MASTER_ADDR="127.0.0.1", MASTER_PORT=str(port))
