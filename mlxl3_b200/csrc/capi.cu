@@ -408,7 +408,8 @@ int b200exl3_unpack_states(const uint16_t* d_packed, int64_t tiles, int k, int c
     if (valid_format(k, cb)) return -1;
     if (tiles < 0) return fail("packed length is not a whole tile");
     if (tiles > 0 && (!d_packed || (!d_states && !d_values))) return fail("NULL buffer");
-    if (check_places({{d_packed, sizeof(uint16_t)}, {d_states, sizeof(uint16_t)}, {d_values, sizeof(uint16_t)}})) return -1;
+    // the kernel reads a tile's words 32 bits at a time
+    if (check_places({{d_packed, sizeof(uint16_t)}, {d_states, sizeof(uint16_t)}, {d_values, sizeof(uint16_t)}, {d_packed, sizeof(uint32_t)}})) return -1;
     return check(launch_unpack_states(d_packed, tiles, k, cb, d_states, reinterpret_cast<__half*>(d_values), as_stream(s)),
                  "unpack_states");
 }

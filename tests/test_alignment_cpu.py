@@ -43,6 +43,7 @@ def test_refused_before_a_launch(name, args):
     ("b200exl3_expert_mapped", (BASE, F16, BASE + 2, 8, BASE, BASE, BASE, 1, 128, 128, 1, 0, 4, 0, 0, 0, BASE, None), 4),
     ("b200exl3_expert_mapped", (BASE, F16, BASE, 8, None, None, BASE, 1, 128, 128, 1, 0, 4, 0, 1, 1, BASE + 8, None), 16),
     ("b200exl3_unpack_states", (BASE + 1, 1, 4, 0, BASE, None, None), 2),
+    ("b200exl3_unpack_states", (BASE + 2, 1, 4, 0, BASE, None, None), 4),
     ("b200exl3_codebook", (None, 8, 0, BASE + 1, None), 2),
 ])
 def test_what_a_kernel_reads_several_at_a_time_lies_on_that_many_bytes(name, args, bytes_):
