@@ -16,7 +16,11 @@
  * 16-byte aligned, with one exception: the rows x and y of the linear, group and rotation calls, the
  * rows x of the expert block and the scales and bias of the rotation calls may start at any element
  * of a larger buffer (input rows are then read element by element, and 9 or more output rows that do
- * not start on a multiple of four elements go through the few-row kernel).  Handles are immutable
+ * not start on a multiple of four elements go through the few-row kernel).  Outputs must not overlap
+ * what a call reads, except where a call says so and in one case: the outputs of a linear or group
+ * forward call, plain or with a SwiGLU prologue, may lie over its own rows x (the rows are then
+ * rotated by a launch of their own before anything is stored; more than 256 rows only with outputs of
+ * the inputs' size at the same address, because such a call may go in passes).  Handles are immutable
  * after creation, so one handle may be used from several threads and streams at once, each with its
  * own workspace; calls that share a workspace must be ordered on one stream.
  */

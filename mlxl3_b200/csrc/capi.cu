@@ -514,10 +514,7 @@ int b200exl3_linear_output_dims(const b200exl3_linear* h) { return h ? h->c.out 
 
 static size_t round256(size_t v) { return (v + 255) / 256 * 256; }
 
-// workspace = [counters + status | partial tiles | rotated activations (only when the kernel does not rotate)]
-static size_t xhat_bytes(const LayerCore& c, int64_t rows) {
-    return rows > kQmvFusedRows ? round256(static_cast<size_t>(c.groups) * rows * c.in * sizeof(__half)) : 0;
-}
+static size_t xhat_bytes(const LayerCore& c, int64_t rows) { return round256(static_cast<size_t>(c.groups) * rows * c.in * sizeof(__half)); }
 
 // From this many rows on, a plain layer's forward runs the tensor-core product (rotate all rows, tcgen05 product with the
 // output rotation in its epilogue) instead of the fused kernel, whose two-block form takes twice its one-block form's time.
@@ -544,16 +541,31 @@ static QmmLayout qmm_layout(const LayerCore& c, int64_t rows, bool whole_items =
     return l;
 }
 
-// few-row path: [counters | parts of shared column blocks | rotated rows, when the kernel does not rotate]
-static size_t qmv_workspace_bytes(const LayerCore& c, int64_t rows) {
+// few-row path: [counters | parts of shared column blocks | rotated rows, when a launch of its own rotates them: `rotate`, or more
+// rows than the kernel rotates itself]
+static size_t qmv_workspace_bytes(const LayerCore& c, int64_t rows, bool rotate = true) {
     const QmvPlan plan = plan_qmv(c.in, c.out, c.k, rows, true);             // the larger of the two grids
-    return kCounterBytes + qmv_partial_bytes(plan, c.out, rows) + xhat_bytes(c, rows);
+    return kCounterBytes + qmv_partial_bytes(plan, c.out, rows) + (rotate || rows > kQmvFusedRows ? xhat_bytes(c, rows) : 0);
 }
 
-static int core_workspace_bytes(const LayerCore& c, int64_t rows, size_t* out_bytes) {
+// Do the outputs lie over the rows the call reads?  The few-row kernels rotate their inputs themselves, each CTA when it comes to
+// run, while others already store outputs.
+static bool writes_over_input(const LayerCore& c, const void* d_x, int x_dtype, int64_t rows, void* const* ys, const float* d_yhat) {
+    const size_t size = dtype_size(x_dtype);
+    const char* x = static_cast<const char*>(d_x);
+    auto meets = [&](const void* p, size_t bytes) {
+        const char* at = static_cast<const char*>(p);
+        return at != nullptr && at < x + static_cast<size_t>(rows) * c.in * size && x < at + bytes;
+    };
+    bool over = d_yhat && meets(d_yhat, static_cast<size_t>(rows) * c.out * sizeof(float));
+    for (int g = 0; ys && g < c.groups; ++g) over = over || meets(ys[g], static_cast<size_t>(rows) * c.gout[g] * size);
+    return over;
+}
+
+static int core_workspace_bytes(const LayerCore& c, int64_t rows, bool rotate, size_t* out_bytes) {
     if (!out_bytes) return fail("NULL argument");
     if (rows <= 0) return fail("EXL3 linear input cannot be empty");
-    size_t bytes = qmv_workspace_bytes(c, rows);
+    size_t bytes = qmv_workspace_bytes(c, rows, rotate);
     if (rows >= kQmmMinRows) {
         bytes = std::max(bytes, qmm_layout(c, rows).total);
         if (c.groups == 1) bytes = std::max(bytes, qmm_layout(c, rows, false, true).total);      // the layer may be a row shard
@@ -564,17 +576,18 @@ static int core_workspace_bytes(const LayerCore& c, int64_t rows, size_t* out_by
 
 int b200exl3_linear_workspace_bytes(const b200exl3_linear* h, int64_t rows, size_t* out_bytes) {
     if (!h) return fail("NULL argument");
-    return core_workspace_bytes(h->c, rows, out_bytes);
+    return core_workspace_bytes(h->c, rows, true, out_bytes);
 }
 
 static TpPeers tp_peers(const b200exl3_tp* tp);
 
 // Exactly one of d_x / d_xhat is given; ys (one pointer per group) selects the rotated output, otherwise the summed fp32
 // product goes to d_yhat.  With a `layout` (rows that are to be rotated and stored rotated) the many-row product, without one
-// a fused launch per batch of up to kMaxBatchRows rows.  The caller has checked that `ws` holds what that path needs.
+// a fused launch per batch of up to kMaxBatchRows rows.  `rotate`: the input rotation is a launch of its own, whatever the rows.
+// The caller has checked that `ws` holds what that path needs.
 static int run_forward(const LayerCore& c, const void* d_x, int x_dtype, const uint16_t* d_xhat, int64_t rows, void* const* ys,
                        float* d_yhat, void* ws, cudaStream_t stream, const b200exl3_tp* tp, const b200exl3_prologue* pro,
-                       const QmmLayout* layout) {
+                       const QmmLayout* layout, bool rotate) {
     char* base = static_cast<char*>(ws);
     const bool exact = (c.flags & B200EXL3_EXACT_WEIGHTS) != 0;
     const size_t x_size = dtype_size(x_dtype);
@@ -584,8 +597,9 @@ static int run_forward(const LayerCore& c, const void* d_x, int x_dtype, const u
     // prologue (the only one taken with that many rows) is applied there
     // -- of a row shard too: a rank's sums are the same with the exchange inside the kernel and without one
     const BlockPlan block = plan_block(c.in, c.out, c.k, rows);
+    rotate = rotate || (rows > kQmvFusedRows && !block.use);
     const __half* glu_up = nullptr;
-    if (pro && pro->kind == 2 && rows > kQmvFusedRows && !block.use) {
+    if (pro && pro->kind == 2 && rotate) {
         glu_up = reinterpret_cast<const __half*>(pro->d_aux);
         pro = nullptr;
     }
@@ -622,8 +636,8 @@ static int run_forward(const LayerCore& c, const void* d_x, int x_dtype, const u
         }
         return 0;
     }
-    if (!xhat && rows > kQmvFusedRows && !block.use) {
-        // more than two rows: rotate all of them once per group, the product kernel reads the rotated rows
+    if (!xhat && rotate) {
+        // all rows rotated once per group, the product kernel reads the rotated rows
         const QmvPlan first = plan_qmv(c.in, c.out, c.k, rows);
         __half* buf = reinterpret_cast<__half*>(base + kCounterBytes + qmv_partial_bytes(first, c.out, rows));
         B200_TRY(launch_prepare(d_x, x_dtype, c.suh, 1, rows, c.in, buf, stream, glu_up, c.groups), "prepare");
@@ -693,7 +707,9 @@ static int forward_common(const LayerCore& c, const void* d_x, int x_dtype, cons
                           void* const* ys, float* d_yhat, void* ws, size_t ws_bytes, cudaStream_t stream,
                           const b200exl3_tp* tp = nullptr, const b200exl3_prologue* pro = nullptr) {
     size_t need = 0;
-    if (core_workspace_bytes(c, rows, &need)) return -1;
+    // outputs over the call's own rows: those are rotated by a launch of their own, which has read them before anything is stored
+    const bool rotate = rows > 0 && !d_xhat && (!pro || (pro->kind == 2 && pro->epilogue == 0)) && writes_over_input(c, d_x, x_dtype, rows, ys, d_yhat);
+    if (core_workspace_bytes(c, rows, rotate, &need)) return -1;
     QmmLayout layout{};                                       // planned once: what is checked is what runs
     const bool tensor_cores = rows >= kQmmMinRows && ys && !d_xhat && takes_tensor_cores(c, x_dtype, ys, tp);
     if (tensor_cores) {
@@ -702,7 +718,7 @@ static int forward_common(const LayerCore& c, const void* d_x, int x_dtype, cons
     }
     if (!ws || ws_bytes < need) return fail("workspace too small: %zu bytes given, %zu needed", ws_bytes, need);
     if (!aligned16(ws)) return fail("device pointers must be 16-byte aligned");
-    return run_forward(c, d_x, x_dtype, d_xhat, rows, ys, d_yhat, ws, stream, tp, pro, tensor_cores ? &layout : nullptr);
+    return run_forward(c, d_x, x_dtype, d_xhat, rows, ys, d_yhat, ws, stream, tp, pro, tensor_cores ? &layout : nullptr, rotate);
 }
 
 int b200exl3_workspace_status(const void* ws, int* out_status) {
@@ -847,7 +863,8 @@ int b200exl3_linear_forward_static(const b200exl3_linear* h, const void* d_x, in
         layout = qmm_layout(c, rows);
         if (layout.total > kStaticScratchBytes) layout = qmm_layout(c, rows, true);       // without parts the call needs less
     }
-    size_t need = tensor_cores ? layout.total : qmv_workspace_bytes(c, rows);
+    const bool rotate = writes_over_input(c, d_x, x_dtype, rows, ys, nullptr);
+    size_t need = tensor_cores ? layout.total : qmv_workspace_bytes(c, rows, rotate);
     if (rows >= kQmmMinRows) {
         // the limit as it is promised to callers, whatever the path keeps where: the rotated rows and one fp32 copy of the result
         need = std::max(need, qmm_layout(c, rows, true).total + static_cast<size_t>(rows) * c.out * sizeof(float));
@@ -862,7 +879,7 @@ int b200exl3_linear_forward_static(const b200exl3_linear* h, const void* d_x, in
     // last word of the header) is left alone, so a failure stays visible to b200exl3_static_status
     // until that call clears it, as it does in a caller's workspace.
     B200_TRY(cudaMemsetAsync(scratch, 0, kCounterBytes - sizeof(unsigned int), as_stream(s)), "clear static scratch");
-    return run_forward(c, d_x, x_dtype, nullptr, rows, ys, nullptr, scratch, as_stream(s), nullptr, nullptr, tensor_cores ? &layout : nullptr);
+    return run_forward(c, d_x, x_dtype, nullptr, rows, ys, nullptr, scratch, as_stream(s), nullptr, nullptr, tensor_cores ? &layout : nullptr, rotate);
 }
 
 int b200exl3_static_status(int* out_status, int clear) {
@@ -946,7 +963,7 @@ int b200exl3_group_count(const b200exl3_group* h) { return h ? h->c.groups : fai
 
 int b200exl3_group_workspace_bytes(const b200exl3_group* h, int64_t rows, size_t* out_bytes) {
     if (!h) return fail("NULL argument");
-    return core_workspace_bytes(h->c, rows, out_bytes);
+    return core_workspace_bytes(h->c, rows, true, out_bytes);
 }
 
 int b200exl3_group_forward(const b200exl3_group* h, const void* d_x, int x_dtype, int64_t rows, void* const* d_ys, void* ws,

@@ -187,3 +187,36 @@ def test_graph_replay_and_dependent_launch(gpu):
             assert gpu.workspace_status(ws) == 0
         finally:
             gpu.set_option("pdl", 0)
+
+
+@pytest.mark.parametrize("n_in,n_out,rows", [(256, 256, 1), (4096, 4096, 1), (4096, 4096, 2), (4096, 4096, 5), (2176, 2176, 8), (1024, 1024, 12),
+                                             (512, 4096, 1), (512, 4096, 7), (512, 28672, 2)])
+def test_outputs_over_the_rows(gpu, n_in, n_out, rows):
+    """Outputs stored where the inputs lie: read before anything is stored, so the bits of outputs elsewhere."""
+    from mlxl3_b200.runtime import DeviceBuffer, Stream
+    rng = np.random.default_rng(n_in + n_out + rows)
+    layer = gpu.Exl3Linear(*random_layer(rng, n_in, n_out, 4, signs=False), None, 4, 0)
+    stream = Stream()
+    x = rng.standard_normal((rows, n_in)).astype(np.float16)
+    d_x, d_y = DeviceBuffer(max(x.nbytes, rows * n_out * 2)), DeviceBuffer(rows * n_out * 2)
+    ws = gpu.new_workspace(layer.workspace_bytes(rows))
+    calls = {"forward": lambda d: layer.forward_device(d_x.ptr, gpu.F16, rows, d, ws, stream),
+             "static": lambda d: layer.forward_static_device(d_x.ptr, gpu.F16, rows, d, stream)}
+    for name, call in calls.items():
+        d_x.upload(x, stream)
+        call(d_y.ptr)
+        want = d_y.download((rows, n_out), np.float16, stream)
+        for _ in range(5):
+            d_x.upload(x, stream)
+            call(d_x.ptr)
+            assert np.array_equal(bits(d_x.download((rows, n_out), np.float16, stream)), bits(want)), name
+    # gate rows replaced by the block's outputs
+    up = DeviceBuffer.from_numpy(rng.standard_normal((rows, n_in)).astype(np.float16))
+    d_x.upload(x, stream)
+    layer.forward_fused_device(gpu.Prologue.swiglu(up.ptr), d_x.ptr, rows, d_y.ptr, ws, stream)
+    want = d_y.download((rows, n_out), np.float16, stream).astype(np.float32)
+    layer.forward_fused_device(gpu.Prologue.swiglu(up.ptr), d_x.ptr, rows, d_x.ptr, ws, stream)
+    got = d_x.download((rows, n_out), np.float16, stream).astype(np.float32)
+    assert (np.abs(got - want) <= 2e-3 * np.abs(want).max(axis=1, keepdims=True)).all()      # other order of the fp32 sums
+    assert gpu.workspace_status(ws) == 0 and gpu.static_status() == 0
+    layer.close()
