@@ -171,6 +171,7 @@ int b200exl3_linear_create(const uint16_t* d_trellis, const void* d_suh, const v
 void b200exl3_linear_free(b200exl3_linear* handle);
 int b200exl3_linear_input_dims(const b200exl3_linear* handle);    /* Exl3Linear::input_dims  */
 int b200exl3_linear_output_dims(const b200exl3_linear* handle);   /* Exl3Linear::output_dims */
+/* What a workspace has to hold for calls of up to `rows` rows (here and in the other *_workspace_bytes). */
 int b200exl3_linear_workspace_bytes(const b200exl3_linear* handle, int64_t rows, size_t* out_bytes);
 /* Waits for the device and reads the status word of a workspace: 0 = every kernel that used it ran to
  * completion, 1 = a bounded device-side wait gave up (the results of that call are invalid).  The

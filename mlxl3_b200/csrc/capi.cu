@@ -562,21 +562,39 @@ static bool writes_over_input(const LayerCore& c, const void* d_x, int x_dtype, 
     return over;
 }
 
-static int core_workspace_bytes(const LayerCore& c, int64_t rows, bool rotate, size_t* out_bytes) {
-    if (!out_bytes) return fail("NULL argument");
+// Bytes that a call of `rows` rows is checked for.
+static int core_workspace_need(const LayerCore& c, int64_t rows, bool rotate, size_t* need) {
     if (rows <= 0) return fail("EXL3 linear input cannot be empty");
-    size_t bytes = qmv_workspace_bytes(c, rows, rotate);
+    *need = qmv_workspace_bytes(c, rows, rotate);
     if (rows >= kQmmMinRows) {
-        bytes = std::max(bytes, qmm_layout(c, rows).total);
-        if (c.groups == 1) bytes = std::max(bytes, qmm_layout(c, rows, false, true).total);      // the layer may be a row shard
+        *need = std::max(*need, qmm_layout(c, rows).total);
+        if (c.groups == 1) *need = std::max(*need, qmm_layout(c, rows, false, true).total);      // the layer may be a row shard
     }
-    *out_bytes = bytes;
+    return 0;
+}
+
+// Bytes that every call of up to `rows` rows can do with: a smaller batch may leave more parts (768 rows 14336 -> 4096 need 54 MB,
+// 1024 rows 29).  The few-row path's need grows with the rows beyond those of one launch; the many-row plan is the same for all rows
+// with as many whole sixteens, of which the most rows need the most.  Going down from `rows`, what is left cannot need more once its
+// rotated rows, its sums and the most parts that a plan has stay below what was found.
+static int core_workspace_bytes(const LayerCore& c, int64_t rows, size_t* out_bytes) {
+    if (!out_bytes) return fail("NULL argument");
+    if (core_workspace_need(c, rows, true, out_bytes)) return -1;
+    for (int64_t r = std::min<int64_t>(rows, kQmvMaxRows); r >= 1; --r) *out_bytes = std::max(*out_bytes, qmv_workspace_bytes(c, r));
+    for (int64_t r = (rows - 1) / 16 * 16; r >= kQmmMinRows; r -= 16) {
+        const size_t most = kCounterBytes + xhat_bytes(c, r) + qmm_most_piece_bytes(r) +
+                            (c.groups == 1 ? round256(static_cast<size_t>(std::min(r, shard_pass_rows(c.out))) * c.out * sizeof(float)) : 0) + 256;
+        if (most <= *out_bytes) break;
+        size_t need = 0;
+        if (core_workspace_need(c, r, true, &need)) return -1;
+        *out_bytes = std::max(*out_bytes, need);
+    }
     return 0;
 }
 
 int b200exl3_linear_workspace_bytes(const b200exl3_linear* h, int64_t rows, size_t* out_bytes) {
     if (!h) return fail("NULL argument");
-    return core_workspace_bytes(h->c, rows, true, out_bytes);
+    return core_workspace_bytes(h->c, rows, out_bytes);
 }
 
 static TpPeers tp_peers(const b200exl3_tp* tp);
@@ -709,7 +727,7 @@ static int forward_common(const LayerCore& c, const void* d_x, int x_dtype, cons
     size_t need = 0;
     // outputs over the call's own rows: those are rotated by a launch of their own, which has read them before anything is stored
     const bool rotate = rows > 0 && !d_xhat && (!pro || (pro->kind == 2 && pro->epilogue == 0)) && writes_over_input(c, d_x, x_dtype, rows, ys, d_yhat);
-    if (core_workspace_bytes(c, rows, rotate, &need)) return -1;
+    if (core_workspace_need(c, rows, rotate, &need)) return -1;
     QmmLayout layout{};                                       // planned once: what is checked is what runs
     const bool tensor_cores = rows >= kQmmMinRows && ys && !d_xhat && takes_tensor_cores(c, x_dtype, ys, tp);
     if (tensor_cores) {
@@ -963,7 +981,7 @@ int b200exl3_group_count(const b200exl3_group* h) { return h ? h->c.groups : fai
 
 int b200exl3_group_workspace_bytes(const b200exl3_group* h, int64_t rows, size_t* out_bytes) {
     if (!h) return fail("NULL argument");
-    return core_workspace_bytes(h->c, rows, true, out_bytes);
+    return core_workspace_bytes(h->c, rows, out_bytes);
 }
 
 int b200exl3_group_forward(const b200exl3_group* h, const void* d_x, int x_dtype, int64_t rows, void* const* d_ys, void* ws,

@@ -373,6 +373,7 @@ struct QmmPlan {
 };
 // `out` counts all members of a group; `whole_items`: no item is shared, so no scratch for pieces
 QmmPlan plan_qmm(int in, int out, int64_t rows, bool whole_items = false);
+size_t qmm_most_piece_bytes(int64_t rows);     // no plan of a batch of up to `rows` rows has more for parts of shared items
 constexpr int kQmmStageIn = 128;     // inputs of a stage
 // CTAs of a launch over `items` items of `stages` stages
 int64_t qmm_grid(const QmmPlan& plan, int64_t items, int64_t stages);

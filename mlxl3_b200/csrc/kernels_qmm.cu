@@ -780,6 +780,12 @@ int64_t qmm_grid(const QmmPlan& plan, int64_t items, int64_t stages) {
 }
 static size_t qmm_piece_count(int64_t items, int64_t grid) { return static_cast<size_t>(items < grid ? grid + items : 2 * grid); }
 
+// at most one wave of CTAs shares items, so there are two parts per CTA or fewer, of at most 256 tokens (a forced split: any number)
+size_t qmm_most_piece_bytes(int64_t rows) {
+    if (g_qmm_splits.load() > 0) return size_t{1} << 60;
+    return static_cast<size_t>(sm_count()) * 2 * static_cast<size_t>(std::min<int64_t>(256, (rows + 15) / 16 * 16)) * 128 * sizeof(float);
+}
+
 // How a batch is cut up: tokens per item and CTAs per item (or one wave of equal runs).  The estimate below is fitted to 1160
 // measured launches (512 to 14336 inputs, 512 to 25600 outputs, 16 to 2000 rows, 3, 4 and 6 bits; its choice is 1.2 % above
 // the best measured one on average): a fixed part; a stage, mostly decode, with a share that grows with the tokens; the epilogue
