@@ -92,6 +92,10 @@ int b200exl3_set_option(const char* name, int64_t value);
  * partition arithmetic, layer accepted}. */
 int b200exl3_plan_query(const char* kind, int in, int out, int k, int64_t rows, int64_t* out_values, int capacity);
 
+/* The same for the expert block: {1 = slots sorted by expert, rows per pass, estimated nanoseconds of one row per slot, of the
+ * sorted form}. */
+int b200exl3_moe_plan_query(int experts, int in, int hidden, int top_k, int k, int64_t rows, int64_t* out_values, int capacity);
+
 /* Plain device-memory plumbing for hosts that have no CUDA binding of their own (replaces
  * mlxl3_array_from_bytes, mlxl3_array_copy_bytes, mlxl3_array_free and mlxl3_synchronize,
  * native/ffi/mlx_bridge.cpp:337, 610, 233, 192).  Streams are created non-blocking. */
@@ -257,10 +261,12 @@ int b200exl3_moe_workspace_bytes(const b200exl3_moe* handle, int64_t rows, size_
 /* x [rows, in] in x_dtype; selected [rows, top_k] expert ids (u32; ids past the bank are clamped to the last
  * expert instead of reading out of bounds); scores [rows, top_k] routing weights in score_dtype (fp16 = 9 or
  * fp32 = 10); y [rows, in] in score_dtype (the reference's result dtype: fp16 products promoted by the scores).
- * Small batches run one activation row per (token, choice) slot against the slot's expert's columns.  From 33
- * slots and two slots per expert on, the slots are grouped by expert on the device (the reference's route_plan, native/src/moe.rs:66-182) into
- * segments of up to 64 rows (tensor cores), so that an expert's columns are decoded once per segment; rows are
- * processed in passes of at most 16384 slots.  No host synchronisation either way.
+ * Small batches run one activation row per (token, choice) slot against the slot's expert's columns.  Where an
+ * estimate says that it is faster (b200exl3_moe_plan_query), the slots are grouped by expert on the device (the
+ * reference's route_plan, native/src/moe.rs:66-182) into segments of up to 64 rows (tensor cores), so that an
+ * expert's columns are decoded once per segment; rows are processed in passes of at most 16384 slots.  The sorted
+ * form multiplies the exact fp16 weight, the other one the weight that the flags of the handle ask for.  No host
+ * synchronisation either way.
  * The workspace follows the rules of the linear layer's workspace. */
 int b200exl3_moe_forward(const b200exl3_moe* handle, const void* d_x, int x_dtype, int64_t rows,
                          const uint32_t* d_selected, const void* d_scores, int score_dtype, void* d_y,

@@ -6,6 +6,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <initializer_list>
 #include <mutex>
@@ -1198,10 +1199,8 @@ static MoeLayout moe_layout(const b200exl3_moe* h, int64_t rows) {
     return l;
 }
 
-// Expert-sorted form, used from this many slots on: slots are grouped by expert into segments of kQmmSegRows rows,
-// so an expert's columns are decoded once per segment instead of once per slot.
-constexpr int64_t kMoeSortedMinSlots = 33;
-
+// Expert-sorted form: slots are grouped by expert into segments of kQmmSegRows rows, so an expert's columns are decoded once per
+// segment instead of once per slot.
 static int64_t moe_max_segments(const b200exl3_moe* h, int64_t slots) {
     return std::min<int64_t>(h->experts, slots) + slots / kQmmSegRows;   // one partly filled segment per expert at most
 }
@@ -1242,20 +1241,28 @@ static MoeSortedLayout moe_sorted_layout(const b200exl3_moe* h, int64_t rows) {
     return l;
 }
 
+// Estimated microseconds of a batch in either form.  One row per slot decodes an expert's columns for every slot; the sorted form
+// once per expert asked for (and per segment), at the price of two more launches and the tensor-core kernel's start, at a rate that
+// depends on the bits alone.  How many experts a batch asks for only the device knows: a little fewer than uniform routes would, as
+// routers favour some.  Fitted to the calls that moe_slots_us was fitted to; over 90 more, drawn, with 8 to 128 experts of 512 to 5120 <->
+// 256 to 14336, the form with the cheaper estimate is 0.14 % slower than the faster one on average, 4.4 % at most.
+// One row per slot / sorted in us: 128 experts, top 8, 2048 <-> 768, 3 bits, 24 slots 48 / 62, 80 112 / 107, 248 359 / 139; 64,
+// top 6, 2048 <-> 1408, 4 bits, 36 slots 89 / 91, 48 110 / 100; 32, 1024 <-> 256, 3 bits, 96 slots 39 / 40, 128 45 / 40; 8, top 1 and 2,
+// 4096 <-> 14336, 4 bits, 1 slot 90 / 68, 2 115 / 107, 16 730 / 320; 32, top 8, 7168 <-> 2048, 4 bits, 8 slots 98 / 112, 24 242 / 183.
+static void moe_estimates(const b200exl3_moe* h, int64_t rows, double* one_per_slot, double* sorted) {
+    const int64_t slots = rows * h->top_k, pass = std::min(rows, moe_chunk_rows(h));
+    *one_per_slot = moe_slots_us(h->in, h->hidden, h->top_k, h->k, pass * h->top_k) * static_cast<double>(rows) / static_cast<double>(pass);
+    const double per = h->k == 3 ? 1.13 : h->k == 4 ? 1.04 : h->k == 8 ? 1.16 : h->k >= 5 ? 1.29 : 1.10;
+    const double asked = 0.9 * h->experts * (1.0 - pow(1.0 - static_cast<double>(h->top_k) / h->experts, static_cast<double>(rows)));
+    *sorted = 31.0 + (asked + 0.9 * static_cast<double>(slots) / kQmmSegRows) * (0.12 + per * static_cast<double>(h->in) * h->hidden / (2048.0 * 768.0));
+}
+
 static bool moe_sorted(const b200exl3_moe* h, int64_t rows) {
     const int mode = g_moe_sorted.load();
-    const int64_t slots = rows * h->top_k;
     if (mode == 0 || !g_qmm_enabled) return false;
-    // One row per slot decodes an expert's columns for every slot, the sorted form once per expert asked for (at most min(slots,
-    // experts) of them), at the price of two more launches and the tensor-core kernel's start.  In units of the columns of a
-    // 2048 <-> 768 expert a slot costs 1.4 us and an expert of the sorted form 0.9; small experts cost a slot more than their columns.
-    // One row per slot / sorted in us: 128 experts, top 8, 2048 <-> 768, 3 bits, 40 slots 66 / 71, 64 94 / 84, 248 359 / 139; 64,
-    // top 6, 2048 <-> 1408, 4 bits, 24 slots 65 / 70, 36 87 / 80; 60, 1024 <-> 512, 2 bits, 48 slots 37 / 41, 100 53 / 44; 32,
-    // 1024 <-> 256, 3 bits, 64 slots 33 / 39, 96 39 / 40; 8, 512 <-> 256, 4 bits, 100 slots 29 / 32, 200 37 / 32.
-    const double expert = static_cast<double>(h->in) * h->hidden / (2048.0 * 768.0);
-    const double gain = expert * (1.4 * slots - 0.9 * std::min<int64_t>(slots, h->experts));
-    const bool worth = gain > (slots >= std::max<int64_t>(kMoeSortedMinSlots, 2 * static_cast<int64_t>(h->experts)) ? 17.0 : 24.0);
-    if (!worth && mode != 2) return false;
+    double one_per_slot = 0.0, sorted = 0.0;
+    moe_estimates(h, rows, &one_per_slot, &sorted);
+    if (sorted >= one_per_slot && mode != 2) return false;
     // the route plan keeps 2 * experts + 1 counters and one 16-bit expert id per slot of a pass in 48 KiB of shared
     // memory; shapes beyond that keep one row per slot
     const size_t plan_smem = (2 * static_cast<size_t>(h->experts) + 1) * sizeof(int) +
@@ -1320,6 +1327,22 @@ int b200exl3_moe_workspace_bytes(const b200exl3_moe* h, int64_t rows, size_t* ou
     if (!h || !out_bytes) return fail("NULL argument");
     if (rows <= 0) return fail("invalid SwitchGLU input/routes");
     *out_bytes = moe_sorted(h, rows) ? moe_sorted_layout(h, rows).total : moe_layout(h, rows).total;
+    return 0;
+}
+
+int b200exl3_moe_plan_query(int experts, int in, int hidden, int top_k, int k, int64_t rows, int64_t* out_values, int capacity) {
+    if (!out_values || capacity < 4) return fail("plan query needs room for 4 values");
+    if (experts <= 0 || top_k <= 0 || top_k > experts || in <= 0 || hidden <= 0 || in % 128 || hidden % 128 || k < 1 || k > 8 || k == 7 || rows <= 0 ||
+        top_k * moe_blocks_per_slot(in, hidden) > static_cast<int64_t>(kCounterBytes / sizeof(unsigned int)) - 2)
+        return fail("invalid plan query");
+    b200exl3_moe h{};
+    h.experts = experts; h.in = in; h.hidden = hidden; h.top_k = top_k; h.k = k;
+    double one_per_slot = 0.0, sorted = 0.0;
+    moe_estimates(&h, rows, &one_per_slot, &sorted);
+    out_values[0] = moe_sorted(&h, rows) ? 1 : 0;
+    out_values[1] = out_values[0] ? moe_sorted_chunk_rows(&h, rows) : std::min(rows, moe_chunk_rows(&h));
+    out_values[2] = static_cast<int64_t>(one_per_slot * 1000.0);
+    out_values[3] = static_cast<int64_t>(sorted * 1000.0);
     return 0;
 }
 

@@ -183,6 +183,8 @@ struct BlockPlan {
 enum class BlockUse { kLayer, kMapped, kGateUp, kDown };
 // `top_k`: of kMapped the parts that a column block's inputs are cut into (0: one, if a wave holds all blocks).
 BlockPlan plan_block(int in, int out, int k, int64_t rows, BlockUse use = BlockUse::kLayer, int top_k = 0);
+// Estimated microseconds of the expert block with one row per slot (at least one).
+double moe_slots_us(int in, int hidden, int top_k, int k, int64_t slots);
 cudaError_t launch_block(QmvArgs args, int k, int cb, bool exact, const BlockPlan& plan, cudaStream_t stream);
 void block_set_tuning(int cluster);  // 0 automatic, -1 never, else the CTAs of a cluster
 

@@ -146,6 +146,46 @@ cudaError_t block_dispatch_k8(const QmvArgs&, int, bool, const BlockPlan&, cudaS
 static std::atomic<int> g_block_cluster{0};
 void block_set_tuning(int cluster) { g_block_cluster = cluster < -1 ? 0 : std::min(cluster, kBlockCluster); }
 
+// Clusters of 1..8 CTAs that a B200 holds at one CTA per SM (a cluster lies inside one processing cluster of SMs); a constant, so
+// that a layer's sums are added in the same order on every GPU.
+static constexpr int kResident[kBlockCluster] = {148, 74, 45, 33, 26, 22, 15, 15};
+
+// Microseconds fitted to sweeps of 1..8 CTAs over 22 shapes (512..14336 inputs, 128..28672 outputs, 2, 3, 4 and 6 bits, one
+// row; the choice is 1 % above the best measured on average): `rb` rows of 16 inputs over `parts` CTAs, a row of 16 inputs per
+// warp, the sum over a cluster, a second wave of single CTAs.
+static double block_us(int64_t rb, int parts, int cluster, int64_t waves, int k) {
+    const bool even = k == 4 || k == 8;                      // the cheapest widths to decode
+    const double warp_rows = 0.5 * (static_cast<double>(((rb + parts - 1) / parts + kBlockWarps - 1) / kBlockWarps) + static_cast<double>(rb) / (parts * kBlockWarps));
+    return 0.7 + waves * (2.7 + (even ? 0.89 : 1.04) * warp_rows) + (cluster > 1 ? 1.0 + 0.04 * cluster : 0.0);
+}
+
+// Fitted to 159 measured calls (8 to 128 experts of 512 <-> 256 to 4096 <-> 14336, top 1 to 8, 1 to 300 slots, 1 to 8 bits; 2 %
+// off on average): products that a wave of clusters holds, products that are dealt out over the grid by rows of 16 inputs per warp
+// (a warp holds one column block's rows at most, so many slots of a large expert take more than a wave of CTAs), glue launches.
+// Independent of the options that change how a product is cut, as the form decides what a workspace holds.
+double moe_slots_us(int in, int hidden, int top_k, int k, int64_t slots) {
+    const double row = k == 3 ? 1.12 : k == 5 || k == 6 ? 1.23 : k == 8 ? 1.07 : 1.01;
+    const int64_t sms = sm_count();
+    auto dealt = [&](int64_t rb, int64_t blocks) {
+        const int64_t rt = rb * blocks, warps = (rt + rb - 2) / (rb - 1) + 1;
+        const int64_t grid = std::max(std::max<int64_t>(1, std::min(2 * sms, rt / kQmvWarps)), (warps + kQmvWarps - 1) / kQmvWarps);
+        const int64_t waves = (grid + 2 * sms - 1) / (2 * sms), rows = (rt + grid * kQmvWarps - 1) / (grid * kQmvWarps);
+        return 6.9 + row * static_cast<double>(waves * rows) * (grid > sms ? 1.0 : 0.7);
+    };
+    const int64_t gu_rows = in / 16, gu_blocks = slots * 2 * hidden / 128, down_rows = hidden / 16, down_blocks = slots * in / 128;
+    double us = 0.0, fused = 0.0;
+    for (int n = 1; 2 * n <= kBlockCluster; ++n)
+        if (gu_blocks / 2 <= kResident[2 * n - 1]) {
+            const double t = block_us(gu_rows, n, 2 * n, 1, k);
+            if (fused == 0.0 || t < fused) fused = t;
+        }
+    if (fused > 0.0) us += 1.06 * fused;
+    else us += 3.3 + (gu_blocks <= kResident[0] ? 1.06 * block_us(gu_rows, 1, 1, 1, k) : dealt(gu_rows, gu_blocks));
+    us += down_blocks <= kResident[0] ? 1.06 * block_us(down_rows, 1, 1, 1, k) : dealt(down_rows, down_blocks);
+    if (top_k > kBlockCluster || down_blocks / top_k > kResident[top_k - 1]) us += 3.3;
+    return us;
+}
+
 BlockPlan plan_block(int in, int out, int k, int64_t rows, BlockUse use, int top_k) {
     BlockPlan plan{};
     const int forced = g_block_cluster.load();
@@ -168,9 +208,6 @@ BlockPlan plan_block(int in, int out, int k, int64_t rows, BlockUse use, int top
         plan.smem_bytes = std::max(plan.smem_bytes, kQmvSharedSmemBytes + 4096);
         return plan.smem_bytes <= static_cast<size_t>(kQmvMaxSmemBytes);
     };
-    // Clusters of 1..8 CTAs that a B200 holds at one CTA per SM (a cluster lies inside one processing cluster of SMs); a constant, so
-    // that a layer's sums are added in the same order on every GPU.
-    constexpr int kResident[kBlockCluster] = {148, 74, 45, 33, 26, 22, 15, 15};
     int cluster = 1, parts = 1;
     int64_t clusters = blocks;
     if (use == BlockUse::kMapped) {
@@ -182,9 +219,7 @@ BlockPlan plan_block(int in, int out, int k, int64_t rows, BlockUse use, int top
         clusters = blocks / top_k;
         plan.use = lay_out(cluster, 1, rows) && clusters <= kResident[top_k - 1];
     } else {
-        // Microseconds fitted to sweeps of 1..8 CTAs over 22 shapes (512..14336 inputs, 128..28672 outputs, 2, 3, 4 and 6 bits, one
-        // row; the choice is 1 % above the best measured on average): a row of 16 inputs per warp, the sum over a cluster, a second
-        // wave of single CTAs; against the other kernel's launch, its decode over all SMs and the parts of its blocks.  The row
+        // The cluster's cost against the other kernel's launch, its decode over all SMs and the parts of its blocks.  The row
         // count is left out, so that a row's sums are added in the same order in every batch of up to 8 (with 8 rows the other
         // kernel is further behind where the inputs are few, because its input rotation is a launch of its own).
         const int projections = use == BlockUse::kGateUp ? 2 : 1;
@@ -195,8 +230,7 @@ BlockPlan plan_block(int in, int out, int k, int64_t rows, BlockUse use, int top
             const int64_t waves = m == 1 && blocks > kResident[0] ? 2 : 1;
             if (forced > 0 && projections == 1 ? m != forced : blocks / projections > waves * kResident[m - 1]) continue;
             if (!lay_out(m, n, projections > 1 ? 1 : kBlockRows)) continue;
-            const double warp_rows = 0.5 * (static_cast<double>(((rb + n - 1) / n + kBlockWarps - 1) / kBlockWarps) + static_cast<double>(rb) / (n * kBlockWarps));
-            const double t = 0.7 + waves * (2.7 + (even ? 0.89 : 1.04) * warp_rows) + (m > 1 ? 1.0 + 0.04 * m : 0.0);
+            const double t = block_us(rb, n, m, waves, k);
             if (t < best) { best = t; cluster = m; parts = n; plan.use = true; }
         }
         clusters = blocks / projections;
