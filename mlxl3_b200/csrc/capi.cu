@@ -1199,6 +1199,16 @@ static MoeLayout moe_layout(const b200exl3_moe* h, int64_t rows) {
     return l;
 }
 
+// Parts of shared column blocks that the products of up to `slots` slots can leave: CTAs + blocks of a launch number them, and each
+// block's last place may stay empty.
+static size_t moe_most_partials(const b200exl3_moe* h, int64_t slots) {
+    auto most = [&](int in, int64_t out) {
+        const QmvPlan plan = plan_qmv(in, static_cast<int>(out), h->k, 1, true);
+        return round256((static_cast<size_t>(plan.grid) + 2 * plan.col_blocks) * 128 * sizeof(float));
+    };
+    return std::max(most(h->in, slots * 2 * h->hidden), most(h->hidden, slots * h->in));
+}
+
 // Expert-sorted form: slots are grouped by expert into segments of kQmmSegRows rows, so an expert's columns are decoded once per
 // segment instead of once per slot.
 static int64_t moe_max_segments(const b200exl3_moe* h, int64_t slots) {
@@ -1257,17 +1267,20 @@ static void moe_estimates(const b200exl3_moe* h, int64_t rows, double* one_per_s
     *sorted = 31.0 + (asked + 0.9 * static_cast<double>(slots) / kQmmSegRows) * (0.12 + per * static_cast<double>(h->in) * h->hidden / (2048.0 * 768.0));
 }
 
+// The route plan keeps 2 * experts + 1 counters and one 16-bit expert id per slot of a pass in 48 KiB of shared memory: rows of a pass
+// that fit, 0 or less for none.  Shapes beyond that keep one row per slot.
+static int64_t moe_plan_rows(const b200exl3_moe* h) {
+    const int64_t left = 48 * 1024 - (2 * static_cast<int64_t>(h->experts) + 1) * static_cast<int64_t>(sizeof(int));
+    return left <= 0 ? 0 : left / static_cast<int64_t>(sizeof(unsigned short)) / h->top_k;
+}
+
 static bool moe_sorted(const b200exl3_moe* h, int64_t rows) {
     const int mode = g_moe_sorted.load();
     if (mode == 0 || !g_qmm_enabled) return false;
     double one_per_slot = 0.0, sorted = 0.0;
     moe_estimates(h, rows, &one_per_slot, &sorted);
     if (sorted >= one_per_slot && mode != 2) return false;
-    // the route plan keeps 2 * experts + 1 counters and one 16-bit expert id per slot of a pass in 48 KiB of shared
-    // memory; shapes beyond that keep one row per slot
-    const size_t plan_smem = (2 * static_cast<size_t>(h->experts) + 1) * sizeof(int) +
-                             static_cast<size_t>(moe_sorted_chunk_rows(h, rows)) * h->top_k * sizeof(unsigned short);
-    return plan_smem <= 48 * 1024 && h->experts <= 65535;
+    return moe_sorted_chunk_rows(h, rows) <= moe_plan_rows(h) && h->experts <= 65535;
 }
 
 int b200exl3_moe_create(const uint16_t* d_gu_trellis, const void* d_gu_suh, const void* d_gu_svh,
@@ -1326,7 +1339,20 @@ void b200exl3_moe_free(b200exl3_moe* h) {
 int b200exl3_moe_workspace_bytes(const b200exl3_moe* h, int64_t rows, size_t* out_bytes) {
     if (!h || !out_bytes) return fail("NULL argument");
     if (rows <= 0) return fail("invalid SwitchGLU input/routes");
-    *out_bytes = moe_sorted(h, rows) ? moe_sorted_layout(h, rows).total : moe_layout(h, rows).total;
+    // Every call of up to `rows` rows can do with it: of the form with one row per slot, and of the sorted form with the most rows that
+    // take it (its need grows with the rows of a pass; few rows take it only where the two estimates lie close).
+    const int64_t few = std::min(rows, moe_chunk_rows(h));
+    *out_bytes = moe_layout(h, few).partials + moe_most_partials(h, few * h->top_k);
+    if (moe_sorted(h, rows)) *out_bytes = std::max(*out_bytes, moe_sorted_layout(h, rows).total);
+    for (int64_t r = std::min({rows, std::max<int64_t>(1, kMoeSortedPassSlots / h->top_k), moe_plan_rows(h)}); r >= 1; --r) {
+        if (moe_sorted(h, r)) {
+            *out_bytes = std::max(*out_bytes, moe_sorted_layout(h, r).total);
+            break;
+        }
+        double one_per_slot = 0.0, sorted = 0.0;
+        moe_estimates(h, r, &one_per_slot, &sorted);
+        if (one_per_slot < 0.8 * sorted) break;
+    }
     return 0;
 }
 
@@ -1702,7 +1728,8 @@ static MoeEpLayout moe_ep_layout(const b200exl3_moe* h, int64_t slots) {
 int b200exl3_moe_ep_workspace_bytes(const b200exl3_moe* h, int64_t rows, size_t* out_bytes) {
     if (!h || !out_bytes) return fail("NULL argument");
     if (rows <= 0) return fail("invalid SwitchGLU input/routes");
-    *out_bytes = moe_ep_layout(h, std::min(rows, moe_chunk_rows(h)) * h->top_k).total;
+    const int64_t slots = std::min(rows, moe_chunk_rows(h)) * h->top_k;
+    *out_bytes = moe_ep_layout(h, slots).partials + moe_most_partials(h, slots);      // every call of up to `rows` rows can do with it
     return 0;
 }
 

@@ -82,3 +82,34 @@ def test_sorted_form_with_few_slots(gpu, experts, top_k, rows):
     check(got, oracle.switch_glu_forward(*bank, top_k, k, 0, x, selected, scores), rms=3e-3)
     assert gpu.workspace_status(moe._workspace) == 0
     moe.close()
+
+
+@pytest.mark.parametrize("experts,top_k,n_in,hidden", [(128, 8, 512, 256), (8, 2, 256, 640), (300, 1, 128, 128)])
+def test_a_workspace_covers_smaller_batches(gpu, experts, top_k, n_in, hidden):
+    """Made for the largest batch, used for any: below the sizes where the forms change, and where a pass ends."""
+    from mlxl3_b200 import ep
+    from mlxl3_b200.runtime import DeviceBuffer, Stream
+    rng = np.random.default_rng(experts)
+    bank = make_bank(rng, experts, n_in, hidden, 2)
+    moe = gpu.Exl3SwitchGlu(*bank, top_k, 2, 0)
+    sizes = [moe.workspace_bytes(r) for r in range(1, 700)]
+    assert all(a <= b for a, b in zip(sizes, sizes[1:]))
+    most = 400
+    selected, scores = routes(rng, most, experts, top_k)
+    stream, ws = Stream(), gpu.new_workspace(moe.workspace_bytes(most))
+    d_x, d_y = DeviceBuffer.from_numpy(rng.standard_normal((most, n_in)).astype(np.float16)), DeviceBuffer(most * n_in * 2)
+    d_sel, d_scores = DeviceBuffer.from_numpy(selected), DeviceBuffer.from_numpy(scores)
+    for rows in (400, 257, 256, 255, 128, 65, 37, 33, 32, 31, 16, 9, 4, 3, 2, 1):
+        moe.forward_device(d_x.ptr, gpu.F16, rows, d_sel.ptr, d_scores.ptr, gpu.F16, d_y.ptr, ws, stream)
+    stream.sync()
+    assert gpu.workspace_status(ws) == 0
+    ctx = ep.EpContext(0, 1, 256, n_in, lambda raw: [raw])
+    sharded = ep.Exl3SwitchGluEp(*bank, top_k, 2, 0, ctx)
+    sizes = [sharded.workspace_bytes(r) for r in range(1, 300)]
+    assert all(a <= b for a, b in zip(sizes, sizes[1:]))
+    ws = gpu.new_workspace(sharded.workspace_bytes(256))
+    for rows in (256, 200, 31, 30, 7, 1):
+        sharded.forward_device(d_x.ptr, gpu.F16, rows, d_sel.ptr, d_scores.ptr, gpu.F16, d_y.ptr, ws, stream)
+    stream.sync()
+    assert ctx.status() == 0 and gpu.workspace_status(ws) == 0
+    sharded.close(), ctx.close(), moe.close()
