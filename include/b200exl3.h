@@ -89,7 +89,9 @@ int b200exl3_set_option(const char* name, int64_t value);
  * of a launch, items of a launch (tile x 128 columns), 128-input stages of an item, tokens per tile, CTAs per item
  * (0 = one wave of CTAs with equal runs of stages), rows per launch, bytes for parts of shared items}; "stack":
  * {CTAs, bound on CTAs per block, column blocks, warps per CTA, shared memory, warps that share the layer, 32-bit
- * partition arithmetic, layer accepted}. */
+ * partition arithmetic, layer accepted}; "block" (up to 8 rows): {1 = a cluster of CTAs per column block, CTAs of a cluster, CTAs,
+ * warps per CTA, shared memory per CTA, of it a warp's, halves between rotated rows, where the cluster's sums lie}; "clusters" (asks
+ * the current device): clusters of 1..8 such CTAs that it holds at once. */
 int b200exl3_plan_query(const char* kind, int in, int out, int k, int64_t rows, int64_t* out_values, int capacity);
 
 /* The same for the expert block: {1 = slots sorted by expert, rows per pass, estimated nanoseconds of one row per slot, of the

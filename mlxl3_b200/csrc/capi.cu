@@ -239,6 +239,14 @@ int b200exl3_plan_query(const char* kind, int in, int out, int k, int64_t rows, 
         out_values[7] = ok ? 1 : 0;
         return 0;
     }
+    if (!strcmp(kind, "clusters")) {
+        for (int n = 1; n <= kBlockCluster; ++n) {
+            int clusters = 0;
+            B200_TRY(block_resident_clusters(n, &clusters), "cudaOccupancyMaxActiveClusters");
+            out_values[n - 1] = clusters;
+        }
+        return 0;
+    }
     return fail("unknown plan kind %s", kind);
 }
 

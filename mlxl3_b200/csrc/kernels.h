@@ -186,6 +186,7 @@ BlockPlan plan_block(int in, int out, int k, int64_t rows, BlockUse use = BlockU
 // Estimated microseconds of the expert block with one row per slot (at least one).
 double moe_slots_us(int in, int hidden, int top_k, int k, int64_t slots);
 cudaError_t launch_block(QmvArgs args, int k, int cb, bool exact, const BlockPlan& plan, cudaStream_t stream);
+cudaError_t block_resident_clusters(int cluster, int* clusters);     // clusters of that many CTAs that the current device holds at once
 void block_set_tuning(int cluster);  // 0 automatic, -1 never, else the CTAs of a cluster
 
 // ---- a whole decode step in one persistent launch (kernels_stack*.cu) ------------------------------------------

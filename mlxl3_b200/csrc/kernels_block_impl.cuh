@@ -488,6 +488,25 @@ cudaError_t block_launch_one(const QmvArgs& p, const BlockPlan& plan, cudaStream
     return cudaLaunchKernelEx(&cfg, kernel, p);
 }
 
+// Clusters of `cluster` CTAs that the current device holds at once, with as much shared memory as one CTA per SM may take.
+template <int K, int CB, int MODE, int FUSED>
+cudaError_t block_resident(int cluster, int* clusters) {
+    auto kernel = block_kernel<K, CB, MODE, FUSED>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kQmvMaxSmemBytes);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(static_cast<unsigned>(cluster));
+    cfg.blockDim = dim3(kBlockWarps * 32);
+    cfg.dynamicSmemBytes = kQmvMaxSmemBytes;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = static_cast<unsigned>(cluster);
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaOccupancyMaxActiveClusters(clusters, kernel, &cfg);
+}
+
 template <int K, int CB, int MODE>
 cudaError_t block_launch_fused(const QmvArgs& p, const BlockPlan& plan, cudaStream_t stream) {
     if (p.epilogue == 4) return block_launch_one<K, CB, MODE, 2>(p, plan, stream);

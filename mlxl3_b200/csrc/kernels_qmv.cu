@@ -147,7 +147,8 @@ static std::atomic<int> g_block_cluster{0};
 void block_set_tuning(int cluster) { g_block_cluster = cluster < -1 ? 0 : std::min(cluster, kBlockCluster); }
 
 // Clusters of 1..8 CTAs that a B200 holds at one CTA per SM (a cluster lies inside one processing cluster of SMs); a constant, so
-// that a layer's sums are added in the same order on every GPU.
+// that a layer's sums are added in the same order on every GPU.  A board whose SMs lie otherwise may hold fewer, and a layer then runs in
+// two waves; a GPU test compares (b200exl3_plan_query, "clusters").
 static constexpr int kResident[kBlockCluster] = {148, 74, 45, 33, 26, 22, 15, 15};
 
 // Microseconds fitted to sweeps of 1..8 CTAs over 22 shapes (512..14336 inputs, 128..28672 outputs, 2, 3, 4 and 6 bits, one

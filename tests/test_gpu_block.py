@@ -77,3 +77,12 @@ def test_expert_block_with_and_without_its_glue(gpu, experts, top_k, n_in, hidde
     check(got, oracle.switch_glu_forward(*bank, top_k, 4, 0, x, selected, scores), rms=4e-3)
     assert gpu.workspace_status(moe._workspace) == 0
     moe.close()
+
+
+def test_the_device_holds_the_clusters_that_plans_count_on(gpu):
+    """A wave of clusters is a constant of the plans, so that sums have one order on every GPU; a board that holds fewer would run
+    full layers in two waves."""
+    from tests.test_block_plan import RESIDENT
+    from tests.test_plan_invariants import query
+    held = query("clusters", 128, 128, 4, 1)
+    assert len(held) == len(RESIDENT) and all(h >= r for h, r in zip(held, RESIDENT)), held
