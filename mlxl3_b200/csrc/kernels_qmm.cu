@@ -16,7 +16,8 @@
 //  * B operand: rotated activations, two TMA tensor copies of [tile tokens, 64 in] fp16 per stage, 128-byte swizzle;
 //  * packed words: one bulk copy per stage (8 tile rows x 8 tiles are contiguous in the quad layout);
 //  * one thread issues the stage's eight products and one commit, which frees the A stage and the activation slot.
-//  * tiles of up to 64 tokens: two accumulators, so that four more warps finish an item while the next one is multiplied.
+//  * tiles of up to 64 tokens, several of them on a CTA: two accumulators, so that four more warps finish an item while the next one
+//    is multiplied.
 //
 // What bounds it: up to 64 rows the decode, and of it the issue slots: the decode loop alone (words resident in shared memory,
 // tensor-memory stores and nothing else) executes 43 warp instructions per 16x16 tile at 4 bits and 48 at 3, in 47 to 49 and 51 to 53
@@ -49,17 +50,20 @@ constexpr int kMmaWarp = 0, kWeightWarp = 1, kActWarp = 2, kFirstDecoder = 4;
 constexpr int kStageCols = 64;                         // tensor-memory columns of an A stage: two fp16 inputs each
 constexpr int kChunk = 16;                             // tokens four warps finish at a time
 
-template <int K, int NT>
+template <int K, int NT, bool FIN>
 struct QmmShape {
     static constexpr int kGroups = 2;                  // groups of eight decoder warps that take alternate stages
     static constexpr int kDecoders = 8 * kGroups;
-    // Small tiles: two accumulators, and four warps that finish an item while the next one is decoded and multiplied; the decoders
-    // finish only the CTA's last item.  Before, the pipeline drained at every item (5000 cycles, 2000 of them waiting for the last
-    // products): 16 rows 5120->2x25600, 3 bits, 84.8 -> 80.1 us; expert block 37 / 256 tokens 176 -> 165 / 250 -> 230.  Large tiles
-    // leave no tensor memory for a second accumulator: their decoders finish every item.
+    // Small tiles: two accumulators, and with FIN four warps that finish an item while the next one is decoded and multiplied; the
+    // decoders finish only the CTA's last item.  Before, the pipeline drained at every item (5000 cycles, 2000 of them waiting for the last
+    // products): 16 rows 5120->2x25600, 3 bits, 84.8 -> 80.1 us; expert block 37 / 256 tokens 176 -> 165 / 250 -> 230.  Without FIN a
+    // CTA has one item: the warps would have nothing to do but to start with the CTA and to leave the decoders 80 registers.  Us with /
+    // without them, 4 bits: 24 rows 2048->2048 9.3 / 9.05, 4096->4096 12.4 / 11.9, 64 rows 14336->4096 25.8 / 25.4, 4096->14336 21.7 / 21.55.
+    // (The loop over several items that large tiles take instead spills here: 24 rows 4096->14336 22.7.)
+    // Large tiles leave no tensor memory for a second accumulator: their decoders finish every item.
     static constexpr uint32_t kAccums = NT == 64 ? 2 : 1;
     static constexpr int kFinishers = NT == 64 ? 4 : kDecoders;
-    static constexpr int kThreads = 32 * (kFirstDecoder + kDecoders + (NT == 64 ? kFinishers : 0));
+    static constexpr int kThreads = 32 * (kFirstDecoder + kDecoders + (FIN ? kFinishers : 0));
     static constexpr int kSlots = NT == 64 ? 6 : 4;    // A stages in tensor memory beside the accumulators
     // Packed stages (2048 * K bytes) in flight.  A multiple of the decoder groups, so that a slot always belongs to one group:
     // parity alone does not tell a phase from the one after the next, and a group that met a slot only every other time could
@@ -70,12 +74,12 @@ struct QmmShape {
     static constexpr int kBSlots = NT == 64 ? kSlots : 2;   // activation stages in shared memory; divides kSlots
     static constexpr uint32_t kBHalfBytes = NT * 128;  // NT tokens x 64 fp16
     static constexpr uint32_t kBSlotBytes = 2 * kBHalfBytes;
-    static constexpr uint32_t kEpilogueBytes = (kDecoders / 4 + (NT == 64 ? 1 : 0)) * 2 * kChunk * 128 * sizeof(__half);
+    static constexpr uint32_t kEpilogueBytes = (kDecoders / 4 + (NT == 64 && FIN ? 1 : 0)) * 2 * kChunk * 128 * sizeof(__half);
     static_assert(kAccums * NT + kSlots * kStageCols <= 512 && kSlots % kGroups == 0 && kSlots % kBSlots == 0, "tensor memory");
 };
-template <int K, int NT>
+template <int K, int NT, bool FIN>
 constexpr size_t qmm_smem_bytes() {
-    using S = QmmShape<K, NT>;
+    using S = QmmShape<K, NT, FIN>;
     return 1024 + S::kBSlots * S::kBSlotBytes + static_cast<size_t>(S::kRaw) * 2048 * K + S::kEpilogueBytes;
 }
 
@@ -268,10 +272,10 @@ __device__ __forceinline__ void qmm_finish4(__half* rows, const QmmArgs& p, cons
     __syncwarp();
 }
 
-template <int K, int CB, int NT>
-__global__ void __launch_bounds__(QmmShape<K, NT>::kThreads, 1)
+template <int K, int CB, int NT, bool FIN>
+__global__ void __launch_bounds__(QmmShape<K, NT, FIN>::kThreads, 1)
 qmm_kernel(const __grid_constant__ CUtensorMap xmap, const QmmArgs p) {
-    using S = QmmShape<K, NT>;
+    using S = QmmShape<K, NT, FIN>;
     // Dependent launch: this kernel may be scheduled under the tail of the kernel before it (the input rotation, the
     // glue of the expert block).  The packed weights are nobody's output, so the barriers, the tensor memory and the
     // first weight copies do not wait; what that kernel wrote -- the rotated rows, the segment table -- is read only
@@ -457,7 +461,7 @@ qmm_kernel(const __grid_constant__ CUtensorMap xmap, const QmmArgs p) {
         }
     };
 
-    if (warp >= kFirstDecoder + S::kDecoders) {
+    if (FIN && warp >= kFirstDecoder + S::kDecoders) {
         // ================= finishing warps: every item of the CTA but its last, while the next one is decoded =================
         pdl_wait();
         const int w = warp - kFirstDecoder - S::kDecoders;
@@ -734,36 +738,46 @@ bool encode_rows(CUtensorMap* map, const __half* xhat, int in, int64_t rows, int
                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int K, int CB, int NT>
+template <int K, int CB, int NT, bool FIN>
 cudaError_t qmm_launch_shape(const CUtensorMap& map, const QmmArgs& p, int grid, cudaStream_t stream) {
-    constexpr size_t smem = qmm_smem_bytes<K, NT>();
-    auto kernel = qmm_kernel<K, CB, NT>;
+    constexpr size_t smem = qmm_smem_bytes<K, NT, FIN>();
+    auto kernel = qmm_kernel<K, CB, NT, FIN>;
     static PerDeviceOnce attribute;                         // once per kernel and device
     if (attribute.needed()) {
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
         if (e != cudaSuccess) return e;
         attribute.mark();
     }
-    return launch_dependent(kernel, dim3(static_cast<unsigned>(grid)), dim3(QmmShape<K, NT>::kThreads), smem, stream, map, p);
+    return launch_dependent(kernel, dim3(static_cast<unsigned>(grid)), dim3(QmmShape<K, NT, FIN>::kThreads), smem, stream, map, p);
+}
+
+// What a CTA is built for: tiles of up to 64 tokens, where every item has CTAs of its own or where a CTA holds several; large tiles.
+enum class QmmForm { kSmall, kSmallItems, kLarge };
+
+template <int K, int CB>
+cudaError_t qmm_launch_form(const CUtensorMap& map, const QmmArgs& p, int grid, QmmForm form, cudaStream_t stream) {
+    if (form == QmmForm::kSmall) return qmm_launch_shape<K, CB, 64, false>(map, p, grid, stream);
+    if (form == QmmForm::kSmallItems) return qmm_launch_shape<K, CB, 64, true>(map, p, grid, stream);
+    return qmm_launch_shape<K, CB, 256, false>(map, p, grid, stream);
 }
 
 template <int K>
-cudaError_t qmm_launch_k(int cb, const CUtensorMap& map, const QmmArgs& p, int grid, bool small, cudaStream_t stream) {
-    if (cb == 0) return small ? qmm_launch_shape<K, 0, 64>(map, p, grid, stream) : qmm_launch_shape<K, 0, 256>(map, p, grid, stream);
-    if (cb == 1) return small ? qmm_launch_shape<K, 1, 64>(map, p, grid, stream) : qmm_launch_shape<K, 1, 256>(map, p, grid, stream);
-    return small ? qmm_launch_shape<K, 2, 64>(map, p, grid, stream) : qmm_launch_shape<K, 2, 256>(map, p, grid, stream);
+cudaError_t qmm_launch_k(int cb, const CUtensorMap& map, const QmmArgs& p, int grid, QmmForm form, cudaStream_t stream) {
+    if (cb == 0) return qmm_launch_form<K, 0>(map, p, grid, form, stream);
+    if (cb == 1) return qmm_launch_form<K, 1>(map, p, grid, form, stream);
+    return qmm_launch_form<K, 2>(map, p, grid, form, stream);
 }
 
-cudaError_t qmm_dispatch(int k, int cb, const CUtensorMap& map, const QmmArgs& p, int grid, bool small, cudaStream_t stream) {
+cudaError_t qmm_dispatch(int k, int cb, const CUtensorMap& map, const QmmArgs& p, int grid, QmmForm form, cudaStream_t stream) {
     switch (k) {
-        case 1: return qmm_launch_k<1>(cb, map, p, grid, small, stream);
-        case 2: return qmm_launch_k<2>(cb, map, p, grid, small, stream);
-        case 3: return qmm_launch_k<3>(cb, map, p, grid, small, stream);
-        case 4: return qmm_launch_k<4>(cb, map, p, grid, small, stream);
-        case 5: return qmm_launch_k<5>(cb, map, p, grid, small, stream);
-        case 6: return qmm_launch_k<6>(cb, map, p, grid, small, stream);
-        case 7: return qmm_launch_k<7>(cb, map, p, grid, small, stream);
-        case 8: return qmm_launch_k<8>(cb, map, p, grid, small, stream);
+        case 1: return qmm_launch_k<1>(cb, map, p, grid, form, stream);
+        case 2: return qmm_launch_k<2>(cb, map, p, grid, form, stream);
+        case 3: return qmm_launch_k<3>(cb, map, p, grid, form, stream);
+        case 4: return qmm_launch_k<4>(cb, map, p, grid, form, stream);
+        case 5: return qmm_launch_k<5>(cb, map, p, grid, form, stream);
+        case 6: return qmm_launch_k<6>(cb, map, p, grid, form, stream);
+        case 7: return qmm_launch_k<7>(cb, map, p, grid, form, stream);
+        case 8: return qmm_launch_k<8>(cb, map, p, grid, form, stream);
         default: return cudaErrorInvalidValue;
     }
 }
@@ -858,7 +872,8 @@ cudaError_t launch_qmm(QmmArgs p, const __half* xhat, int k, int cb, const QmmPl
     p.trace = g_qmm_trace.load();
     const int64_t stages = p.in / kQmmStageIn, grid = qmm_grid(plan, p.items, stages);
     if (p.items * stages * grid >= (int64_t{1} << 32)) return cudaErrorInvalidValue;
-    return qmm_dispatch(k, cb, map, p, static_cast<int>(grid), plan.tile_tokens <= 64, stream);
+    const QmmForm form = plan.tile_tokens > 64 ? QmmForm::kLarge : plan.splits > 0 ? QmmForm::kSmall : QmmForm::kSmallItems;
+    return qmm_dispatch(k, cb, map, p, static_cast<int>(grid), form, stream);
 }
 
 size_t qmm_mapped_piece_bytes() { return static_cast<size_t>(sm_count()) * 2 * kQmmSegRows * 128 * sizeof(float); }
@@ -873,7 +888,7 @@ cudaError_t launch_qmm_mapped(QmmArgs p, const __half* xhat, int max_segments, i
     p.groups = 1; p.gcol0[0] = 0;
     p.tile_tokens = kQmmSegRows; p.box_rows = box;
     p.trace = nullptr;
-    return qmm_dispatch(k, cb, map, p, sm_count(), true, stream);
+    return qmm_dispatch(k, cb, map, p, sm_count(), QmmForm::kSmallItems, stream);
 }
 
 }  // namespace b200exl3

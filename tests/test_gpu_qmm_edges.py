@@ -119,3 +119,23 @@ def test_many_items_on_a_cta(gpu, n_in, n_out, k, rows):
     pick = np.unique([0, 15, rows // 2, rows - 1])
     _close(got[pick], oracle.linear_forward(trellis, k, 0, suh, svh, None, x[pick]))
     layer.close()
+
+
+@pytest.mark.parametrize("splits", [1, 3, 8])
+@pytest.mark.parametrize("n_in,n_out,k,rows", [(128, 256, 4, 9), (1152, 384, 3, 17), (1024, 128, 8, 64), (2176, 640, 5, 33), (4224, 256, 2, 16)])
+def test_items_with_ctas_of_their_own(gpu, splits, n_in, n_out, k, rows):
+    """Tiles of up to 64 tokens without finishing warps: whole items, and items shared by CTAs that do not get equal stages."""
+    rng = np.random.default_rng(n_in + rows + splits)
+    trellis, suh, svh = random_layer(rng, n_in, n_out, k)
+    x = rng.standard_normal((rows, n_in)).astype(np.float16)
+    gpu.set_option("qmm_splits", splits)
+    try:
+        layer = gpu.Exl3Linear(trellis, suh, svh, None, k, 0)
+        got = layer.forward(x)
+        for _ in range(5):
+            assert np.array_equal(bits(layer.forward(x)), bits(got))
+        assert gpu.workspace_status(layer._workspace) == 0
+        layer.close()
+    finally:
+        gpu.set_option("qmm_splits", 0)
+    _close(got, oracle.linear_forward(trellis, k, 0, suh, svh, None, x))
