@@ -57,13 +57,18 @@ struct QmmShape {
     // Small tiles: two accumulators, and with FIN four warps that finish an item while the next one is decoded and multiplied; the
     // decoders finish only the CTA's last item.  Before, the pipeline drained at every item (5000 cycles, 2000 of them waiting for the last
     // products): 16 rows 5120->2x25600, 3 bits, 84.8 -> 80.1 us; expert block 37 / 256 tokens 176 -> 165 / 250 -> 230.  Without FIN a
-    // CTA has one item: the warps would have nothing to do but to start with the CTA and to leave the decoders 80 registers.  Us with /
-    // without them, 4 bits: 24 rows 2048->2048 9.3 / 9.05, 4096->4096 12.4 / 11.9, 64 rows 14336->4096 25.8 / 25.4, 4096->14336 21.7 / 21.55.
-    // (The loop over several items that large tiles take instead spills here: 24 rows 4096->14336 22.7.)
+    // CTA has one item, and the warps would have nothing to do but to start with it.  Us with / without them, 4 bits: 24 rows 2048->2048
+    // 9.3 / 9.05, 4096->4096 12.4 / 11.9, 64 rows 14336->4096 25.8 / 25.4, 4096->14336 21.7 / 21.55.  (The loop over several items that
+    // large tiles take instead spills here: 24 rows 4096->14336 22.7.)
     // Large tiles leave no tensor memory for a second accumulator: their decoders finish every item.
     static constexpr uint32_t kAccums = NT == 64 ? 2 : 1;
     static constexpr int kFinishers = NT == 64 ? 4 : kDecoders;
     static constexpr int kThreads = 32 * (kFirstDecoder + kDecoders + (FIN ? kFinishers : 0));
+    // Small tiles get the registers of 768 threads, 80 each, also when 640 start: that leaves room on the SM for a CTA of the kernel after
+    // this one, whose 256 threads rotate the next call's input and may lie there until this kernel is done.  With 89 registers they
+    // waited for SMs that a full wave does not leave: us with 89 / 80, 4 bits, 64 rows 4096->4096 14.9 / 12.8, 24 rows 8192->2048 14.5 / 12.8,
+    // 16 rows 14336->4096 22.5 / 20.4, 48 rows 10240->1280 15.5 / 13.6; level where the grid leaves 20 SMs or more.
+    static constexpr int kBoundThreads = NT == 64 ? 768 : kThreads;
     static constexpr int kSlots = NT == 64 ? 6 : 4;    // A stages in tensor memory beside the accumulators
     // Packed stages (2048 * K bytes) in flight.  A multiple of the decoder groups, so that a slot always belongs to one group:
     // parity alone does not tell a phase from the one after the next, and a group that met a slot only every other time could
@@ -273,7 +278,7 @@ __device__ __forceinline__ void qmm_finish4(__half* rows, const QmmArgs& p, cons
 }
 
 template <int K, int CB, int NT, bool FIN>
-__global__ void __launch_bounds__(QmmShape<K, NT, FIN>::kThreads, 1)
+__global__ void __launch_bounds__(QmmShape<K, NT, FIN>::kBoundThreads, 1)
 qmm_kernel(const __grid_constant__ CUtensorMap xmap, const QmmArgs p) {
     using S = QmmShape<K, NT, FIN>;
     // Dependent launch: this kernel may be scheduled under the tail of the kernel before it (the input rotation, the
