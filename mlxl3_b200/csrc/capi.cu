@@ -223,7 +223,7 @@ int b200exl3_plan_query(const char* kind, int in, int out, int k, int64_t rows, 
         return 0;
     }
     if (!strcmp(kind, "qmm")) {
-        const QmmPlan p = plan_qmm(in, out, rows);
+        const QmmPlan p = plan_qmm(in, out, k, rows);
         const int64_t tiles = (p.pass_rows + p.tile_tokens - 1) / p.tile_tokens, items = tiles * (out / 128), stages = in / kQmmStageIn;
         out_values[0] = qmm_grid(p, items, stages); out_values[1] = tiles; out_values[2] = items; out_values[3] = stages;
         out_values[4] = p.tile_tokens; out_values[5] = p.splits; out_values[6] = p.pass_rows; out_values[7] = static_cast<int64_t>(p.piece_bytes);
@@ -542,7 +542,7 @@ struct QmmLayout { QmmPlan plan; size_t xhat, pieces, sums, total; };
 static QmmLayout qmm_layout(const LayerCore& c, int64_t rows, bool whole_items = false, bool row_shard = false) {
     QmmLayout l;
     if (row_shard) rows = std::min(rows, shard_pass_rows(c.out));
-    l.plan = plan_qmm(c.in, c.out, rows, whole_items);
+    l.plan = plan_qmm(c.in, c.out, c.k, rows, whole_items);
     l.xhat = kCounterBytes;
     l.pieces = l.xhat + xhat_bytes(c, std::min(rows, l.plan.pass_rows));
     l.sums = l.pieces + round256(l.plan.piece_bytes);

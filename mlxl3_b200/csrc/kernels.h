@@ -46,6 +46,7 @@ cudaError_t launch_reconstruct(const uint16_t* trellis, int tiles_k, int tiles_n
 constexpr int64_t kQuadRotationUnits = 8192;
 // xhat[r, :] = H128(half(half(x[r, :]) * suh[(r % scale_rows), :])); scale_rows is 1 or rows.  With groups > 1 (scale_rows
 // 1) the rows are rotated once per member: suh [groups, in], xhat [groups, rows, in].
+int64_t prepare_ctas(int64_t rows, int in);          // CTAs of launch_prepare
 cudaError_t launch_prepare(const void* x, int x_dtype, const __half* suh, int64_t scale_rows, int64_t rows, int in,
                            __half* xhat, cudaStream_t stream, const __half* glu_up = nullptr, int groups = 1);
 // y = half(H128(half(sum_s partials[s, r, :]))) * svh (+ bias), written in y_dtype.
@@ -375,7 +376,7 @@ struct QmmPlan {
     size_t piece_bytes;  // scratch for the parts of items that CTAs share
 };
 // `out` counts all members of a group; `whole_items`: no item is shared, so no scratch for pieces
-QmmPlan plan_qmm(int in, int out, int64_t rows, bool whole_items = false);
+QmmPlan plan_qmm(int in, int out, int k, int64_t rows, bool whole_items = false);
 size_t qmm_most_piece_bytes(int64_t rows);     // no plan of a batch of up to `rows` rows has more for parts of shared items
 constexpr int kQmmStageIn = 128;     // inputs of a stage
 // CTAs of a launch over `items` items of `stages` stages

@@ -805,28 +805,41 @@ size_t qmm_most_piece_bytes(int64_t rows) {
     return static_cast<size_t>(sm_count()) * 2 * static_cast<size_t>(std::min<int64_t>(256, (rows + 15) / 16 * 16)) * 128 * sizeof(float);
 }
 
-// How a batch is cut up: tokens per item and CTAs per item (or one wave of equal runs).  The estimate below is fitted to 1160
-// measured launches (512 to 14336 inputs, 512 to 25600 outputs, 16 to 2000 rows, 3, 4 and 6 bits; its choice is 1.2 % above
-// the best measured one on average): a fixed part; a stage, mostly decode, with a share that grows with the tokens; the epilogue
-// of every item or part of one; parts that are written, counted and read again by the last CTA; and a run that starts in one item
-// and ends in another.  So small tiles (every tile decodes the weights again) win where the layer alone gives the SMs too little
-// to do: 256 rows of 2048 -> 2048 take 15.7 us as 4 tiles of 64 rows and 39 as one tile in 148 equal runs.
-// What it does not say: the bits are no term (64 rows 4096 -> 14336 at 4 bits come out at 29 us, measured 24.4; 1, 2, 5, 7 and 8
-// bits were not in the fit), so it ranks the ways to cut one layer and predicts no times.  `load` makes a launch dearer the more
-// SMs it takes although a stage takes the same cycles on 37 SMs as on 148: the launches were timed back to back with dependent
-// launch, where the next call starts on the SMs that are left (37 CTAs 29.0 us, 148 CTAs 33.4; without dependent launch 33.3, 34.4).
-static double qmm_cost_us(int64_t sms, int64_t items, int64_t stages, int tile, int64_t splits) {
+// How a batch is cut up: tokens per item and CTAs per item (or one wave of equal runs).  Microseconds fitted to 40000 measured launches
+// (76 layers of 512 to 14336 inputs and 512 to 25600 outputs, 9 to 2000 rows, 1 to 6 and 8 bits, calls back to back with dependent
+// launch), small and large tiles, items with CTAs of their own and equal runs each for themselves: a launch; a stage, mostly decode, with
+// a share that grows with the tokens and one that grows with the SMs at work; an end of an item or of a part of one; parts that
+// are written, counted and read again by the last CTA; and the next call's input rotation, whose CTAs lie on the SMs that the last
+// wave leaves (eight each) and, beside a small tile's CTA of the form without finishing warps, one on the others: where they do not all
+// find a place the next call starts later (100 rows 4096->1024: 96 CTAs 12.2 us, 144 CTAs 14.4).
+// Over those 2311 batches the choice is 0.8 % above the best one measured on average (1.0 % over layers left out of the fit).  The
+// estimate before it, fitted to an older form of the kernel and without the bits, was at 2.3 %: of 1014 batches of 26 layers that neither
+// was fitted to, 217 are cut in another way now, 7 % faster on average; 12 lost more than 3 %, at most 10 % (24 rows 5888->4736, 4 bits,
+// 13.4 -> 14.8 us).  Us, 4 bits: 90 rows 2304->8704 17.8 -> 14.4, 400 rows 640->10752 28.7 -> 23.7, 64 rows 4096->14336 21.55 ->
+// 21.4, 512 rows 4096<->14336 (MLP block, 3 bits) 227 -> 224, 1999 rows 4096->6144 (group, 6 bits) 152 -> 143.5.
+struct QmmCost { double launch, load, rotate, late, late_cta, stage_tile, stage, stage_load, end, end_tile, shared, shared_tile, part, part_tile; };
+static constexpr QmmCost kQmmCost[2][2] = {                                  // [tiles above 64 tokens][equal runs]
+    {{1.38, 0.967, 1.21, 1.03, 0.14, 0.056, 0.351, 0.118, 2.8, 0.717, 1.43, 0.521, 0.104, 0.248},
+     {7.08, 0.138, 0.807, 0.047, 0.326, 0.0, 0.469, 0.0, 0.038, 1.45, 0.4, 1.72, 0.043, 0.306}},
+    {{1.29, 2.21, 0.771, 0.732, 0.005, 0.029, 0.521, 0.036, 2.03, 1.86, 1.77, 0.249, 0.245, 0.18},
+     {0.0, 0.0, 0.663, 5.88, 0.0, 0.08, 0.477, 0.0, 1.67, 1.1, 1.02, 0.093, 0.403, 0.11}}};
+
+static double qmm_cost_us(int64_t sms, int64_t rows, int in, int k, int64_t items, int64_t stages, int tile, int64_t splits) {
+    const QmmCost& c = kQmmCost[tile > 64][splits == 0];
     const int64_t grid = splits > 0 ? items * splits : std::min(sms, items * stages);
     const int64_t waves = (grid + sms - 1) / sms, run = splits > 0 ? (stages + splits - 1) / splits : (items * stages + grid - 1) / grid;
     const bool whole = splits == 0 && items % grid == 0;                     // equal runs of whole items
     const double parts = splits > 0 ? static_cast<double>(splits) : whole ? 1.0 : static_cast<double>(items < grid ? (grid + items - 1) / items + 1 : 2);
     const double ends = splits > 0 ? 1.0 : static_cast<double>(whole ? items / grid : (run + stages - 1) / stages + 1);
-    const double load = static_cast<double>(grid) / static_cast<double>(sms * waves);
-    return 4.4 + 2.24 * load + waves * (run * (0.414 + 0.001 * tile) * (1 + 0.48 * load) + ends * (0.38 + 0.0306 * tile)) +
-           (parts > 1 ? 1.8 + 0.1 * parts + 0.003 * tile * parts : 0.0) + (splits > 0 ? 0.0 : 1.27);
+    const double bits = k == 4 || k == 8 ? 1.0 : k == 3 ? 1.09 : k < 3 ? 1.06 : 1.15;         // of a tile's decode
+    const double t = tile / 64.0, load = static_cast<double>(std::min(grid, sms)) / static_cast<double>(sms);
+    const int64_t busy = grid - (waves - 1) * sms, late = std::max<int64_t>(0, prepare_ctas(rows, in) - (sms - busy) * 8 - (tile <= 64 && splits > 0 ? busy : 0));
+    return c.launch + c.load * load + c.rotate * 1e-6 * static_cast<double>(rows * in) + (late > 0 ? c.late : 0.0) + c.late_cta * late / sms +
+           waves * (run * (c.stage_tile * t + bits * (c.stage + c.stage_load * load)) + ends * (c.end + c.end_tile * t)) +
+           (parts > 1 ? c.shared + c.shared_tile * t + parts * (c.part + c.part_tile * t) : 0.0);
 }
 
-static QmmPlan make_qmm_plan(int in, int out, int64_t rows, bool whole_items, int forced, int64_t sms) {
+static QmmPlan make_qmm_plan(int in, int out, int k, int64_t rows, bool whole_items, int forced, int64_t sms) {
     QmmPlan plan{};
     const int64_t col_blocks = out / 128, stages = in / kQmmStageIn;
     // the items of one launch need an arrival counter each, and stages x CTAs must fit 32 bits: more rows go in passes
@@ -834,21 +847,23 @@ static QmmPlan make_qmm_plan(int in, int out, int64_t rows, bool whole_items, in
     const int64_t max_tiles = std::max<int64_t>(1, max_items / col_blocks);
     plan.pass_rows = std::min(rows, max_tiles * 256);
     double best = 0;
-    for (const int target : {16, 32, 64, 96, 128, 192, 256}) {
+    for (const int target : {16, 32, 48, 64, 96, 128, 192, 256}) {
         const int64_t tiles = (plan.pass_rows + target - 1) / target;
         if (tiles > max_tiles) continue;
         // equal tiles of whole sixteens: N of the MMA is a multiple of 16
         const int tile = static_cast<int>(((plan.pass_rows + tiles - 1) / tiles + 15) / 16 * 16);
         const int64_t items = tiles * col_blocks;
         auto consider = [&](int64_t splits) {
-            const double t = qmm_cost_us(sms, items, stages, tile, splits);
+            // of whole sixteens, so that all rows with as many are cut alike: workspace sizes step by them
+            const double t = qmm_cost_us(sms, (plan.pass_rows + 15) / 16 * 16, in, k, items, stages, tile, splits);
             if (best == 0 || t < best) { best = t; plan.tile_tokens = tile; plan.splits = static_cast<int>(splits); }
         };
         if (whole_items) consider(1);
         else if (forced) consider(std::max<int64_t>(1, std::min<int64_t>(forced, stages)));
         else {
-            for (int64_t splits = 1; splits <= stages && items * splits <= sms; ++splits) consider(splits);
-            consider(0);
+            // whole items also in up to three waves: their stages are not cut, and nothing waits for parts
+            for (int64_t splits = 1; splits <= stages && items * splits <= (splits == 1 ? 3 * sms : sms); ++splits) consider(splits);
+            if (items * stages > sms) consider(0);
         }
     }
     const int64_t items = (plan.pass_rows + plan.tile_tokens - 1) / plan.tile_tokens * col_blocks;
@@ -857,13 +872,13 @@ static QmmPlan make_qmm_plan(int in, int out, int64_t rows, bool whole_items, in
 }
 
 // Weighing the choices takes a few microseconds of the host and a call asks twice: a thread remembers its last plans.
-QmmPlan plan_qmm(int in, int out, int64_t rows, bool whole_items) {
-    struct Entry { int in, out, forced, sms; int64_t rows; bool whole; QmmPlan plan; };
+QmmPlan plan_qmm(int in, int out, int k, int64_t rows, bool whole_items) {
+    struct Entry { int in, out, k, forced, sms; int64_t rows; bool whole; QmmPlan plan; };
     thread_local Entry cache[64] = {};
     const int forced = g_qmm_splits.load(), sms = sm_count();
     Entry& e = cache[(static_cast<unsigned>(in) / 128 * 7 + static_cast<unsigned>(out) / 128 * 3 + static_cast<unsigned>(rows)) % 64];
-    if (e.in != in || e.out != out || e.rows != rows || e.whole != whole_items || e.forced != forced || e.sms != sms)
-        e = {in, out, forced, sms, rows, whole_items, make_qmm_plan(in, out, rows, whole_items, forced, sms)};
+    if (e.in != in || e.out != out || e.k != k || e.rows != rows || e.whole != whole_items || e.forced != forced || e.sms != sms)
+        e = {in, out, k, forced, sms, rows, whole_items, make_qmm_plan(in, out, k, rows, whole_items, forced, sms)};
     return e.plan;
 }
 

@@ -146,6 +146,11 @@ static unsigned grid_for(int64_t units) {
     return static_cast<unsigned>(blocks < cap ? (blocks > 0 ? blocks : 1) : cap);
 }
 
+int64_t prepare_ctas(int64_t rows, int in) {
+    const int64_t units = rows * (in / 128);
+    return grid_for(units > kQuadRotationUnits ? (units + 3) / 4 : units);
+}
+
 cudaError_t launch_prepare(const void* x, int x_dtype, const __half* suh, int64_t scale_rows, int64_t rows, int in,
                            __half* xhat, cudaStream_t stream, const __half* glu_up, int groups) {
     if (rows == 0) return cudaSuccess;
@@ -154,11 +159,11 @@ cudaError_t launch_prepare(const void* x, int x_dtype, const __half* suh, int64_
     const int64_t units = rows * (in / 128);
     if (units > kQuadRotationUnits) {
         const bool wide = sixteen_bytes_at_once(x) && sixteen_bytes_at_once(suh) && sixteen_bytes_at_once(glu_up);
-        return launch_dependent(wide ? prepare_quads_kernel<true> : prepare_quads_kernel<false>, dim3(grid_for((units + 3) / 4)), dim3(256), 0, stream, x,
+        return launch_dependent(wide ? prepare_quads_kernel<true> : prepare_quads_kernel<false>, dim3(static_cast<unsigned>(prepare_ctas(rows, in))), dim3(256), 0, stream, x,
                                 x_dtype, suh, scale_rows, rows, in, xhat, glu_up, groups);
     }
     const bool wide = four_at_once(x, x_dtype) && four_at_once(suh, kF16);
-    return launch_dependent(wide ? prepare_kernel<true> : prepare_kernel<false>, dim3(grid_for(units)), dim3(256), 0, stream, x, x_dtype, suh, scale_rows, rows, in, xhat,
+    return launch_dependent(wide ? prepare_kernel<true> : prepare_kernel<false>, dim3(static_cast<unsigned>(prepare_ctas(rows, in))), dim3(256), 0, stream, x, x_dtype, suh, scale_rows, rows, in, xhat,
                             glu_up, groups);
 }
 
