@@ -9,6 +9,7 @@ file so that it is found by :mod:`mlxl3_b200._lib` and travels with the source t
 from __future__ import annotations
 
 import os
+import re
 import shutil
 import subprocess
 import sys
@@ -39,6 +40,11 @@ def _newest_header() -> float:
     return max(h.stat().st_mtime for h in headers)
 
 
+def _included(src: Path) -> float:
+    """Newest of the sources that a source includes."""
+    return max(((CSRC / name).stat().st_mtime for name in re.findall(r'#include "(\w+\.cu)"', src.read_text())), default=0.0)
+
+
 def build(force: bool = False, verbose: bool = False) -> Path:
     sources = sorted(CSRC.glob("*.cu"))
     OBJ.mkdir(parents=True, exist_ok=True)
@@ -47,7 +53,7 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     jobs = []
     for src in sources:
         obj = OBJ / (src.stem + ".o")
-        stale = force or not obj.exists() or obj.stat().st_mtime < max(src.stat().st_mtime, header_time)
+        stale = force or not obj.exists() or obj.stat().st_mtime < max(src.stat().st_mtime, header_time, _included(src))
         if stale:
             jobs.append((src, obj))
 

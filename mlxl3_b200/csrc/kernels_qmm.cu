@@ -43,6 +43,9 @@
 
 namespace b200exl3 {
 
+// What a CTA is built for: tiles of up to 64 tokens, where every item has CTAs of its own or where a CTA holds several; large tiles.
+enum class QmmForm { kSmall, kSmallItems, kLarge };
+
 namespace {
 
 // The single-thread roles take the lowest warp numbers: the scheduler favours older warps.
@@ -716,6 +719,44 @@ qmm_kernel(const __grid_constant__ CUtensorMap xmap, const QmmArgs p) {
     }
 }
 
+template <int K, int CB, int NT, bool FIN>
+cudaError_t qmm_launch_shape(const CUtensorMap& map, const QmmArgs& p, int grid, cudaStream_t stream) {
+    constexpr size_t smem = qmm_smem_bytes<K, NT, FIN>();
+    auto kernel = qmm_kernel<K, CB, NT, FIN>;
+    static PerDeviceOnce attribute;                         // once per kernel and device
+    if (attribute.needed()) {
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+        if (e != cudaSuccess) return e;
+        attribute.mark();
+    }
+    return launch_dependent(kernel, dim3(static_cast<unsigned>(grid)), dim3(QmmShape<K, NT, FIN>::kThreads), smem, stream, map, p);
+}
+
+template <int K, int CB>
+cudaError_t qmm_launch_form(const CUtensorMap& map, const QmmArgs& p, int grid, QmmForm form, cudaStream_t stream) {
+    if (form == QmmForm::kSmall) return qmm_launch_shape<K, CB, 64, false>(map, p, grid, stream);
+    if (form == QmmForm::kSmallItems) return qmm_launch_shape<K, CB, 64, true>(map, p, grid, stream);
+    return qmm_launch_shape<K, CB, 256, false>(map, p, grid, stream);
+}
+
+}  // namespace
+
+#ifdef B200_QMM_K
+
+// One width per translation unit (kernels_qmm_k1.cu and its neighbours): they compile side by side, and the first call of a program
+// loads the kernels of its width alone: 2.6 ms, 41 with all widths in one module.
+template <int K>
+cudaError_t qmm_launch_k(int cb, const CUtensorMap& map, const QmmArgs& p, int grid, QmmForm form, cudaStream_t stream) {
+    if (cb == 0) return qmm_launch_form<K, 0>(map, p, grid, form, stream);
+    if (cb == 1) return qmm_launch_form<K, 1>(map, p, grid, form, stream);
+    return qmm_launch_form<K, 2>(map, p, grid, form, stream);
+}
+template cudaError_t qmm_launch_k<B200_QMM_K>(int, const CUtensorMap&, const QmmArgs&, int, QmmForm, cudaStream_t);
+
+#else
+
+namespace {
+
 using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                               const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                               CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -743,37 +784,12 @@ bool encode_rows(CUtensorMap* map, const __half* xhat, int in, int64_t rows, int
                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int K, int CB, int NT, bool FIN>
-cudaError_t qmm_launch_shape(const CUtensorMap& map, const QmmArgs& p, int grid, cudaStream_t stream) {
-    constexpr size_t smem = qmm_smem_bytes<K, NT, FIN>();
-    auto kernel = qmm_kernel<K, CB, NT, FIN>;
-    static PerDeviceOnce attribute;                         // once per kernel and device
-    if (attribute.needed()) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-        if (e != cudaSuccess) return e;
-        attribute.mark();
-    }
-    return launch_dependent(kernel, dim3(static_cast<unsigned>(grid)), dim3(QmmShape<K, NT, FIN>::kThreads), smem, stream, map, p);
-}
-
-// What a CTA is built for: tiles of up to 64 tokens, where every item has CTAs of its own or where a CTA holds several; large tiles.
-enum class QmmForm { kSmall, kSmallItems, kLarge };
-
-template <int K, int CB>
-cudaError_t qmm_launch_form(const CUtensorMap& map, const QmmArgs& p, int grid, QmmForm form, cudaStream_t stream) {
-    if (form == QmmForm::kSmall) return qmm_launch_shape<K, CB, 64, false>(map, p, grid, stream);
-    if (form == QmmForm::kSmallItems) return qmm_launch_shape<K, CB, 64, true>(map, p, grid, stream);
-    return qmm_launch_shape<K, CB, 256, false>(map, p, grid, stream);
-}
+}  // namespace
 
 template <int K>
-cudaError_t qmm_launch_k(int cb, const CUtensorMap& map, const QmmArgs& p, int grid, QmmForm form, cudaStream_t stream) {
-    if (cb == 0) return qmm_launch_form<K, 0>(map, p, grid, form, stream);
-    if (cb == 1) return qmm_launch_form<K, 1>(map, p, grid, form, stream);
-    return qmm_launch_form<K, 2>(map, p, grid, form, stream);
-}
+cudaError_t qmm_launch_k(int cb, const CUtensorMap& map, const QmmArgs& p, int grid, QmmForm form, cudaStream_t stream);
 
-cudaError_t qmm_dispatch(int k, int cb, const CUtensorMap& map, const QmmArgs& p, int grid, QmmForm form, cudaStream_t stream) {
+static cudaError_t qmm_dispatch(int k, int cb, const CUtensorMap& map, const QmmArgs& p, int grid, QmmForm form, cudaStream_t stream) {
     switch (k) {
         case 1: return qmm_launch_k<1>(cb, map, p, grid, form, stream);
         case 2: return qmm_launch_k<2>(cb, map, p, grid, form, stream);
@@ -786,8 +802,6 @@ cudaError_t qmm_dispatch(int k, int cb, const CUtensorMap& map, const QmmArgs& p
         default: return cudaErrorInvalidValue;
     }
 }
-
-}  // namespace
 
 std::atomic<unsigned long long*> g_qmm_trace{nullptr};
 static std::atomic<int> g_qmm_splits{0};                              // 0 = one wave of CTAs with equal runs of stages
@@ -910,5 +924,7 @@ cudaError_t launch_qmm_mapped(QmmArgs p, const __half* xhat, int max_segments, i
     p.trace = nullptr;
     return qmm_dispatch(k, cb, map, p, sm_count(), QmmForm::kSmallItems, stream);
 }
+
+#endif
 
 }  // namespace b200exl3
