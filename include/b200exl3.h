@@ -274,18 +274,18 @@ int b200exl3_moe_forward(const b200exl3_moe* handle, const void* d_x, int x_dtyp
                          const uint32_t* d_selected, const void* d_scores, int score_dtype, void* d_y,
                          void* d_workspace, size_t workspace_bytes, b200exl3_stream stream);
 
-/* ---- layers with a fused prologue (fp16; 1 to 8 rows, the SwiGLU prologue alone any number of rows) --------------
+/* ---- layers with a fused prologue (fp16; 1 or 2 rows, the SwiGLU prologue alone any number of rows) --------------
  * The reference fuses the operators around a projection into its prologue kernels where dispatch count matters
  * (flash_up_finish_swiglu_prepare and its neighbours, native/shaders/exl3.metal:240-291).  Here the layer kernel's own
  * input rotation takes the operator in front of it:
  *   kind 1  RMSNorm: s = half(x + aux) (aux = residual rows or NULL), input = weight * half(s * rsqrt(mean(s^2) + eps));
  *           s is also stored to d_sum when that is not NULL (it must not be x: other warps still read x);
- *   kind 2  SwiGLU: input = half(half(x * half(sigmoid(x))) * aux), x = gate rows, aux = up rows.  With more than 8
- *           rows (prefill: the tensor-core product) it is applied by the input-rotation kernel, so a dense MLP block
- *           is [gate | up] -> down with no kernel between them.
+ *   kind 2  SwiGLU: input = half(half(x * half(sigmoid(x))) * aux), x = gate rows, aux = up rows.  Where a
+ *           launch of its own rotates the input (9 rows and more; from 3 on for layers too wide for clusters) that launch
+ *           applies it, so a dense MLP block is [gate | up] -> down with no kernel between them.
  * Same arithmetic as b200exl3_rms_norm / b200exl3_swiglu followed by the plain forward; the row sum of the norm is added
- * in another order, so the last fp32 bit of 1/rms may differ from the stand-alone kernel's.  Kind 1 makes every warp
- * add up the whole row; the cheaper pairing is the residual EPILOGUE of the layer before (which already holds each
+ * in another order, so the last fp32 bit of 1/rms may differ from the stand-alone kernel's.  Kind 1 makes every CTA
+ * (every warp, for layers too wide for clusters) add up the whole row; the cheaper pairing is the residual EPILOGUE of the layer before (which already holds each
  * output block in registers) with a kind-3 prologue. */
 typedef struct {
     int kind;
@@ -325,8 +325,8 @@ int b200exl3_group_forward_fused(const b200exl3_group* handle, const b200exl3_pr
  * Replaces the reference's recorded decode step (mlxl3_replay_capture / mlxl3_replay_apply,
  * native/ffi/mlx_bridge.cpp:150-175): `count` (1..256) layers (Exl3Linear or Exl3Group), each with its input and output
  * pointers, become one object, and b200exl3_stack_forward runs them all, in order, in a single persistent kernel:
- * the result is what the per-layer forward calls issued in that order on one stream would give (same kernels'
- * arithmetic, same summation order), but the weight stream does not stop at layer boundaries and a boundary costs
+ * the result is what the per-layer forward calls issued in that order on one stream would give (the same arithmetic;
+ * the fp32 sums of a layer are added in an order of their own), but the weight stream does not stop at layer boundaries and a boundary costs
  * a counter instead of a launch.  Layer i+1 may read anything layer i wrote.
  *   - all layers share bit width, codebook and weight mode; 1..2 activation rows in `x_dtype`; outputs in x_dtype;
  *   - pointers are fixed at creation (as a recorded graph fixes them); the object owns its scratch memory, so

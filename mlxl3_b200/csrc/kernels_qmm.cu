@@ -29,7 +29,7 @@
 // decoders that keep the integer pipes full: an instruction of theirs takes about eight cycles, a stage of any of them 400 to
 // 600.  For the same reason the issuing loop is unrolled over the ring and its thread picked by elect.sync; the producers'
 // loops stay rolled (all three unrolled: 714 ns per 64 inputs against 523).  Us per call with the input rotation: 64 rows
-// 4096->14336, 4 bits, 21.7; 16 rows 5120->2x25600, 3 bits, 72.0.
+// 4096->14336, 4 bits, 21.4; 16 rows 5120->2x25600, 3 bits, 72.0.
 // Every wait is bounded in time; a wait that gives up sets the status word and the kernel still releases its tensor memory.
 #include <cuda.h>
 

@@ -74,7 +74,7 @@ def static_status(clear: bool = False) -> int:
 
 class Prologue(ctypes.Structure):
     """``b200exl3_prologue``: the operators fused in front of a layer's input rotation and behind its output rotation
-    (fp16; 1 to 8 rows, the SwiGLU prologue alone any number of rows)."""
+    (fp16; 1 or 2 rows, the SwiGLU prologue alone any number of rows)."""
     _fields_ = [("kind", ctypes.c_int), ("d_aux", c_void_p), ("d_weight", c_void_p), ("d_sum", c_void_p), ("eps", ctypes.c_float),
                 ("d_sumsq", c_void_p), ("epilogue", ctypes.c_int), ("d_residual", c_void_p), ("d_residual_out", c_void_p),
                 ("d_sumsq_out", c_void_p), ("d_pos", c_void_p), ("theta", ctypes.c_float), ("max_ctx", ctypes.c_int),
@@ -82,7 +82,7 @@ class Prologue(ctypes.Structure):
 
     @classmethod
     def rms_norm(cls, d_weight: int, eps: float, d_residual: int = 0, d_sum: int = 0) -> "Prologue":
-        """Every warp adds up the whole row (+ residual) itself."""
+        """Every CTA (every warp, for layers too wide for clusters) adds up the whole row (+ residual) itself."""
         return cls(1, d_residual or None, d_weight, d_sum or None, eps)
 
     @classmethod
