@@ -73,7 +73,7 @@ int b200exl3_version(void);
  * column block: CTAs of a cluster, 0 = chosen by a cost model, -1 = never), "qmm_trace_buffer" (device address of a uint64 [CTAs, 8] array that receives nanosecond
  * stamps of the tensor-core kernel's phases: start, set up, first epilogue begins, products issued, (unused),
  * epilogues done, end, activation copies issued; 0 = off), "tp_wait_ms" (how long a rank waits for the other ranks'
- * words inside a tensor- or expert-parallel kernel before it gives up with status 4; default 4000), "stack_wait_ms"
+ * words inside a tensor- or expert-parallel kernel before it gives up with status 4 or 7; default 4000), "stack_wait_ms"
  * (the same bound for every wait inside the decode-step kernel: status 5 = a layer never completed, 6 = a piece of
  * a column block never arrived; default 2000), "stack_trace_buffer" (device address of a uint64
  * [layers, CTAs, 20] array that receives nanosecond stamps of the decode-step kernel: boundary passed, activations

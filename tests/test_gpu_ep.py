@@ -68,6 +68,33 @@ def test_few_slots_give_the_bytes_of_the_block(gpu, rows, experts, top_k, n_in, 
     sharded.close(), whole.close(), ctx.close()
 
 
+def test_clusters_of_slots_that_are_not_local(gpu):
+    """Fewer local slots than the call has: their clusters return at once, and the slots behind them move up.  An id past the bank is
+    local to no rank, so the sum of its token gives up after the wait limit; the other token's bytes are the block's."""
+    from mlxl3_b200 import ep
+    rng = np.random.default_rng(8)
+    experts, top_k, n_in, hidden, k = 8, 4, 2048, 768, 3
+    bank = make_bank(rng, experts, n_in, hidden, k)
+    whole = gpu.Exl3SwitchGlu(*bank, top_k, k, 0)
+    x = rng.standard_normal((2, n_in)).astype(np.float16)
+    selected, scores = routes(rng, 2, experts, top_k)
+    want = whole.forward(x, selected, scores)
+    gpu.set_option("tp_wait_ms", 30)
+    try:
+        for token in (0, 1):
+            ctx = ep.EpContext(0, 1, 64, n_in, lambda raw: [raw])
+            sharded = ep.Exl3SwitchGluEp(*bank, top_k, k, 0, ctx)
+            partly = selected.copy()
+            partly[token, 1:3] = experts + 5
+            got = sharded.forward(x, partly, scores)
+            assert np.array_equal(bits(got[1 - token]), bits(want[1 - token]))
+            assert ctx.status() == 7 and gpu.workspace_status(sharded._workspace) == 0
+            sharded.close(), ctx.close()
+    finally:
+        gpu.set_option("tp_wait_ms", 4000)
+    whole.close()
+
+
 def _rank(rank, world, port, out):
     import torch.distributed as dist
     os.environ.update(MASTER_ADDR="127.0.0.1", MASTER_PORT=str(port))

@@ -122,9 +122,10 @@ def test_many_items_on_a_cta(gpu, n_in, n_out, k, rows):
 
 
 @pytest.mark.parametrize("splits", [1, 3, 8])
-@pytest.mark.parametrize("n_in,n_out,k,rows", [(128, 256, 4, 9), (1152, 384, 3, 17), (1024, 128, 8, 64), (2176, 640, 5, 33), (4224, 256, 2, 16)])
+@pytest.mark.parametrize("n_in,n_out,k,rows", [(128, 256, 4, 9), (1152, 384, 3, 17), (1024, 128, 8, 64), (2176, 640, 5, 33), (4224, 256, 2, 16), (256, 25600, 6, 48)])
 def test_items_with_ctas_of_their_own(gpu, splits, n_in, n_out, k, rows):
-    """Tiles of up to 64 tokens without finishing warps: whole items, and items shared by CTAs that do not get equal stages."""
+    """Tiles of up to 64 tokens without finishing warps: whole items, items shared by CTAs that do not get equal stages, and more CTAs
+    than a wave holds."""
     rng = np.random.default_rng(n_in + rows + splits)
     trellis, suh, svh = random_layer(rng, n_in, n_out, k)
     x = rng.standard_normal((rows, n_in)).astype(np.float16)
